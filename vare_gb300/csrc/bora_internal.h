@@ -123,6 +123,12 @@ struct BoraReduceDev
     uint32_t* done;      // [BORA_RING] block-arrival counters
     uint32_t* err;       // set non-zero by a kernel that met an inconsistent stencil code
     double* mirror;      // [BORA_RING] host-mapped copy of the slot values, or null
+    // the solver chain's sums, finished by the kernel that consumes them (reduce.cuh): one
+    // double-float partial per producer block, and the finished values as double-float pairs
+    float2* part_dq;     // [kBoraMaxReduceBlocks] d.q, from the direction kernel
+    float2* part_rz;     // r.z, from the preconditioner's last kernel
+    float2* part_rr;     // r.r, from the residual update
+    float2* ringf;       // [BORA_RING]
 };
 
 // ---- launchers -----------------------------------------------------------------------
@@ -196,30 +202,33 @@ void bora_launch_mic_factor( const BoraGridDev& g, int ntiles, const uint16_t* c
 // r = b, x = 0, e = 0, d = 0, q = 0; partial sums of ||b||^2 and max|b| -> ring slots
 void bora_launch_solve_init( int ntiles, const float* b, const uint16_t* code, BoraSolverDev s, BoraReduceDev red,
                              int slot_norm2, int slot_max, cudaStream_t st );
-// e += alpha d; r -= alpha q; z = M^-1 r; rz, rr -> ring slots (alpha = rz_in / dq_in, or 0 when slot_rz_in < 0)
+// r -= alpha q; z = M^-1 r; partial sums of rz and rr (alpha = rz_in / dq, or 0 when slot_rz_in < 0; dq is
+// finished from the direction kernel's partials into slot_dq_in). bora_pcg_update_grid: its blocks.
+int bora_pcg_update_grid( int ntiles );
 void bora_launch_pcg_update( int ntiles, const uint16_t* code, BoraSolverDev s, BoraReduceDev red, int slot_rz_in,
-                             int slot_dq_in, int slot_rz_out, int slot_rr_out, cudaStream_t st );
-// d' = z + beta d; q = A d'; dq -> ring slot (beta = rz_new / rz_old, or 0 when slot_rz_old < 0)
+                             int slot_dq_in, cudaStream_t st );
+int bora_pcg_direction_grid( int ntiles );
 // One refinement pass of the plain form's inner PCG in one cooperative launch with bounded
 // grid barriers (projection.cu). Outputs: ring slots slot_a_rz / slot_a_dq (the last
-// update's alpha, whose e += alpha d is pending), slot_rr (the last r.r), *iters. bar: two
+// update's alpha, whose e += alpha d is pending), part_rr[0] (the last r.r), *iters. bar: two
 // zeroed words; part: 3 * bora_pcg_persistent_grid() doubles. never_release: every barrier
 // wait runs out (a test of the error path). Returns 0, or -1 when the launch is refused.
 #define BORA_REDUCE_ERR_BARRIER 0x100u  // a grid barrier wait ran out
 int bora_pcg_persistent_grid();
 int bora_launch_pcg_persistent( int ntiles, const int32_t* nbr, const uint16_t* code, BoraSolverDev s, BoraReduceDev red,
                                 int dsel, int slot_rz_prev, int max_inner, double target, int slot_a_rz, int slot_a_dq,
-                                int slot_rr, uint32_t* iters, unsigned* bar, double* part, bool never_release,
-                                cudaStream_t st );
+                                uint32_t* iters, unsigned* bar, double* part, bool never_release, cudaStream_t st );
+// d' = z + beta d; q = A d'; partial sums of dq (beta = rz_new / rz_old, or 0 when slot_rz_old < 0). Finishes rz
+// and rr from nparts producer blocks' partials into slot_rz_new and slot_rr (host_rr: rr also for the host).
 void bora_launch_pcg_direction( const BoraGridDev& g, int ntiles, BoraTilesDev t, const uint16_t* code, BoraSolverDev s,
-                                int dsel_in, BoraReduceDev red, int slot_rz_new, int slot_rz_old, int slot_dq_out,
-                                int slot_a_rz, int slot_a_dq, cudaStream_t st );
-// x += e (FP64); e = 0; d = 0; q = 0
+                                int dsel_in, BoraReduceDev red, int nparts, int slot_rz_new, int slot_rr, int slot_rz_old,
+                                int slot_a_rz, int slot_a_dq, bool host_rr, cudaStream_t st );
+// x += e (FP64); e = 0; d = 0; q = 0; finishes the last update's rr into slot_rr (also for the host)
 // x = the last step's pressure on fluid cells, read through the previous tile table (the warm start)
 void bora_launch_solve_warm( int ntiles, const uint16_t* code, const int32_t* tile_of, const int32_t* slot_prev,
                              const float* pres, BoraSolverDev s, cudaStream_t st );
-void bora_launch_refine_accumulate( int ntiles, const uint16_t* code, BoraSolverDev s, int dsel, const double* ring,
-                                    int slot_a_rz, int slot_a_dq, cudaStream_t st );
+void bora_launch_refine_accumulate( int ntiles, const uint16_t* code, BoraSolverDev s, int dsel, BoraReduceDev red,
+                                    int nparts, int slot_rr, int slot_a_rz, int slot_a_dq, cudaStream_t st );
 // r = b - A x in FP64 (stored FP32); ||r||^2 and max|r| -> ring slots
 void bora_launch_refine_residual( const BoraGridDev& g, int ntiles, BoraTilesDev t, const float* b, const uint16_t* code,
                                   BoraSolverDev s, BoraReduceDev red, int slot_norm2, int slot_max, cudaStream_t st );
@@ -245,17 +254,17 @@ struct BoraLevelDev
 
 // The tiled levels' passes of a V-cycle (mg_passes.cu): level l (E = 8, 4 or 2) pre-smoothed
 // and restricted into level l + 1's r (down), or prolonged from the coarser correction ec and
-// post-smoothed (up: level 0 into the PCG's z with r.z -> slot_rz, the others into z1).
+// post-smoothed (up: level 0 into the PCG's z with partial sums of r.z, the others into z1).
 // scratch: an FP32 vector of level 0's size. Level 0's down passes first apply the PCG's
-// residual update r -= alpha q, alpha = ring[slot_rz_in] / ring[slot_dq_in] (none when
-// slot_rz_in < 0), and sum the updated r.r into slot_rr_out; slot_rr gives the scale.
+// residual update r -= alpha q, alpha = rz / dq of slots slot_rz_in and slot_dq_in (none when
+// slot_rz_in < 0; the first pass finishes dq from the direction kernel's partials), with partial
+// sums of the updated r.r; slot_rr gives the scale.
 int bora_mg_pass_grid( int E, int ntiles, int v );  // v < 0: level 0's fixed up-2 shape
 void bora_mg_pass_down( const BoraLevelDev* levels, int l, const BoraTilesDev& t, int ntiles, float* r0, const float* q,
                         float* scratch, const BoraReduceDev& red, int slot_rr, int slot_rz_in, int slot_dq_in,
-                        int slot_rr_out, cudaStream_t st );
+                        cudaStream_t st );
 void bora_mg_pass_up( const BoraLevelDev* levels, int l, const __half* ec, const BoraTilesDev& t, int ntiles,
-                      const float* r0, float* scratch, const BoraReduceDev& red, int slot_rr, float* z, int slot_rz,
-                      cudaStream_t st );
+                      const float* r0, float* scratch, const BoraReduceDev& red, int slot_rr, float* z, cudaStream_t st );
 
 // ---- launch-shape autotuner (tune.cu) ------------------------------------------------------
 // Kernel groups with interchangeable launch shapes (bit-identical results): the multigrid
@@ -291,9 +300,9 @@ void bora_tune_resolve();
 // mid_image: the buffer for the coarse levels' cluster image (bora_mg_mid_image_bytes), or null
 void bora_mg_setup( const BoraGridDev& g, BoraLevelDev* levels, int nlevels, BoraTilesDev t, void* mid_image,
                     uint32_t* err, cudaStream_t st );
-// One preconditioned PCG update: r -= alpha q (alpha = ring[slot_rz_in] / ring[slot_dq_in],
-// none when slot_rz_in < 0), r.r -> slot_rr_out, then one V-cycle z = M^-1 r (FP32 in and out,
-// FP16 inside, scaled by 1 / sqrt(ring[slot_scale])); r.z -> slot_rz (FP64-accurate).
+// One preconditioned PCG update: r -= alpha q (alpha = rz / dq of slots slot_rz_in and slot_dq_in,
+// none when slot_rz_in < 0), then one V-cycle z = M^-1 r (FP32 in and out, FP16 inside, scaled by
+// 1 / sqrt(ring[slot_scale])); partial sums of r.r and r.z, bora_mg_pass_grid( 8, ntiles, -1 ) blocks each.
 // Kernel launches of one bora_mg_vcycle call for this hierarchy.
 int bora_mg_vcycle_launches( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t,
                              const void* mid_image );
@@ -310,7 +319,7 @@ int bora_mg_mid_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nl
                         const void* image, uint32_t* err, int sweeps, cudaStream_t st, bool launch );
 void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t, const void* mid_image,
                      float* r, const float* q, float* z, float* scratch, BoraReduceDev red, int slot_rz_in,
-                     int slot_dq_in, int slot_rr_out, int slot_scale, int slot_rz, int coarse_sweeps, cudaStream_t st );
+                     int slot_dq_in, int slot_scale, int coarse_sweeps, cudaStream_t st );
 // ---- batched solve: several simulations, one launch per kernel ---------------------------
 // A batched launch packs the blocks of the simulations taking part back to back into one
 // 1-D grid: simulation k owns blocks start[k] .. start[k+1] - 1, exactly the grid its own
@@ -320,9 +329,9 @@ void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nleve
 // any batch, and no block of a batched launch idles. Arguments come from device arrays.
 enum BoraMemberGrid
 {
-    kGridDir = 0, kGridUpd, kGridCells, kGridResidual,
+    kGridDir = 0, kGridCells, kGridResidual,
     kGridPass0, kGridPass0R, kGridPass1, kGridPass2,  // the multigrid passes of levels 0, 1, 2 (mg_passes.cu);
-                                                      // 0R: level 0's up 2, which reduces r.z
+                                                      // 0R: level 0's down 1 and up 2, which reduce
     kGridCount
 };
 struct BoraMemberSolve
@@ -342,9 +351,11 @@ struct BoraMemberSlots  // ring slots of one batched launch sequence
 {
     int active;                          // 0: this simulation sits the launch out
     int dsel;                            // which search-direction buffer is the current one
-    int rz_new, rz_old, dq, a_rz, a_dq;  // direction (beta = rz_new / rz_old; pending alpha)
-    int rz_in, dq_in, rr_out;            // update (alpha = rz_in / dq_in), r.r out
-    int rr, rz;                          // V-cycle: the scale's r.r, r.z out
+    int rz_new, rr_new, rz_old, a_rz, a_dq;  // direction (finishes rz_new and rr_new; beta = rz_new / rz_old; pending
+                                             // alpha); refinement: rr_new, a_rz, a_dq
+    int chk;                             // the host reads rr_new
+    int rz_in, dq_in;                    // residual update (alpha = rz_in / dq_in; dq_in is finished there)
+    int rr;                              // V-cycle: the scale's r.r
     int n2, mx;                          // solve init / refinement residual: ||r||^2, max|r|
 };
 struct BoraBatchLaunch
@@ -387,7 +398,6 @@ void bora_launch_pcg_direction_batch( const BoraBatchLaunch& L, int blocks, cuda
 void bora_launch_refine_accumulate_batch( const BoraBatchLaunch& L, int blocks, cudaStream_t st );
 void bora_launch_refine_residual_batch( const BoraBatchLaunch& L, int blocks, cudaStream_t st );
 void bora_launch_write_pressure_batch( const BoraBatchLaunch& L, int blocks, cudaStream_t st );
-void bora_launch_pcg_update_noprec_batch( const BoraBatchLaunch& L, int blocks, cudaStream_t st );
 // pass `pass` (0, 1 down; 2, 3 up) of multigrid level l (0, 1, 2) for the batch, launch
 // shape v (level 0's up 2 has a fixed shape)
 void bora_launch_mg_pass_batch( int l, int pass, int v, const BoraBatchLaunch& L, int blocks, cudaStream_t st );
@@ -396,6 +406,3 @@ void bora_launch_mg_pass_batch( int l, int pass, int v, const BoraBatchLaunch& L
 void bora_member_grids( int ntiles, int* grid, const int* v );
 void bora_projection_grids( int ntiles, int* grid );  // the kGridDir, kGridCells and kGridResidual entries
 
-// e += alpha d; r -= alpha q; r.r -> ring slot (alpha = rz / dq, or 0 when slot_rz < 0)
-void bora_launch_pcg_update_noprec( int ntiles, BoraSolverDev s, BoraReduceDev red, int slot_rz, int slot_dq,
-                                    int slot_rr_out, cudaStream_t st );

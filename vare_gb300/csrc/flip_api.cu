@@ -154,6 +154,7 @@ struct bora_flip_sim
 
     // reductions
     DevBuf ring, partials, done;
+    DevBuf sums;     // the solver chain's partial sums (d.q, r.z, r.r) and the finished pairs
     DevBuf gbar;     // the persistent solver's grid barrier: count, generation
     int fault = 0;   // BORA_FAULT_*
     int next_slot = 0;
@@ -189,8 +190,6 @@ struct bora_flip_sim
     double* d_hring = nullptr;  // its device address
     double* h_mirror = nullptr;  // pinned, mapped: reductions' slot values as the host sees them
     double* d_mirror = nullptr;  // its device address
-    static constexpr int kChecks = 8;
-    cudaEvent_t ev_chk[kChecks] = {};
 
     bora_flip_stats stats{};
     int last_status = BORA_OK;
@@ -251,8 +250,10 @@ struct bora_flip_sim
     }
     BoraReduceDev reducer()
     {
+        float2* p = P<float2>( sums );
         return BoraReduceDev{ P<double>( ring ), P<double>( partials ), P<uint32_t>( done ), P<uint32_t>( counters ) + 5,
-                              d_mirror };
+                              d_mirror, p, p + kBoraMaxReduceBlocks, p + 2 * kBoraMaxReduceBlocks,
+                              p + 3 * kBoraMaxReduceBlocks };
     }
     int slot()
     {
@@ -443,6 +444,26 @@ double read_ring( bora_flip_sim* s, int slot, int* status )
     if( e == cudaSuccess ) e = cudaStreamSynchronize( s->st );
     if( e != cudaSuccess ) { *status = cuda_status( e ); return 0.0; }
     return ( (volatile double*)s->h_ring )[0];
+}
+
+// A value that a kernel writes to mapped host memory (BoraReduceDev::mirror): marked as not
+// arrived before the launch, then polled. Sums of squares and maxima are never negative.
+constexpr double kNotArrived = -1.0;
+void arm_mirror( bora_flip_sim* s, int slot ) { ( (volatile double*)s->h_mirror )[slot] = kNotArrived; }
+int poll_mirror( bora_flip_sim* s, int slot, cudaStream_t st, double* v )
+{
+    volatile double* p = s->h_mirror + slot;
+    for( unsigned n = 1;; ++n )
+    {
+        *v = *p;
+        if( *v != kNotArrived ) return BORA_OK;
+        if( n % 8192 ) continue;
+        const cudaError_t e = cudaStreamQuery( st );  // an error, or nothing left that could write it
+        if( e == cudaErrorNotReady ) continue;
+        if( e != cudaSuccess ) return cuda_status( e );
+        *v = *p;
+        return *v != kNotArrived ? BORA_OK : BORA_ERR_INTERNAL;
+    }
 }
 
 // ---- stages --------------------------------------------------------------------------
@@ -696,11 +717,13 @@ int stage_solve( bora_flip_sim* s )
         s->stats.mg_vcycle_launches = mixed ? vlaunch : 0;
         // the mixed form's update r -= alpha q (alpha = rz_in / dq_in) and r.r run inside the
         // V-cycle's first passes, which scale the FP16 levels by the last known residual norm
-        auto precondition = [&]( int rz_in, int dq_in, int rr_out, int scale, int rz_out ) {
+        auto precondition = [&]( int rz_in, int dq_in, int scale ) {
             KTimer t( s, BORA_KERNEL_MG, vlaunch );
             bora_mg_vcycle( s->g, s->levels, s->nlevels, s->tiles(), mid_img, sv.r, sv.q, sv.z, sv.minv, red, rz_in, dq_in,
-                            rr_out, scale, rz_out, 16, st );
+                            scale, 16, st );
         };
+        // blocks of the kernels that leave partial sums of r.z and r.r
+        int nparts = mixed ? bora_mg_pass_grid( 8, s->ntiles, -1 ) : bora_pcg_update_grid( s->ntiles );
         int rz_cur = s->slot(), rr_cur = s->slot();
         int it = 0;
         int a_rz = -1, a_dq = -1;  // alpha of the last update, whose e += alpha d is still pending
@@ -712,7 +735,7 @@ int stage_solve( bora_flip_sim* s )
             {
                 KTimer t( s, BORA_KERNEL_PCG_UPDATE, 1 );
                 if( bora_launch_pcg_persistent( s->ntiles, P<int32_t>( s->nbr ), code, sv, red, dsel, rz_prev, max_inner, target,
-                                                s_a_rz, s_a_dq, rr_cur, P<uint32_t>( s->counters ) + 8,
+                                                s_a_rz, s_a_dq, P<uint32_t>( s->counters ) + 8,
                                                 P<unsigned>( s->gbar ), P<double>( s->partials ),
                                                 s->fault == BORA_FAULT_BARRIER, st ) != 0 )
                     return BORA_ERR_CUDA;
@@ -725,41 +748,43 @@ int stage_solve( bora_flip_sim* s )
             a_rz = s_a_rz;
             a_dq = s_a_dq;
             rz_prev = s_a_rz;
+            nparts = 1;
         }
         else if( mixed )
         {
-            precondition( -1, -1, rr_cur, scale_slot, rz_cur );
+            precondition( -1, -1, scale_slot );
         }
         else
         {
             KTimer t( s, BORA_KERNEL_PCG_UPDATE, 1 );
-            bora_launch_pcg_update( s->ntiles, code, sv, red, -1, -1, rz_cur, rr_cur, st );
+            bora_launch_pcg_update( s->ntiles, code, sv, red, -1, -1, st );
         }
-        // Convergence checks do not stall the device: the reductions also write their
-        // results to mapped host memory, an event marks the end of iteration i, and the
-        // host waits for it only once iteration i + 1 is queued (a converged solve runs one
-        // extra iteration, which only lowers the residual further).
-        struct Check { int it, q, slot; };
-        Check pend[bora_flip_sim::kChecks];
-        int npend = 0, nchk = 0;
+        // Convergence checks do not stall the device: the direction kernel of iteration i + 1
+        // finishes iteration i's r.r and also writes it to mapped host memory, where the host
+        // polls for it once the rest of iteration i + 1 is queued (a converged solve runs one
+        // extra iteration, which only lowers the residual further). No event stands between the
+        // kernels, which would end their programmatic overlap.
+        int chk_slot = -1;  // r.r of the last iteration, to be checked
         bool done = a_rz >= 0;  // the persistent pass has run
         while( it < max_inner && !done )
         {
             const int s_dq = s->slot();
+            if( chk_slot >= 0 ) arm_mirror( s, chk_slot );
             {
                 KTimer t( s, BORA_KERNEL_PCG_DIRECTION, 1 );
-                bora_launch_pcg_direction( s->g, s->ntiles, s->tiles(), code, sv, dsel, red, rz_cur, rz_prev, s_dq, a_rz, a_dq, st );
+                bora_launch_pcg_direction( s->g, s->ntiles, s->tiles(), code, sv, dsel, red, nparts, rz_cur, rr_cur, rz_prev,
+                                           a_rz, a_dq, chk_slot >= 0, st );
             }
             dsel ^= 1;
             const int rz_new = s->slot(), rr_new = s->slot();
             if( mixed )
             {
-                precondition( rz_cur, s_dq, rr_new, rr_cur, rz_new );
+                precondition( rz_cur, s_dq, rr_cur );
             }
             else
             {
                 KTimer t( s, BORA_KERNEL_PCG_UPDATE, 1 );
-                bora_launch_pcg_update( s->ntiles, code, sv, red, rz_cur, s_dq, rz_new, rr_new, st );
+                bora_launch_pcg_update( s->ntiles, code, sv, red, rz_cur, s_dq, st );
             }
             a_rz = rz_cur;
             a_dq = s_dq;
@@ -767,20 +792,17 @@ int stage_solve( bora_flip_sim* s )
             rz_cur = rz_new;
             rr_cur = rr_new;
             ++it;
+            if( chk_slot >= 0 )
+            {
+                double rr = 0.0;
+                BORA_TRYS( poll_mirror( s, chk_slot, st, &rr ) );
+                if( !( rr > 0.0 ) || std::sqrt( rr ) <= target ) done = true;
+            }
+            chk_slot = -1;
             if( it % check == 0 )
             {
                 BORA_TRYS( check_launch( s ) );
-                const int q = nchk++ % bora_flip_sim::kChecks;
-                BORA_TRY( cudaEventRecord( s->ev_chk[q], st ) );
-                pend[npend++] = Check{ it, q, rr_cur };
-            }
-            while( npend > 0 && ( it - pend[0].it >= 1 || npend == bora_flip_sim::kChecks || it >= max_inner ) )
-            {
-                BORA_TRY( cudaEventSynchronize( s->ev_chk[pend[0].q] ) );
-                const double rr = ( (volatile double*)s->h_mirror )[pend[0].slot];
-                for( int k = 1; k < npend; ++k ) pend[k - 1] = pend[k];
-                --npend;
-                if( !( rr > 0.0 ) || std::sqrt( rr ) <= target ) { done = true; break; }
+                chk_slot = rr_cur;
             }
         }
         total_it += it;
@@ -788,7 +810,7 @@ int stage_solve( bora_flip_sim* s )
         const int s_n2 = s->slot(), s_mx = s->slot();
         {
             KTimer t( s, BORA_KERNEL_REFINE, 2 );
-            bora_launch_refine_accumulate( s->ntiles, code, sv, dsel, P<double>( s->ring ), a_rz, a_dq, st );
+            bora_launch_refine_accumulate( s->ntiles, code, sv, dsel, red, nparts, rr_cur, a_rz, a_dq, st );
             bora_launch_refine_residual( s->g, s->ntiles, s->tiles(), b, code, sv, red, s_n2, s_mx, st );
         }
         BORA_TRYS( check_launch( s ) );
@@ -1000,7 +1022,7 @@ void for_each_buffer( bora_flip_sim* s, F&& f )
     DevBuf* all[] = { &s->tile_flag, &s->tile_act, &s->tile_excl, &s->slot_of, &s->tile_of, &s->nbr, &s->mass, &s->surf,
                       &s->pres, &s->vx, &s->vy, &s->vz, &s->cx, &s->cy, &s->cz, &s->flag, &s->code, &s->rhs, &s->sx,
                       &s->se, &s->sr, &s->sd0, &s->sd1, &s->sq, &s->sz, &s->sminv, &s->cell_count, &s->cell_start,
-                      &s->ring, &s->partials, &s->done, &s->adj, &s->vkey, &s->key, &s->idx, &s->scan_scratch,
+                      &s->ring, &s->partials, &s->done, &s->sums, &s->adj, &s->vkey, &s->key, &s->idx, &s->scan_scratch,
                       &s->counters, &s->stage_in, &s->stage_out, &s->live_flag, &s->col_phi, &s->col_vel,
                       &s->col_tslot, &s->col_tnear, &s->col_tphi, &s->col_tvel, &s->gbar };
     for( DevBuf* b : all ) f( *b );
@@ -1096,8 +1118,6 @@ int bora_flip_create( const bora_grid_desc* grid, const bora_flip_params* params
     if( st == BORA_OK ) st = cuda_status( cudaHostGetDevicePointer( (void**)&s->d_hring, s->h_ring, 0 ) );
     if( st == BORA_OK ) st = cuda_status( cudaHostAlloc( (void**)&s->h_mirror, BORA_RING * 8, cudaHostAllocMapped ) );
     if( st == BORA_OK ) st = cuda_status( cudaHostGetDevicePointer( (void**)&s->d_mirror, s->h_mirror, 0 ) );
-    for( int q = 0; q < bora_flip_sim::kChecks && st == BORA_OK; ++q )
-        st = cuda_status( cudaEventCreateWithFlags( &s->ev_chk[q], cudaEventDisableTiming ) );
     if( st == BORA_OK ) st = cuda_status( grow( s->tile_flag, s->ntv, false, s->st ) );
     if( st == BORA_OK ) st = cuda_status( grow( s->tile_act, s->ntv * 4, false, s->st ) );
     if( st == BORA_OK ) st = cuda_status( grow( s->tile_excl, s->ntv * 4, false, s->st ) );
@@ -1106,6 +1126,7 @@ int bora_flip_create( const bora_grid_desc* grid, const bora_flip_params* params
     if( st == BORA_OK ) st = cuda_status( grow( s->counters, 64, false, s->st ) );
     if( st == BORA_OK ) st = cuda_status( grow( s->ring, BORA_RING * 8, false, s->st ) );
     if( st == BORA_OK ) st = cuda_status( grow( s->done, BORA_RING * 4, false, s->st ) );
+    if( st == BORA_OK ) st = cuda_status( grow( s->sums, ( 3 * kBoraMaxReduceBlocks + BORA_RING ) * 8, false, s->st ) );
     if( st == BORA_OK ) st = cuda_status( grow( s->gbar, 16, false, s->st ) );
     if( st == BORA_OK ) st = cuda_status( cudaMemsetAsync( s->done.p, 0, BORA_RING * 4, s->st ) );
     if( st == BORA_OK ) st = cuda_status( cudaMemsetAsync( s->ring.p, 0, BORA_RING * 8, s->st ) );
@@ -1134,8 +1155,6 @@ int bora_flip_destroy( bora_flip_handle s )
     for( cudaEvent_t e : s->evpool ) cudaEventDestroy( e );
     for( int q = 0; q < 2; ++q )
         if( s->ev_step[q] ) cudaEventDestroy( s->ev_step[q] );
-    for( cudaEvent_t e : s->ev_chk )
-        if( e ) cudaEventDestroy( e );
     if( s->ev_join ) cudaEventDestroy( s->ev_join );
     if( s->h_cnt ) cudaFreeHost( s->h_cnt );
     if( s->h_ring ) cudaFreeHost( s->h_ring );
@@ -1418,9 +1437,7 @@ struct BatchMember
     bool converged = false, inner_done = false;
     int rz_prev = -1, dsel = 0, rz_cur = -1, rr_cur = -1, a_rz = -1, a_dq = -1;
     int s_b2 = -1, s_bmax = -1, s_n2 = -1, s_mx = -1;
-    struct Check { int it, tick, slot; };
-    Check pend[bora_flip_sim::kChecks];
-    int npend = 0;
+    int chk_slot = -1;  // r.r of the last iteration, to be checked once the next one is queued
 
     double mirror( int slot ) const { return ( (volatile double*)s->h_mirror )[slot]; }
     // the check at the top of stage_solve's pass loop
@@ -1441,7 +1458,7 @@ struct BatchBuffers
     DevBuf ms, sl, mid;
 };
 
-int batch_solve( std::vector<BatchMember>& M, cudaStream_t st, BatchBuffers& bb, bora_flip_sim* host_of_events )
+int batch_solve( std::vector<BatchMember>& M, cudaStream_t st, BatchBuffers& bb )
 {
     const int n = (int)M.size();
     // static per-simulation records: solver vectors, reductions, levels, own grids, and the
@@ -1570,9 +1587,6 @@ int batch_solve( std::vector<BatchMember>& M, cudaStream_t st, BatchBuffers& bb,
         b.check = std::max( 1, b.s->prm.check_every );
         b.decide();
     }
-    int tick = 0;
-    cudaEvent_t* tev = host_of_events->ev_chk;
-    constexpr int kTicks = bora_flip_sim::kChecks;
     for( ;; )
     {
         // passes that start: the first V-cycle z = M^-1 r with r.r (no residual update; scaled
@@ -1588,12 +1602,10 @@ int batch_solve( std::vector<BatchMember>& M, cudaStream_t st, BatchBuffers& bb,
             sl[k].active = 1;
             sl[k].rz_in = -1;
             sl[k].dq_in = -1;
-            sl[k].rr_out = b.rr_cur;
             sl[k].rr = b.passes == 0 ? b.s_b2 : b.s_n2;
-            sl[k].rz = b.rz_cur;
             b.phase = BatchMember::kInner;
             b.it = 0;
-            b.npend = 0;
+            b.chk_slot = -1;
             b.a_rz = b.a_dq = -1;
             b.inner_done = false;
             b.s->stats.mg_vcycle_launches = 13;
@@ -1616,9 +1628,11 @@ int batch_solve( std::vector<BatchMember>& M, cudaStream_t st, BatchBuffers& bb,
             BoraMemberSlots& q = sl[k];
             q.active = 1;
             q.dsel = b.dsel;
-            q.rz_new = b.rz_cur; q.rz_old = b.rz_prev; q.dq = s_dq; q.a_rz = b.a_rz; q.a_dq = b.a_dq;
-            q.rz_in = b.rz_cur; q.dq_in = s_dq; q.rr_out = rr_new;
-            q.rr = b.rr_cur; q.rz = rz_new;  // the V-cycle's scale: the previous r.r
+            q.rz_new = b.rz_cur; q.rr_new = b.rr_cur; q.rz_old = b.rz_prev; q.a_rz = b.a_rz; q.a_dq = b.a_dq;
+            q.rz_in = b.rz_cur; q.dq_in = s_dq;
+            q.rr = b.rr_cur;  // the V-cycle's scale: the previous r.r
+            q.chk = b.chk_slot >= 0;
+            if( q.chk ) arm_mirror( b.s, b.chk_slot );
             b.dsel ^= 1;
             b.a_rz = b.rz_cur;
             b.a_dq = s_dq;
@@ -1635,23 +1649,19 @@ int batch_solve( std::vector<BatchMember>& M, cudaStream_t st, BatchBuffers& bb,
             ++launches;
             vcycle();  // with the residual update
             BORA_TRYS( check_launch( nullptr ) );
-            BORA_TRY( cudaEventRecord( tev[tick % kTicks], st ) );
             for( int k = 0; k < n; ++k )
             {
                 if( !sl[k].active ) continue;
                 BatchMember& b = M[k];
-                if( b.it % b.check == 0 ) b.pend[b.npend++] = BatchMember::Check{ b.it, tick, b.rr_cur };
                 // the convergence check of stage_solve: iteration i is read once i + 1 is queued
-                while( b.npend > 0 && ( b.it - b.pend[0].it >= 1 || b.npend == kTicks || b.it >= b.max_inner ) )
+                if( b.chk_slot >= 0 )
                 {
-                    BORA_TRY( cudaEventSynchronize( tev[b.pend[0].tick % kTicks] ) );
-                    const double rr = b.mirror( b.pend[0].slot );
-                    for( int q = 1; q < b.npend; ++q ) b.pend[q - 1] = b.pend[q];
-                    --b.npend;
-                    if( !( rr > 0.0 ) || std::sqrt( rr ) <= b.target ) { b.inner_done = true; break; }
+                    double rr = 0.0;  // the direction kernel finished the previous iteration's r.r
+                    BORA_TRYS( poll_mirror( b.s, b.chk_slot, st, &rr ) );
+                    if( !( rr > 0.0 ) || std::sqrt( rr ) <= b.target ) b.inner_done = true;
                 }
+                b.chk_slot = b.it % b.check == 0 ? b.rr_cur : -1;
             }
-            ++tick;
         }
         // passes that end: refinement (x += e; r = b - A x in double-float arithmetic)
         bool refine = false;
@@ -1664,6 +1674,7 @@ int batch_solve( std::vector<BatchMember>& M, cudaStream_t st, BatchBuffers& bb,
             b.s_mx = b.s->slot();
             sl[k].active = 1;
             sl[k].dsel = b.dsel;
+            sl[k].rr_new = b.rr_cur;
             sl[k].a_rz = b.a_rz;
             sl[k].a_dq = b.a_dq;
             sl[k].n2 = b.s_n2;
@@ -1812,7 +1823,7 @@ int bora_flip_step_batch( bora_flip_handle* hs, int n, float dt, int* status )
         static std::mutex bb_mu;
         std::lock_guard<std::mutex> lk( bb_mu );
         BatchBuffers& bb = bb_cache[dev >= 0 && dev < 64 ? dev : 0];
-        const int solve = batch_solve( M, st, bb, h0 );
+        const int solve = batch_solve( M, st, bb );
         if( solve < 0 ) return solve;
     }
     const auto t2 = std::chrono::steady_clock::now();

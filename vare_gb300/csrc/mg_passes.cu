@@ -269,9 +269,8 @@ struct Pass0Args
     float* zout;          // up 2: the PCG's z
     BoraReduceDev red;
     int slot_rr;          // the scale's r.r
-    int slot_rz;          // up 2: r.z out
     int slot_rz_in, slot_dq_in;  // down 1, 2: alpha = rz_in / dq_in (slot_rz_in < 0: no update)
-    int slot_rr_out;      // down 1: r.r of the updated residual out
+    int ndq;              // down 1: partial sums of dq to finish into slot_dq_in
 };
 
 // pass P of level 0: 0 = down 1, 1 = down 2, 2 = up 1, 3 = up 2; W tiles (warps) per block
@@ -299,16 +298,20 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
     };
     int s = (int)bid * W + ( threadIdx.x >> 5 );
     fetch( s );
-    __shared__ float s_alpha;
+    __shared__ float2 s_dq[W];
     bora_pdl_wait();  // the previous kernel's results are complete from here
-    if( threadIdx.x == 0 )
-    {
-        s_sc = scale_from( a.red.ring, a.slot_rr );
-        s_alpha = a.slot_rz_in < 0 ? 0.f : (float)( a.red.ring[a.slot_rz_in] / a.red.ring[a.slot_dq_in] );
-    }
-    __syncthreads();
-    const float sc = s_sc, alpha = s_alpha;
+    if( threadIdx.x == 0 ) s_sc = scale_from( a.red.ring, a.slot_rr );
     const bool upd = ( P == 0 || P == 1 ) && a.slot_rz_in >= 0;  // down 1, 2 apply r -= alpha q
+    float alpha = 0.f;
+    if( P == 0 && upd )
+    {
+        const DF dq = part_collect( a.red.part_dq, a.ndq, s_dq );
+        alpha = df_ratio( a.red.ringf[a.slot_rz_in], make_float2( dq.hi, dq.lo ) );
+        if( bid == 0 && threadIdx.x == 0 ) ring_store( a.red, a.slot_dq_in, dq, false );
+    }
+    if( P == 1 && upd ) alpha = df_ratio( a.red.ringf[a.slot_rz_in], a.red.ringf[a.slot_dq_in] );
+    __syncthreads();
+    const float sc = s_sc;
     DF acc{ 0.f, 0.f };  // down 1: r.r of the updated residual; up 2: r.z
     for( ; s < a.ntiles; s += stride )
     {
@@ -454,8 +457,8 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
             acc = df_add_f( acc, trz );
         }
     }
-    if constexpr( P == 3 ) reduce2_publish_warp( df_warp_sum( acc ), 0.0, 0, a.red, a.slot_rz, -1, bid, G );
-    if constexpr( P == 0 ) reduce2_publish_warp( df_warp_sum( acc ), 0.0, 0, a.red, a.slot_rr_out, -1, bid, G );
+    if constexpr( P == 3 ) part_publish( acc, DF{ 0.f, 0.f }, a.red.part_rz, nullptr, bid );
+    if constexpr( P == 0 ) part_publish( acc, DF{ 0.f, 0.f }, a.red.part_rr, nullptr, bid );
 }
 
 template <int W, int P>
@@ -482,10 +485,9 @@ __global__ void __launch_bounds__( 32 * W, 16 / W ) k_mg_pass0_batch( const __gr
     a.zout = m.sv.z;
     a.red = m.red;
     a.slot_rr = q.rr;
-    a.slot_rz = q.rz;
     a.slot_rz_in = q.rz_in;
     a.slot_dq_in = q.dq_in;
-    a.slot_rr_out = q.rr_out;
+    a.ndq = m.grid[kGridDir];
     pass0_body<W, P>( a, bid, (unsigned)m.grid[P == 0 || P == 3 ? kGridPass0R : kGridPass0] );
 }
 
@@ -679,7 +681,7 @@ int bora_mg_pass_grid( int E, int ntiles, int v )
 
 void bora_mg_pass_down( const BoraLevelDev* levels, int l, const BoraTilesDev& t, int ntiles, float* r0, const float* q,
                         float* scratch, const BoraReduceDev& red, int slot_rr, int slot_rz_in, int slot_dq_in,
-                        int slot_rr_out, cudaStream_t st )
+                        cudaStream_t st )
 {
     const int group = l == 0 ? kBoraTuneL0 : ( l == 1 ? kBoraTuneL1 : kBoraTuneL2 );
     const BoraTunePick pick = bora_tune_pick( group, ntiles );
@@ -689,8 +691,8 @@ void bora_mg_pass_down( const BoraLevelDev* levels, int l, const BoraTilesDev& t
     {
         Pass0Args a{};
         a.ntiles = ntiles; a.nbr = t.nbr; a.F = levels[0]; a.C = levels[1]; a.r0 = r0; a.q = q; a.scratch = scratch;
-        a.red = red; a.slot_rr = slot_rr; a.slot_rz = -1;
-        a.slot_rz_in = slot_rz_in; a.slot_dq_in = slot_dq_in; a.slot_rr_out = slot_rr_out;
+        a.red = red; a.slot_rr = slot_rr;
+        a.slot_rz_in = slot_rz_in; a.slot_dq_in = slot_dq_in; a.ndq = bora_pcg_direction_grid( ntiles );
         // down 1 sums r.r over its blocks: the fixed shape
         const int g = bora_mg_pass_grid( 8, ntiles, -1 );
         if( g > 0 ) bora_launch_pdl( k_mg_pass0<kReduceWarps, 0>, dim3( g ), dim3( 32 * kReduceWarps ), 0, st, a );
@@ -704,8 +706,7 @@ void bora_mg_pass_down( const BoraLevelDev* levels, int l, const BoraTilesDev& t
 }
 
 void bora_mg_pass_up( const BoraLevelDev* levels, int l, const __half* ec, const BoraTilesDev& t, int ntiles,
-                      const float* r0, float* scratch, const BoraReduceDev& red, int slot_rr, float* z, int slot_rz,
-                      cudaStream_t st )
+                      const float* r0, float* scratch, const BoraReduceDev& red, int slot_rr, float* z, cudaStream_t st )
 {
     const int group = l == 0 ? kBoraTuneL0 : ( l == 1 ? kBoraTuneL1 : kBoraTuneL2 );
     const int v = bora_tune_pick( group, ntiles ).variant;
@@ -713,8 +714,8 @@ void bora_mg_pass_up( const BoraLevelDev* levels, int l, const __half* ec, const
     {
         Pass0Args a{};
         a.ntiles = ntiles; a.nbr = t.nbr; a.F = levels[0]; a.C = levels[1]; a.C.z1 = const_cast<__half*>( ec );
-        a.r0 = const_cast<float*>( r0 ); a.scratch = scratch; a.zout = z; a.red = red; a.slot_rr = slot_rr; a.slot_rz = slot_rz;
-        a.slot_rz_in = -1; a.slot_dq_in = -1; a.slot_rr_out = -1;
+        a.r0 = const_cast<float*>( r0 ); a.scratch = scratch; a.zout = z; a.red = red; a.slot_rr = slot_rr;
+        a.slot_rz_in = -1; a.slot_dq_in = -1;
         launch_pass0<2>( a, v, st );
         // r.z: the fixed shape
         const int g = bora_mg_pass_grid( 8, ntiles, -1 );

@@ -186,12 +186,6 @@ __global__ void k_mg_codes( LevelNav nav, float voxel_wall )
 // neighbour table), dense levels use their small extents. Kernels only visit the
 // neighbours that the stencil code marks as fluid, which always exist.
 
-__device__ inline float scale_of( const double* ring, int slot )
-{
-    const double rr = ring[slot];
-    return rr > 0.0 ? (float)( 1.0 / sqrt( rr ) ) : 1.f;
-}
-
 template <int E>
 struct TiledNav
 {
@@ -263,14 +257,11 @@ struct DenseNav
     }
 };
 
-// Level residual r' of a cell: level 0 reads the PCG residual (FP32) times the scale,
-// coarser levels read their FP16 residual.
+// Level residual r' of a cell (level 0 runs in mg_passes.cu).
 struct RIn
 {
-    const float* r0;
-    float s;
     const __half* rh;
-    __device__ inline float operator()( long long c ) const { return r0 ? r0[c] * s : __half2float( rh[c] ); }
+    __device__ inline float operator()( long long c ) const { return __half2float( rh[c] ); }
 };
 
 __device__ inline float ldh( const __half* z, long long c ) { return __half2float( z[c] ); }
@@ -464,13 +455,11 @@ __device__ inline void prolong_smooth_cells( const Nav& nav, const BoraLevelDev&
     }
 }
 
-// Final Jacobi sweep of a level: z = z1 + w (r' - S z1)/d, written to z0. On level 0 the
-// result is unscaled to FP32 into zout and r.z is accumulated (double-float).
+// Final Jacobi sweep of a level: z = z1 + w (r' - S z1)/d, written to z0.
 template <class Nav>
-__device__ inline DF smooth_last_cells( const Nav& nav, const BoraLevelDev& L, const RIn& R, float* __restrict__ zout,
-                                        uint32_t* err, long long i0, long long stride )
+__device__ inline void smooth_last_cells( const Nav& nav, const BoraLevelDev& L, const RIn& R, uint32_t* err, long long i0,
+                                          long long stride )
 {
-    DF rz{ 0.f, 0.f };
     for( long long cell = i0; cell < (long long)L.ncells; cell += stride )
     {
         const uint16_t cc = L.code[cell];
@@ -490,18 +479,8 @@ __device__ inline DF smooth_last_cells( const Nav& nav, const BoraLevelDev& L, c
             }
             zc = zb + kOmegaA * ( R( cell ) - ( (float)dg * zb - sum ) ) / (float)dg;
         }
-        if( zout )
-        {
-            const float zf = zc / R.s;  // undo the FP16 scaling of the residual
-            zout[cell] = zf;
-            if( cc & BORA_CODE_FLUID ) rz = df_add( rz, df_prod( R.r0[cell], zf ) );
-        }
-        else
-        {
-            L.z0[cell] = __float2half_rn( zc );
-        }
+        L.z0[cell] = __float2half_rn( zc );
     }
-    return rz;
 }
 
 // Grid-wide kernels, one per operation.
@@ -509,26 +488,17 @@ __device__ inline long long gtid() { return blockIdx.x * (long long)blockDim.x +
 __device__ inline long long gstride() { return (long long)gridDim.x * blockDim.x; }
 
 template <class Nav>
-__global__ void __launch_bounds__( 256 ) k_mg_smooth0( Nav nav, BoraLevelDev L, const float* __restrict__ r0,
-                                                       int slot_rr, const double* __restrict__ ring, uint32_t* err )
+__global__ void __launch_bounds__( 256 ) k_mg_smooth0( Nav nav, BoraLevelDev L, uint32_t* err )
 {
-    __shared__ float s_scale;
-    if( threadIdx.x == 0 ) s_scale = r0 ? scale_of( ring, slot_rr ) : 1.f;
-    __syncthreads();
-    smooth0_cells( nav, L, RIn{ r0, s_scale, L.r }, err, gtid(), gstride() );
+    smooth0_cells( nav, L, RIn{ L.r }, err, gtid(), gstride() );
 }
 
 template <class FNav, int MODE, int EC>
 __global__ void __launch_bounds__( 256 ) k_mg_restrict( FNav fnav, BoraLevelDev F, BoraLevelDev C,
-                                                        const float* __restrict__ r0, int slot_rr,
-                                                        const double* __restrict__ ring,
                                                         const int32_t* __restrict__ slot_of, int tx, int ty, int tz,
                                                         uint32_t* err )
 {
-    __shared__ float s_scale;
-    if( threadIdx.x == 0 ) s_scale = r0 ? scale_of( ring, slot_rr ) : 1.f;
-    __syncthreads();
-    restrict_cells<FNav, MODE, EC>( fnav, F, C, RIn{ r0, s_scale, F.r }, slot_of, tx, ty, tz, err, gtid(), gstride() );
+    restrict_cells<FNav, MODE, EC>( fnav, F, C, RIn{ F.r }, slot_of, tx, ty, tz, err, gtid(), gstride() );
 }
 
 template <class Nav>
@@ -540,25 +510,15 @@ __global__ void __launch_bounds__( 512 ) k_mg_coarsest( Nav nav, BoraLevelDev L,
 
 template <class Nav>
 __global__ void __launch_bounds__( 256 ) k_mg_prolong_smooth( Nav nav, BoraLevelDev F, const __half* __restrict__ ec,
-                                                              const float* __restrict__ r0, int slot_rr,
-                                                              const double* __restrict__ ring, uint32_t* err )
+                                                              uint32_t* err )
 {
-    __shared__ float s_scale;
-    if( threadIdx.x == 0 ) s_scale = r0 ? scale_of( ring, slot_rr ) : 1.f;
-    __syncthreads();
-    prolong_smooth_cells( nav, F, ec, RIn{ r0, s_scale, F.r }, err, gtid(), gstride() );
+    prolong_smooth_cells( nav, F, ec, RIn{ F.r }, err, gtid(), gstride() );
 }
 
 template <class Nav>
-__global__ void __launch_bounds__( 256 ) k_mg_smooth_last( Nav nav, BoraLevelDev L, const float* __restrict__ r0,
-                                                           int slot_rr, BoraReduceDev red, float* __restrict__ zout,
-                                                           int slot_rz )
+__global__ void __launch_bounds__( 256 ) k_mg_smooth_last( Nav nav, BoraLevelDev L, uint32_t* err )
 {
-    __shared__ float s_scale;
-    if( threadIdx.x == 0 ) s_scale = r0 ? scale_of( red.ring, slot_rr ) : 1.f;
-    __syncthreads();
-    const DF rz = smooth_last_cells( nav, L, RIn{ r0, s_scale, L.r }, zout, red.err, gtid(), gstride() );
-    if( zout ) reduce2_publish_warp( df_warp_sum( rz ), 0.0, 0, red, slot_rz, -1 );
+    smooth_last_cells( nav, L, RIn{ L.r }, err, gtid(), gstride() );
 }
 
 // The small tail of the hierarchy in one thread-block cluster: levels that are dense or
@@ -602,7 +562,7 @@ __global__ void __launch_bounds__( kTailThreads ) k_mg_tail( const __grid_consta
     };
     for( int t = 0; t + 1 < d.n; ++t )
     {
-        const RIn R{ nullptr, 1.f, d.L[t].r };
+        const RIn R{ d.L[t].r };
         with_level( t, [&]( auto nav ) { smooth0_cells( nav, d.L[t], R, err, i0, st ); } );
         cluster_barrier();
         with_level( t, [&]( auto nav ) {
@@ -617,58 +577,16 @@ __global__ void __launch_bounds__( kTailThreads ) k_mg_tail( const __grid_consta
     cluster_barrier();
     for( int t = d.n - 2; t >= 0; --t )
     {
-        const RIn R{ nullptr, 1.f, d.L[t].r };
+        const RIn R{ d.L[t].r };
         with_level( t, [&]( auto nav ) { prolong_smooth_cells( nav, d.L[t], d.L[t + 1].z0, R, err, i0, st ); } );
         cluster_barrier();
-        with_level( t, [&]( auto nav ) { (void)smooth_last_cells( nav, d.L[t], R, nullptr, err, i0, st ); } );
+        with_level( t, [&]( auto nav ) { smooth_last_cells( nav, d.L[t], R, err, i0, st ); } );
         cluster_barrier();
     }
 }
 
 // ---- tiled levels with E >= 2 -----------------------------------------------------------
 // Levels 0, 1 and 2 (E = 8, 4, 2) run as stencil passes (mg_passes.cu).
-
-// PCG update without a preconditioner sweep: r -= alpha q; r.r (e += alpha d is applied by
-// the next direction kernel or the refinement step).
-__device__ __forceinline__ void pcg_update_noprec_body( size_t ncells, const BoraSolverDev& sv, const BoraReduceDev& red,
-                                                        int slot_rz, int slot_dq, int slot_rr_out, unsigned bid, unsigned G )
-{
-    __shared__ float s_alpha;
-    bora_pdl_trigger();
-    bora_pdl_wait();
-    if( threadIdx.x == 0 ) s_alpha = slot_rz < 0 ? 0.f : (float)( red.ring[slot_rz] / red.ring[slot_dq] );
-    __syncthreads();
-    const float alpha = s_alpha;
-    DF rr{ 0.f, 0.f };
-    const size_t n4 = ncells / 4;
-    float4* __restrict__ r4 = reinterpret_cast<float4*>( sv.r );
-    const float4* __restrict__ q4 = reinterpret_cast<const float4*>( sv.q );
-    for( size_t v = bid * (size_t)blockDim.x + threadIdx.x; v < n4; v += (size_t)G * blockDim.x )
-    {
-        float4 r = r4[v];
-        const float4 q = q4[v];
-        r.x = fmaf( -alpha, q.x, r.x ); r.y = fmaf( -alpha, q.y, r.y ); r.z = fmaf( -alpha, q.z, r.z ); r.w = fmaf( -alpha, q.w, r.w );
-        r4[v] = r;
-        rr = df_add_f( rr, dot4( r, r ) );
-    }
-    reduce2_publish_warp( df_warp_sum( rr ), 0.0, 0, red, slot_rr_out, -1, bid, G );
-}
-
-__global__ void __launch_bounds__( 256 ) k_pcg_update_noprec( size_t ncells, BoraSolverDev sv, BoraReduceDev red,
-                                                              int slot_rz, int slot_dq, int slot_rr_out )
-{
-    pcg_update_noprec_body( ncells, sv, red, slot_rz, slot_dq, slot_rr_out, blockIdx.x, gridDim.x );
-}
-
-__global__ void __launch_bounds__( 256 ) k_pcg_update_noprec_batch( const __grid_constant__ BoraBatchLaunch L )
-{
-    unsigned bid;
-    const int k = bora_batch_member( L, blockIdx.x, &bid );
-    const BoraMemberSolve& m = L.ms[k];
-    const BoraMemberSlots& q = L.sl[k];
-    pcg_update_noprec_body( (size_t)m.ntiles * 512, m.sv, m.red, q.rz_in, q.dq_in, q.rr_out, bid,
-                            (unsigned)m.grid[kGridUpd] );
-}
 
 int sm_count()
 {
@@ -788,13 +706,12 @@ int bora_mg_vcycle_launches( const BoraGridDev& g, const BoraLevelDev* levels, i
     const int stop = std::min( first, nlevels - 1 );
     int n = 1;  // the tail kernel, or the coarsest-level kernel
     for( int l = 0; l < stop; ++l ) n += 4;
-    if( !( stop > 0 && pass_level( levels[0] ) ) ) n += 1;  // the residual update on its own
     return n;
 }
 
 void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t, const void* mid_image,
                      float* r, const float* q, float* z, float* scratch, BoraReduceDev red, int slot_rz_in,
-                     int slot_dq_in, int slot_rr_out, int slot_scale, int slot_rz, int coarse_sweeps, cudaStream_t st )
+                     int slot_dq_in, int slot_scale, int coarse_sweeps, cudaStream_t st )
 {
     if( nlevels < 2 ) return;  // the caller always builds at least two levels
     if( levels[0].ncells == 0 ) return;
@@ -805,41 +722,29 @@ void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nleve
     const bool mid = bora_mg_mid_vcycle( g, levels, nlevels, t, ntiles, mid_image, red.err, coarse_sweeps, st, false ) != 0;
     const int first = mid ? 3 : tail_start( levels, nlevels );  // levels [first, last] run in one kernel
     const int stop = std::min( first, last );                     // levels [0, stop) restrict/prolong here
-    // the residual update runs in level 0's down passes; when level 0 itself is in the tail
-    // kernel, it runs first on its own, and the V-cycle is scaled by its r.r
-    int slot_rr = slot_scale;
-    if( !( stop > 0 && pass_level( levels[0] ) ) )
-    {
-        BoraSolverDev sv{};
-        sv.r = r;
-        sv.q = const_cast<float*>( q );
-        bora_launch_pcg_update_noprec( ntiles, sv, red, slot_rz_in, slot_dq_in, slot_rr_out, st );
-        slot_rr = slot_rr_out;
-    }
     // down: pre-smooth and restrict
     for( int l = 0; l < stop; ++l )
     {
         const BoraLevelDev& F = levels[l];
         const BoraLevelDev& C = levels[l + 1];
-        const float* r0 = l == 0 ? r : nullptr;
         if( pass_level( F ) )
         {
-            bora_mg_pass_down( levels, l, t, ntiles, r, q, scratch, red, slot_rr, slot_rz_in, slot_dq_in, slot_rr_out, st );
+            bora_mg_pass_down( levels, l, t, ntiles, r, q, scratch, red, slot_scale, slot_rz_in, slot_dq_in, st );
             continue;
         }
         with_nav( g, levels, nlevels, l, t, [&]( auto nav ) {
-            k_mg_smooth0<<<blocks_for( F.ncells ), 256, 0, st>>>( nav, F, r0, slot_rr, red.ring, red.err );
+            k_mg_smooth0<<<blocks_for( F.ncells ), 256, 0, st>>>( nav, F, red.err );
             const int nb = blocks_for( C.ncells * 8 );
             using N = decltype( nav );
             if( C.kind == 1 )
             {
                 if( F.kind == 1 )
-                    k_mg_restrict<N, 2, 1><<<nb, 256, 0, st>>>( nav, F, C, r0, slot_rr, red.ring, t.slot_of, g.tx, g.ty, g.tz, red.err );
+                    k_mg_restrict<N, 2, 1><<<nb, 256, 0, st>>>( nav, F, C, t.slot_of, g.tx, g.ty, g.tz, red.err );
                 else
-                    k_mg_restrict<N, 1, 1><<<nb, 256, 0, st>>>( nav, F, C, r0, slot_rr, red.ring, t.slot_of, g.tx, g.ty, g.tz, red.err );
+                    k_mg_restrict<N, 1, 1><<<nb, 256, 0, st>>>( nav, F, C, t.slot_of, g.tx, g.ty, g.tz, red.err );
             }
             else
-                k_mg_restrict<N, 0, 1><<<nb, 256, 0, st>>>( nav, F, C, r0, slot_rr, red.ring, t.slot_of, g.tx, g.ty, g.tz, red.err );
+                k_mg_restrict<N, 0, 1><<<nb, 256, 0, st>>>( nav, F, C, t.slot_of, g.tx, g.ty, g.tz, red.err );
         } );
     }
     if( mid )
@@ -881,20 +786,17 @@ void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nleve
     for( int l = stop - 1; l >= 0; --l )
     {
         const BoraLevelDev& F = levels[l];
-        const float* r0 = l == 0 ? r : nullptr;
         if( pass_level( F ) )
         {
             // a coarser level that ran its passes left its correction in z1, the others in z0
             const bool cf = l + 1 < stop && pass_level( levels[l + 1] );
             const __half* ec = cf ? levels[l + 1].z1 : levels[l + 1].z0;
-            bora_mg_pass_up( levels, l, ec, t, ntiles, r, scratch, red, slot_rr, z, slot_rz, st );
+            bora_mg_pass_up( levels, l, ec, t, ntiles, r, scratch, red, slot_scale, z, st );
             continue;
         }
         with_nav( g, levels, nlevels, l, t, [&]( auto nav ) {
-            k_mg_prolong_smooth<<<blocks_for( F.ncells ), 256, 0, st>>>( nav, F, levels[l + 1].z0, r0, slot_rr, red.ring,
-                                                                         red.err );
-            k_mg_smooth_last<<<blocks_for( F.ncells ), 256, 0, st>>>( nav, F, r0, slot_rr, red, l == 0 ? z : nullptr,
-                                                                      slot_rz );
+            k_mg_prolong_smooth<<<blocks_for( F.ncells ), 256, 0, st>>>( nav, F, levels[l + 1].z0, red.err );
+            k_mg_smooth_last<<<blocks_for( F.ncells ), 256, 0, st>>>( nav, F, red.err );
         } );
     }
 }
@@ -902,22 +804,8 @@ void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nleve
 void bora_member_grids( int ntiles, int* grid, const int* v )
 {
     bora_projection_grids( ntiles, grid );
-    grid[kGridUpd] = blocks_for( (size_t)std::max( ntiles, 0 ) * 512 / 4 );
     grid[kGridPass0] = bora_mg_pass_grid( 8, ntiles, v[0] );
     grid[kGridPass0R] = bora_mg_pass_grid( 8, ntiles, -1 );
     grid[kGridPass1] = bora_mg_pass_grid( 4, ntiles, v[1] );
     grid[kGridPass2] = bora_mg_pass_grid( 2, ntiles, v[2] );
-}
-
-void bora_launch_pcg_update_noprec_batch( const BoraBatchLaunch& L, int blocks, cudaStream_t st )
-{
-    if( blocks > 0 ) bora_launch_pdl( k_pcg_update_noprec_batch, dim3( blocks ), dim3( 256 ), 0, st, L );
-}
-
-
-void bora_launch_pcg_update_noprec( int ntiles, BoraSolverDev s, BoraReduceDev red, int slot_rz, int slot_dq,
-                                    int slot_rr_out, cudaStream_t st )
-{
-    const size_t nc = (size_t)ntiles * 512;
-    bora_launch_pdl( k_pcg_update_noprec, blocks_for( nc / 4 ), 256, 0, st, nc, s, red, slot_rz, slot_dq, slot_rr_out );
 }

@@ -425,22 +425,27 @@ __device__ __forceinline__ void pcg_update_tiles( int ntiles, const BoraSolverDe
 }
 
 __global__ void __launch_bounds__( 32 * kUpdWarps, 5 ) k_pcg_update( int ntiles, BoraSolverDev sv, BoraReduceDev red,
-                                                                  int slot_rz_in, int slot_dq_in, int slot_rz_out,
-                                                                  int slot_rr_out )
+                                                                  int ndq, int slot_rz_in, int slot_dq_in )
 {
     using namespace micsweep;
     __shared__ __align__( 16 ) float sval[kUpdWarps][kBuf];
     __shared__ __align__( 16 ) float spiv[kUpdWarps][kBuf];
-    __shared__ float s_alpha;
+    __shared__ float2 s_dq[kUpdWarps];
     bora_pdl_trigger();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for( int q = lane; q < kBuf; q += 32 ) { sval[w][q] = 0.f; spiv[w][q] = 0.f; }
     bora_pdl_wait();  // the previous kernel's results are complete from here
-    if( threadIdx.x == 0 ) s_alpha = slot_rz_in < 0 ? 0.f : (float)( red.ring[slot_rz_in] / red.ring[slot_dq_in] );
-    __syncthreads();
+    float alpha = 0.f;
+    if( slot_rz_in >= 0 )
+    {
+        const DF dq = part_collect( red.part_dq, ndq, s_dq );
+        alpha = df_ratio( red.ringf[slot_rz_in], make_float2( dq.hi, dq.lo ) );
+        if( blockIdx.x == 0 && threadIdx.x == 0 ) ring_store( red, slot_dq_in, dq, false );
+    }
     DF prz{ 0.f, 0.f }, prr{ 0.f, 0.f };
-    pcg_update_tiles( ntiles, sv, s_alpha, blockIdx.x * kUpdWarps + w, gridDim.x * kUpdWarps, sval[w], spiv[w], prz, prr );
-    reduce2_publish_df( prz, prr, red, slot_rz_out, slot_rr_out );
+    __syncwarp();
+    pcg_update_tiles( ntiles, sv, alpha, blockIdx.x * kUpdWarps + w, gridDim.x * kUpdWarps, sval[w], spiv[w], prz, prr );
+    part_publish( prz, prr, red.part_rz, red.part_rr, blockIdx.x );
 }
 
 // Global index of the face neighbour of cell (slot s, local l) in direction q
@@ -600,30 +605,37 @@ __device__ __forceinline__ DF pcg_direction_tiles( int ntiles, const int32_t* __
 
 __device__ __forceinline__ void pcg_direction_body( int ntiles, const int32_t* __restrict__ nbr,
                                                     const uint16_t* __restrict__ code, const BoraSolverDev& sv, int dsel_in,
-                                                    const BoraReduceDev& red, int slot_rz_new, int slot_rz_old,
-                                                    int slot_dq_out, int slot_a_rz, int slot_a_dq, unsigned bid, unsigned G )
+                                                    const BoraReduceDev& red, int nparts, int slot_rz_new, int slot_rr,
+                                                    int slot_rz_old, int slot_a_rz, int slot_a_dq, bool host_rr, unsigned bid,
+                                                    unsigned G )
 {
-    __shared__ float s_beta, s_alpha;
+    __shared__ float2 s_rz[kDirWarps], s_rr[kDirWarps];
     bora_pdl_trigger();
-    bora_pdl_wait();  // the previous kernel's results (ring, z, d, e) are complete from here
-    if( threadIdx.x == 0 )
+    bora_pdl_wait();  // the previous kernel's results (ring, partial sums, z, d, e) are complete from here
+    const DF rz = part_collect( red.part_rz, nparts, s_rz );
+    const float beta = slot_rz_old < 0 ? 0.f : df_ratio( make_float2( rz.hi, rz.lo ), red.ringf[slot_rz_old] );
+    const float alpha = slot_a_rz < 0 ? 0.f : df_ratio( red.ringf[slot_a_rz], red.ringf[slot_a_dq] );
+    if( bid == G - 1 )  // the last block (never the one with more tiles) finishes rr for the host
     {
-        s_beta = slot_rz_old < 0 ? 0.f : (float)( red.ring[slot_rz_new] / red.ring[slot_rz_old] );
-        s_alpha = slot_a_rz < 0 ? 0.f : (float)( red.ring[slot_a_rz] / red.ring[slot_a_dq] );
+        const DF rr = part_collect( red.part_rr, nparts, s_rr );
+        if( threadIdx.x == 0 )
+        {
+            ring_store( red, slot_rz_new, rz, false );
+            ring_store( red, slot_rr, rr, host_rr );
+        }
     }
-    __syncthreads();
-    const DF pdq = pcg_direction_tiles( ntiles, nbr, code, sv, dsel_in, s_beta, s_alpha, slot_a_rz >= 0, bid, G );
-    reduce2_publish_warp( df_warp_sum( pdq ), 0.0, 0, red, slot_dq_out, -1, bid, G );
+    const DF pdq = pcg_direction_tiles( ntiles, nbr, code, sv, dsel_in, beta, alpha, slot_a_rz >= 0, bid, G );
+    part_publish( pdq, DF{ 0.f, 0.f }, red.part_dq, nullptr, bid );
 }
 
 __global__ void __launch_bounds__( 32 * kDirWarps, 7 ) k_pcg_direction( int ntiles, const int32_t* __restrict__ nbr,
                                                                     const uint16_t* __restrict__ code, BoraSolverDev sv,
-                                                                    int dsel_in, BoraReduceDev red, int slot_rz_new,
-                                                                    int slot_rz_old, int slot_dq_out, int slot_a_rz,
-                                                                    int slot_a_dq )
+                                                                    int dsel_in, BoraReduceDev red, int nparts,
+                                                                    int slot_rz_new, int slot_rr, int slot_rz_old,
+                                                                    int slot_a_rz, int slot_a_dq, bool host_rr )
 {
-    pcg_direction_body( ntiles, nbr, code, sv, dsel_in, red, slot_rz_new, slot_rz_old, slot_dq_out, slot_a_rz, slot_a_dq,
-                        blockIdx.x, gridDim.x );
+    pcg_direction_body( ntiles, nbr, code, sv, dsel_in, red, nparts, slot_rz_new, slot_rr, slot_rz_old, slot_a_rz, slot_a_dq,
+                        host_rr, blockIdx.x, gridDim.x );
 }
 
 // Batched: each simulation on its own grid of m.grid[kGridDir] blocks.
@@ -633,8 +645,8 @@ __global__ void __launch_bounds__( 32 * kDirWarps ) k_pcg_direction_batch( const
     const int k = bora_batch_member( L, blockIdx.x, &bid );
     const BoraMemberSolve& m = L.ms[k];
     const BoraMemberSlots& q = L.sl[k];
-    pcg_direction_body( m.ntiles, m.nbr, m.code, m.sv, q.dsel, m.red, q.rz_new, q.rz_old, q.dq, q.a_rz, q.a_dq, bid,
-                        (unsigned)m.grid[kGridDir] );
+    pcg_direction_body( m.ntiles, m.nbr, m.code, m.sv, q.dsel, m.red, m.grid[kGridPass0R], q.rz_new, q.rr_new, q.rz_old,
+                        q.a_rz, q.a_dq, q.chk != 0, bid, (unsigned)m.grid[kGridDir] );
 }
 
 // ---------------------------------------------------------------------------------
@@ -660,8 +672,8 @@ struct PcgPersistArgs
     int slot_rz_prev;          // r.z before the last update of the previous pass, or -1 (restart)
     int max_inner;
     double target;             // stop once ||r|| <= target
-    int slot_a_rz, slot_a_dq;  // out: the last update's alpha = a_rz / a_dq (its e += alpha d is pending)
-    int slot_rr;               // out: the last r.r
+    int slot_a_rz, slot_a_dq;  // out: the last update's alpha = a_rz / a_dq (its e += alpha d is pending);
+                               // the last r.r is left as the one partial sum part_rr[0]
     uint32_t* iters;           // out: iterations run
     unsigned* bar;             // barrier count and generation (zeroed before the launch)
     unsigned expect;           // blocks a barrier waits for (gridDim.x)
@@ -789,15 +801,10 @@ __global__ void __launch_bounds__( 32 * kUpdWarps, 3 ) k_pcg_persistent( const _
     }
     if( blockIdx.x == 0 && threadIdx.x == 0 )
     {
-        a.red.ring[a.slot_a_rz] = a_rz;
-        a.red.ring[a.slot_a_dq] = a_dq;
-        a.red.ring[a.slot_rr] = rr;
-        if( a.red.mirror )
-        {
-            a.red.mirror[a.slot_a_rz] = a_rz;
-            a.red.mirror[a.slot_a_dq] = a_dq;
-            a.red.mirror[a.slot_rr] = rr;
-        }
+        auto pair = []( double v ) { return DF{ (float)v, (float)( v - (double)(float)v ) }; };
+        ring_store( a.red, a.slot_a_rz, pair( a_rz ), false );
+        ring_store( a.red, a.slot_a_dq, pair( a_dq ), false );
+        a.red.part_rr[0] = make_float2( pair( rr ).hi, pair( rr ).lo );  // finished by the refinement
         *a.iters = (uint32_t)it;
     }
 }
@@ -859,13 +866,17 @@ __global__ void k_solve_init_batch( const __grid_constant__ BoraBatchLaunch L )
 // x += e (+ the last update's pending alpha d), then clear e and q; the direction d is kept
 // (the next refinement pass continues the recurrence from it).
 __device__ __forceinline__ void refine_accumulate_body( size_t ncells, const uint16_t* __restrict__ code,
-                                                        const BoraSolverDev& sv, int dsel, const double* __restrict__ ring,
-                                                        int slot_a_rz, int slot_a_dq, unsigned bid, unsigned G )
+                                                        const BoraSolverDev& sv, int dsel, const BoraReduceDev& red,
+                                                        int nparts, int slot_rr, int slot_a_rz, int slot_a_dq, unsigned bid,
+                                                        unsigned G )
 {
-    __shared__ float s_alpha;
-    if( threadIdx.x == 0 ) s_alpha = slot_a_rz < 0 ? 0.f : (float)( ring[slot_a_rz] / ring[slot_a_dq] );
-    __syncthreads();
-    const float alpha = s_alpha;
+    __shared__ float2 s_rr[8];  // 256 threads
+    if( bid == G - 1 )          // the last update's r.r, for the host
+    {
+        const DF rr = part_collect( red.part_rr, nparts, s_rr );
+        if( threadIdx.x == 0 ) ring_store( red, slot_rr, rr, true );
+    }
+    const float alpha = slot_a_rz < 0 ? 0.f : df_ratio( red.ringf[slot_a_rz], red.ringf[slot_a_dq] );
     const float* __restrict__ d = dsel ? sv.d[1] : sv.d[0];
     for( size_t i = bid * (size_t)blockDim.x + threadIdx.x; i < ncells; i += (size_t)G * blockDim.x )
     {
@@ -882,9 +893,9 @@ __device__ __forceinline__ void refine_accumulate_body( size_t ncells, const uin
 }
 
 __global__ void k_refine_accumulate( size_t ncells, const uint16_t* __restrict__ code, BoraSolverDev sv, int dsel,
-                                     const double* __restrict__ ring, int slot_a_rz, int slot_a_dq )
+                                     BoraReduceDev red, int nparts, int slot_rr, int slot_a_rz, int slot_a_dq )
 {
-    refine_accumulate_body( ncells, code, sv, dsel, ring, slot_a_rz, slot_a_dq, blockIdx.x, gridDim.x );
+    refine_accumulate_body( ncells, code, sv, dsel, red, nparts, slot_rr, slot_a_rz, slot_a_dq, blockIdx.x, gridDim.x );
 }
 
 __global__ void k_refine_accumulate_batch( const __grid_constant__ BoraBatchLaunch L )
@@ -893,8 +904,8 @@ __global__ void k_refine_accumulate_batch( const __grid_constant__ BoraBatchLaun
     const int k = bora_batch_member( L, blockIdx.x, &bid );
     const BoraMemberSolve& m = L.ms[k];
     const BoraMemberSlots& q = L.sl[k];
-    refine_accumulate_body( (size_t)m.ntiles * 512, m.code, m.sv, q.dsel, m.red.ring, q.a_rz, q.a_dq, bid,
-                            (unsigned)m.grid[kGridCells] );
+    refine_accumulate_body( (size_t)m.ntiles * 512, m.code, m.sv, q.dsel, m.red, m.grid[kGridPass0R], q.rr_new, q.a_rz,
+                            q.a_dq, bid, (unsigned)m.grid[kGridCells] );
 }
 
 // r = b - A x in double-float arithmetic (A from the stencil code, x the double-float
@@ -1102,10 +1113,8 @@ void bora_launch_solve_init( int ntiles, const float* b, const uint16_t*, BoraSo
     k_solve_init<<<grid_for( nc, 256 ), 256, 0, st>>>( nc, b, s, red, slot_norm2, slot_max );
 }
 
-void bora_launch_pcg_update( int ntiles, const uint16_t* code, BoraSolverDev s, BoraReduceDev red, int slot_rz_in,
-                             int slot_dq_in, int slot_rz_out, int slot_rr_out, cudaStream_t st )
+int bora_pcg_update_grid( int ntiles )
 {
-    (void)code;
     static BoraPerDevice per_sm;
     const int bps = per_sm.get( [] {
         int v = 0;
@@ -1115,15 +1124,20 @@ void bora_launch_pcg_update( int ntiles, const uint16_t* code, BoraSolverDev s, 
     // that every warp gets that many tiles (no warp waits in the reduction for a straggler)
     const int cap = std::max( 1, std::min( bps * num_sms(), kBoraMaxReduceBlocks ) ) * kUpdWarps;
     const int rounds = std::max( 1, ( ntiles + cap - 1 ) / cap );  // one block even for no tiles: it publishes the sums
-    const int nb = std::max( 1, ( ntiles + kUpdWarps * rounds - 1 ) / ( kUpdWarps * rounds ) );
-    bora_launch_pdl( k_pcg_update, nb, 32 * kUpdWarps, 0, st, ntiles, s, red, slot_rz_in, slot_dq_in, slot_rz_out,
-                     slot_rr_out );
+    return std::max( 1, ( ntiles + kUpdWarps * rounds - 1 ) / ( kUpdWarps * rounds ) );
 }
 
-namespace {
+void bora_launch_pcg_update( int ntiles, const uint16_t* code, BoraSolverDev s, BoraReduceDev red, int slot_rz_in,
+                             int slot_dq_in, cudaStream_t st )
+{
+    (void)code;
+    bora_launch_pdl( k_pcg_update, bora_pcg_update_grid( ntiles ), 32 * kUpdWarps, 0, st, ntiles, s, red,
+                     bora_pcg_direction_grid( ntiles ), slot_rz_in, slot_dq_in );
+}
+
 // Grid of the direction kernel: every warp gets the same number of tiles; at most
 // kBoraMaxReduceBlocks CTAs (partial sums capacity).
-int direction_grid( int ntiles )
+int bora_pcg_direction_grid( int ntiles )
 {
     if( ntiles <= 0 ) return 0;
     static BoraPerDevice per_sm;
@@ -1135,13 +1149,15 @@ int direction_grid( int ntiles )
     const int rounds = ( ntiles + cap - 1 ) / cap;
     return std::max( 1, ( ntiles + kDirWarps * rounds - 1 ) / ( kDirWarps * rounds ) );
 }
+
+namespace {
 int residual_grid( size_t nc ) { return (int)std::max<size_t>( 1, std::min<size_t>( ( nc + 255 ) / 256, (size_t)num_sms() * 8 ) ); }
 }  // namespace
 
 void bora_projection_grids( int ntiles, int* grid )
 {
     const size_t nc = (size_t)std::max( ntiles, 0 ) * 512;
-    grid[kGridDir] = direction_grid( ntiles );
+    grid[kGridDir] = bora_pcg_direction_grid( ntiles );
     grid[kGridCells] = grid_for( nc, 256 );
     grid[kGridResidual] = residual_grid( nc );
 }
@@ -1183,15 +1199,14 @@ int bora_pcg_persistent_grid()
 
 int bora_launch_pcg_persistent( int ntiles, const int32_t* nbr, const uint16_t* code, BoraSolverDev s, BoraReduceDev red,
                                 int dsel, int slot_rz_prev, int max_inner, double target, int slot_a_rz, int slot_a_dq,
-                                int slot_rr, uint32_t* iters, unsigned* bar, double* part, bool never_release,
-                                cudaStream_t st )
+                                uint32_t* iters, unsigned* bar, double* part, bool never_release, cudaStream_t st )
 {
     const int grid = bora_pcg_persistent_grid();
     if( grid <= 0 ) return -1;
     PcgPersistArgs a{};
     a.ntiles = ntiles; a.nbr = nbr; a.code = code; a.sv = s; a.red = red;
     a.dsel = dsel; a.slot_rz_prev = slot_rz_prev; a.max_inner = max_inner; a.target = target;
-    a.slot_a_rz = slot_a_rz; a.slot_a_dq = slot_a_dq; a.slot_rr = slot_rr; a.iters = iters;
+    a.slot_a_rz = slot_a_rz; a.slot_a_dq = slot_a_dq; a.iters = iters;
     a.bar = bar; a.part = part;
     // a barrier that waits for one block more than there are never releases: every wait runs
     // out (fault injection for tests), after a short limit
@@ -1206,13 +1221,12 @@ int bora_launch_pcg_persistent( int ntiles, const int32_t* nbr, const uint16_t* 
 }
 
 void bora_launch_pcg_direction( const BoraGridDev&, int ntiles, BoraTilesDev t, const uint16_t* code, BoraSolverDev s,
-                                int dsel_in, BoraReduceDev red, int slot_rz_new, int slot_rz_old, int slot_dq_out,
-                                int slot_a_rz, int slot_a_dq, cudaStream_t st )
+                                int dsel_in, BoraReduceDev red, int nparts, int slot_rz_new, int slot_rr, int slot_rz_old,
+                                int slot_a_rz, int slot_a_dq, bool host_rr, cudaStream_t st )
 {
     if( ntiles <= 0 ) return;
-    const int grid = direction_grid( ntiles );
-    bora_launch_pdl( k_pcg_direction, grid, 32 * kDirWarps, 0, st, ntiles, (const int32_t*)t.nbr, code, s, dsel_in, red,
-                     slot_rz_new, slot_rz_old, slot_dq_out, slot_a_rz, slot_a_dq );
+    bora_launch_pdl( k_pcg_direction, bora_pcg_direction_grid( ntiles ), 32 * kDirWarps, 0, st, ntiles, (const int32_t*)t.nbr,
+                     code, s, dsel_in, red, nparts, slot_rz_new, slot_rr, slot_rz_old, slot_a_rz, slot_a_dq, host_rr );
 }
 
 void bora_launch_solve_warm( int ntiles, const uint16_t* code, const int32_t* tile_of, const int32_t* slot_prev,
@@ -1222,11 +1236,12 @@ void bora_launch_solve_warm( int ntiles, const uint16_t* code, const int32_t* ti
     if( nc ) k_solve_warm<<<grid_for( nc, 256 ), 256, 0, st>>>( nc, code, tile_of, slot_prev, pres, s.x );
 }
 
-void bora_launch_refine_accumulate( int ntiles, const uint16_t* code, BoraSolverDev s, int dsel, const double* ring,
-                                    int slot_a_rz, int slot_a_dq, cudaStream_t st )
+void bora_launch_refine_accumulate( int ntiles, const uint16_t* code, BoraSolverDev s, int dsel, BoraReduceDev red,
+                                    int nparts, int slot_rr, int slot_a_rz, int slot_a_dq, cudaStream_t st )
 {
     const size_t nc = (size_t)ntiles * 512;
-    if( nc ) k_refine_accumulate<<<grid_for( nc, 256 ), 256, 0, st>>>( nc, code, s, dsel, ring, slot_a_rz, slot_a_dq );
+    if( nc )
+        k_refine_accumulate<<<grid_for( nc, 256 ), 256, 0, st>>>( nc, code, s, dsel, red, nparts, slot_rr, slot_a_rz, slot_a_dq );
 }
 
 void bora_launch_refine_residual( const BoraGridDev&, int ntiles, BoraTilesDev t, const float* b, const uint16_t* code,

@@ -128,7 +128,12 @@ __device__ __forceinline__ void reduce2_publish_warp( double v0, double v1, int 
     {
         double ta = 0.0, tb = 0.0;
         for( int q = 0; q < nw; ++q ) { ta += w0[q]; tb = op1 ? fmax( tb, w1[q] ) : tb + w1[q]; }
-        if( slot0 >= 0 ) red.ring[slot0] = ta;
+        if( slot0 >= 0 )
+        {
+            red.ring[slot0] = ta;
+            const float hi = (float)ta;
+            red.ringf[slot0] = make_float2( hi, (float)( ta - (double)hi ) );
+        }
         if( slot1 >= 0 ) red.ring[slot1] = tb;
         if( red.mirror )  // host-visible once the kernel has completed
         {
@@ -170,6 +175,95 @@ __device__ __forceinline__ void reduce2_publish_dfmax( DF v0, float vmax, BoraRe
     reduce2_publish_dfmax( v0, vmax, red, slot0, slot1, blockIdx.x, gridDim.x );
 }
 
+
+// ---------------------------------------------------------------------------------
+// Sums finished by their consumer. The solver's inner kernels run as a chain in which the next
+// kernel needs the previous one's sum: a producer's block stores its partial sum as a
+// double-float pair and exits, and every block of the consumer adds all partials in the same
+// fixed order while its first tile's loads are in flight, so each holds the same bits. Against
+// a last block that finishes the sum (fence, arrival counter, second pass, 7 us at the end of
+// every reducing kernel on GB300: 13.8 against 6.4 us for level 0's down passes with and
+// without a sum at 240 tiles), the producer's tail is one store. Partials are float pairs
+// (48 bits): FP64 additions by every block would be bound by the narrow FP64 pipe. Measured
+// with the host polling r.r instead of waiting for events: a plain PCG iteration at 240 tiles
+// 18 -> 13 us, the 256^3 plain step's solve 32 -> 27 ms, a V-cycle 6 us less.
+
+__device__ __forceinline__ DF df_warp_sum_df( DF v )
+{
+#pragma unroll
+    for( int o = 16; o > 0; o >>= 1 )
+        v = df_add( v, DF{ __shfl_xor_sync( 0xffffffffu, v.hi, o ), __shfl_xor_sync( 0xffffffffu, v.lo, o ) } );
+    return v;
+}
+
+// (float)( a / b ) of two double-float values: the quotient of the high parts corrected by one
+// residual step (within an ulp of the rounded quotient).
+__device__ __forceinline__ float df_ratio( float2 a, float2 b )
+{
+    const float q = a.x / b.x;
+    const float rem = fmaf( -q, b.x, a.x ) + fmaf( -q, b.y, a.y );
+    const float c = rem / b.x;
+    return isfinite( c ) ? q + c : q;
+}
+
+// The block's sums of v0 and v1 into part0[bid] and part1[bid] (part1 may be null). Called once per
+// kernel, by every thread of the block.
+__device__ __forceinline__ void part_publish( DF v0, DF v1, float2* part0, float2* part1, unsigned bid )
+{
+    __shared__ float4 w[32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = ( blockDim.x + 31 ) >> 5;
+    v0 = df_warp_sum_df( v0 );
+    if( part1 ) v1 = df_warp_sum_df( v1 );
+    if( lane == 0 ) w[wid] = make_float4( v0.hi, v0.lo, v1.hi, v1.lo );
+    __syncthreads();
+    if( threadIdx.x == 0 )
+    {
+        DF a{ w[0].x, w[0].y }, b{ w[0].z, w[0].w };
+        for( int q = 1; q < nw; ++q )
+        {
+            a = df_add( a, DF{ w[q].x, w[q].y } );
+            b = df_add( b, DF{ w[q].z, w[q].w } );
+        }
+        part0[bid] = make_float2( a.hi, a.lo );
+        if( part1 ) part1[bid] = make_float2( b.hi, b.lo );
+    }
+}
+
+// The sum of part[0 .. n) in a fixed order that depends on n and the block's size alone, returned in
+// every thread. Every thread of the block calls it; w is shared memory of the caller, one
+// float2 per warp, not used by anything else since the last block barrier.
+__device__ __forceinline__ DF part_collect( const float2* part, int n, float2* w )
+{
+    constexpr int kAhead = 8;  // independent loads in flight per thread
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = ( blockDim.x + 31 ) >> 5;
+    DF a{ 0.f, 0.f };
+    for( int base = threadIdx.x; base < n; base += kAhead * (int)blockDim.x )
+    {
+        float2 p[kAhead];
+#pragma unroll
+        for( int q = 0; q < kAhead; ++q )
+        {
+            const int i = base + q * (int)blockDim.x;
+            p[q] = i < n ? __ldcg( part + i ) : make_float2( 0.f, 0.f );
+        }
+#pragma unroll
+        for( int q = 0; q < kAhead; ++q ) a = df_add( a, DF{ p[q].x, p[q].y } );
+    }
+    a = df_warp_sum_df( a );
+    if( lane == 0 ) w[wid] = make_float2( a.hi, a.lo );
+    __syncthreads();
+    DF t{ w[0].x, w[0].y };
+    for( int q = 1; q < nw; ++q ) t = df_add( t, DF{ w[q].x, w[q].y } );
+    return t;
+}
+
+// A finished sum for the kernels after this one, and (mirror) for the host. One thread calls it.
+__device__ __forceinline__ void ring_store( const BoraReduceDev& red, int slot, DF v, bool mirror )
+{
+    red.ringf[slot] = make_float2( v.hi, v.lo );
+    red.ring[slot] = (double)v.hi + (double)v.lo;
+    if( mirror && red.mirror ) red.mirror[slot] = (double)v.hi + (double)v.lo;
+}
 
 }  // namespace bora_reduce
 
