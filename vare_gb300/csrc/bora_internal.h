@@ -195,7 +195,7 @@ struct BoraSolverDev
     float* d[2];    // search directions (ping-pong)
     float* q;       // A d
     float* z;       // preconditioned residual
-    float* minv;    // block-MIC(0) inverse pivots
+    float* minv;    // squared block-MIC(0) inverse pivots, each row of a tile rotated (projection.cu)
 };
 
 void bora_launch_mic_factor( const BoraGridDev& g, int ntiles, const uint16_t* code, float* minv, cudaStream_t st );

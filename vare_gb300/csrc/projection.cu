@@ -182,8 +182,8 @@ __device__ inline void load_plane_tables( uint16_t* pc, uint16_t* ps )
 __device__ inline int code_diag( uint16_t c ) { return ( c >> 8 ) & 15; }
 
 // Block-MIC(0) pivots (MIC(0) of BLAS.cu:211-262 with tau = 0.97, restricted to the
-// couplings inside each 8^3 tile so that tiles factor independently). One warp per
-// tile, persistent over tiles.
+// couplings inside each 8^3 tile so that tiles factor independently), stored squared and
+// rotated (mic_sweeps). One warp per tile, persistent over tiles.
 constexpr int kTilesPerCta = 4;
 
 __global__ void __launch_bounds__( 32 * kTilesPerCta ) k_mic_factor( int ntiles, const uint16_t* __restrict__ code,
@@ -247,7 +247,9 @@ __global__ void __launch_bounds__( 32 * kTilesPerCta ) k_mic_factor( int ntiles,
             }
             __syncwarp();
         }
-        for( int l = lane; l < 512; l += 32 ) minv[base + l] = sm[w][l];
+        // squared, each row rotated as mic_sweeps reads it
+        for( int l = lane; l < 512; l += 32 )
+            minv[base + ( l & ~7 ) + ( ( l + ( l >> 3 & 7 ) + ( l >> 6 ) + 1 ) & 7 )] = sm[w][l] * sm[w][l];
         __syncwarp();
     }
 }
@@ -256,195 +258,164 @@ __global__ void __launch_bounds__( 32 * kTilesPerCta ) k_mic_factor( int ntiles,
 // PCG update: r -= alpha q; z = M^-1 r (block-MIC(0) forward and backward sweeps over the
 // tile's 22 wavefront planes i+j+k = p); rz = r.z and rr = r.r, FP64-accurate. The matching
 // e += alpha d is applied by the next direction kernel (which reads d anyway) or by the
-// refinement step. One warp per tile, persistent over tiles (every warp gets the same
-// number of tiles; the next tile's r, q and pivots are loaded into registers during the
-// current tile's sweeps, the one after into L2); alpha is formed once per CTA.
+// refinement step. One warp per tile, persistent over tiles (every warp gets the same number
+// of tiles).
 //
-// Sweep schedule: each lane owns two x-rows of the tile, (j, kq) and (j, kq + 4) with
-// j = lane & 7, kq = lane >> 3, i.e. tile rows lane and lane + 32; the tile's values and
-// pivots are staged in shared memory at cell address i + 8 j + 73 k, where the plane pitch
-// 73 makes every step's 32 accesses fall in distinct banks. Step u of a sweep handles cell
-// i = u - (j + k) - 1 of every row at once, so a lane's cell address is its own row offset
-// plus the compile-time u, and the -y, -z (+y, +z) neighbours sit 8 and 73 cells below
-// (above) it, computed in the previous step. The -x (+x) neighbour is the lane's own previous
-// step, kept in registers. Steps outside a row's eight cells compute with pivot 0 (so they
-// yield 0 and feed the row's first cell a zero neighbour) and store nothing; neighbours
-// outside the tile (j = 0 / 7, k = 0 / 7) are masked, and zeroed guard cells keep every read
-// inside the warp's buffers and finite. The floating-point operations per cell are those of
-// the wavefront form: forward y_c = (r_c + M_x y_x + M_y y_y + M_z y_z) M_c as three chained
-// FMAs in the order -x, -y, -z; backward z_c = (y_c + M_c (z_x + z_y + z_z)) M_c with the sum
-// in the order +x, +y, +z. Non-fluid cells have M = 0 (k_mic_factor) and r = 0.
-namespace micsweep {
-constexpr int kPlane = 73;                          // buffer pitch of a z-plane (64 cells + 9)
-constexpr int kGuard = 80;                          // cells before the tile (reads reach -73)
-constexpr int kBuf = kGuard + 7 * kPlane + 64 + kPlane + 7;  // reads reach 574 + 73
-constexpr int kWarps = 4;  // 4 x 5.9 KB of buffers per CTA; five CTAs per SM at 96 registers
-}  // namespace micsweep
-constexpr int kUpdWarps = micsweep::kWarps;
+// The sweeps run in registers. Each lane owns two x-rows of the tile that are neighbours in z,
+// row A = (j, k = 2 kq) and row B = (j, k + 1), j = lane & 7, kq = lane >> 3. Step u of a sweep
+// handles cell i = u - (j + k) - 1 of every row at once. In the scaled unknowns w = M y and the
+// squared pivots M2 = M^2 (which k_mic_factor stores) the sweeps are
+//   forward   w = M2 t, t = r + (w_-x + w_-y + w_-z)
+//   backward  z = w + M2 (z_+x + z_+y + z_+z),
+// so a step needs its neighbours' single values of the step before: -x and the z neighbour
+// inside the pair are the lane's own registers, the other y and z neighbours are three
+// shuffles. A row's cells sit in eight registers rotated by (j + k + 1) mod 8, so that step u
+// finds its cell in register u mod 8 in every lane (r is rotated in three select stages; M2 is
+// stored rotated). Steps outside a row's eight cells yield 0, which feeds the row's first cell a
+// zero neighbour. r.z = sum of w t (r.M^-1 r = y.y), all terms >= 0. Non-fluid
+// cells have M2 = 0 and r = 0.
+//
+// Bound by latency and issue: 44 dependent steps of a shuffle and three arithmetic
+// instructions, about 900 warp instructions per tile. The earlier form kept the tile in shared
+// memory (11 shared accesses per row and step pair, 78 % of the shared pipe): 32.5 us per launch
+// at 256^3 (7926 tiles), now 22 us with an event on either side, 3.7 TB/s of its 20 B per cell;
+// 8.4 against 11.9 us at 64^3 (240 tiles). 16 warps per SM without spills beat 20 .. 32 with
+// (23.3 against 23.5 .. 26.1 ms per 256^3 step), and loading the next tile during the sweeps
+// gains nothing (23.3 .. 24.3 ms).
+constexpr int kUpdWarps = 4;
 
-// The update of the warp's tiles first, first + tstride, ...: r -= alpha q, z = M^-1 r; r.z and
-// r.r accumulated into prz, prr. sv_w, sp_w: the warp's two sweep buffers (kBuf floats each,
-// zeroed before the first call; the sweeps keep their guard cells zero).
-__device__ __forceinline__ void pcg_update_tiles( int ntiles, const BoraSolverDev& sv, float alpha, int first, int tstride,
-                                                  float* sv_w, float* sp_w, DF& prz, DF& prr )
+// v[i] -> v[(i + rho) mod 8]
+__device__ __forceinline__ void rotate8( float* v, int rho )
 {
-    using namespace micsweep;
-    const int lane = threadIdx.x & 31;
-    float* const V = sv_w + kGuard;  // tile cell (i, j, k) at V[i + 8 j + kPlane k]
-    float* const P = sp_w + kGuard;
-    const int j = lane & 7, kq = lane >> 3, sA = j + kq;  // plane offset of row A; row B: sA + 4
-    const bool has_ym = j > 0, has_yp = j < 7, has_zmA = kq > 0, has_zpB = kq < 3;
-    // cell of row A at step u: VA + u (row B: VB + u)
-    const int rA = 8 * j + kPlane * kq, rB = rA + 4 * kPlane;  // element 0 of rows A and B
-    const int oA = rA - sA - 1, oB = rB - ( sA + 4 ) - 1;
-    float4* const r4 = reinterpret_cast<float4*>( sv.r );
-    float4* const z4 = reinterpret_cast<float4*>( sv.z );
-    const float4* __restrict__ q4 = reinterpret_cast<const float4*>( sv.q );
-    const float4* __restrict__ m4 = reinterpret_cast<const float4*>( sv.minv );
-    // Step u of a row with plane offset s. The operands that do not depend on the previous
-    // step (the cell's own value and pivot, the neighbours' pivots) are read one step ahead,
-    // so that only the two neighbour values computed in the previous step are waited for.
-    struct FwdOps { float r, p, py, pz; };
-    auto fwd_load = [&]( int o, bool zm ) -> FwdOps {
-        return { V[o], P[o], has_ym ? P[o - 8] : 0.f, zm ? P[o - kPlane] : 0.f };
-    };
-    // y = (r + M_x y_x + M_y y_y + M_z y_z) M
-    auto fwd_step = [&]( int o, int u, int s, const FwdOps& c, float& y, float& m ) {
-        const bool act = (unsigned)( u - s - 1 ) < 8u;
-        const float vy = V[o - 8], vz = V[o - kPlane];
-        float t = fmaf( m, y, c.r );
-        t = fmaf( c.py, vy, t );
-        t = fmaf( c.pz, vz, t );
-        m = act ? c.p : 0.f;
-        y = t * m;
-        if( act ) V[o] = y;
-    };
-    struct BwdOps { float y, p; };
-    auto bwd_load = [&]( int o ) -> BwdOps { return { V[o], P[o] }; };
-    // z = (y + M (z_x + z_y + z_z)) M
-    auto bwd_step = [&]( int o, int u, int s, bool zp, const BwdOps& c, float& z ) {
-        const bool act = (unsigned)( u - s - 1 ) < 8u;
-        const float zy = has_yp ? V[o + 8] : 0.f, zz = zp ? V[o + kPlane] : 0.f;
-        float acc = 0.f;
-        acc += z;
-        acc += zy;
-        acc += zz;
-        const float m = act ? c.p : 0.f;
-        z = fmaf( m, acc, c.y ) * m;
-        if( act ) V[o] = z;
-    };
-    // global traffic in whole-warp 512-byte float4 runs: float4 c = lane + 32 m of a tile holds
-    // cells 4c .. 4c + 3, which sit at buffer address 4c + 9 k, k = c >> 4
-    const int cbase = 4 * lane + 9 * ( lane >> 4 );  // + 146 m
-    auto prefetch_tile = [&]( int s ) {  // the tile's r, q and pivots into L2
-        if( s < ntiles && lane < 3 )
-        {
-            const float* src = ( lane == 0 ? sv.r : lane == 1 ? sv.q : sv.minv ) + (size_t)s * 512;
-            asm volatile( "cp.async.bulk.prefetch.L2.global [%0], 2048;" ::"l"( src ) : "memory" );
-        }
-    };
-    // the next tile's r, q and pivots are loaded into registers before this tile's sweeps
-    float4 rn[4], qn[4], mn[4];
-    auto load_tile = [&]( int s ) {
-        if( s >= ntiles ) return;
 #pragma unroll
-        for( int m = 0; m < 4; ++m )
-        {
-            const size_t o = (size_t)s * 128 + lane + 32 * m;
-            rn[m] = r4[o];
-            qn[m] = q4[o];
-            mn[m] = m4[o];
-        }
-    };
-    load_tile( first );
-    for( int s = first; s < ntiles; s += tstride )
+    for( int b = 1; b < 8; b <<= 1 )
     {
-        const size_t b4 = (size_t)s * 128 + lane;
-        float4 r[4];
+        float t[8];
+        const bool on = ( rho & b ) != 0;
 #pragma unroll
-        for( int m = 0; m < 4; ++m )
-        {
-            r[m] = rn[m];
-            const float4 q = qn[m];
-            const float4 mv = mn[m];
-            r[m].x = fmaf( -alpha, q.x, r[m].x ); r[m].y = fmaf( -alpha, q.y, r[m].y );
-            r[m].z = fmaf( -alpha, q.z, r[m].z ); r[m].w = fmaf( -alpha, q.w, r[m].w );
-            r4[b4 + 32 * m] = r[m];
-            const int c = cbase + 146 * m;
-            V[c] = r[m].x; V[c + 1] = r[m].y; V[c + 2] = r[m].z; V[c + 3] = r[m].w;
-            P[c] = mv.x; P[c + 1] = mv.y; P[c + 2] = mv.z; P[c + 3] = mv.w;
-            prr = df_add_f( prr, dot4( r[m], r[m] ) );
-        }
-        load_tile( s + tstride );
-        prefetch_tile( s + 2 * tstride );
-        __syncwarp();
-        // forward: row A holds cells at u = 1 .. 18, row B at u = 5 .. 22
-        {
-            float yA = 0.f, mA = 0.f, yB = 0.f, mB = 0.f;  // the -x neighbour (previous step)
-            FwdOps cA = fwd_load( oA + 1, has_zmA ), cB = { 0.f, 0.f, 0.f, 0.f };
+        for( int i = 0; i < 8; ++i ) t[i] = on ? v[( i - b ) & 7] : v[i];
 #pragma unroll
-            for( int u = 1; u <= 22; ++u )
-            {
-                FwdOps nA = { 0.f, 0.f, 0.f, 0.f }, nB = { 0.f, 0.f, 0.f, 0.f };
-                if( u + 1 <= 18 ) nA = fwd_load( oA + u + 1, has_zmA );
-                if( u + 1 >= 5 && u + 1 <= 22 ) nB = fwd_load( oB + u + 1, true );
-                if( u <= 18 ) fwd_step( oA + u, u, sA, cA, yA, mA );
-                if( u >= 5 ) fwd_step( oB + u, u, sA + 4, cB, yB, mB );
-                cA = nA;
-                cB = nB;
-                __syncwarp();
-            }
-        }
-        // backward, in place over y
-        {
-            float zA = 0.f, zB = 0.f;  // the +x neighbour (previous step)
-            BwdOps cB = bwd_load( oB + 22 ), cA = { 0.f, 0.f };
-#pragma unroll
-            for( int u = 22; u >= 1; --u )
-            {
-                BwdOps nA = { 0.f, 0.f }, nB = { 0.f, 0.f };
-                if( u - 1 >= 5 ) nB = bwd_load( oB + u - 1 );
-                if( u - 1 >= 1 && u - 1 <= 18 ) nA = bwd_load( oA + u - 1 );
-                if( u >= 5 ) bwd_step( oB + u, u, sA + 4, has_zpB, cB, zB );
-                if( u <= 18 ) bwd_step( oA + u, u, sA, true, cA, zA );
-                cA = nA;
-                cB = nB;
-                __syncwarp();
-            }
-        }
-#pragma unroll
-        for( int m = 0; m < 4; ++m )
-        {
-            const int c = cbase + 146 * m;
-            const float4 z = make_float4( V[c], V[c + 1], V[c + 2], V[c + 3] );
-            z4[b4 + 32 * m] = z;
-            prz = df_add_f( prz, dot4( r[m], z ) );
-        }
-        __syncwarp();
+        for( int i = 0; i < 8; ++i ) v[i] = t[i];
     }
 }
 
-__global__ void __launch_bounds__( 32 * kUpdWarps, 5 ) k_pcg_update( int ntiles, BoraSolverDev sv, BoraReduceDev red,
+__device__ __forceinline__ void load8( const float* __restrict__ p, float* v )
+{
+    const float4 a = reinterpret_cast<const float4*>( p )[0], b = reinterpret_cast<const float4*>( p )[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
+__device__ __forceinline__ void store8( float* __restrict__ p, const float* v )
+{
+    reinterpret_cast<float4*>( p )[0] = make_float4( v[0], v[1], v[2], v[3] );
+    reinterpret_cast<float4*>( p )[1] = make_float4( v[4], v[5], v[6], v[7] );
+}
+
+// z = M^-1 r of one tile: rA, rB hold the lane's rows of r and return z (both in cell order);
+// mA, mB the rows' squared pivots as stored (rotated). Returns the lane's part of r.z.
+__device__ __forceinline__ float mic_sweeps( float* rA, float* rB, const float* mA, const float* mB )
+{
+    constexpr unsigned kAllLanes = 0xffffffffu;
+    const int lane = threadIdx.x & 31, j = lane & 7, kq = lane >> 3, sA = j + 2 * kq, rho = ( sA + 1 ) & 7;
+    const float ym = j > 0 ? 1.f : 0.f, yp = j < 7 ? 1.f : 0.f, zm = kq > 0 ? 1.f : 0.f, zp = kq < 3 ? 1.f : 0.f;
+    const unsigned live = 0xffu << ( sA + 1 );  // bit u: row A has a cell at step u (row B: at step u + 1)
+    rotate8( rA, rho );
+    rotate8( rB, rho );  // row B's cell of step u is register (u - 1) mod 8
+    float wA = 0.f, wB = 0.f, rzA = 0.f, rzB = 0.f;
+#pragma unroll
+    for( int u = 1; u <= 22; ++u )
+    {
+        const bool a = ( live >> u ) & 1u, b = ( live >> ( u - 1 ) ) & 1u;
+        const float yA = __shfl_up_sync( kAllLanes, wA, 1 ), yB = __shfl_up_sync( kAllLanes, wB, 1 );
+        const float zA = __shfl_up_sync( kAllLanes, wB, 8 );
+        float& cA = rA[u & 7];
+        float& cB = rB[( u - 1 ) & 7];
+        const float tA = fmaf( zm, zA, fmaf( ym, yA, cA + wA ) );
+        const float tB = fmaf( ym, yB, ( cB + wB ) + wA );
+        wA = a ? mA[u & 7] * tA : 0.f;
+        wB = b ? mB[u & 7] * tB : 0.f;
+        rzA = fmaf( wA, tA, rzA );
+        rzB = fmaf( wB, tB, rzB );
+        cA = a ? wA : cA;
+        cB = b ? wB : cB;
+    }
+    float zA = 0.f, zB = 0.f;
+#pragma unroll
+    for( int u = 22; u >= 1; --u )
+    {
+        const bool a = ( live >> u ) & 1u, b = ( live >> ( u - 1 ) ) & 1u;
+        const float yA = __shfl_down_sync( kAllLanes, zA, 1 ), yB = __shfl_down_sync( kAllLanes, zB, 1 );
+        const float nB = __shfl_down_sync( kAllLanes, zA, 8 );
+        float& cA = rA[u & 7];
+        float& cB = rB[( u - 1 ) & 7];
+        const float sumA = fmaf( yp, yA, zA + zB ), sumB = fmaf( zp, nB, fmaf( yp, yB, zB ) );
+        zA = a ? fmaf( mA[u & 7], sumA, cA ) : 0.f;
+        zB = b ? fmaf( mB[u & 7], sumB, cB ) : 0.f;
+        cA = a ? zA : cA;
+        cB = b ? zB : cB;
+    }
+    rotate8( rA, ( 8 - rho ) & 7 );
+    rotate8( rB, ( 8 - rho ) & 7 );
+    return rzA + rzB;
+}
+
+// The update of the warp's tiles first, first + tstride, ...: r -= alpha q, z = M^-1 r; r.z and
+// r.r accumulated into prz, prr. alpha_of() is called once, by every thread of the block, after
+// the first tile's loads have been issued.
+template <class AlphaOf>
+__device__ __forceinline__ void pcg_update_tiles( int ntiles, const BoraSolverDev& sv, AlphaOf alpha_of, int first, int tstride,
+                                                  DF& prz, DF& prr )
+{
+    const int lane = threadIdx.x & 31;
+    const size_t row = 8 * (size_t)( ( lane & 7 ) + 16 * ( lane >> 3 ) );  // row A; row B follows 64 cells on
+    float rA[8], rB[8], qA[8], qB[8], mA[8], mB[8];
+    auto load_tile = [&]( int s ) {
+        const size_t o = (size_t)s * 512 + row;
+        load8( sv.r + o, rA ); load8( sv.r + o + 64, rB );
+        load8( sv.q + o, qA ); load8( sv.q + o + 64, qB );
+    };
+    if( first < ntiles ) load_tile( first );
+    const float alpha = alpha_of();
+    for( int s = first; s < ntiles; s += tstride )
+    {
+        const size_t o = (size_t)s * 512 + row;
+        if( s != first ) load_tile( s );
+        load8( sv.minv + o, mA );  // not with the first loads: the registers they take there cost more (spills)
+        load8( sv.minv + o + 64, mB );
+#pragma unroll
+        for( int i = 0; i < 8; ++i )
+        {
+            rA[i] = fmaf( -alpha, qA[i], rA[i] );
+            rB[i] = fmaf( -alpha, qB[i], rB[i] );
+        }
+        store8( sv.r + o, rA );
+        store8( sv.r + o + 64, rB );
+#pragma unroll
+        for( int h = 0; h < 8; h += 4 )
+        {
+            prr = df_add_f( prr, dot4( make_float4( rA[h], rA[h + 1], rA[h + 2], rA[h + 3] ), make_float4( rA[h], rA[h + 1], rA[h + 2], rA[h + 3] ) ) );
+            prr = df_add_f( prr, dot4( make_float4( rB[h], rB[h + 1], rB[h + 2], rB[h + 3] ), make_float4( rB[h], rB[h + 1], rB[h + 2], rB[h + 3] ) ) );
+        }
+        prz = df_add_f( prz, mic_sweeps( rA, rB, mA, mB ) );
+        store8( sv.z + o, rA );
+        store8( sv.z + o + 64, rB );
+    }
+}
+
+__global__ void __launch_bounds__( 32 * kUpdWarps, 4 ) k_pcg_update( int ntiles, BoraSolverDev sv, BoraReduceDev red,
                                                                   int ndq, int slot_rz_in, int slot_dq_in )
 {
-    using namespace micsweep;
-    __shared__ __align__( 16 ) float sval[kUpdWarps][kBuf];
-    __shared__ __align__( 16 ) float spiv[kUpdWarps][kBuf];
     __shared__ float2 s_dq[kUpdWarps];
     bora_pdl_trigger();
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for( int q = lane; q < kBuf; q += 32 ) { sval[w][q] = 0.f; spiv[w][q] = 0.f; }
     bora_pdl_wait();  // the previous kernel's results are complete from here
-    float alpha = 0.f;
-    if( slot_rz_in >= 0 )
-    {
-        const DF dq = part_collect( red.part_dq, ndq, s_dq );
-        alpha = df_ratio( red.ringf[slot_rz_in], make_float2( dq.hi, dq.lo ) );
-        if( blockIdx.x == 0 && threadIdx.x == 0 ) ring_store( red, slot_dq_in, dq, false );
-    }
     DF prz{ 0.f, 0.f }, prr{ 0.f, 0.f };
-    __syncwarp();
-    pcg_update_tiles( ntiles, sv, alpha, blockIdx.x * kUpdWarps + w, gridDim.x * kUpdWarps, sval[w], spiv[w], prz, prr );
+    auto alpha_of = [&]() -> float {
+        if( slot_rz_in < 0 ) return 0.f;
+        const DF dq = part_collect( red.part_dq, ndq, s_dq );
+        if( blockIdx.x == 0 && threadIdx.x == 0 ) ring_store( red, slot_dq_in, dq, false );
+        return df_ratio( red.ringf[slot_rz_in], make_float2( dq.hi, dq.lo ) );
+    };
+    pcg_update_tiles( ntiles, sv, alpha_of, blockIdx.x * kUpdWarps + ( threadIdx.x >> 5 ), gridDim.x * kUpdWarps, prz, prr );
     part_publish( prz, prr, red.part_rz, red.part_rr, blockIdx.x );
 }
 
@@ -754,22 +725,16 @@ __device__ __forceinline__ double grid_sum( const double* part, unsigned nb )
 
 __global__ void __launch_bounds__( 32 * kUpdWarps, 3 ) k_pcg_persistent( const __grid_constant__ PcgPersistArgs a )
 {
-    using namespace micsweep;
     static_assert( kUpdWarps == kDirWarps, "both phases run one tile per warp" );
-    __shared__ __align__( 16 ) float sval[kUpdWarps][kBuf];
-    __shared__ __align__( 16 ) float spiv[kUpdWarps][kBuf];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for( int q = lane; q < kBuf; q += 32 ) { sval[w][q] = 0.f; spiv[w][q] = 0.f; }
-    __syncwarp();
     const unsigned G = gridDim.x;
     double* const pd = a.part;                // d'.q
     double* const pz = a.part + G;            // r.z
     double* const pr = a.part + 2 * (size_t)G;  // r.r
-    const int first = blockIdx.x * kUpdWarps + w, stride = G * kUpdWarps;
+    const int first = blockIdx.x * kUpdWarps + ( threadIdx.x >> 5 ), stride = G * kUpdWarps;
     double rz_prev = a.slot_rz_prev >= 0 ? a.red.ring[a.slot_rz_prev] : -1.0;
     // the pass's first update: z = M^-1 r (alpha 0)
     DF prz{ 0.f, 0.f }, prr{ 0.f, 0.f };
-    pcg_update_tiles( a.ntiles, a.sv, 0.f, first, stride, sval[w], spiv[w], prz, prr );
+    pcg_update_tiles( a.ntiles, a.sv, [] { return 0.f; }, first, stride, prz, prr );
     block_sum_store( df_warp_sum( prz ), pz );
     block_sum_store( df_warp_sum( prr ), pr );
     if( !grid_barrier( a ) ) return;
@@ -787,7 +752,8 @@ __global__ void __launch_bounds__( 32 * kUpdWarps, 3 ) k_pcg_persistent( const _
         dsel ^= 1;
         prz = DF{ 0.f, 0.f };
         prr = DF{ 0.f, 0.f };
-        pcg_update_tiles( a.ntiles, a.sv, (float)( rz / dq ), first, stride, sval[w], spiv[w], prz, prr );
+        const float alpha = (float)( rz / dq );
+        pcg_update_tiles( a.ntiles, a.sv, [=] { return alpha; }, first, stride, prz, prr );
         block_sum_store( df_warp_sum( prz ), pz );
         block_sum_store( df_warp_sum( prr ), pr );
         if( !grid_barrier( a ) ) return;
