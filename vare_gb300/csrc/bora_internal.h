@@ -50,6 +50,24 @@ private:
 __device__ __forceinline__ void bora_pdl_trigger() { asm volatile( "griddepcontrol.launch_dependents;" ::: "memory" ); }
 __device__ __forceinline__ void bora_pdl_wait() { asm volatile( "griddepcontrol.wait;" ::: "memory" ); }
 
+// Eight consecutive floats (an x-row of a tile, 32-byte aligned) in one 256-bit access (sm_100
+// and later). A lane that owns a row would otherwise read its two halves in two 16-byte accesses
+// of 32-byte stride, each of which touches every sector of the warp's rows: twice the L1 sector
+// accesses (929 per tile in the PCG direction kernel). Volatile, so that no access moves across
+// a dependency wait or a barrier.
+__device__ __forceinline__ void bora_ld8( const float* p, float* v )
+{
+    asm volatile( "ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                  : "=f"( v[0] ), "=f"( v[1] ), "=f"( v[2] ), "=f"( v[3] ), "=f"( v[4] ), "=f"( v[5] ), "=f"( v[6] ), "=f"( v[7] )
+                  : "l"( p ) );
+}
+__device__ __forceinline__ void bora_st8( float* p, const float* v )
+{
+    asm volatile( "st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"( p ), "f"( v[0] ), "f"( v[1] ), "f"( v[2] ),
+                  "f"( v[3] ), "f"( v[4] ), "f"( v[5] ), "f"( v[6] ), "f"( v[7] )
+                  : "memory" );
+}
+
 template <typename... KArgs, typename... Args>
 cudaError_t bora_launch_pdl( void ( *kernel )( KArgs... ), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                              Args&&... args )

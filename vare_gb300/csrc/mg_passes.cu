@@ -90,15 +90,10 @@ __device__ __forceinline__ void codes8( const uint16_t* __restrict__ code, size_
 
 __device__ __forceinline__ void f32x8( const float* __restrict__ p, size_t g, float* v )
 {
-    const float4 a = *reinterpret_cast<const float4*>( p + g ), b = *reinterpret_cast<const float4*>( p + g + 4 );
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    bora_ld8( p + g, v );
 }
 
-__device__ __forceinline__ void st_f32x8( float* __restrict__ p, size_t g, const float* v )
-{
-    reinterpret_cast<float4*>( p + g )[0] = make_float4( v[0], v[1], v[2], v[3] );
-    reinterpret_cast<float4*>( p + g )[1] = make_float4( v[4], v[5], v[6], v[7] );
-}
+__device__ __forceinline__ void st_f32x8( float* __restrict__ p, size_t g, const float* v ) { bora_st8( p + g, v ); }
 
 __device__ __forceinline__ float hbits( uint32_t w, int q ) { return __half2float( __ushort_as_half( (unsigned short)( w >> ( 16 * q ) ) ) ); }
 

@@ -299,18 +299,6 @@ __device__ __forceinline__ void rotate8( float* v, int rho )
     }
 }
 
-__device__ __forceinline__ void load8( const float* __restrict__ p, float* v )
-{
-    const float4 a = reinterpret_cast<const float4*>( p )[0], b = reinterpret_cast<const float4*>( p )[1];
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-}
-
-__device__ __forceinline__ void store8( float* __restrict__ p, const float* v )
-{
-    reinterpret_cast<float4*>( p )[0] = make_float4( v[0], v[1], v[2], v[3] );
-    reinterpret_cast<float4*>( p )[1] = make_float4( v[4], v[5], v[6], v[7] );
-}
-
 // z = M^-1 r of one tile: rA, rB hold the lane's rows of r and return z (both in cell order);
 // mA, mB the rows' squared pivots as stored (rotated). Returns the lane's part of r.z.
 __device__ __forceinline__ float mic_sweeps( float* rA, float* rB, const float* mA, const float* mB )
@@ -371,8 +359,8 @@ __device__ __forceinline__ void pcg_update_tiles( int ntiles, const BoraSolverDe
     float rA[8], rB[8], qA[8], qB[8], mA[8], mB[8];
     auto load_tile = [&]( int s ) {
         const size_t o = (size_t)s * 512 + row;
-        load8( sv.r + o, rA ); load8( sv.r + o + 64, rB );
-        load8( sv.q + o, qA ); load8( sv.q + o + 64, qB );
+        bora_ld8( sv.r + o, rA ); bora_ld8( sv.r + o + 64, rB );
+        bora_ld8( sv.q + o, qA ); bora_ld8( sv.q + o + 64, qB );
     };
     if( first < ntiles ) load_tile( first );
     const float alpha = alpha_of();
@@ -380,16 +368,16 @@ __device__ __forceinline__ void pcg_update_tiles( int ntiles, const BoraSolverDe
     {
         const size_t o = (size_t)s * 512 + row;
         if( s != first ) load_tile( s );
-        load8( sv.minv + o, mA );  // not with the first loads: the registers they take there cost more (spills)
-        load8( sv.minv + o + 64, mB );
+        bora_ld8( sv.minv + o, mA );  // not with the first loads: the registers they take there cost more (spills)
+        bora_ld8( sv.minv + o + 64, mB );
 #pragma unroll
         for( int i = 0; i < 8; ++i )
         {
             rA[i] = fmaf( -alpha, qA[i], rA[i] );
             rB[i] = fmaf( -alpha, qB[i], rB[i] );
         }
-        store8( sv.r + o, rA );
-        store8( sv.r + o + 64, rB );
+        bora_st8( sv.r + o, rA );
+        bora_st8( sv.r + o + 64, rB );
 #pragma unroll
         for( int h = 0; h < 8; h += 4 )
         {
@@ -397,8 +385,8 @@ __device__ __forceinline__ void pcg_update_tiles( int ntiles, const BoraSolverDe
             prr = df_add_f( prr, dot4( make_float4( rB[h], rB[h + 1], rB[h + 2], rB[h + 3] ), make_float4( rB[h], rB[h + 1], rB[h + 2], rB[h + 3] ) ) );
         }
         prz = df_add_f( prz, mic_sweeps( rA, rB, mA, mB ) );
-        store8( sv.z + o, rA );
-        store8( sv.z + o + 64, rB );
+        bora_st8( sv.z + o, rA );
+        bora_st8( sv.z + o + 64, rB );
     }
 }
 
@@ -442,134 +430,111 @@ __device__ inline size_t face_nbr( const int32_t* __restrict__ nbr, size_t cell,
 
 // ---------------------------------------------------------------------------------
 // PCG direction: e += alpha d (the previous update's step, pending); d' = z + beta d;
-// q = A d'; dq = d'.q (d double-buffered). One warp per tile, persistent over tiles. Each
-// lane owns two x-rows of the tile, (j, kq) and (j, kq + 4) with j = lane & 7, kq = lane >> 3
-// (tile rows lane and lane + 32), read and written as 16-byte vectors. The stencil's x
-// neighbours are the lane's own registers, its y and z neighbours inside the tile come from
-// other lanes by shuffles, and the cells of the six face-neighbour tiles that the tile's
-// boundary rows need are loaded by the lanes that own those rows (d' formed the same way;
-// an inactive neighbour tile contributes 0). Non-fluid cells hold d = z = 0, so the stencil
-// sum runs over all six neighbours in the fixed order -x, +x, -y, +y, -z, +z; the dot
-// product adds d'.q of cells (i, j, k) and (i, j, k + 4) in float, then into a double-float
-// sum.
+// q = A d'; dq = d'.q (d double-buffered). One warp per half tile (the z-layers 0..3 or 4..7),
+// persistent over half tiles; a lane owns one x-row (lane = j + 8 (k mod 4)), read and written as
+// 32-byte vectors. The stencil's x neighbours are the lane's own registers, its y and z neighbours
+// inside the half come from other lanes by shuffles, and the rows across the half's faces (the
+// other half, the face-neighbour tiles) are loaded by the lanes that need them (d' formed the same
+// way; an inactive neighbour tile contributes 0). Non-fluid cells hold d = z = 0, so the stencil
+// sum runs over all six neighbours in the fixed order -x, +x, -y, +y, -z, +z; the dot product adds
+// d'.q of two x-neighbour cells in float, then into a double-float sum.
+//
+// Waits on its loads (long scoreboard), so it wants warps in flight and few sectors per load: a
+// lane with two rows needs 122 registers for the same loads in flight (31.2 us per launch with
+// 16-byte loads at 72 registers, 256^3, an event on either side; 26.8 us now).
 constexpr int kDirWarps = 4;
 
-// The direction step of the warp's tiles bid * kDirWarps + warp, then every G * kDirWarps:
-// returns the thread's d'.q. upd_e: the previous update's e += alpha d is still pending.
+// The direction step of the warp's half tiles bid * kDirWarps + warp, then every G * kDirWarps:
+// returns the thread's d'.q. coef(): the pair (beta, alpha of the pending e += alpha d), called
+// once by every thread of the block after the first half tile's loads have been issued; upd_e:
+// that update is pending.
+template <class Coef>
 __device__ __forceinline__ DF pcg_direction_tiles( int ntiles, const int32_t* __restrict__ nbr,
                                                    const uint16_t* __restrict__ code, const BoraSolverDev& sv, int dsel_in,
-                                                   float beta, float alpha, bool upd_e, unsigned bid, unsigned G )
+                                                   Coef coef, bool upd_e, unsigned bid, unsigned G )
 {
-    const float* __restrict__ dold = dsel_in ? sv.d[1] : sv.d[0];  // selects keep sv out of local memory
-    float* __restrict__ dnew = dsel_in ? sv.d[0] : sv.d[1];
-    const int lane = threadIdx.x & 31, j = lane & 7, kq = lane >> 3;
+    const float* dold = dsel_in ? sv.d[1] : sv.d[0];  // selects keep sv out of local memory
+    float* dnew = dsel_in ? sv.d[0] : sv.d[1];
+    const int lane = threadIdx.x & 31, j = lane & 7, kk = lane >> 3;
     constexpr unsigned kAll = 0xffffffffu;
-    // d' of 8 consecutive cells starting at cell c of tile slot t (0 when t < 0)
-    auto halo8 = [&]( int t, int c, float* v ) {
-        if( t < 0 ) { for( int i = 0; i < 8; ++i ) v[i] = 0.f; return; }
-        const size_t g = (size_t)t * 512 + c;
-        const float4 d0 = *reinterpret_cast<const float4*>( dold + g ), d1 = *reinterpret_cast<const float4*>( dold + g + 4 );
-        const float4 z0 = *reinterpret_cast<const float4*>( sv.z + g ), z1 = *reinterpret_cast<const float4*>( sv.z + g + 4 );
-        v[0] = fmaf( beta, d0.x, z0.x ); v[1] = fmaf( beta, d0.y, z0.y ); v[2] = fmaf( beta, d0.z, z0.z ); v[3] = fmaf( beta, d0.w, z0.w );
-        v[4] = fmaf( beta, d1.x, z1.x ); v[5] = fmaf( beta, d1.y, z1.y ); v[6] = fmaf( beta, d1.z, z1.z ); v[7] = fmaf( beta, d1.w, z1.w );
-    };
-    auto halo1 = [&]( int t, int c ) { return t < 0 ? 0.f : fmaf( beta, dold[(size_t)t * 512 + c], sv.z[(size_t)t * 512 + c] ); };
     DF pdq{ 0.f, 0.f };
-    for( int s = (int)bid * kDirWarps + ( threadIdx.x >> 5 ); s < ntiles; s += (int)G * kDirWarps )
+    float beta = 0.f, alpha = 0.f;
+    float d[8], z[8];
+    const int nh = 2 * ntiles;
+    int h = (int)bid * kDirWarps + ( threadIdx.x >> 5 );
+    auto load_rows = [&]( int h ) {
+        const size_t g = (size_t)h * 256 + 8 * lane;
+        bora_ld8( dold + g, d );
+        bora_ld8( sv.z + g, z );
+    };
+    if( h < nh ) load_rows( h );
     {
+        const float2 c = coef();
+        beta = c.x;
+        alpha = c.y;
+    }
+    for( bool head = true; h < nh; h += (int)G * kDirWarps, head = false )
+    {
+        const int s = h >> 1, hi = h & 1;
         const int32_t* __restrict__ nb = nbr + (size_t)s * 27;  // tile tables: not written by the solver chain
         const int smx = nb[bora_dir( -1, 0, 0 )], spx = nb[bora_dir( 1, 0, 0 )];
         const int smy = nb[bora_dir( 0, -1, 0 )], spy = nb[bora_dir( 0, 1, 0 )];
-        const int smz = nb[bora_dir( 0, 0, -1 )], spz = nb[bora_dir( 0, 0, 1 )];
-        const size_t gA = (size_t)s * 512 + 8 * lane, gB = gA + 256;
-        // own rows: d' = z + beta d and the pending e += alpha d, both stored right away
-        float dA[8], dB[8];
-        uint16_t cA[8], cB[8];
+        const int sz = nb[bora_dir( 0, 0, hi ? 1 : -1 )];
+        const int cA = hi * 256 + 8 * lane;
+        const size_t g = (size_t)h * 256 + 8 * lane;
+        if( !head ) load_rows( h );
+        const uint4 w = *reinterpret_cast<const uint4*>( code + g );
+        float e[8];
+        if( upd_e ) bora_ld8( sv.e + g, e );
+        auto halo1 = [&]( int t, int c ) { return t < 0 ? 0.f : fmaf( beta, dold[(size_t)t * 512 + c], sv.z[(size_t)t * 512 + c] ); };
+        auto halo8 = [&]( int t, int c, float* v ) {
+            if( t < 0 ) { for( int i = 0; i < 8; ++i ) v[i] = 0.f; return; }
+            float dd[8];
+            bora_ld8( dold + (size_t)t * 512 + c, dd );
+            bora_ld8( sv.z + (size_t)t * 512 + c, v );
 #pragma unroll
-        for( int r = 0; r < 2; ++r )
-        {
-            const size_t g = r ? gB : gA;
-            float* dn = r ? dB : dA;
-            uint16_t* cc = r ? cB : cA;
-            halo8( s, (int)( g - (size_t)s * 512 ), dn );
-            reinterpret_cast<float4*>( dnew + g )[0] = make_float4( dn[0], dn[1], dn[2], dn[3] );
-            reinterpret_cast<float4*>( dnew + g )[1] = make_float4( dn[4], dn[5], dn[6], dn[7] );
-            const uint4 cw = *reinterpret_cast<const uint4*>( code + g );
-            const uint32_t w4[4] = { cw.x, cw.y, cw.z, cw.w };
-#pragma unroll
-            for( int i = 0; i < 4; ++i ) { cc[2 * i] = (uint16_t)( w4[i] & 0xffffu ); cc[2 * i + 1] = (uint16_t)( w4[i] >> 16 ); }
-            if( upd_e )
-            {
-                const float4 d0 = *reinterpret_cast<const float4*>( dold + g ), d1 = *reinterpret_cast<const float4*>( dold + g + 4 );
-                float4 e0 = *reinterpret_cast<const float4*>( sv.e + g ), e1 = *reinterpret_cast<const float4*>( sv.e + g + 4 );
-                e0.x = fmaf( alpha, d0.x, e0.x ); e0.y = fmaf( alpha, d0.y, e0.y ); e0.z = fmaf( alpha, d0.z, e0.z ); e0.w = fmaf( alpha, d0.w, e0.w );
-                e1.x = fmaf( alpha, d1.x, e1.x ); e1.y = fmaf( alpha, d1.y, e1.y ); e1.z = fmaf( alpha, d1.z, e1.z ); e1.w = fmaf( alpha, d1.w, e1.w );
-                reinterpret_cast<float4*>( sv.e + g )[0] = e0;
-                reinterpret_cast<float4*>( sv.e + g )[1] = e1;
-            }
-        }
-        // neighbour-tile cells: x ends of both rows; the y face row of lanes j = 0 / 7 (row A
-        // here, row B after row A's stencil); the z face row of row A at k = 0 (-z) and of row
-        // B at k = 7 (+z)
-        const float xmA = halo1( smx, 8 * lane + 7 ), xpA = halo1( spx, 8 * lane );
-        const float xmB = halo1( smx, 256 + 8 * lane + 7 ), xpB = halo1( spx, 256 + 8 * lane );
-        const int yt = j == 0 ? smy : ( j == 7 ? spy : -1 );
-        const int yc = 8 * ( lane - j ) + ( j == 0 ? 56 : 0 );  // row (7 or 0, kq) of the neighbour tile
-        float yh[8], zh[8];
+            for( int i = 0; i < 8; ++i ) v[i] = fmaf( beta, dd[i], v[i] );
+        };
+        const float xm = halo1( smx, cA + 7 ), xp = halo1( spx, cA );
+        const int yt = j == 0 ? smy : ( j == 7 ? spy : -1 ), yc = cA + ( j == 0 ? 56 : -56 );
+        // the z neighbour rows outside the warp's half: the other half, or the neighbour tile
+        const int zt = kk == 0 ? ( hi ? s : sz ) : ( kk == 3 ? ( hi ? sz : s ) : -1 );
+        const int zc = 8 * j + ( kk == 0 ? ( hi ? 192 : 448 ) : ( hi ? 0 : 256 ) );
+        float yh[8], zh[8], q[8];
         halo8( yt, yc, yh );
+        halo8( zt, zc, zh );
+        if( upd_e )
         {
-            const int zt = kq == 0 ? smz : ( kq == 3 ? spz : -1 );
-            const int zc = 8 * j + ( kq == 0 ? 448 : 0 );  // row (j, 7) or (j, 0) of the neighbour tile
-            halo8( zt, zc, zh );
+#pragma unroll
+            for( int i = 0; i < 8; ++i ) e[i] = fmaf( alpha, d[i], e[i] );
+            bora_st8( sv.e + g, e );
         }
-        // q = A d' and d'.q, row A then row B (both rows' d' feed the z shuffles)
-        float q[8], tA[8];
+#pragma unroll
+        for( int i = 0; i < 8; ++i ) d[i] = fmaf( beta, d[i], z[i] );
+        bora_st8( dnew + g, d );
+        const uint32_t cw[4] = { w.x, w.y, w.z, w.w };
 #pragma unroll
         for( int i = 0; i < 8; ++i )
         {
-            float ymA = __shfl_up_sync( kAll, dA[i], 1 ), ypA = __shfl_down_sync( kAll, dA[i], 1 );
-            if( j == 0 ) ymA = yh[i];
-            if( j == 7 ) ypA = yh[i];
-            float zmA = __shfl_up_sync( kAll, dA[i], 8 );
-            if( kq == 0 ) zmA = zh[i];
-            const float zpA = __shfl_sync( kAll, kq == 0 ? dB[i] : dA[i], ( lane + 8 ) & 31 );
-            const float xmA_ = i > 0 ? dA[i > 0 ? i - 1 : 0] : xmA, xpA_ = i < 7 ? dA[i < 7 ? i + 1 : 7] : xpA;
+            float ym = __shfl_up_sync( kAll, d[i], 1 ), yp = __shfl_down_sync( kAll, d[i], 1 );
+            if( j == 0 ) ym = yh[i];
+            if( j == 7 ) yp = yh[i];
+            float zm = __shfl_up_sync( kAll, d[i], 8 ), zp = __shfl_down_sync( kAll, d[i], 8 );
+            if( kk == 0 ) zm = zh[i];
+            if( kk == 3 ) zp = zh[i];
+            const uint32_t c = i & 1 ? cw[i >> 1] >> 16 : cw[i >> 1] & 0xffffu;
             q[i] = 0.f;
-            tA[i] = 0.f;
-            if( cA[i] & BORA_CODE_FLUID )
+            if( c & BORA_CODE_FLUID )
             {
                 float acc = 0.f;
-                acc += xmA_; acc += xpA_; acc += ymA; acc += ypA; acc += zmA; acc += zpA;
-                q[i] = fmaf( (float)code_diag( cA[i] ), dA[i], -acc );
-                tA[i] = fmaf( dA[i], q[i], 0.f );
+                acc += i > 0 ? d[i > 0 ? i - 1 : 0] : xm; acc += i < 7 ? d[i < 7 ? i + 1 : 7] : xp;
+                acc += ym; acc += yp; acc += zm; acc += zp;
+                q[i] = fmaf( (float)code_diag( (uint16_t)c ), d[i], -acc );
             }
         }
-        reinterpret_cast<float4*>( sv.q + gA )[0] = make_float4( q[0], q[1], q[2], q[3] );
-        reinterpret_cast<float4*>( sv.q + gA )[1] = make_float4( q[4], q[5], q[6], q[7] );
-        halo8( yt, yc + 256, yh );
 #pragma unroll
-        for( int i = 0; i < 8; ++i )
-        {
-            float ymB = __shfl_up_sync( kAll, dB[i], 1 ), ypB = __shfl_down_sync( kAll, dB[i], 1 );
-            if( j == 0 ) ymB = yh[i];
-            if( j == 7 ) ypB = yh[i];
-            const float zmB = __shfl_sync( kAll, kq == 3 ? dA[i] : dB[i], ( lane + 24 ) & 31 );
-            float zpB = __shfl_down_sync( kAll, dB[i], 8 );
-            if( kq == 3 ) zpB = zh[i];
-            const float xmB_ = i > 0 ? dB[i > 0 ? i - 1 : 0] : xmB, xpB_ = i < 7 ? dB[i < 7 ? i + 1 : 7] : xpB;
-            q[i] = 0.f;
-            float t = tA[i];
-            if( cB[i] & BORA_CODE_FLUID )
-            {
-                float acc = 0.f;
-                acc += xmB_; acc += xpB_; acc += ymB; acc += ypB; acc += zmB; acc += zpB;
-                q[i] = fmaf( (float)code_diag( cB[i] ), dB[i], -acc );
-                t = fmaf( dB[i], q[i], t );
-            }
-            pdq = df_add_f( pdq, t );
-        }
-        reinterpret_cast<float4*>( sv.q + gB )[0] = make_float4( q[0], q[1], q[2], q[3] );
-        reinterpret_cast<float4*>( sv.q + gB )[1] = make_float4( q[4], q[5], q[6], q[7] );
+        for( int i = 0; i < 8; i += 2 ) pdq = df_add_f( pdq, fmaf( d[i + 1], q[i + 1], d[i] * q[i] ) );
+        bora_st8( sv.q + g, q );
     }
     return pdq;
 }
@@ -583,23 +548,25 @@ __device__ __forceinline__ void pcg_direction_body( int ntiles, const int32_t* _
     __shared__ float2 s_rz[kDirWarps], s_rr[kDirWarps];
     bora_pdl_trigger();
     bora_pdl_wait();  // the previous kernel's results (ring, partial sums, z, d, e) are complete from here
-    const DF rz = part_collect( red.part_rz, nparts, s_rz );
-    const float beta = slot_rz_old < 0 ? 0.f : df_ratio( make_float2( rz.hi, rz.lo ), red.ringf[slot_rz_old] );
-    const float alpha = slot_a_rz < 0 ? 0.f : df_ratio( red.ringf[slot_a_rz], red.ringf[slot_a_dq] );
-    if( bid == G - 1 )  // the last block (never the one with more tiles) finishes rr for the host
-    {
-        const DF rr = part_collect( red.part_rr, nparts, s_rr );
-        if( threadIdx.x == 0 )
+    auto coef = [&]() -> float2 {
+        const DF rz = part_collect( red.part_rz, nparts, s_rz );
+        if( bid == G - 1 )  // the last block (never the one with more tiles) finishes rr for the host
         {
-            ring_store( red, slot_rz_new, rz, false );
-            ring_store( red, slot_rr, rr, host_rr );
+            const DF rr = part_collect( red.part_rr, nparts, s_rr );
+            if( threadIdx.x == 0 )
+            {
+                ring_store( red, slot_rz_new, rz, false );
+                ring_store( red, slot_rr, rr, host_rr );
+            }
         }
-    }
-    const DF pdq = pcg_direction_tiles( ntiles, nbr, code, sv, dsel_in, beta, alpha, slot_a_rz >= 0, bid, G );
+        return make_float2( slot_rz_old < 0 ? 0.f : df_ratio( make_float2( rz.hi, rz.lo ), red.ringf[slot_rz_old] ),
+                            slot_a_rz < 0 ? 0.f : df_ratio( red.ringf[slot_a_rz], red.ringf[slot_a_dq] ) );
+    };
+    const DF pdq = pcg_direction_tiles( ntiles, nbr, code, sv, dsel_in, coef, slot_a_rz >= 0, bid, G );
     part_publish( pdq, DF{ 0.f, 0.f }, red.part_dq, nullptr, bid );
 }
 
-__global__ void __launch_bounds__( 32 * kDirWarps, 7 ) k_pcg_direction( int ntiles, const int32_t* __restrict__ nbr,
+__global__ void __launch_bounds__( 32 * kDirWarps, 6 ) k_pcg_direction( int ntiles, const int32_t* __restrict__ nbr,
                                                                     const uint16_t* __restrict__ code, BoraSolverDev sv,
                                                                     int dsel_in, BoraReduceDev red, int nparts,
                                                                     int slot_rz_new, int slot_rr, int slot_rz_old,
@@ -725,7 +692,7 @@ __device__ __forceinline__ double grid_sum( const double* part, unsigned nb )
 
 __global__ void __launch_bounds__( 32 * kUpdWarps, 3 ) k_pcg_persistent( const __grid_constant__ PcgPersistArgs a )
 {
-    static_assert( kUpdWarps == kDirWarps, "both phases run one tile per warp" );
+    static_assert( kUpdWarps == kDirWarps, "one block shape for both phases" );
     const unsigned G = gridDim.x;
     double* const pd = a.part;                // d'.q
     double* const pz = a.part + G;            // r.z
@@ -745,7 +712,8 @@ __global__ void __launch_bounds__( 32 * kUpdWarps, 3 ) k_pcg_persistent( const _
     {
         const float beta = rz_prev < 0.0 ? 0.f : (float)( rz / rz_prev );
         const float alpha_e = a_rz < 0.0 ? 0.f : (float)( a_rz / a_dq );
-        const DF pdq = pcg_direction_tiles( a.ntiles, a.nbr, a.code, a.sv, dsel, beta, alpha_e, a_rz >= 0.0, blockIdx.x, G );
+        const DF pdq = pcg_direction_tiles( a.ntiles, a.nbr, a.code, a.sv, dsel, [=] { return make_float2( beta, alpha_e ); },
+                                            a_rz >= 0.0, blockIdx.x, G );
         block_sum_store( df_warp_sum( pdq ), pd );
         if( !grid_barrier( a ) ) return;
         const double dq = grid_sum( pd, G );
@@ -1101,7 +1069,7 @@ void bora_launch_pcg_update( int ntiles, const uint16_t* code, BoraSolverDev s, 
                      bora_pcg_direction_grid( ntiles ), slot_rz_in, slot_dq_in );
 }
 
-// Grid of the direction kernel: every warp gets the same number of tiles; at most
+// Grid of the direction kernel: every warp gets the same number of half tiles; at most
 // kBoraMaxReduceBlocks CTAs (partial sums capacity).
 int bora_pcg_direction_grid( int ntiles )
 {
@@ -1112,8 +1080,8 @@ int bora_pcg_direction_grid( int ntiles )
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor( &v, k_pcg_direction, 32 * kDirWarps, 0 ) == cudaSuccess && v > 0 ? v : 1;
     } );
     const int cap = std::max( 1, std::min( b * num_sms(), kBoraMaxReduceBlocks ) ) * kDirWarps;
-    const int rounds = ( ntiles + cap - 1 ) / cap;
-    return std::max( 1, ( ntiles + kDirWarps * rounds - 1 ) / ( kDirWarps * rounds ) );
+    const int rounds = ( 2 * ntiles + cap - 1 ) / cap;
+    return std::max( 1, ( 2 * ntiles + kDirWarps * rounds - 1 ) / ( kDirWarps * rounds ) );
 }
 
 namespace {
