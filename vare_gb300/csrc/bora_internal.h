@@ -128,6 +128,20 @@ struct BoraTilesDev
     const int32_t* nbr;       // [slots * 27] -> neighbour slot or -1
 };
 
+// The solver's tiles: the active tiles that hold at least one fluid cell, in slot order. The other
+// active tiles (the margin the activation rule adds around the particles: a sixth of the tiles of
+// the 256^3 dam break) have no unknowns, so no kernel of the solve visits them: their entries in
+// the solver's vectors are neither written nor read, which also keeps more of the vectors in L2
+// (256^3 plain step: 22.3 -> 18.5 ms of GPU time; mixed 4.92 -> 4.74 ms). tab: two int4
+// per solver tile, (-x, +x, -y, +y) and (-z, +z, own, 0): the slots of the face neighbours (-1: not
+// a solver tile) and its own.
+struct BoraSolveTilesDev
+{
+    const int4* tab;
+    const uint32_t* count;  // their number, on the device
+    int n;                  // the same on the host, once known
+};
+
 // Scalars that the solver kernels exchange on the device (ring of FP64 reductions).
 #define BORA_RING 64
 // Largest grid of a kernel that reduces through BoraReduceDev::partials (one slot pair per
@@ -167,7 +181,14 @@ void bora_launch_scatter( size_t n, const uint32_t* key, const uint32_t* start, 
 void bora_launch_order_bins( size_t nbins, const uint32_t* start, uint32_t* idx, cudaStream_t st );
 void bora_launch_p2g( const BoraGridDev& g, int ntiles, BoraTilesDev t, BoraParticlesDev p, const uint32_t* idx,
                       const uint32_t* start, BoraCellsDev c, cudaStream_t st );
-void bora_launch_rhs( const BoraGridDev& g, int ntiles, BoraTilesDev t, BoraCellsDev c, uint32_t* nfluid, cudaStream_t st );
+// tile_fluid: 1 for the tiles with a fluid cell
+void bora_launch_rhs( const BoraGridDev& g, int ntiles, BoraTilesDev t, BoraCellsDev c, uint32_t* nfluid, uint8_t* tile_fluid,
+                      cudaStream_t st );
+// the same flags from stencil codes that the caller has set
+void bora_launch_tile_fluid( int ntiles, const uint16_t* code, uint8_t* tile_fluid, cudaStream_t st );
+// the solver's tile table and count (also written to host_count, mapped host memory) from the flags
+void bora_launch_solve_tiles( int ntiles, BoraTilesDev t, const uint8_t* tile_fluid, int4* tab, uint32_t* count,
+                              uint32_t* host_count, cudaStream_t st );
 void bora_launch_vel_update( const BoraGridDev& g, int ntiles, BoraTilesDev t, BoraCellsDev c, cudaStream_t st );
 void bora_launch_g2p( const BoraGridDev& g, int ntiles, size_t nsorted, BoraTilesDev t, const uint32_t* start, BoraCellsDev c,
                       BoraParticlesDev src, const uint32_t* idx, BoraParticlesDev dst, float* adj, float dt,
@@ -216,15 +237,16 @@ struct BoraSolverDev
     float* minv;    // squared block-MIC(0) inverse pivots, each row of a tile rotated (projection.cu)
 };
 
-void bora_launch_mic_factor( const BoraGridDev& g, int ntiles, const uint16_t* code, float* minv, cudaStream_t st );
+// (ntiles: an upper bound for the grid; the kernels read the number of solver tiles on the device)
+void bora_launch_mic_factor( int ntiles, BoraSolveTilesDev t, const uint16_t* code, float* minv, cudaStream_t st );
 // r = b, x = 0, e = 0, d = 0, q = 0; partial sums of ||b||^2 and max|b| -> ring slots
-void bora_launch_solve_init( int ntiles, const float* b, const uint16_t* code, BoraSolverDev s, BoraReduceDev red,
+void bora_launch_solve_init( int ntiles, BoraSolveTilesDev t, const float* b, BoraSolverDev s, BoraReduceDev red,
                              int slot_norm2, int slot_max, cudaStream_t st );
 // r -= alpha q; z = M^-1 r; partial sums of rz and rr (alpha = rz_in / dq, or 0 when slot_rz_in < 0; dq is
 // finished from the direction kernel's partials into slot_dq_in). bora_pcg_update_grid: its blocks.
 int bora_pcg_update_grid( int ntiles );
-void bora_launch_pcg_update( int ntiles, const uint16_t* code, BoraSolverDev s, BoraReduceDev red, int slot_rz_in,
-                             int slot_dq_in, cudaStream_t st );
+void bora_launch_pcg_update( BoraSolveTilesDev t, BoraSolverDev s, BoraReduceDev red, int slot_rz_in, int slot_dq_in,
+                             cudaStream_t st );
 int bora_pcg_direction_grid( int ntiles );
 // One refinement pass of the plain form's inner PCG in one cooperative launch with bounded
 // grid barriers (projection.cu). Outputs: ring slots slot_a_rz / slot_a_dq (the last
@@ -233,23 +255,22 @@ int bora_pcg_direction_grid( int ntiles );
 // wait runs out (a test of the error path). Returns 0, or -1 when the launch is refused.
 #define BORA_REDUCE_ERR_BARRIER 0x100u  // a grid barrier wait ran out
 int bora_pcg_persistent_grid();
-int bora_launch_pcg_persistent( int ntiles, const int32_t* nbr, const uint16_t* code, BoraSolverDev s, BoraReduceDev red,
+int bora_launch_pcg_persistent( BoraSolveTilesDev t, const uint16_t* code, BoraSolverDev s, BoraReduceDev red,
                                 int dsel, int slot_rz_prev, int max_inner, double target, int slot_a_rz, int slot_a_dq,
                                 uint32_t* iters, unsigned* bar, double* part, bool never_release, cudaStream_t st );
 // d' = z + beta d; q = A d'; partial sums of dq (beta = rz_new / rz_old, or 0 when slot_rz_old < 0). Finishes rz
 // and rr from nparts producer blocks' partials into slot_rz_new and slot_rr (host_rr: rr also for the host).
-void bora_launch_pcg_direction( const BoraGridDev& g, int ntiles, BoraTilesDev t, const uint16_t* code, BoraSolverDev s,
-                                int dsel_in, BoraReduceDev red, int nparts, int slot_rz_new, int slot_rr, int slot_rz_old,
+void bora_launch_pcg_direction( BoraSolveTilesDev t, const uint16_t* code, BoraSolverDev s, int dsel_in, BoraReduceDev red, int nparts, int slot_rz_new, int slot_rr, int slot_rz_old,
                                 int slot_a_rz, int slot_a_dq, bool host_rr, cudaStream_t st );
 // x += e (FP64); e = 0; d = 0; q = 0; finishes the last update's rr into slot_rr (also for the host)
 // x = the last step's pressure on fluid cells, read through the previous tile table (the warm start)
 void bora_launch_solve_warm( int ntiles, const uint16_t* code, const int32_t* tile_of, const int32_t* slot_prev,
                              const float* pres, BoraSolverDev s, cudaStream_t st );
-void bora_launch_refine_accumulate( int ntiles, const uint16_t* code, BoraSolverDev s, int dsel, BoraReduceDev red,
+void bora_launch_refine_accumulate( BoraSolveTilesDev t, const uint16_t* code, BoraSolverDev s, int dsel, BoraReduceDev red,
                                     int nparts, int slot_rr, int slot_a_rz, int slot_a_dq, cudaStream_t st );
 // r = b - A x in FP64 (stored FP32); ||r||^2 and max|r| -> ring slots
-void bora_launch_refine_residual( const BoraGridDev& g, int ntiles, BoraTilesDev t, const float* b, const uint16_t* code,
-                                  BoraSolverDev s, BoraReduceDev red, int slot_norm2, int slot_max, cudaStream_t st );
+void bora_launch_refine_residual( BoraSolveTilesDev t, const float* b, const uint16_t* code, BoraSolverDev s,
+                                  BoraReduceDev red, int slot_norm2, int slot_max, cudaStream_t st );
 // pres = (float) x on fluid cells, 0 elsewhere
 void bora_launch_write_pressure( int ntiles, const uint16_t* code, const float2* x, float* pres, cudaStream_t st );
 
@@ -278,11 +299,11 @@ struct BoraLevelDev
 // slot_rz_in < 0; the first pass finishes dq from the direction kernel's partials), with partial
 // sums of the updated r.r; slot_rr gives the scale.
 int bora_mg_pass_grid( int E, int ntiles, int v );  // v < 0: level 0's fixed up-2 shape
-void bora_mg_pass_down( const BoraLevelDev* levels, int l, const BoraTilesDev& t, int ntiles, float* r0, const float* q,
+void bora_mg_pass_down( const BoraLevelDev* levels, int l, const BoraSolveTilesDev& t, float* r0, const float* q,
                         float* scratch, const BoraReduceDev& red, int slot_rr, int slot_rz_in, int slot_dq_in,
                         cudaStream_t st );
-void bora_mg_pass_up( const BoraLevelDev* levels, int l, const __half* ec, const BoraTilesDev& t, int ntiles,
-                      const float* r0, float* scratch, const BoraReduceDev& red, int slot_rr, float* z, cudaStream_t st );
+void bora_mg_pass_up( const BoraLevelDev* levels, int l, const __half* ec, const BoraSolveTilesDev& t, const float* r0,
+                      float* scratch, const BoraReduceDev& red, int slot_rr, float* z, cudaStream_t st );
 
 // ---- launch-shape autotuner (tune.cu) ------------------------------------------------------
 // Kernel groups with interchangeable launch shapes (bit-identical results): the multigrid
@@ -335,8 +356,8 @@ void bora_mg_mid_setup( const BoraGridDev& g, const BoraLevelDev* levels, int nl
                         void* image, cudaStream_t st );
 int bora_mg_mid_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t, int ntiles,
                         const void* image, uint32_t* err, int sweeps, cudaStream_t st, bool launch );
-void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t, const void* mid_image,
-                     float* r, const float* q, float* z, float* scratch, BoraReduceDev red, int slot_rz_in,
+void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t, BoraSolveTilesDev ft,
+                     const void* mid_image, float* r, const float* q, float* z, float* scratch, BoraReduceDev red, int slot_rz_in,
                      int slot_dq_in, int slot_scale, int coarse_sweeps, cudaStream_t st );
 // ---- batched solve: several simulations, one launch per kernel ---------------------------
 // A batched launch packs the blocks of the simulations taking part back to back into one
@@ -354,8 +375,8 @@ enum BoraMemberGrid
 };
 struct BoraMemberSolve
 {
-    int ntiles;
-    const int32_t* nbr;
+    int ntiles;            // active tiles (the pressure's)
+    BoraSolveTilesDev ft;  // the solver's tiles
     const uint16_t* code;
     const float* b;
     float* pres;
@@ -421,6 +442,7 @@ void bora_launch_write_pressure_batch( const BoraBatchLaunch& L, int blocks, cud
 void bora_launch_mg_pass_batch( int l, int pass, int v, const BoraBatchLaunch& L, int blocks, cudaStream_t st );
 // this simulation's own grid per batched kernel (what its single launches use), with the
 // multigrid passes of levels 0, 1, 2 in launch shapes v[0..2]
-void bora_member_grids( int ntiles, int* grid, const int* v );
-void bora_projection_grids( int ntiles, int* grid );  // the kGridDir, kGridCells and kGridResidual entries
+// (of a simulation with nft solver tiles)
+void bora_member_grids( int nft, int* grid, const int* v );
+void bora_projection_grids( int nft, int* grid );  // the kGridDir, kGridCells and kGridResidual entries
 

@@ -106,11 +106,6 @@ __global__ void k_to_host_u32( const uint32_t* __restrict__ src, uint32_t* dst, 
     for( int i = threadIdx.x; i < n; i += blockDim.x ) ( (volatile uint32_t*)dst )[i] = src[i];
 }
 
-__global__ void k_to_host_f64( const double* __restrict__ src, double* dst, int n )
-{
-    for( int i = threadIdx.x; i < n; i += blockDim.x ) ( (volatile double*)dst )[i] = src[i];
-}
-
 int grid_blocks( size_t n )
 {
     const size_t b = ( n + 255 ) / 256;
@@ -154,6 +149,9 @@ struct bora_flip_sim
 
     // reductions
     DevBuf ring, partials, done;
+    DevBuf tile_fluid, solve_tab;  // the solver's tiles: a flag per tile, the table (BoraSolveTilesDev)
+    bool solve_tiles_valid = false;  // the table describes the stencil codes
+    int nft = 0;                     // solver tiles, known to the host from the solve's start on
     DevBuf sums;     // the solver chain's partial sums (d.q, r.z, r.r) and the finished pairs
     DevBuf gbar;     // the persistent solver's grid barrier: count, generation
     int fault = 0;   // BORA_FAULT_*
@@ -186,8 +184,6 @@ struct bora_flip_sim
     DevBuf scan_scratch, counters, stage_in, stage_out, live_flag;
     uint32_t* h_cnt = nullptr;  // pinned, mapped: counters as the host sees them
     uint32_t* d_cnt = nullptr;  // its device address
-    double* h_ring = nullptr;   // pinned, mapped
-    double* d_hring = nullptr;  // its device address
     double* h_mirror = nullptr;  // pinned, mapped: reductions' slot values as the host sees them
     double* d_mirror = nullptr;  // its device address
 
@@ -239,6 +235,7 @@ struct bora_flip_sim
                              P<float>( vz ), P<float>( cx ), P<float>( cy ), P<float>( cz ), P<uint8_t>( flag ),
                              P<uint16_t>( code ), P<float>( rhs ) };
     }
+    BoraSolveTilesDev solve_tiles() { return BoraSolveTilesDev{ P<int4>( solve_tab ), P<uint32_t>( counters ) + 9, nft }; }
     BoraTilesDev tiles() { return BoraTilesDev{ P<int32_t>( slot_of ), P<int32_t>( tile_of ), P<int32_t>( nbr ) }; }
     BoraSolverDev solver()
     {
@@ -412,6 +409,8 @@ int ensure_cells( bora_flip_sim* s, int ntiles )
     BORA_TRY( grow( s->cell_start, ( nc + 2 ) * 4, false, s->st ) );
     BORA_TRY( grow( s->tile_of, cap * 4, false, s->st ) );
     BORA_TRY( grow( s->nbr, cap * 27 * 4, false, s->st ) );
+    BORA_TRY( grow( s->tile_fluid, ( cap + 15 ) / 16 * 16, false, s->st ) );
+    BORA_TRY( grow( s->solve_tab, cap * 32, false, s->st ) );
     // two values per block for the reductions; three for the persistent solver's
     BORA_TRY( grow( s->partials, ( std::max<size_t>( cap, kBoraMaxReduceBlocks ) + 16 ) * 3 * 8, false, s->st ) );
     BORA_TRYS( ensure_scan_scratch( s, std::max( nc + 2, s->ntv ) ) );
@@ -436,34 +435,28 @@ int read_counters( bora_flip_sim* s, int first, int count )
     return BORA_OK;
 }
 
-double read_ring( bora_flip_sim* s, int slot, int* status )
-{
-    s->stats.kernel_launches += 1;
-    k_to_host_f64<<<1, 32, 0, s->st>>>( P<double>( s->ring ) + slot, s->d_hring, 1 );
-    cudaError_t e = cudaGetLastError();
-    if( e == cudaSuccess ) e = cudaStreamSynchronize( s->st );
-    if( e != cudaSuccess ) { *status = cuda_status( e ); return 0.0; }
-    return ( (volatile double*)s->h_ring )[0];
-}
-
 // A value that a kernel writes to mapped host memory (BoraReduceDev::mirror): marked as not
 // arrived before the launch, then polled. Sums of squares and maxima are never negative.
 constexpr double kNotArrived = -1.0;
-void arm_mirror( bora_flip_sim* s, int slot ) { ( (volatile double*)s->h_mirror )[slot] = kNotArrived; }
-int poll_mirror( bora_flip_sim* s, int slot, cudaStream_t st, double* v )
+template <class T>
+int poll_mapped( volatile T* p, T none, cudaStream_t st, T* v )
 {
-    volatile double* p = s->h_mirror + slot;
     for( unsigned n = 1;; ++n )
     {
         *v = *p;
-        if( *v != kNotArrived ) return BORA_OK;
+        if( *v != none ) return BORA_OK;
         if( n % 8192 ) continue;
         const cudaError_t e = cudaStreamQuery( st );  // an error, or nothing left that could write it
         if( e == cudaErrorNotReady ) continue;
         if( e != cudaSuccess ) return cuda_status( e );
         *v = *p;
-        return *v != kNotArrived ? BORA_OK : BORA_ERR_INTERNAL;
+        return *v != none ? BORA_OK : BORA_ERR_INTERNAL;
     }
+}
+void arm_mirror( bora_flip_sim* s, int slot ) { ( (volatile double*)s->h_mirror )[slot] = kNotArrived; }
+int poll_mirror( bora_flip_sim* s, int slot, cudaStream_t st, double* v )
+{
+    return poll_mapped( (volatile double*)s->h_mirror + slot, kNotArrived, st, v );
 }
 
 // ---- stages --------------------------------------------------------------------------
@@ -508,6 +501,7 @@ int rebuild_sort( bora_flip_sim* s )
     const int ntiles = (int)s->h_cnt[0];
     BORA_TRYS( ensure_cells( s, std::max( ntiles, 1 ) ) );
     s->ntiles = ntiles;
+    s->solve_tiles_valid = false;
     const uint32_t ncell = (uint32_t)ntiles * BORA_TILE_CELLS;
     {
         KTimer t( s, BORA_KERNEL_TILES, ntiles > 0 ? 2 : 1 );
@@ -623,11 +617,33 @@ int build_hierarchy( bora_flip_sim* s )
     return BORA_OK;
 }
 
+// The table of the solver's tiles from the per-tile flags; the count reaches the host later
+// (wait_solve_tiles).
+constexpr uint32_t kCountNotArrived = 0xFFFFFFFFu;
+void issue_solve_tiles( bora_flip_sim* s )
+{
+    ( (volatile uint32_t*)s->h_cnt )[9] = kCountNotArrived;
+    s->stats.kernel_launches += s->ntiles > 0 ? 2 : 1;
+    bora_launch_solve_tiles( s->ntiles, s->tiles(), P<uint8_t>( s->tile_fluid ), P<int4>( s->solve_tab ),
+                             P<uint32_t>( s->counters ) + 9, s->d_cnt + 9, s->st );
+    s->solve_tiles_valid = true;
+}
+
+int wait_solve_tiles( bora_flip_sim* s )
+{
+    uint32_t n = 0;
+    BORA_TRYS( poll_mapped( (volatile uint32_t*)s->h_cnt + 9, kCountNotArrived, s->st, &n ) );
+    if( n > (uint32_t)std::max( s->ntiles, 0 ) ) return BORA_ERR_INTERNAL;
+    s->nft = (int)n;
+    return BORA_OK;
+}
+
 int stage_build_system( bora_flip_sim* s )
 {
     KTimer t( s, BORA_KERNEL_RHS, s->ntiles > 0 ? 1 : 0 );
     BORA_TRY( cudaMemsetAsync( P<uint32_t>( s->counters ) + 6, 0, 4, s->st ) );
-    bora_launch_rhs( s->g, s->ntiles, s->tiles(), s->cells(), P<uint32_t>( s->counters ) + 6, s->st );
+    bora_launch_rhs( s->g, s->ntiles, s->tiles(), s->cells(), P<uint32_t>( s->counters ) + 6, P<uint8_t>( s->tile_fluid ), s->st );
+    issue_solve_tiles( s );
     if( s->ntiles <= 0 ) return check_launch( s );
     if( s->prm.solver == BORA_SOLVER_MIXED )
     {
@@ -639,7 +655,7 @@ int stage_build_system( bora_flip_sim* s )
     else
     {
         s->stats.kernel_launches += 1;
-        bora_launch_mic_factor( s->g, s->ntiles, P<uint16_t>( s->code ), P<float>( s->sminv ), s->st );
+        bora_launch_mic_factor( s->ntiles, s->solve_tiles(), P<uint16_t>( s->code ), P<float>( s->sminv ), s->st );
     }
     return check_launch( s );
 }
@@ -653,17 +669,27 @@ int stage_solve( bora_flip_sim* s )
     const uint16_t* code = P<uint16_t>( s->code );
     const float* b = P<float>( s->rhs );
     cudaStream_t st = s->st;
-    int status = BORA_OK;
     const double dx = s->scale[0];
 
     BORA_TRY( cudaMemsetAsync( P<uint32_t>( s->counters ) + 5, 0, 4, st ) );
+    if( !s->solve_tiles_valid )  // codes that did not come from this system's build
+    {
+        s->stats.kernel_launches += 1;
+        bora_launch_tile_fluid( s->ntiles, code, P<uint8_t>( s->tile_fluid ), st );
+        issue_solve_tiles( s );
+    }
     const int s_b2 = s->slot(), s_bmax = s->slot();
-    { KTimer t( s, BORA_KERNEL_REFINE, 1 ); bora_launch_solve_init( s->ntiles, b, code, sv, red, s_b2, s_bmax, st ); }
+    arm_mirror( s, s_b2 );
+    arm_mirror( s, s_bmax );
+    { KTimer t( s, BORA_KERNEL_REFINE, 1 ); bora_launch_solve_init( s->ntiles, s->solve_tiles(), b, sv, red, s_b2, s_bmax, st ); }
     BORA_TRYS( check_launch( s ) );
-    const double bnorm = std::sqrt( read_ring( s, s_b2, &status ) );
-    BORA_TRYS( status );
-    double rnorm = bnorm, rmax = read_ring( s, s_bmax, &status );
-    BORA_TRYS( status );
+    double b2 = 0.0, rmax = 0.0;
+    BORA_TRYS( wait_solve_tiles( s ) );
+    BORA_TRYS( poll_mirror( s, s_b2, st, &b2 ) );
+    BORA_TRYS( poll_mirror( s, s_bmax, st, &rmax ) );
+    const BoraSolveTilesDev ft = s->solve_tiles();
+    const double bnorm = std::sqrt( b2 );
+    double rnorm = bnorm;
     int total_it = 0, passes = 0;
     bool converged = false;
     const int max_inner = std::max( 1, p.proj_iteration );
@@ -678,17 +704,19 @@ int stage_solve( bora_flip_sim* s )
         // warm start: x = the last step's pressure, r = b - A x; kept only if closer than x = 0
         s->warm_ready = false;
         const int w_n2 = s->slot(), w_mx = s->slot();
+        arm_mirror( s, w_n2 );
+        arm_mirror( s, w_mx );
         {
             KTimer t( s, BORA_KERNEL_REFINE, 2 );
             bora_launch_solve_warm( s->ntiles, code, P<int32_t>( s->tile_of ), P<int32_t>( s->slot_prev ),
                                     P<float>( s->pres ), sv, st );
-            bora_launch_refine_residual( s->g, s->ntiles, s->tiles(), b, code, sv, red, w_n2, w_mx, st );
+            bora_launch_refine_residual( ft, b, code, sv, red, w_n2, w_mx, st );
         }
         BORA_TRYS( check_launch( s ) );
-        const double wnorm = std::sqrt( read_ring( s, w_n2, &status ) );
-        BORA_TRYS( status );
-        const double wmax = read_ring( s, w_mx, &status );
-        BORA_TRYS( status );
+        double w2 = 0.0, wmax = 0.0;
+        BORA_TRYS( poll_mirror( s, w_n2, st, &w2 ) );
+        BORA_TRYS( poll_mirror( s, w_mx, st, &wmax ) );
+        const double wnorm = std::sqrt( w2 );
         if( wnorm < rnorm )
         {
             rnorm = wnorm;
@@ -698,7 +726,7 @@ int stage_solve( bora_flip_sim* s )
         else
         {
             const int c_b2 = s->slot(), c_bmax = s->slot();  // back to x = 0, r = b
-            { KTimer t( s, BORA_KERNEL_REFINE, 1 ); bora_launch_solve_init( s->ntiles, b, code, sv, red, c_b2, c_bmax, st ); }
+            { KTimer t( s, BORA_KERNEL_REFINE, 1 ); bora_launch_solve_init( s->ntiles, ft, b, sv, red, c_b2, c_bmax, st ); }
             BORA_TRYS( check_launch( s ) );
             scale_slot = c_b2;
         }
@@ -719,11 +747,11 @@ int stage_solve( bora_flip_sim* s )
         // V-cycle's first passes, which scale the FP16 levels by the last known residual norm
         auto precondition = [&]( int rz_in, int dq_in, int scale ) {
             KTimer t( s, BORA_KERNEL_MG, vlaunch );
-            bora_mg_vcycle( s->g, s->levels, s->nlevels, s->tiles(), mid_img, sv.r, sv.q, sv.z, sv.minv, red, rz_in, dq_in,
+            bora_mg_vcycle( s->g, s->levels, s->nlevels, s->tiles(), ft, mid_img, sv.r, sv.q, sv.z, sv.minv, red, rz_in, dq_in,
                             scale, 16, st );
         };
         // blocks of the kernels that leave partial sums of r.z and r.r
-        int nparts = mixed ? bora_mg_pass_grid( 8, s->ntiles, -1 ) : bora_pcg_update_grid( s->ntiles );
+        int nparts = mixed ? bora_mg_pass_grid( 8, ft.n, -1 ) : bora_pcg_update_grid( ft.n );
         int rz_cur = s->slot(), rr_cur = s->slot();
         int it = 0;
         int a_rz = -1, a_dq = -1;  // alpha of the last update, whose e += alpha d is still pending
@@ -734,7 +762,7 @@ int stage_solve( bora_flip_sim* s )
             BORA_TRY( cudaMemsetAsync( P<uint32_t>( s->counters ) + 8, 0, 4, st ) );
             {
                 KTimer t( s, BORA_KERNEL_PCG_UPDATE, 1 );
-                if( bora_launch_pcg_persistent( s->ntiles, P<int32_t>( s->nbr ), code, sv, red, dsel, rz_prev, max_inner, target,
+                if( bora_launch_pcg_persistent( ft, code, sv, red, dsel, rz_prev, max_inner, target,
                                                 s_a_rz, s_a_dq, P<uint32_t>( s->counters ) + 8,
                                                 P<unsigned>( s->gbar ), P<double>( s->partials ),
                                                 s->fault == BORA_FAULT_BARRIER, st ) != 0 )
@@ -757,7 +785,7 @@ int stage_solve( bora_flip_sim* s )
         else
         {
             KTimer t( s, BORA_KERNEL_PCG_UPDATE, 1 );
-            bora_launch_pcg_update( s->ntiles, code, sv, red, -1, -1, st );
+            bora_launch_pcg_update( ft, sv, red, -1, -1, st );
         }
         // Convergence checks do not stall the device: the direction kernel of iteration i + 1
         // finishes iteration i's r.r and also writes it to mapped host memory, where the host
@@ -772,7 +800,7 @@ int stage_solve( bora_flip_sim* s )
             if( chk_slot >= 0 ) arm_mirror( s, chk_slot );
             {
                 KTimer t( s, BORA_KERNEL_PCG_DIRECTION, 1 );
-                bora_launch_pcg_direction( s->g, s->ntiles, s->tiles(), code, sv, dsel, red, nparts, rz_cur, rr_cur, rz_prev,
+                bora_launch_pcg_direction( ft, code, sv, dsel, red, nparts, rz_cur, rr_cur, rz_prev,
                                            a_rz, a_dq, chk_slot >= 0, st );
             }
             dsel ^= 1;
@@ -784,7 +812,7 @@ int stage_solve( bora_flip_sim* s )
             else
             {
                 KTimer t( s, BORA_KERNEL_PCG_UPDATE, 1 );
-                bora_launch_pcg_update( s->ntiles, code, sv, red, rz_cur, s_dq, st );
+                bora_launch_pcg_update( ft, sv, red, rz_cur, s_dq, st );
             }
             a_rz = rz_cur;
             a_dq = s_dq;
@@ -808,17 +836,19 @@ int stage_solve( bora_flip_sim* s )
         total_it += it;
         ++passes;
         const int s_n2 = s->slot(), s_mx = s->slot();
+        arm_mirror( s, s_n2 );
+        arm_mirror( s, s_mx );
         {
             KTimer t( s, BORA_KERNEL_REFINE, 2 );
-            bora_launch_refine_accumulate( s->ntiles, code, sv, dsel, red, nparts, rr_cur, a_rz, a_dq, st );
-            bora_launch_refine_residual( s->g, s->ntiles, s->tiles(), b, code, sv, red, s_n2, s_mx, st );
+            bora_launch_refine_accumulate( ft, code, sv, dsel, red, nparts, rr_cur, a_rz, a_dq, st );
+            bora_launch_refine_residual( ft, b, code, sv, red, s_n2, s_mx, st );
         }
         BORA_TRYS( check_launch( s ) );
-        rnorm = std::sqrt( read_ring( s, s_n2, &status ) );
+        double n2 = 0.0;
+        BORA_TRYS( poll_mirror( s, s_n2, st, &n2 ) );
+        BORA_TRYS( poll_mirror( s, s_mx, st, &rmax ) );
+        rnorm = std::sqrt( n2 );
         scale_slot = s_n2;
-        BORA_TRYS( status );
-        rmax = read_ring( s, s_mx, &status );
-        BORA_TRYS( status );
         if( !std::isfinite( rnorm ) ) break;
         // Continue the recurrence only while the refined residual still agrees with the
         // recursive one (the device finished the pass, so its last r.r is in mapped memory);
@@ -1022,7 +1052,7 @@ void for_each_buffer( bora_flip_sim* s, F&& f )
     DevBuf* all[] = { &s->tile_flag, &s->tile_act, &s->tile_excl, &s->slot_of, &s->tile_of, &s->nbr, &s->mass, &s->surf,
                       &s->pres, &s->vx, &s->vy, &s->vz, &s->cx, &s->cy, &s->cz, &s->flag, &s->code, &s->rhs, &s->sx,
                       &s->se, &s->sr, &s->sd0, &s->sd1, &s->sq, &s->sz, &s->sminv, &s->cell_count, &s->cell_start,
-                      &s->ring, &s->partials, &s->done, &s->sums, &s->adj, &s->vkey, &s->key, &s->idx, &s->scan_scratch,
+                      &s->ring, &s->partials, &s->done, &s->sums, &s->tile_fluid, &s->solve_tab, &s->adj, &s->vkey, &s->key, &s->idx, &s->scan_scratch,
                       &s->counters, &s->stage_in, &s->stage_out, &s->live_flag, &s->col_phi, &s->col_vel,
                       &s->col_tslot, &s->col_tnear, &s->col_tphi, &s->col_tvel, &s->gbar };
     for( DevBuf* b : all ) f( *b );
@@ -1114,8 +1144,6 @@ int bora_flip_create( const bora_grid_desc* grid, const bora_flip_params* params
     if( st == BORA_OK ) st = cuda_status( cudaEventCreateWithFlags( &s->ev_join, cudaEventDisableTiming ) );
     if( st == BORA_OK ) st = cuda_status( cudaHostAlloc( (void**)&s->h_cnt, 64, cudaHostAllocMapped ) );
     if( st == BORA_OK ) st = cuda_status( cudaHostGetDevicePointer( (void**)&s->d_cnt, s->h_cnt, 0 ) );
-    if( st == BORA_OK ) st = cuda_status( cudaHostAlloc( (void**)&s->h_ring, 64, cudaHostAllocMapped ) );
-    if( st == BORA_OK ) st = cuda_status( cudaHostGetDevicePointer( (void**)&s->d_hring, s->h_ring, 0 ) );
     if( st == BORA_OK ) st = cuda_status( cudaHostAlloc( (void**)&s->h_mirror, BORA_RING * 8, cudaHostAllocMapped ) );
     if( st == BORA_OK ) st = cuda_status( cudaHostGetDevicePointer( (void**)&s->d_mirror, s->h_mirror, 0 ) );
     if( st == BORA_OK ) st = cuda_status( grow( s->tile_flag, s->ntv, false, s->st ) );
@@ -1157,7 +1185,6 @@ int bora_flip_destroy( bora_flip_handle s )
         if( s->ev_step[q] ) cudaEventDestroy( s->ev_step[q] );
     if( s->ev_join ) cudaEventDestroy( s->ev_join );
     if( s->h_cnt ) cudaFreeHost( s->h_cnt );
-    if( s->h_ring ) cudaFreeHost( s->h_ring );
     if( s->h_mirror ) cudaFreeHost( s->h_mirror );
     if( s->st ) cudaStreamDestroy( s->st );
     delete s;
@@ -1471,7 +1498,11 @@ int batch_solve( std::vector<BatchMember>& M, cudaStream_t st, BatchBuffers& bb 
     // the launch shapes of the multigrid passes for this batch (the autotuner's choice for
     // the batch's total size; every shape gives the same results)
     int total_tiles = 0;
-    for( int k = 0; k < n; ++k ) total_tiles += M[k].s->ntiles;
+    for( int k = 0; k < n; ++k )
+    {
+        BORA_TRYS( wait_solve_tiles( M[k].s ) );
+        total_tiles += M[k].s->nft;
+    }
     const int tgroup[3] = { kBoraTuneL0Batch, kBoraTuneL1Batch, kBoraTuneL2Batch };
     BoraTunePick tpick[3];
     int tv[3];
@@ -1485,7 +1516,7 @@ int batch_solve( std::vector<BatchMember>& M, cudaStream_t st, BatchBuffers& bb 
         bora_flip_sim* s = M[k].s;
         BoraMemberSolve& m = ms[k];
         m.ntiles = s->ntiles;
-        m.nbr = P<int32_t>( s->nbr );
+        m.ft = s->solve_tiles();
         m.code = P<uint16_t>( s->code );
         m.b = P<float>( s->rhs );
         m.pres = P<float>( s->pres );
@@ -1493,7 +1524,7 @@ int batch_solve( std::vector<BatchMember>& M, cudaStream_t st, BatchBuffers& bb 
         m.red = s->reducer();
         for( int l = 0; l < 4; ++l ) m.L[l] = s->levels[l];
         m.z3 = s->levels[3].z0;
-        bora_member_grids( s->ntiles, m.grid, tv );
+        bora_member_grids( s->nft, m.grid, tv );
         size_t sm = 0;
         int c = 0;
         if( !bora_mg_mid_describe( s->g, s->levels, s->nlevels, s->tiles(), s->ntiles, s->mg_mid.p,
@@ -2254,6 +2285,7 @@ int bora_flip_set_field( bora_flip_handle s, int which, const void* in, size_t b
     BORA_TRYS( field_bufs( s, which, b, &nc, &es ) );
     const size_t ncell = (size_t)s->ntiles * BORA_TILE_CELLS;
     if( bytes < ncell * nc * es ) return BORA_ERR_CAPACITY;
+    if( which == BORA_FIELD_CODE ) s->solve_tiles_valid = false;  // the solve looks at the codes themselves
     if( nc == 1 )
     {
         BORA_TRY( cudaMemcpyAsync( b[0]->p, in, ncell * es, cudaMemcpyHostToDevice, s->st ) );

@@ -254,8 +254,7 @@ __device__ __forceinline__ void row_sums( const F& f, const int* nf, int lane, c
 
 struct Pass0Args
 {
-    int ntiles;
-    const int32_t* nbr;
+    BoraSolveTilesDev ft;
     BoraLevelDev F;       // level 0
     BoraLevelDev C;       // level 1 (down 2 writes its r; up 1 reads its z1)
     float* r0;            // the PCG residual (down 2 stores its update)
@@ -278,21 +277,27 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
     init_weights( w );
     const int lane = threadIdx.x & 31, j = lane & 7, kq = lane >> 3;
     const int stride = (int)G * W;
-    // what no kernel of the solve writes - the tile's face neighbours and the rows' codes - is
-    // read a tile ahead, the first tile's before the dependency wait
-    int nfn[6] = { -1, -1, -1, -1, -1, -1 };
+    // what no kernel of the solve writes is read ahead, the first tile's before the dependency
+    // wait: the rows' codes a tile ahead, the tile table (which says where they are) two
+    int4 n0 = make_int4( -1, -1, -1, -1 ), n1 = n0;  // table entry of the tile after the next fetch
     uint4 cwA = make_uint4( 0u, 0u, 0u, 0u ), cwB = cwA;
-    auto fetch = [&]( int t ) {
-        if( t >= a.ntiles ) return;
-        const int32_t* __restrict__ nb = a.nbr + (size_t)t * 27;
-        nfn[0] = nb[bora_dir( -1, 0, 0 )]; nfn[1] = nb[bora_dir( 1, 0, 0 )];
-        nfn[2] = nb[bora_dir( 0, -1, 0 )]; nfn[3] = nb[bora_dir( 0, 1, 0 )];
-        nfn[4] = nb[bora_dir( 0, 0, -1 )]; nfn[5] = nb[bora_dir( 0, 0, 1 )];
-        cwA = *reinterpret_cast<const uint4*>( a.F.code + (size_t)t * 512 + 8 * lane );
-        cwB = *reinterpret_cast<const uint4*>( a.F.code + (size_t)t * 512 + 256 + 8 * lane );
+    int nfn[6] = { -1, -1, -1, -1, -1, -1 }, sn = 0;
+    auto entry = [&]( int t ) {
+        if( t >= a.ft.n ) return;
+        n0 = __ldg( a.ft.tab + 2 * (size_t)t );
+        n1 = __ldg( a.ft.tab + 2 * (size_t)t + 1 );
     };
-    int s = (int)bid * W + ( threadIdx.x >> 5 );
-    fetch( s );
+    auto fetch = [&]( int t ) {  // from the entry read before; reads the one after
+        if( t >= a.ft.n ) return;
+        nfn[0] = n0.x; nfn[1] = n0.y; nfn[2] = n0.z; nfn[3] = n0.w; nfn[4] = n1.x; nfn[5] = n1.y;
+        sn = n1.z;
+        cwA = *reinterpret_cast<const uint4*>( a.F.code + (size_t)sn * 512 + 8 * lane );
+        cwB = *reinterpret_cast<const uint4*>( a.F.code + (size_t)sn * 512 + 256 + 8 * lane );
+        entry( t + stride );
+    };
+    int t = (int)bid * W + ( threadIdx.x >> 5 );
+    entry( t );
+    fetch( t );
     __shared__ float2 s_dq[W];
     bora_pdl_wait();  // the previous kernel's results are complete from here
     if( threadIdx.x == 0 ) s_sc = scale_from( a.red.ring, a.slot_rr );
@@ -308,8 +313,9 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
     __syncthreads();
     const float sc = s_sc;
     DF acc{ 0.f, 0.f };  // down 1: r.r of the updated residual; up 2: r.z
-    for( ; s < a.ntiles; s += stride )
+    for( ; t < a.ft.n; t += stride )
     {
+        const int s = sn;
         int nf[6];
 #pragma unroll
         for( int q = 0; q < 6; ++q ) nf[q] = nfn[q];
@@ -324,7 +330,7 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
                 cB[2 * i] = (uint16_t)( wb[i] & 0xffffu ); cB[2 * i + 1] = (uint16_t)( wb[i] >> 16 );
             }
         }
-        fetch( s + stride );
+        fetch( t + stride );
         float rA[8], rB[8];  // r' on fluid cells
         f32x8( a.r0, gA, rA );
         f32x8( a.r0, gB, rB );
@@ -347,10 +353,10 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
         }
         if constexpr( P == 0 )
         {
-            float t = 0.f;
+            float p = 0.f;
 #pragma unroll
-            for( int i = 0; i < 8; ++i ) { t = fmaf( rA[i], rA[i], t ); t = fmaf( rB[i], rB[i], t ); }
-            acc = df_add_f( acc, t );
+            for( int i = 0; i < 8; ++i ) { p = fmaf( rA[i], rA[i], p ); p = fmaf( rB[i], rB[i], p ); }
+            acc = df_add_f( acc, p );
         }
 #pragma unroll
         for( int i = 0; i < 8; ++i )
@@ -470,8 +476,7 @@ __global__ void __launch_bounds__( 32 * W, 16 / W ) k_mg_pass0_batch( const __gr
     const BoraMemberSolve& m = L.ms[k];
     const BoraMemberSlots& q = L.sl[k];
     Pass0Args a;
-    a.ntiles = m.ntiles;
-    a.nbr = m.nbr;
+    a.ft = m.ft;
     a.F = m.L[0];
     a.C = m.L[1];
     a.r0 = m.sv.r;
@@ -490,8 +495,7 @@ __global__ void __launch_bounds__( 32 * W, 16 / W ) k_mg_pass0_batch( const __gr
 
 struct PassFArgs
 {
-    int ntiles;
-    const int32_t* nbr;
+    BoraSolveTilesDev ft;
     BoraLevelDev F;     // this level (E = 4 or 2)
     BoraLevelDev C;     // the coarser one (down 2 writes its r)
     const __half* ec;   // up 1: the coarser level's correction
@@ -511,10 +515,11 @@ __device__ __forceinline__ void passf_body( const PassFArgs& a, unsigned bid )
     __shared__ float res[T];
     bora_pdl_trigger();
     init_weights( w );
-    const size_t ncells = (size_t)a.ntiles * E3;
-    const size_t base = (size_t)bid * T, g = base + threadIdx.x;
-    const bool live = g < ncells;
+    // cell i of the solver's tiles: cell g of the level
+    const size_t base = (size_t)bid * T, i = base + threadIdx.x;
+    const bool live = i < (size_t)a.ft.n * E3;
     const BoraLevelDev& F = a.F;
+    size_t g = 0;
     int s = 0, x = 0, y = 0, z = 0;
     uint16_t cc = 0;
     int64_t gn[6];     // neighbour cells -x +x -y +y -z +z (-1: none)
@@ -522,11 +527,13 @@ __device__ __forceinline__ void passf_body( const PassFArgs& a, unsigned bid )
     int pn[6];         // up 1: the neighbours' parents on the coarser level
     if( live )
     {
-        s = (int)( g / E3 );
-        const int l = (int)( g % E3 );
+        const int l = (int)( i % E3 );
+        const int4 n0 = __ldg( a.ft.tab + 2 * ( i / E3 ) ), n1 = __ldg( a.ft.tab + 2 * ( i / E3 ) + 1 );
+        const int nf[6] = { n0.x, n0.y, n0.z, n0.w, n1.x, n1.y };
+        s = n1.z;
+        g = (size_t)s * E3 + l;
         x = l % E; y = ( l / E ) % E; z = l / ( E * E );
         cc = F.code[g];
-        const int32_t* __restrict__ nb = a.nbr + (size_t)s * 27;
 #pragma unroll
         for( int q = 0; q < 6; ++q )
         {
@@ -535,7 +542,7 @@ __device__ __forceinline__ void passf_body( const PassFArgs& a, unsigned bid )
             int xx = x + dx, yy = y + dy, zz = z + dz, t = s;
             if( xx < 0 || xx >= E || yy < 0 || yy >= E || zz < 0 || zz >= E )
             {
-                t = nb[bora_dir( dx, dy, dz )];
+                t = nf[q];
                 xx &= E - 1; yy &= E - 1; zz &= E - 1;
             }
             gn[q] = t < 0 ? -1 : (int64_t)t * E3 + xx + E * ( yy + E * zz );
@@ -578,9 +585,9 @@ __device__ __forceinline__ void passf_body( const PassFArgs& a, unsigned bid )
         if( threadIdx.x < kParents )
         {
             const int p = threadIdx.x, tl = p / H3, pl = p % H3;
-            const size_t tile = base / E3 + tl;
-            if( tile < (size_t)a.ntiles )
+            if( base / E3 + tl < (size_t)a.ft.n )
             {
+                const size_t tile = (size_t)__ldg( &a.ft.tab[2 * ( base / E3 + tl ) + 1].z );
                 const int pa = pl % H, pb = ( pl / H ) % H, pc = pl / ( H * H );
                 const int l = tl * E3 + 2 * pa + E * ( 2 * pb + E * 2 * pc );
                 const float sum = ( ( res[l] + res[l + 1] ) + ( res[l + E] + res[l + E + 1] ) ) +
@@ -605,8 +612,7 @@ __global__ void __launch_bounds__( T ) k_mg_passf_batch( const __grid_constant__
     const int k = bora_batch_member( L, blockIdx.x, &bid );
     const BoraMemberSolve& m = L.ms[k];
     PassFArgs a;
-    a.ntiles = m.ntiles;
-    a.nbr = m.nbr;
+    a.ft = m.ft;
     a.F = m.L[l];
     a.C = m.L[l + 1];
     a.ec = l == 1 ? m.L[2].z1 : m.z3;
@@ -628,7 +634,7 @@ int num_sms_pass()
 template <int E, int P>
 void launch_passf( const PassFArgs& a, int v, cudaStream_t st )
 {
-    const int g = bora_mg_pass_grid( E, a.ntiles, v );
+    const int g = bora_mg_pass_grid( E, a.ft.n, v );
     if( g <= 0 ) return;
     switch( v )
     {
@@ -642,7 +648,7 @@ void launch_passf( const PassFArgs& a, int v, cudaStream_t st )
 template <int P>
 void launch_pass0( const Pass0Args& a, int v, cudaStream_t st )
 {
-    const int g = bora_mg_pass_grid( 8, a.ntiles, v );
+    const int g = bora_mg_pass_grid( 8, a.ft.n, v );
     if( g <= 0 ) return;
     switch( v )
     {
@@ -674,51 +680,51 @@ int bora_mg_pass_grid( int E, int ntiles, int v )
     return (int)( ( n + T - 1 ) / T );
 }
 
-void bora_mg_pass_down( const BoraLevelDev* levels, int l, const BoraTilesDev& t, int ntiles, float* r0, const float* q,
+void bora_mg_pass_down( const BoraLevelDev* levels, int l, const BoraSolveTilesDev& t, float* r0, const float* q,
                         float* scratch, const BoraReduceDev& red, int slot_rr, int slot_rz_in, int slot_dq_in,
                         cudaStream_t st )
 {
     const int group = l == 0 ? kBoraTuneL0 : ( l == 1 ? kBoraTuneL1 : kBoraTuneL2 );
-    const BoraTunePick pick = bora_tune_pick( group, ntiles );
-    BoraTuneTimer timer( pick, group, ntiles, st );  // times the level's two down passes
+    const BoraTunePick pick = bora_tune_pick( group, t.n );
+    BoraTuneTimer timer( pick, group, t.n, st );  // times the level's two down passes
     const int v = pick.variant;
     if( levels[l].E == 8 )
     {
         Pass0Args a{};
-        a.ntiles = ntiles; a.nbr = t.nbr; a.F = levels[0]; a.C = levels[1]; a.r0 = r0; a.q = q; a.scratch = scratch;
+        a.ft = t; a.F = levels[0]; a.C = levels[1]; a.r0 = r0; a.q = q; a.scratch = scratch;
         a.red = red; a.slot_rr = slot_rr;
-        a.slot_rz_in = slot_rz_in; a.slot_dq_in = slot_dq_in; a.ndq = bora_pcg_direction_grid( ntiles );
+        a.slot_rz_in = slot_rz_in; a.slot_dq_in = slot_dq_in; a.ndq = bora_pcg_direction_grid( t.n );
         // down 1 sums r.r over its blocks: the fixed shape
-        const int g = bora_mg_pass_grid( 8, ntiles, -1 );
+        const int g = bora_mg_pass_grid( 8, t.n, -1 );
         if( g > 0 ) bora_launch_pdl( k_mg_pass0<kReduceWarps, 0>, dim3( g ), dim3( 32 * kReduceWarps ), 0, st, a );
         launch_pass0<1>( a, v, st );
         return;
     }
     PassFArgs a{};
-    a.ntiles = ntiles; a.nbr = t.nbr; a.F = levels[l]; a.C = levels[l + 1]; a.scratch = scratch;
+    a.ft = t; a.F = levels[l]; a.C = levels[l + 1]; a.scratch = scratch;
     if( levels[l].E == 4 ) { launch_passf<4, 0>( a, v, st ); launch_passf<4, 1>( a, v, st ); }
     else { launch_passf<2, 0>( a, v, st ); launch_passf<2, 1>( a, v, st ); }
 }
 
-void bora_mg_pass_up( const BoraLevelDev* levels, int l, const __half* ec, const BoraTilesDev& t, int ntiles,
-                      const float* r0, float* scratch, const BoraReduceDev& red, int slot_rr, float* z, cudaStream_t st )
+void bora_mg_pass_up( const BoraLevelDev* levels, int l, const __half* ec, const BoraSolveTilesDev& t, const float* r0,
+                      float* scratch, const BoraReduceDev& red, int slot_rr, float* z, cudaStream_t st )
 {
     const int group = l == 0 ? kBoraTuneL0 : ( l == 1 ? kBoraTuneL1 : kBoraTuneL2 );
-    const int v = bora_tune_pick( group, ntiles ).variant;
+    const int v = bora_tune_pick( group, t.n ).variant;
     if( levels[l].E == 8 )
     {
         Pass0Args a{};
-        a.ntiles = ntiles; a.nbr = t.nbr; a.F = levels[0]; a.C = levels[1]; a.C.z1 = const_cast<__half*>( ec );
+        a.ft = t; a.F = levels[0]; a.C = levels[1]; a.C.z1 = const_cast<__half*>( ec );
         a.r0 = const_cast<float*>( r0 ); a.scratch = scratch; a.zout = z; a.red = red; a.slot_rr = slot_rr;
         a.slot_rz_in = -1; a.slot_dq_in = -1;
         launch_pass0<2>( a, v, st );
         // r.z: the fixed shape
-        const int g = bora_mg_pass_grid( 8, ntiles, -1 );
+        const int g = bora_mg_pass_grid( 8, t.n, -1 );
         if( g > 0 ) bora_launch_pdl( k_mg_pass0<kReduceWarps, 3>, dim3( g ), dim3( 32 * kReduceWarps ), 0, st, a );
         return;
     }
     PassFArgs a{};
-    a.ntiles = ntiles; a.nbr = t.nbr; a.F = levels[l]; a.C = levels[l + 1]; a.ec = ec; a.scratch = scratch;
+    a.ft = t; a.F = levels[l]; a.C = levels[l + 1]; a.ec = ec; a.scratch = scratch;
     if( levels[l].E == 4 ) { launch_passf<4, 2>( a, v, st ); launch_passf<4, 3>( a, v, st ); }
     else { launch_passf<2, 2>( a, v, st ); launch_passf<2, 3>( a, v, st ); }
 }

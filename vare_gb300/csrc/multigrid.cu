@@ -709,8 +709,8 @@ int bora_mg_vcycle_launches( const BoraGridDev& g, const BoraLevelDev* levels, i
     return n;
 }
 
-void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t, const void* mid_image,
-                     float* r, const float* q, float* z, float* scratch, BoraReduceDev red, int slot_rz_in,
+void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t, BoraSolveTilesDev ft,
+                     const void* mid_image, float* r, const float* q, float* z, float* scratch, BoraReduceDev red, int slot_rz_in,
                      int slot_dq_in, int slot_scale, int coarse_sweeps, cudaStream_t st )
 {
     if( nlevels < 2 ) return;  // the caller always builds at least two levels
@@ -729,7 +729,7 @@ void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nleve
         const BoraLevelDev& C = levels[l + 1];
         if( pass_level( F ) )
         {
-            bora_mg_pass_down( levels, l, t, ntiles, r, q, scratch, red, slot_scale, slot_rz_in, slot_dq_in, st );
+            bora_mg_pass_down( levels, l, ft, r, q, scratch, red, slot_scale, slot_rz_in, slot_dq_in, st );
             continue;
         }
         with_nav( g, levels, nlevels, l, t, [&]( auto nav ) {
@@ -791,7 +791,7 @@ void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nleve
             // a coarser level that ran its passes left its correction in z1, the others in z0
             const bool cf = l + 1 < stop && pass_level( levels[l + 1] );
             const __half* ec = cf ? levels[l + 1].z1 : levels[l + 1].z0;
-            bora_mg_pass_up( levels, l, ec, t, ntiles, r, scratch, red, slot_scale, z, st );
+            bora_mg_pass_up( levels, l, ec, ft, r, scratch, red, slot_scale, z, st );
             continue;
         }
         with_nav( g, levels, nlevels, l, t, [&]( auto nav ) {
@@ -801,11 +801,11 @@ void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nleve
     }
 }
 
-void bora_member_grids( int ntiles, int* grid, const int* v )
+void bora_member_grids( int nft, int* grid, const int* v )
 {
-    bora_projection_grids( ntiles, grid );
-    grid[kGridPass0] = bora_mg_pass_grid( 8, ntiles, v[0] );
-    grid[kGridPass0R] = bora_mg_pass_grid( 8, ntiles, -1 );
-    grid[kGridPass1] = bora_mg_pass_grid( 4, ntiles, v[1] );
-    grid[kGridPass2] = bora_mg_pass_grid( 2, ntiles, v[2] );
+    bora_projection_grids( nft, grid );
+    grid[kGridPass0] = bora_mg_pass_grid( 8, nft, v[0] );
+    grid[kGridPass0R] = bora_mg_pass_grid( 8, nft, -1 );
+    grid[kGridPass1] = bora_mg_pass_grid( 4, nft, v[1] );
+    grid[kGridPass2] = bora_mg_pass_grid( 2, nft, v[2] );
 }

@@ -53,7 +53,8 @@ __device__ inline float absr( float x ) { return x < 0.f ? -x : x; }  // MathUti
 
 // ---------------------------------------------------------------------------------
 // Right-hand side and stencil code (FluidProjection.cu:203-266).
-__global__ void __launch_bounds__( 512 ) k_rhs( BoraGridDev g, BoraTilesDev t, BoraCellsDev c, uint32_t* nfluid )
+__global__ void __launch_bounds__( 512 ) k_rhs( BoraGridDev g, BoraTilesDev t, BoraCellsDev c, uint32_t* nfluid,
+                                                 uint8_t* __restrict__ tile_fluid )
 {
     using HL = Halo<1>;
     __shared__ int32_t nb[27];
@@ -80,6 +81,8 @@ __global__ void __launch_bounds__( 512 ) k_rhs( BoraGridDev g, BoraTilesDev t, B
     const bool fluid = sf[h] == BORA_FLUID;
     const unsigned fl = __ballot_sync( 0xffffffffu, fluid );  // unknowns of the system, counted per warp
     if( ( threadIdx.x & 31 ) == 0 && fl ) atomicAdd( nfluid, (uint32_t)__popc( fl ) );
+    const int any = __syncthreads_or( fluid );
+    if( threadIdx.x == 0 ) tile_fluid[s] = any ? 1 : 0;
     if( !fluid )
     {
         c.b[cell] = 0.f;
@@ -122,6 +125,93 @@ __global__ void __launch_bounds__( 512 ) k_rhs( BoraGridDev g, BoraTilesDev t, B
     c.b[cell] = d;
     c.code[cell] = (uint16_t)( BORA_CODE_FLUID | ( (uint32_t)diag << 8 ) | mask );
 }
+
+// ---------------------------------------------------------------------------------
+// The solver's tiles (BoraSolveTilesDev): flags -> table.
+__global__ void k_tile_fluid( int ntiles, const uint16_t* __restrict__ code, uint8_t* __restrict__ tile_fluid )
+{
+    for( int s = blockIdx.x * (int)( blockDim.x >> 5 ) + ( threadIdx.x >> 5 ); s < ntiles; s += gridDim.x * (int)( blockDim.x >> 5 ) )
+    {
+        bool any = false;
+        for( int l = threadIdx.x & 31; l < 512; l += 32 ) any = any || ( code[(size_t)s * 512 + l] & BORA_CODE_FLUID );
+        any = __any_sync( 0xffffffffu, any );
+        if( ( threadIdx.x & 31 ) == 0 ) tile_fluid[s] = any ? 1 : 0;
+    }
+}
+
+// One CTA: the slots of the flagged tiles, in order, into the own entries of the table, 16 flags
+// per thread and round (a few microseconds for 50 K tiles), and their number.
+__global__ void __launch_bounds__( 1024 ) k_solve_tiles( int ntiles, const uint8_t* __restrict__ tile_fluid, int32_t* __restrict__ tab,
+                                                         uint32_t* count, uint32_t* host_count )
+{
+    __shared__ int wsum[32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int carry = 0;
+    for( int base = 0; base < ntiles; base += 16 * 1024 )
+    {
+        const int s0 = base + 16 * (int)threadIdx.x;
+        uint32_t w[4] = { 0u, 0u, 0u, 0u };
+        if( s0 < ntiles )  // the flags are padded to a multiple of 16
+        {
+            const uint4 f = *reinterpret_cast<const uint4*>( tile_fluid + s0 );
+            w[0] = f.x; w[1] = f.y; w[2] = f.z; w[3] = f.w;
+#pragma unroll
+            for( int q = 0; q < 4; ++q )
+                for( int b = 0; b < 4; ++b )
+                    if( s0 + 4 * q + b >= ntiles ) w[q] &= ~( 0xffu << ( 8 * b ) );
+        }
+        const int mine = __popc( w[0] ) + __popc( w[1] ) + __popc( w[2] ) + __popc( w[3] );  // flags are 0 or 1
+        int inc = mine;
+#pragma unroll
+        for( int o = 1; o < 32; o <<= 1 )
+        {
+            const int y = __shfl_up_sync( 0xffffffffu, inc, o );
+            if( lane >= o ) inc += y;
+        }
+        if( lane == 31 ) wsum[wid] = inc;
+        __syncthreads();
+        if( wid == 0 )
+        {
+            int v = wsum[lane];
+#pragma unroll
+            for( int o = 1; o < 32; o <<= 1 )
+            {
+                const int y = __shfl_up_sync( 0xffffffffu, v, o );
+                if( lane >= o ) v += y;
+            }
+            wsum[lane] = v;
+        }
+        __syncthreads();
+        int out = carry + inc - mine + ( wid ? wsum[wid - 1] : 0 );
+        for( int b = 0; b < 16; ++b )
+            if( ( w[b >> 2] >> ( 8 * ( b & 3 ) ) ) & 1u ) tab[8 * (size_t)out++ + 6] = s0 + b;
+        carry += wsum[31];
+        __syncthreads();  // wsum is rewritten next
+    }
+    if( threadIdx.x == 0 )
+    {
+        *count = (uint32_t)carry;
+        *(volatile uint32_t*)host_count = (uint32_t)carry;
+    }
+}
+
+// The face neighbours of the solver's tiles (-1: not a solver tile), eight threads per tile.
+__global__ void k_solve_nbrs( const uint32_t* __restrict__ count, const int32_t* __restrict__ nbr,
+                              const uint8_t* __restrict__ tile_fluid, int32_t* __restrict__ tab )
+{
+    const size_t total = (size_t)*count * 8;
+    for( size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < total; q += (size_t)gridDim.x * blockDim.x )
+    {
+        const int f = (int)( q & 7 );
+        if( f == 7 ) tab[q] = 0;
+        if( f >= 6 ) continue;
+        const int sg = ( f & 1 ) ? 1 : -1;
+        const int ns = nbr[(size_t)tab[( q & ~(size_t)7 ) + 6] * 27 + bora_dir( f < 2 ? sg : 0, f == 2 || f == 3 ? sg : 0, f >= 4 ? sg : 0 )];
+        tab[q] = ns >= 0 && tile_fluid[ns] ? ns : -1;
+    }
+}
+
+__device__ __forceinline__ int solve_slot( const int4* tab, int t ) { return __ldg( &tab[2 * (size_t)t + 1].z ); }
 
 // ---------------------------------------------------------------------------------
 // Wavefront tables of an 8^3 tile: cells ordered by plane i+j+k (0..21). Kept in global
@@ -186,7 +276,8 @@ __device__ inline int code_diag( uint16_t c ) { return ( c >> 8 ) & 15; }
 // rotated (mic_sweeps). One warp per tile, persistent over tiles.
 constexpr int kTilesPerCta = 4;
 
-__global__ void __launch_bounds__( 32 * kTilesPerCta ) k_mic_factor( int ntiles, const uint16_t* __restrict__ code,
+__global__ void __launch_bounds__( 32 * kTilesPerCta ) k_mic_factor( BoraSolveTilesDev ft,
+                                                                     const uint16_t* __restrict__ code,
                                                                      float* __restrict__ minv )
 {
     __shared__ float sm[kTilesPerCta][512];
@@ -196,9 +287,10 @@ __global__ void __launch_bounds__( 32 * kTilesPerCta ) k_mic_factor( int ntiles,
     __syncthreads();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float tau = 0.97f;
-    for( int s = blockIdx.x * kTilesPerCta + w; s < ntiles; s += gridDim.x * kTilesPerCta )
+    const int nft = (int)*ft.count;
+    for( int t = blockIdx.x * kTilesPerCta + w; t < nft; t += gridDim.x * kTilesPerCta )
     {
-        const size_t base = (size_t)s * 512;
+        const size_t base = (size_t)solve_slot( ft.tab, t ) * 512;
         for( int l = lane; l < 512; l += 32 ) { sc[w][l] = code[base + l]; sm[w][l] = 0.f; }
         __syncwarp();
         for( int p = 0; p <= 21; ++p )
@@ -351,9 +443,11 @@ __device__ __forceinline__ float mic_sweeps( float* rA, float* rB, const float* 
 // r.r accumulated into prz, prr. alpha_of() is called once, by every thread of the block, after
 // the first tile's loads have been issued.
 template <class AlphaOf>
-__device__ __forceinline__ void pcg_update_tiles( int ntiles, const BoraSolverDev& sv, AlphaOf alpha_of, int first, int tstride,
-                                                  DF& prz, DF& prr )
+__device__ __forceinline__ void pcg_update_tiles( const BoraSolveTilesDev& ft, const BoraSolverDev& sv, AlphaOf alpha_of, int first,
+                                                  int tstride, DF& prz, DF& prr )
 {
+    // the tiles' slots, read a tile ahead (no kernel of the chain writes the table)
+    int next = first < ft.n ? solve_slot( ft.tab, first ) : 0;
     const int lane = threadIdx.x & 31;
     const size_t row = 8 * (size_t)( ( lane & 7 ) + 16 * ( lane >> 3 ) );  // row A; row B follows 64 cells on
     float rA[8], rB[8], qA[8], qB[8], mA[8], mB[8];
@@ -362,12 +456,15 @@ __device__ __forceinline__ void pcg_update_tiles( int ntiles, const BoraSolverDe
         bora_ld8( sv.r + o, rA ); bora_ld8( sv.r + o + 64, rB );
         bora_ld8( sv.q + o, qA ); bora_ld8( sv.q + o + 64, qB );
     };
-    if( first < ntiles ) load_tile( first );
+    bora_pdl_wait();  // the previous kernel's results are complete from here
+    if( first < ft.n ) load_tile( next );
     const float alpha = alpha_of();
-    for( int s = first; s < ntiles; s += tstride )
+    for( int t = first; t < ft.n; t += tstride )
     {
+        const int s = next;
         const size_t o = (size_t)s * 512 + row;
-        if( s != first ) load_tile( s );
+        if( t != first ) load_tile( s );
+        if( t + tstride < ft.n ) next = solve_slot( ft.tab, t + tstride );
         bora_ld8( sv.minv + o, mA );  // not with the first loads: the registers they take there cost more (spills)
         bora_ld8( sv.minv + o + 64, mB );
 #pragma unroll
@@ -390,12 +487,12 @@ __device__ __forceinline__ void pcg_update_tiles( int ntiles, const BoraSolverDe
     }
 }
 
-__global__ void __launch_bounds__( 32 * kUpdWarps, 4 ) k_pcg_update( int ntiles, BoraSolverDev sv, BoraReduceDev red,
-                                                                  int ndq, int slot_rz_in, int slot_dq_in )
+__global__ void __launch_bounds__( 32 * kUpdWarps, 4 ) k_pcg_update( BoraSolveTilesDev ft, BoraSolverDev sv,
+                                                                  BoraReduceDev red, int ndq, int slot_rz_in,
+                                                                  int slot_dq_in )
 {
     __shared__ float2 s_dq[kUpdWarps];
     bora_pdl_trigger();
-    bora_pdl_wait();  // the previous kernel's results are complete from here
     DF prz{ 0.f, 0.f }, prr{ 0.f, 0.f };
     auto alpha_of = [&]() -> float {
         if( slot_rz_in < 0 ) return 0.f;
@@ -403,28 +500,28 @@ __global__ void __launch_bounds__( 32 * kUpdWarps, 4 ) k_pcg_update( int ntiles,
         if( blockIdx.x == 0 && threadIdx.x == 0 ) ring_store( red, slot_dq_in, dq, false );
         return df_ratio( red.ringf[slot_rz_in], make_float2( dq.hi, dq.lo ) );
     };
-    pcg_update_tiles( ntiles, sv, alpha_of, blockIdx.x * kUpdWarps + ( threadIdx.x >> 5 ), gridDim.x * kUpdWarps, prz, prr );
+    pcg_update_tiles( ft, sv, alpha_of, blockIdx.x * kUpdWarps + ( threadIdx.x >> 5 ), gridDim.x * kUpdWarps, prz, prr );
     part_publish( prz, prr, red.part_rz, red.part_rr, blockIdx.x );
 }
 
-// Global index of the face neighbour of cell (slot s, local l) in direction q
-// (0:-x 1:+x 2:-y 3:+y 4:-z 5:+z), or SIZE_MAX when the neighbour tile is not active
+// Global index of the face neighbour of cell `cell` (solver tile t, local l) in direction q
+// (0:-x 1:+x 2:-y 3:+y 4:-z 5:+z), or SIZE_MAX when the neighbour tile is not a solver tile
 // (a stencil code that names a fluid neighbour there is inconsistent; callers record
 // it and skip the access).
-__device__ inline size_t face_nbr( const int32_t* __restrict__ nbr, size_t cell, int s, int l, int q )
+__device__ inline size_t face_nbr( const int4* __restrict__ tab, size_t cell, int t, int l, int q )
 {
     const int li = l & 7, lj = ( l >> 3 ) & 7, lk = l >> 6;
-    int dir, ll;
+    int ll;
     switch( q )
     {
-        case 0: if( li > 0 ) return cell - 1; dir = 12; ll = l + 7; break;
-        case 1: if( li < 7 ) return cell + 1; dir = 14; ll = l - 7; break;
-        case 2: if( lj > 0 ) return cell - 8; dir = 10; ll = l + 56; break;
-        case 3: if( lj < 7 ) return cell + 8; dir = 16; ll = l - 56; break;
-        case 4: if( lk > 0 ) return cell - 64; dir = 4; ll = l + 448; break;
-        default: if( lk < 7 ) return cell + 64; dir = 22; ll = l - 448; break;
+        case 0: if( li > 0 ) return cell - 1; ll = l + 7; break;
+        case 1: if( li < 7 ) return cell + 1; ll = l - 7; break;
+        case 2: if( lj > 0 ) return cell - 8; ll = l + 56; break;
+        case 3: if( lj < 7 ) return cell + 8; ll = l - 56; break;
+        case 4: if( lk > 0 ) return cell - 64; ll = l + 448; break;
+        default: if( lk < 7 ) return cell + 64; ll = l - 448; break;
     }
-    const int ns = nbr[(size_t)s * 27 + dir];
+    const int ns = __ldg( reinterpret_cast<const int*>( tab + 2 * (size_t)t ) + q );
     return ns < 0 ? (size_t)-1 : (size_t)ns * 512 + ll;
 }
 
@@ -449,9 +546,9 @@ constexpr int kDirWarps = 4;
 // once by every thread of the block after the first half tile's loads have been issued; upd_e:
 // that update is pending.
 template <class Coef>
-__device__ __forceinline__ DF pcg_direction_tiles( int ntiles, const int32_t* __restrict__ nbr,
-                                                   const uint16_t* __restrict__ code, const BoraSolverDev& sv, int dsel_in,
-                                                   Coef coef, bool upd_e, unsigned bid, unsigned G )
+__device__ __forceinline__ DF pcg_direction_tiles( const BoraSolveTilesDev& ft, const uint16_t* __restrict__ code,
+                                                   const BoraSolverDev& sv, int dsel_in, Coef coef, bool upd_e, unsigned bid,
+                                                   unsigned G )
 {
     const float* dold = dsel_in ? sv.d[1] : sv.d[0];  // selects keep sv out of local memory
     float* dnew = dsel_in ? sv.d[0] : sv.d[1];
@@ -460,14 +557,16 @@ __device__ __forceinline__ DF pcg_direction_tiles( int ntiles, const int32_t* __
     DF pdq{ 0.f, 0.f };
     float beta = 0.f, alpha = 0.f;
     float d[8], z[8];
-    const int nh = 2 * ntiles;
+    const int nh = 2 * ft.n;
     int h = (int)bid * kDirWarps + ( threadIdx.x >> 5 );
-    auto load_rows = [&]( int h ) {
-        const size_t g = (size_t)h * 256 + 8 * lane;
+    // a half tile's slot, read one ahead (no kernel of the chain writes the table)
+    int next = h < nh ? solve_slot( ft.tab, h >> 1 ) : 0;
+    auto load_rows = [&]( size_t g ) {
         bora_ld8( dold + g, d );
         bora_ld8( sv.z + g, z );
     };
-    if( h < nh ) load_rows( h );
+    bora_pdl_wait();  // the previous kernel's results (ring, partial sums, z, d, e) are complete from here
+    if( h < nh ) load_rows( (size_t)next * 512 + ( h & 1 ) * 256 + 8 * lane );
     {
         const float2 c = coef();
         beta = c.x;
@@ -475,14 +574,13 @@ __device__ __forceinline__ DF pcg_direction_tiles( int ntiles, const int32_t* __
     }
     for( bool head = true; h < nh; h += (int)G * kDirWarps, head = false )
     {
-        const int s = h >> 1, hi = h & 1;
-        const int32_t* __restrict__ nb = nbr + (size_t)s * 27;  // tile tables: not written by the solver chain
-        const int smx = nb[bora_dir( -1, 0, 0 )], spx = nb[bora_dir( 1, 0, 0 )];
-        const int smy = nb[bora_dir( 0, -1, 0 )], spy = nb[bora_dir( 0, 1, 0 )];
-        const int sz = nb[bora_dir( 0, 0, hi ? 1 : -1 )];
+        const int s = next, hi = h & 1;
         const int cA = hi * 256 + 8 * lane;
-        const size_t g = (size_t)h * 256 + 8 * lane;
-        if( !head ) load_rows( h );
+        const size_t g = (size_t)s * 512 + cA;
+        if( !head ) load_rows( g );
+        const int4 n0 = __ldg( ft.tab + 2 * (size_t)( h >> 1 ) ), n1 = __ldg( ft.tab + 2 * (size_t)( h >> 1 ) + 1 );
+        const int smx = n0.x, spx = n0.y, smy = n0.z, spy = n0.w, sz = hi ? n1.y : n1.x;
+        if( h + (int)G * kDirWarps < nh ) next = solve_slot( ft.tab, ( h + (int)G * kDirWarps ) >> 1 );
         const uint4 w = *reinterpret_cast<const uint4*>( code + g );
         float e[8];
         if( upd_e ) bora_ld8( sv.e + g, e );
@@ -539,15 +637,13 @@ __device__ __forceinline__ DF pcg_direction_tiles( int ntiles, const int32_t* __
     return pdq;
 }
 
-__device__ __forceinline__ void pcg_direction_body( int ntiles, const int32_t* __restrict__ nbr,
-                                                    const uint16_t* __restrict__ code, const BoraSolverDev& sv, int dsel_in,
-                                                    const BoraReduceDev& red, int nparts, int slot_rz_new, int slot_rr,
+__device__ __forceinline__ void pcg_direction_body( const BoraSolveTilesDev& ft, const uint16_t* __restrict__ code,
+                                                    const BoraSolverDev& sv, int dsel_in, const BoraReduceDev& red, int nparts, int slot_rz_new, int slot_rr,
                                                     int slot_rz_old, int slot_a_rz, int slot_a_dq, bool host_rr, unsigned bid,
                                                     unsigned G )
 {
     __shared__ float2 s_rz[kDirWarps], s_rr[kDirWarps];
     bora_pdl_trigger();
-    bora_pdl_wait();  // the previous kernel's results (ring, partial sums, z, d, e) are complete from here
     auto coef = [&]() -> float2 {
         const DF rz = part_collect( red.part_rz, nparts, s_rz );
         if( bid == G - 1 )  // the last block (never the one with more tiles) finishes rr for the host
@@ -562,17 +658,17 @@ __device__ __forceinline__ void pcg_direction_body( int ntiles, const int32_t* _
         return make_float2( slot_rz_old < 0 ? 0.f : df_ratio( make_float2( rz.hi, rz.lo ), red.ringf[slot_rz_old] ),
                             slot_a_rz < 0 ? 0.f : df_ratio( red.ringf[slot_a_rz], red.ringf[slot_a_dq] ) );
     };
-    const DF pdq = pcg_direction_tiles( ntiles, nbr, code, sv, dsel_in, coef, slot_a_rz >= 0, bid, G );
+    const DF pdq = pcg_direction_tiles( ft, code, sv, dsel_in, coef, slot_a_rz >= 0, bid, G );
     part_publish( pdq, DF{ 0.f, 0.f }, red.part_dq, nullptr, bid );
 }
 
-__global__ void __launch_bounds__( 32 * kDirWarps, 6 ) k_pcg_direction( int ntiles, const int32_t* __restrict__ nbr,
+__global__ void __launch_bounds__( 32 * kDirWarps, 6 ) k_pcg_direction( BoraSolveTilesDev ft,
                                                                     const uint16_t* __restrict__ code, BoraSolverDev sv,
                                                                     int dsel_in, BoraReduceDev red, int nparts,
                                                                     int slot_rz_new, int slot_rr, int slot_rz_old,
                                                                     int slot_a_rz, int slot_a_dq, bool host_rr )
 {
-    pcg_direction_body( ntiles, nbr, code, sv, dsel_in, red, nparts, slot_rz_new, slot_rr, slot_rz_old, slot_a_rz, slot_a_dq,
+    pcg_direction_body( ft, code, sv, dsel_in, red, nparts, slot_rz_new, slot_rr, slot_rz_old, slot_a_rz, slot_a_dq,
                         host_rr, blockIdx.x, gridDim.x );
 }
 
@@ -583,7 +679,7 @@ __global__ void __launch_bounds__( 32 * kDirWarps ) k_pcg_direction_batch( const
     const int k = bora_batch_member( L, blockIdx.x, &bid );
     const BoraMemberSolve& m = L.ms[k];
     const BoraMemberSlots& q = L.sl[k];
-    pcg_direction_body( m.ntiles, m.nbr, m.code, m.sv, q.dsel, m.red, m.grid[kGridPass0R], q.rz_new, q.rr_new, q.rz_old,
+    pcg_direction_body( m.ft, m.code, m.sv, q.dsel, m.red, m.grid[kGridPass0R], q.rz_new, q.rr_new, q.rz_old,
                         q.a_rz, q.a_dq, q.chk != 0, bid, (unsigned)m.grid[kGridDir] );
 }
 
@@ -601,8 +697,7 @@ __global__ void __launch_bounds__( 32 * kDirWarps ) k_pcg_direction_batch( const
 // then runs out of its own waits and returns too, and the host reports BORA_ERR_INTERNAL.
 struct PcgPersistArgs
 {
-    int ntiles;
-    const int32_t* nbr;
+    BoraSolveTilesDev ft;
     const uint16_t* code;
     BoraSolverDev sv;
     BoraReduceDev red;
@@ -701,7 +796,7 @@ __global__ void __launch_bounds__( 32 * kUpdWarps, 3 ) k_pcg_persistent( const _
     double rz_prev = a.slot_rz_prev >= 0 ? a.red.ring[a.slot_rz_prev] : -1.0;
     // the pass's first update: z = M^-1 r (alpha 0)
     DF prz{ 0.f, 0.f }, prr{ 0.f, 0.f };
-    pcg_update_tiles( a.ntiles, a.sv, [] { return 0.f; }, first, stride, prz, prr );
+    pcg_update_tiles( a.ft, a.sv, [] { return 0.f; }, first, stride, prz, prr );
     block_sum_store( df_warp_sum( prz ), pz );
     block_sum_store( df_warp_sum( prr ), pr );
     if( !grid_barrier( a ) ) return;
@@ -712,7 +807,7 @@ __global__ void __launch_bounds__( 32 * kUpdWarps, 3 ) k_pcg_persistent( const _
     {
         const float beta = rz_prev < 0.0 ? 0.f : (float)( rz / rz_prev );
         const float alpha_e = a_rz < 0.0 ? 0.f : (float)( a_rz / a_dq );
-        const DF pdq = pcg_direction_tiles( a.ntiles, a.nbr, a.code, a.sv, dsel, [=] { return make_float2( beta, alpha_e ); },
+        const DF pdq = pcg_direction_tiles( a.ft, a.code, a.sv, dsel, [=] { return make_float2( beta, alpha_e ); },
                                             a_rz >= 0.0, blockIdx.x, G );
         block_sum_store( df_warp_sum( pdq ), pd );
         if( !grid_barrier( a ) ) return;
@@ -721,7 +816,7 @@ __global__ void __launch_bounds__( 32 * kUpdWarps, 3 ) k_pcg_persistent( const _
         prz = DF{ 0.f, 0.f };
         prr = DF{ 0.f, 0.f };
         const float alpha = (float)( rz / dq );
-        pcg_update_tiles( a.ntiles, a.sv, [=] { return alpha; }, first, stride, prz, prr );
+        pcg_update_tiles( a.ft, a.sv, [=] { return alpha; }, first, stride, prz, prr );
         block_sum_store( df_warp_sum( prz ), pz );
         block_sum_store( df_warp_sum( prr ), pr );
         if( !grid_barrier( a ) ) return;
@@ -744,23 +839,31 @@ __global__ void __launch_bounds__( 32 * kUpdWarps, 3 ) k_pcg_persistent( const _
 }
 
 // ---------------------------------------------------------------------------------
-__device__ __forceinline__ void solve_init_body( size_t ncells, const float* __restrict__ b, const BoraSolverDev& sv,
+// float4 v of the solver's tiles -> its place in the cell vectors
+__device__ __forceinline__ size_t solve_quad( const int4* tab, size_t v ) { return (size_t)solve_slot( tab, (int)( v >> 7 ) ) * 128 + ( v & 127 ); }
+
+__device__ __forceinline__ void solve_init_body( const BoraSolveTilesDev& ft, const float* __restrict__ b, const BoraSolverDev& sv,
                                                  const BoraReduceDev& red, int slot_norm2, int slot_max, unsigned bid,
                                                  unsigned G )
 {
     DF n2{ 0.f, 0.f };
     float mx = 0.f;
-    for( size_t i = bid * (size_t)blockDim.x + threadIdx.x; i < ncells; i += (size_t)G * blockDim.x )
+    const size_t n4 = (size_t)*ft.count * 128;
+    for( size_t v = bid * (size_t)blockDim.x + threadIdx.x; v < n4; v += (size_t)G * blockDim.x )
     {
-        const float bv = b[i];
-        sv.r[i] = bv;
-        sv.x[i] = make_float2( 0.f, 0.f );
-        sv.e[i] = 0.f;
-        sv.d[0][i] = 0.f;
-        sv.d[1][i] = 0.f;
-        sv.q[i] = 0.f;
-        n2 = df_add( n2, df_prod( bv, bv ) );
-        mx = fmaxf( mx, fabsf( bv ) );
+        const size_t i = solve_quad( ft.tab, v );
+        const float4 bv = reinterpret_cast<const float4*>( b )[i], zero = make_float4( 0.f, 0.f, 0.f, 0.f );
+        reinterpret_cast<float4*>( sv.r )[i] = bv;
+        reinterpret_cast<float4*>( sv.x )[2 * i] = zero;
+        reinterpret_cast<float4*>( sv.x )[2 * i + 1] = zero;
+        reinterpret_cast<float4*>( sv.e )[i] = zero;
+        reinterpret_cast<float4*>( sv.d[0] )[i] = zero;
+        reinterpret_cast<float4*>( sv.q )[i] = zero;
+        n2 = df_add( n2, df_prod( bv.x, bv.x ) );
+        n2 = df_add( n2, df_prod( bv.y, bv.y ) );
+        n2 = df_add( n2, df_prod( bv.z, bv.z ) );
+        n2 = df_add( n2, df_prod( bv.w, bv.w ) );
+        mx = fmaxf( fmaxf( mx, fmaxf( fabsf( bv.x ), fabsf( bv.y ) ) ), fmaxf( fabsf( bv.z ), fabsf( bv.w ) ) );
     }
     reduce2_publish_dfmax( n2, mx, red, slot_norm2, slot_max, bid, G );
 }
@@ -782,10 +885,10 @@ __global__ void k_solve_warm( size_t ncells, const uint16_t* __restrict__ code, 
     }
 }
 
-__global__ void k_solve_init( size_t ncells, const float* __restrict__ b, BoraSolverDev sv, BoraReduceDev red,
+__global__ void k_solve_init( BoraSolveTilesDev ft, const float* __restrict__ b, BoraSolverDev sv, BoraReduceDev red,
                               int slot_norm2, int slot_max )
 {
-    solve_init_body( ncells, b, sv, red, slot_norm2, slot_max, blockIdx.x, gridDim.x );
+    solve_init_body( ft, b, sv, red, slot_norm2, slot_max, blockIdx.x, gridDim.x );
 }
 
 __global__ void k_solve_init_batch( const __grid_constant__ BoraBatchLaunch L )
@@ -794,12 +897,12 @@ __global__ void k_solve_init_batch( const __grid_constant__ BoraBatchLaunch L )
     const int k = bora_batch_member( L, blockIdx.x, &bid );
     const BoraMemberSolve& m = L.ms[k];
     const BoraMemberSlots& q = L.sl[k];
-    solve_init_body( (size_t)m.ntiles * 512, m.b, m.sv, m.red, q.n2, q.mx, bid, (unsigned)m.grid[kGridCells] );
+    solve_init_body( m.ft, m.b, m.sv, m.red, q.n2, q.mx, bid, (unsigned)m.grid[kGridCells] );
 }
 
 // x += e (+ the last update's pending alpha d), then clear e and q; the direction d is kept
 // (the next refinement pass continues the recurrence from it).
-__device__ __forceinline__ void refine_accumulate_body( size_t ncells, const uint16_t* __restrict__ code,
+__device__ __forceinline__ void refine_accumulate_body( const BoraSolveTilesDev& ft, const uint16_t* __restrict__ code,
                                                         const BoraSolverDev& sv, int dsel, const BoraReduceDev& red,
                                                         int nparts, int slot_rr, int slot_a_rz, int slot_a_dq, unsigned bid,
                                                         unsigned G )
@@ -810,26 +913,44 @@ __device__ __forceinline__ void refine_accumulate_body( size_t ncells, const uin
         const DF rr = part_collect( red.part_rr, nparts, s_rr );
         if( threadIdx.x == 0 ) ring_store( red, slot_rr, rr, true );
     }
-    const float alpha = slot_a_rz < 0 ? 0.f : df_ratio( red.ringf[slot_a_rz], red.ringf[slot_a_dq] );
-    const float* __restrict__ d = dsel ? sv.d[1] : sv.d[0];
-    for( size_t i = bid * (size_t)blockDim.x + threadIdx.x; i < ncells; i += (size_t)G * blockDim.x )
+    const bool pending = slot_a_rz >= 0;
+    const float alpha = pending ? df_ratio( red.ringf[slot_a_rz], red.ringf[slot_a_dq] ) : 0.f;
+    const float4* __restrict__ d = reinterpret_cast<const float4*>( dsel ? sv.d[1] : sv.d[0] );
+    const size_t n4 = (size_t)ft.n * 128;
+    for( size_t v = bid * (size_t)blockDim.x + threadIdx.x; v < n4; v += (size_t)G * blockDim.x )
     {
-        const float e = slot_a_rz < 0 ? sv.e[i] : fmaf( alpha, d[i], sv.e[i] );
-        if( code[i] & BORA_CODE_FLUID )
+        const size_t i = solve_quad( ft.tab, v );
+        const uint2 cw = reinterpret_cast<const uint2*>( code )[i];
+        float4 e = reinterpret_cast<const float4*>( sv.e )[i];
+        if( pending )
         {
-            const float2 x = sv.x[i];
-            const DF y = df_add_f( DF{ x.x, x.y }, e );
-            sv.x[i] = make_float2( y.hi, y.lo );
+            const float4 dv = d[i];
+            e.x = fmaf( alpha, dv.x, e.x ); e.y = fmaf( alpha, dv.y, e.y );
+            e.z = fmaf( alpha, dv.z, e.z ); e.w = fmaf( alpha, dv.w, e.w );
         }
-        sv.e[i] = 0.f;
-        sv.q[i] = 0.f;
+        float4 x0 = reinterpret_cast<const float4*>( sv.x )[2 * i], x1 = reinterpret_cast<const float4*>( sv.x )[2 * i + 1];
+        auto add = [&]( uint32_t c, float& hi, float& lo, float ev ) {
+            if( !( c & BORA_CODE_FLUID ) ) return;
+            const DF y = df_add_f( DF{ hi, lo }, ev );
+            hi = y.hi;
+            lo = y.lo;
+        };
+        add( cw.x, x0.x, x0.y, e.x );
+        add( cw.x >> 16, x0.z, x0.w, e.y );
+        add( cw.y, x1.x, x1.y, e.z );
+        add( cw.y >> 16, x1.z, x1.w, e.w );
+        reinterpret_cast<float4*>( sv.x )[2 * i] = x0;
+        reinterpret_cast<float4*>( sv.x )[2 * i + 1] = x1;
+        const float4 zero = make_float4( 0.f, 0.f, 0.f, 0.f );
+        reinterpret_cast<float4*>( sv.e )[i] = zero;
+        reinterpret_cast<float4*>( sv.q )[i] = zero;
     }
 }
 
-__global__ void k_refine_accumulate( size_t ncells, const uint16_t* __restrict__ code, BoraSolverDev sv, int dsel,
+__global__ void k_refine_accumulate( BoraSolveTilesDev ft, const uint16_t* __restrict__ code, BoraSolverDev sv, int dsel,
                                      BoraReduceDev red, int nparts, int slot_rr, int slot_a_rz, int slot_a_dq )
 {
-    refine_accumulate_body( ncells, code, sv, dsel, red, nparts, slot_rr, slot_a_rz, slot_a_dq, blockIdx.x, gridDim.x );
+    refine_accumulate_body( ft, code, sv, dsel, red, nparts, slot_rr, slot_a_rz, slot_a_dq, blockIdx.x, gridDim.x );
 }
 
 __global__ void k_refine_accumulate_batch( const __grid_constant__ BoraBatchLaunch L )
@@ -838,31 +959,32 @@ __global__ void k_refine_accumulate_batch( const __grid_constant__ BoraBatchLaun
     const int k = bora_batch_member( L, blockIdx.x, &bid );
     const BoraMemberSolve& m = L.ms[k];
     const BoraMemberSlots& q = L.sl[k];
-    refine_accumulate_body( (size_t)m.ntiles * 512, m.code, m.sv, q.dsel, m.red, m.grid[kGridPass0R], q.rr_new, q.a_rz,
+    refine_accumulate_body( m.ft, m.code, m.sv, q.dsel, m.red, m.grid[kGridPass0R], q.rr_new, q.a_rz,
                             q.a_dq, bid, (unsigned)m.grid[kGridCells] );
 }
 
 // r = b - A x in double-float arithmetic (A from the stencil code, x the double-float
 // iterate); r stored in FP32, ||r||^2 and max|r| reduced. Streaming, one thread per cell.
 // GB300's FP64 pipe is narrow: in FP64 this kernel and the accumulation were bound by it.
-__device__ __forceinline__ void refine_residual_body( size_t ncells, const int32_t* __restrict__ nbr,
-                                                      const float* __restrict__ b, const uint16_t* __restrict__ code,
-                                                      const BoraSolverDev& sv, const BoraReduceDev& red, int slot_norm2,
+__device__ __forceinline__ void refine_residual_body( const BoraSolveTilesDev& ft, const float* __restrict__ b,
+                                                      const uint16_t* __restrict__ code, const BoraSolverDev& sv, const BoraReduceDev& red, int slot_norm2,
                                                       int slot_max, unsigned bid, unsigned G )
 {
     DF n2{ 0.f, 0.f };
     float mx = 0.f;
-    for( size_t cell = bid * (size_t)blockDim.x + threadIdx.x; cell < ncells; cell += (size_t)G * blockDim.x )
+    const size_t n = (size_t)ft.n * 512;
+    for( size_t i = bid * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)G * blockDim.x )
     {
+        const int t = (int)( i >> 9 ), l = (int)( i & 511 );
+        const size_t cell = (size_t)solve_slot( ft.tab, t ) * 512 + l;
         const uint16_t cc = code[cell];
         if( !( cc & BORA_CODE_FLUID ) ) { sv.r[cell] = 0.f; continue; }
-        const int s = (int)( cell >> 9 ), l = (int)( cell & 511 );
         DF acc{ 0.f, 0.f };
 #pragma unroll
         for( int q = 0; q < 6; ++q )
         {
             if( !( cc & ( 1u << q ) ) ) continue;
-            const size_t nc = face_nbr( nbr, cell, s, l, q );
+            const size_t nc = face_nbr( ft.tab, cell, t, l, q );
             if( nc == (size_t)-1 ) { atomicOr( red.err, 2u ); continue; }
             const float2 xn = sv.x[nc];
             acc = df_add( acc, DF{ xn.x, xn.y } );
@@ -870,8 +992,8 @@ __device__ __forceinline__ void refine_residual_body( size_t ncells, const int32
         const float2 xc = sv.x[cell];
         const float dg = (float)code_diag( cc );
         const DF ax = df_add_f( df_prod( xc.x, dg ), xc.y * dg );  // diag * x (diag <= 12)
-        const DF t = df_add( ax, DF{ -acc.hi, -acc.lo } );
-        const DF rv = df_add_f( DF{ -t.hi, -t.lo }, b[cell] );
+        const DF y = df_add( ax, DF{ -acc.hi, -acc.lo } );
+        const DF rv = df_add_f( DF{ -y.hi, -y.lo }, b[cell] );
         const float rf = rv.hi + rv.lo;
         sv.r[cell] = rf;
         n2 = df_add( n2, df_prod( rf, rf ) );
@@ -880,12 +1002,11 @@ __device__ __forceinline__ void refine_residual_body( size_t ncells, const int32
     reduce2_publish_dfmax( n2, mx, red, slot_norm2, slot_max, bid, G );
 }
 
-__global__ void __launch_bounds__( 256 ) k_refine_residual( size_t ncells, const int32_t* __restrict__ nbr,
-                                                            const float* __restrict__ b, const uint16_t* __restrict__ code,
-                                                            BoraSolverDev sv, BoraReduceDev red, int slot_norm2,
-                                                            int slot_max )
+__global__ void __launch_bounds__( 256 ) k_refine_residual( BoraSolveTilesDev ft, const float* __restrict__ b,
+                                                            const uint16_t* __restrict__ code, BoraSolverDev sv,
+                                                            BoraReduceDev red, int slot_norm2, int slot_max )
 {
-    refine_residual_body( ncells, nbr, b, code, sv, red, slot_norm2, slot_max, blockIdx.x, gridDim.x );
+    refine_residual_body( ft, b, code, sv, red, slot_norm2, slot_max, blockIdx.x, gridDim.x );
 }
 
 __global__ void __launch_bounds__( 256 ) k_refine_residual_batch( const __grid_constant__ BoraBatchLaunch L )
@@ -894,7 +1015,7 @@ __global__ void __launch_bounds__( 256 ) k_refine_residual_batch( const __grid_c
     const int k = bora_batch_member( L, blockIdx.x, &bid );
     const BoraMemberSolve& m = L.ms[k];
     const BoraMemberSlots& q = L.sl[k];
-    refine_residual_body( (size_t)m.ntiles * 512, m.nbr, m.b, m.code, m.sv, m.red, q.n2, q.mx, bid,
+    refine_residual_body( m.ft, m.b, m.code, m.sv, m.red, q.n2, q.mx, bid,
                           (unsigned)m.grid[kGridResidual] );
 }
 
@@ -1022,9 +1143,23 @@ int grid_for( size_t n, int threads )
 
 }  // namespace
 
-void bora_launch_rhs( const BoraGridDev& g, int ntiles, BoraTilesDev t, BoraCellsDev c, uint32_t* nfluid, cudaStream_t st )
+void bora_launch_rhs( const BoraGridDev& g, int ntiles, BoraTilesDev t, BoraCellsDev c, uint32_t* nfluid, uint8_t* tile_fluid,
+                      cudaStream_t st )
 {
-    if( ntiles > 0 ) k_rhs<<<ntiles, 512, 0, st>>>( g, t, c, nfluid );
+    if( ntiles > 0 ) k_rhs<<<ntiles, 512, 0, st>>>( g, t, c, nfluid, tile_fluid );
+}
+
+void bora_launch_tile_fluid( int ntiles, const uint16_t* code, uint8_t* tile_fluid, cudaStream_t st )
+{
+    if( ntiles > 0 ) k_tile_fluid<<<grid_for( (size_t)ntiles * 32, 256 ), 256, 0, st>>>( ntiles, code, tile_fluid );
+}
+
+void bora_launch_solve_tiles( int ntiles, BoraTilesDev t, const uint8_t* tile_fluid, int4* tab, uint32_t* count,
+                              uint32_t* host_count, cudaStream_t st )
+{
+    k_solve_tiles<<<1, 1024, 0, st>>>( ntiles, tile_fluid, reinterpret_cast<int32_t*>( tab ), count, host_count );
+    if( ntiles > 0 )
+        k_solve_nbrs<<<grid_for( (size_t)ntiles * 8, 256 ), 256, 0, st>>>( count, t.nbr, tile_fluid, reinterpret_cast<int32_t*>( tab ) );
 }
 
 void bora_launch_vel_update( const BoraGridDev& g, int ntiles, BoraTilesDev t, BoraCellsDev c, cudaStream_t st )
@@ -1032,19 +1167,18 @@ void bora_launch_vel_update( const BoraGridDev& g, int ntiles, BoraTilesDev t, B
     if( ntiles > 0 ) k_vel_update<<<ntiles, 512, 0, st>>>( g, t, c );
 }
 
-void bora_launch_mic_factor( const BoraGridDev&, int ntiles, const uint16_t* code, float* minv, cudaStream_t st )
+void bora_launch_mic_factor( int ntiles, BoraSolveTilesDev t, const uint16_t* code, float* minv, cudaStream_t st )
 {
     ensure_tables();
     if( ntiles <= 0 ) return;
     const int nb = std::min( ( ntiles + kTilesPerCta - 1 ) / kTilesPerCta, num_sms() * 8 );
-    k_mic_factor<<<nb, 32 * kTilesPerCta, 0, st>>>( ntiles, code, minv );
+    k_mic_factor<<<nb, 32 * kTilesPerCta, 0, st>>>( t, code, minv );
 }
 
-void bora_launch_solve_init( int ntiles, const float* b, const uint16_t*, BoraSolverDev s, BoraReduceDev red,
+void bora_launch_solve_init( int ntiles, BoraSolveTilesDev t, const float* b, BoraSolverDev s, BoraReduceDev red,
                              int slot_norm2, int slot_max, cudaStream_t st )
 {
-    const size_t nc = (size_t)ntiles * 512;
-    k_solve_init<<<grid_for( nc, 256 ), 256, 0, st>>>( nc, b, s, red, slot_norm2, slot_max );
+    k_solve_init<<<grid_for( (size_t)ntiles * 128, 256 ), 256, 0, st>>>( t, b, s, red, slot_norm2, slot_max );
 }
 
 int bora_pcg_update_grid( int ntiles )
@@ -1061,12 +1195,11 @@ int bora_pcg_update_grid( int ntiles )
     return std::max( 1, ( ntiles + kUpdWarps * rounds - 1 ) / ( kUpdWarps * rounds ) );
 }
 
-void bora_launch_pcg_update( int ntiles, const uint16_t* code, BoraSolverDev s, BoraReduceDev red, int slot_rz_in,
-                             int slot_dq_in, cudaStream_t st )
+void bora_launch_pcg_update( BoraSolveTilesDev t, BoraSolverDev s, BoraReduceDev red, int slot_rz_in, int slot_dq_in,
+                             cudaStream_t st )
 {
-    (void)code;
-    bora_launch_pdl( k_pcg_update, bora_pcg_update_grid( ntiles ), 32 * kUpdWarps, 0, st, ntiles, s, red,
-                     bora_pcg_direction_grid( ntiles ), slot_rz_in, slot_dq_in );
+    bora_launch_pdl( k_pcg_update, bora_pcg_update_grid( t.n ), 32 * kUpdWarps, 0, st, t, s, red, bora_pcg_direction_grid( t.n ),
+                     slot_rz_in, slot_dq_in );
 }
 
 // Grid of the direction kernel: every warp gets the same number of half tiles; at most
@@ -1088,12 +1221,11 @@ namespace {
 int residual_grid( size_t nc ) { return (int)std::max<size_t>( 1, std::min<size_t>( ( nc + 255 ) / 256, (size_t)num_sms() * 8 ) ); }
 }  // namespace
 
-void bora_projection_grids( int ntiles, int* grid )
+void bora_projection_grids( int nft, int* grid )
 {
-    const size_t nc = (size_t)std::max( ntiles, 0 ) * 512;
-    grid[kGridDir] = bora_pcg_direction_grid( ntiles );
-    grid[kGridCells] = grid_for( nc, 256 );
-    grid[kGridResidual] = residual_grid( nc );
+    grid[kGridDir] = bora_pcg_direction_grid( nft );
+    grid[kGridCells] = grid_for( (size_t)nft * 128, 256 );
+    grid[kGridResidual] = residual_grid( (size_t)nft * 512 );
 }
 
 void bora_launch_solve_init_batch( const BoraBatchLaunch& L, int blocks, cudaStream_t st )
@@ -1131,14 +1263,14 @@ int bora_pcg_persistent_grid()
     return std::min( b * num_sms(), kBoraMaxReduceBlocks );
 }
 
-int bora_launch_pcg_persistent( int ntiles, const int32_t* nbr, const uint16_t* code, BoraSolverDev s, BoraReduceDev red,
+int bora_launch_pcg_persistent( BoraSolveTilesDev t, const uint16_t* code, BoraSolverDev s, BoraReduceDev red,
                                 int dsel, int slot_rz_prev, int max_inner, double target, int slot_a_rz, int slot_a_dq,
                                 uint32_t* iters, unsigned* bar, double* part, bool never_release, cudaStream_t st )
 {
     const int grid = bora_pcg_persistent_grid();
     if( grid <= 0 ) return -1;
     PcgPersistArgs a{};
-    a.ntiles = ntiles; a.nbr = nbr; a.code = code; a.sv = s; a.red = red;
+    a.ft = t; a.code = code; a.sv = s; a.red = red;
     a.dsel = dsel; a.slot_rz_prev = slot_rz_prev; a.max_inner = max_inner; a.target = target;
     a.slot_a_rz = slot_a_rz; a.slot_a_dq = slot_a_dq; a.iters = iters;
     a.bar = bar; a.part = part;
@@ -1154,13 +1286,11 @@ int bora_launch_pcg_persistent( int ntiles, const int32_t* nbr, const uint16_t* 
                : -1;
 }
 
-void bora_launch_pcg_direction( const BoraGridDev&, int ntiles, BoraTilesDev t, const uint16_t* code, BoraSolverDev s,
-                                int dsel_in, BoraReduceDev red, int nparts, int slot_rz_new, int slot_rr, int slot_rz_old,
+void bora_launch_pcg_direction( BoraSolveTilesDev t, const uint16_t* code, BoraSolverDev s, int dsel_in, BoraReduceDev red, int nparts, int slot_rz_new, int slot_rr, int slot_rz_old,
                                 int slot_a_rz, int slot_a_dq, bool host_rr, cudaStream_t st )
 {
-    if( ntiles <= 0 ) return;
-    bora_launch_pdl( k_pcg_direction, bora_pcg_direction_grid( ntiles ), 32 * kDirWarps, 0, st, ntiles, (const int32_t*)t.nbr,
-                     code, s, dsel_in, red, nparts, slot_rz_new, slot_rr, slot_rz_old, slot_a_rz, slot_a_dq, host_rr );
+    if( t.n <= 0 ) return;
+    bora_launch_pdl( k_pcg_direction, bora_pcg_direction_grid( t.n ), 32 * kDirWarps, 0, st, t, code, s, dsel_in, red, nparts, slot_rz_new, slot_rr, slot_rz_old, slot_a_rz, slot_a_dq, host_rr );
 }
 
 void bora_launch_solve_warm( int ntiles, const uint16_t* code, const int32_t* tile_of, const int32_t* slot_prev,
@@ -1170,19 +1300,18 @@ void bora_launch_solve_warm( int ntiles, const uint16_t* code, const int32_t* ti
     if( nc ) k_solve_warm<<<grid_for( nc, 256 ), 256, 0, st>>>( nc, code, tile_of, slot_prev, pres, s.x );
 }
 
-void bora_launch_refine_accumulate( int ntiles, const uint16_t* code, BoraSolverDev s, int dsel, BoraReduceDev red,
+void bora_launch_refine_accumulate( BoraSolveTilesDev t, const uint16_t* code, BoraSolverDev s, int dsel, BoraReduceDev red,
                                     int nparts, int slot_rr, int slot_a_rz, int slot_a_dq, cudaStream_t st )
 {
-    const size_t nc = (size_t)ntiles * 512;
-    if( nc )
-        k_refine_accumulate<<<grid_for( nc, 256 ), 256, 0, st>>>( nc, code, s, dsel, red, nparts, slot_rr, slot_a_rz, slot_a_dq );
+    if( t.n > 0 )
+        k_refine_accumulate<<<grid_for( (size_t)t.n * 128, 256 ), 256, 0, st>>>( t, code, s, dsel, red, nparts, slot_rr, slot_a_rz,
+                                                                              slot_a_dq );
 }
 
-void bora_launch_refine_residual( const BoraGridDev&, int ntiles, BoraTilesDev t, const float* b, const uint16_t* code,
-                                  BoraSolverDev s, BoraReduceDev red, int slot_norm2, int slot_max, cudaStream_t st )
+void bora_launch_refine_residual( BoraSolveTilesDev t, const float* b, const uint16_t* code, BoraSolverDev s, BoraReduceDev red,
+                                  int slot_norm2, int slot_max, cudaStream_t st )
 {
-    const size_t nc = (size_t)ntiles * 512;
-    k_refine_residual<<<residual_grid( nc ), 256, 0, st>>>( nc, t.nbr, b, code, s, red, slot_norm2, slot_max );
+    k_refine_residual<<<residual_grid( (size_t)t.n * 512 ), 256, 0, st>>>( t, b, code, s, red, slot_norm2, slot_max );
 }
 
 void bora_launch_write_pressure( int ntiles, const uint16_t* code, const float2* x, float* pres, cudaStream_t st )
