@@ -95,7 +95,10 @@ typedef struct bora_flip_params
     int persistent;          /* 0: one launch per PCG phase, convergence read back by the host
                                 (check_every); 1: the plain form runs each refinement pass's inner
                                 PCG in one cooperative launch whose phases meet at bounded grid
-                                barriers and which checks convergence itself */
+                                barriers and which checks convergence itself, every iteration. Small
+                                systems (up to 608 tiles with fluid, proj_iteration up to 2^24) run
+                                that way with either value, where it is the faster form, unless the
+                                PCG's phases are being timed (bora_flip_set_profiling) */
     int warm_start;          /* 0: every pressure solve starts from p = 0, as the reference's does
                                 (its pressure field is re-created with the frame each step,
                                 FLIPMethod.cu:28-33, FluidProjection.cu:265); 1: from the last
@@ -325,7 +328,9 @@ int bora_flip_set_field( bora_flip_handle h, int which, const void* in, size_t b
 int bora_flip_get_stats( bora_flip_handle h, bora_flip_stats* out );
 
 /* Record CUDA events around every launch of the kernel classes in `class_mask` (bit c =
- * class c) and accumulate their device time; setting a mask resets the totals. */
+ * class c) and accumulate their device time; setting a mask resets the totals. Timing the PCG's
+ * direction or update class makes small plain systems run per phase too (see persistent), whose
+ * results differ from the one-launch form's by the solver's tolerance. */
 int bora_flip_set_profiling( bora_flip_handle h, uint32_t class_mask );
 /* Time only one in `every` brackets of each profiled class (1, the default: all). A bracket
  * records an event on the handle's stream before and after the class's kernels, which ends the

@@ -35,8 +35,8 @@ def _solve(n, pos, vel, solver, set_codes):
     return out
 
 
-@pytest.mark.parametrize("tiles_per_axis,spacing", [(1, 4), (2, 4), (2, 1), (9, 3)])
 @pytest.mark.parametrize("solver", [flip.SOLVER_PLAIN, flip.SOLVER_MIXED])
+@pytest.mark.parametrize("tiles_per_axis,spacing", [(1, 4), (2, 4), (2, 1), (9, 3)])
 def test_solve_tiles(gpu, tiles_per_axis, spacing, solver):
     n, pos, vel = _droplets(tiles_per_axis, spacing, 11)
     pres, code, rhs, st, status = _solve(n, pos, vel, solver, False)

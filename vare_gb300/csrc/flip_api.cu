@@ -154,6 +154,8 @@ struct bora_flip_sim
     int nft = 0;                     // solver tiles, known to the host from the solve's start on
     DevBuf sums;     // the solver chain's partial sums (d.q, r.z, r.r) and the finished pairs
     DevBuf gbar;     // the persistent solver's grid barrier: count, generation
+    DevBuf meet;     // the resident solver's words
+    uint32_t meet_tag = 1;  // the next launch's first tag
     int fault = 0;   // BORA_FAULT_*
     int next_slot = 0;
 
@@ -755,7 +757,34 @@ int stage_solve( bora_flip_sim* s )
         int rz_cur = s->slot(), rr_cur = s->slot();
         int it = 0;
         int a_rz = -1, a_dq = -1;  // alpha of the last update, whose e += alpha d is still pending
-        if( !mixed && p.persistent && bora_pcg_persistent_grid() > 0 )
+        // the resident form where it is the faster one (bora_pcg_resident_warps), in place of both others
+        constexpr int kResidentMaxInner = 1 << 24;  // bounds a launch's tags
+        // (a caller that times the PCG's two phases gets the form that has them)
+        constexpr uint32_t kPhases = ( 1u << BORA_KERNEL_PCG_DIRECTION ) | ( 1u << BORA_KERNEL_PCG_UPDATE );
+        bool resident = !mixed && !( s->prof_mask & kPhases ) && max_inner <= kResidentMaxInner && bora_pcg_resident_warps( ft.n ) > 0;
+        if( resident )
+        {
+            const int s_a_rz = s->slot();
+            const uint32_t tags = 2 * (uint32_t)max_inner + 2;
+            if( s->meet_tag > 0xFFFFFFFFu - tags )  // tags start over: no word may hold an old one
+            {
+                BORA_TRY( cudaMemsetAsync( s->meet.p, 0, s->meet.bytes, st ) );
+                s->meet_tag = 1;
+            }
+            ( (volatile uint32_t*)s->h_cnt )[8] = kCountNotArrived;
+            s->stats.kernel_launches += 1;
+            resident = bora_launch_pcg_resident( ft, code, sv, red, dsel, rz_prev, max_inner, target, s_a_rz, s->d_cnt + 8,
+                                                 s->meet.p, s->meet_tag, p.persistent && s->fault == BORA_FAULT_BARRIER, st ) == 0;
+            if( resident )
+            {
+                s->meet_tag += tags;
+                rz_prev = s_a_rz;
+                nparts = 1;
+            }
+            else cudaGetLastError();  // the device cannot hold the grid now: the other forms
+        }
+        if( resident ) {}
+        else if( !mixed && p.persistent && bora_pcg_persistent_grid() > 0 )
         {
             // the whole pass in one cooperative launch (convergence checked on the device)
             const int s_a_rz = s->slot(), s_a_dq = s->slot();
@@ -793,7 +822,7 @@ int stage_solve( bora_flip_sim* s )
         // extra iteration, which only lowers the residual further). No event stands between the
         // kernels, which would end their programmatic overlap.
         int chk_slot = -1;  // r.r of the last iteration, to be checked
-        bool done = a_rz >= 0;  // the persistent pass has run
+        bool done = resident || a_rz >= 0;  // the resident or persistent pass has run
         while( it < max_inner && !done )
         {
             const int s_dq = s->slot();
@@ -849,6 +878,12 @@ int stage_solve( bora_flip_sim* s )
         BORA_TRYS( poll_mirror( s, s_mx, st, &rmax ) );
         rnorm = std::sqrt( n2 );
         scale_slot = s_n2;
+        if( resident )  // the pass is complete: its iterations, or a wait that ran out
+        {
+            uint32_t n = 0;
+            BORA_TRYS( poll_mapped( (volatile uint32_t*)s->h_cnt + 8, kCountNotArrived, st, &n ) );
+            total_it += (int)n;
+        }
         if( !std::isfinite( rnorm ) ) break;
         // Continue the recurrence only while the refined residual still agrees with the
         // recursive one (the device finished the pass, so its last r.r is in mapped memory);
@@ -1054,7 +1089,7 @@ void for_each_buffer( bora_flip_sim* s, F&& f )
                       &s->se, &s->sr, &s->sd0, &s->sd1, &s->sq, &s->sz, &s->sminv, &s->cell_count, &s->cell_start,
                       &s->ring, &s->partials, &s->done, &s->sums, &s->tile_fluid, &s->solve_tab, &s->adj, &s->vkey, &s->key, &s->idx, &s->scan_scratch,
                       &s->counters, &s->stage_in, &s->stage_out, &s->live_flag, &s->col_phi, &s->col_vel,
-                      &s->col_tslot, &s->col_tnear, &s->col_tphi, &s->col_tvel, &s->gbar };
+                      &s->col_tslot, &s->col_tnear, &s->col_tphi, &s->col_tvel, &s->gbar, &s->meet };
     for( DevBuf* b : all ) f( *b );
     for( int q = 0; q < 2; ++q )
     {
@@ -1156,6 +1191,8 @@ int bora_flip_create( const bora_grid_desc* grid, const bora_flip_params* params
     if( st == BORA_OK ) st = cuda_status( grow( s->done, BORA_RING * 4, false, s->st ) );
     if( st == BORA_OK ) st = cuda_status( grow( s->sums, ( 3 * kBoraMaxReduceBlocks + BORA_RING ) * 8, false, s->st ) );
     if( st == BORA_OK ) st = cuda_status( grow( s->gbar, 16, false, s->st ) );
+    if( st == BORA_OK ) st = cuda_status( grow( s->meet, bora_pcg_resident_words_bytes(), false, s->st ) );
+    if( st == BORA_OK ) st = cuda_status( cudaMemsetAsync( s->meet.p, 0, s->meet.bytes, s->st ) );
     if( st == BORA_OK ) st = cuda_status( cudaMemsetAsync( s->done.p, 0, BORA_RING * 4, s->st ) );
     if( st == BORA_OK ) st = cuda_status( cudaMemsetAsync( s->ring.p, 0, BORA_RING * 8, s->st ) );
     if( st == BORA_OK ) st = ensure_cells( s, 1 );

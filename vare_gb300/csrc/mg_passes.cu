@@ -313,12 +313,17 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
     __syncthreads();
     const float sc = s_sc;
     DF acc{ 0.f, 0.f };  // down 1: r.r of the updated residual; up 2: r.z
-    for( ; t < a.ft.n; t += stride )
+    // the loop's bound is the block's, not the warp's: control flow that the compiler knows to be
+    // uniform, without a reconvergence around each shuffle; a warp past the last tile has no
+    // neighbours and neither loads nor stores
+#pragma unroll 1
+    for( int base = (int)bid * W; base < a.ft.n; base += stride, t += stride )
     {
+        const bool mine = t < a.ft.n;
         const int s = sn;
         int nf[6];
 #pragma unroll
-        for( int q = 0; q < 6; ++q ) nf[q] = nfn[q];
+        for( int q = 0; q < 6; ++q ) nf[q] = mine ? nfn[q] : -1;
         const size_t gA = (size_t)s * 512 + 8 * lane, gB = gA + 256;
         uint16_t cA[8], cB[8];
         {
@@ -331,10 +336,13 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
             }
         }
         fetch( t + stride );
-        float rA[8], rB[8];  // r' on fluid cells
-        f32x8( a.r0, gA, rA );
-        f32x8( a.r0, gB, rB );
-        if( upd )
+        float rA[8] = {}, rB[8] = {};  // r' on fluid cells
+        if( mine )
+        {
+            f32x8( a.r0, gA, rA );
+            f32x8( a.r0, gB, rB );
+        }
+        if( upd && mine )
         {
             float qA[8], qB[8];
             f32x8( a.q, gA, qA );
@@ -356,7 +364,7 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
             float p = 0.f;
 #pragma unroll
             for( int i = 0; i < 8; ++i ) { p = fmaf( rA[i], rA[i], p ); p = fmaf( rB[i], rB[i], p ); }
-            acc = df_add_f( acc, p );
+            if( mine ) acc = df_add_f( acc, p );
         }
 #pragma unroll
         for( int i = 0; i < 8; ++i )
@@ -380,14 +388,18 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
                 vA[i] = sweep( vA[i], rA[i], cA[i], sA[i], w + 16 );
                 vB[i] = sweep( vB[i], rB[i], cB[i], sB[i], w + 16 );
             }
-            st_f16x8( reinterpret_cast<__half*>( a.scratch ), gA, vA );
-            st_f16x8( reinterpret_cast<__half*>( a.scratch ), gB, vB );
+            if( mine )
+            {
+                st_f16x8( reinterpret_cast<__half*>( a.scratch ), gA, vA );
+                st_f16x8( reinterpret_cast<__half*>( a.scratch ), gB, vB );
+            }
         }
         else if constexpr( P == 1 )
         {
-            f16x8( reinterpret_cast<const __half*>( a.scratch ), gA, vA );
-            f16x8( reinterpret_cast<const __half*>( a.scratch ), gB, vB );
-            row_sums( FieldF16{ reinterpret_cast<const __half*>( a.scratch ) }, nf, lane, vA, vB, sA, sB );
+            const FieldF16 f{ reinterpret_cast<const __half*>( a.scratch ) };
+            f.row( mine ? s : -1, 8 * lane, vA );
+            f.row( mine ? s : -1, 256 + 8 * lane, vB );
+            row_sums( f, nf, lane, vA, vB, sA, sB );
             float qA[8], qB[8];  // residuals
 #pragma unroll
             for( int i = 0; i < 8; ++i )
@@ -395,10 +407,11 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
                 qA[i] = cfluid( cA[i] ) ? rA[i] - ( (float)cdiag( cA[i] ) * vA[i] - sA[i] ) : 0.f;
                 qB[i] = cfluid( cB[i] ) ? rB[i] - ( (float)cdiag( cB[i] ) * vB[i] - sB[i] ) : 0.f;
             }
-            *reinterpret_cast<uint4*>( a.F.z0 + gA ) =
-                make_uint4( pack2( vA[0], vA[1] ), pack2( vA[2], vA[3] ), pack2( vA[4], vA[5] ), pack2( vA[6], vA[7] ) );
-            *reinterpret_cast<uint4*>( a.F.z0 + gB ) =
-                make_uint4( pack2( vB[0], vB[1] ), pack2( vB[2], vB[3] ), pack2( vB[4], vB[5] ), pack2( vB[6], vB[7] ) );
+            if( mine )
+            {
+                st_f16x8( a.F.z0, gA, vA );
+                st_f16x8( a.F.z0, gB, vB );
+            }
             // restriction: x pairs in the row, y pairs from lane j + 1, z pairs from lane + 8
             float pA[4], pB[4];
 #pragma unroll
@@ -411,7 +424,7 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
                 pA[q] = pA[q] + __shfl_down_sync( kAll, pA[q], 8 );
                 pB[q] = pB[q] + __shfl_down_sync( kAll, pB[q], 8 );
             }
-            if( !( j & 1 ) && !( kq & 1 ) )
+            if( mine && !( j & 1 ) && !( kq & 1 ) )
             {
                 __half* cr = a.C.r + (size_t)s * 64 + 4 * ( j >> 1 );
                 *reinterpret_cast<uint2*>( cr + 16 * ( kq >> 1 ) ) =
@@ -423,8 +436,8 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
         else if constexpr( P == 2 )
         {
             const FieldZa f{ a.F.code, a.F.z0, a.C.z1 };
-            f.row( s, 8 * lane, vA );
-            f.row( s, 256 + 8 * lane, vB );
+            f.row( mine ? s : -1, 8 * lane, vA );
+            f.row( mine ? s : -1, 256 + 8 * lane, vB );
             row_sums( f, nf, lane, vA, vB, sA, sB );
 #pragma unroll
             for( int i = 0; i < 8; ++i )
@@ -432,17 +445,24 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
                 vA[i] = sweep( vA[i], rA[i], cA[i], sA[i], w + 16 );
                 vB[i] = sweep( vB[i], rB[i], cB[i], sB[i], w + 16 );
             }
-            st_f16x8( reinterpret_cast<__half*>( a.scratch ), gA, vA );
-            st_f16x8( reinterpret_cast<__half*>( a.scratch ), gB, vB );
+            if( mine )
+            {
+                st_f16x8( reinterpret_cast<__half*>( a.scratch ), gA, vA );
+                st_f16x8( reinterpret_cast<__half*>( a.scratch ), gB, vB );
+            }
         }
         else
         {
-            f16x8( reinterpret_cast<const __half*>( a.scratch ), gA, vA );
-            f16x8( reinterpret_cast<const __half*>( a.scratch ), gB, vB );
-            row_sums( FieldF16{ reinterpret_cast<const __half*>( a.scratch ) }, nf, lane, vA, vB, sA, sB );
-            float rawA[8], rawB[8];
-            f32x8( a.r0, gA, rawA );
-            f32x8( a.r0, gB, rawB );
+            const FieldF16 f{ reinterpret_cast<const __half*>( a.scratch ) };
+            f.row( mine ? s : -1, 8 * lane, vA );
+            f.row( mine ? s : -1, 256 + 8 * lane, vB );
+            row_sums( f, nf, lane, vA, vB, sA, sB );
+            float rawA[8] = {}, rawB[8] = {};
+            if( mine )
+            {
+                f32x8( a.r0, gA, rawA );
+                f32x8( a.r0, gB, rawB );
+            }
             float trz = 0.f;
 #pragma unroll
             for( int i = 0; i < 8; ++i )
@@ -453,9 +473,12 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
                 if( cfluid( cA[i] ) ) trz = fmaf( rawA[i], vA[i], trz );
                 if( cfluid( cB[i] ) ) trz = fmaf( rawB[i], vB[i], trz );
             }
-            st_f32x8( a.zout, gA, vA );
-            st_f32x8( a.zout, gB, vB );
-            acc = df_add_f( acc, trz );
+            if( mine )
+            {
+                st_f32x8( a.zout, gA, vA );
+                st_f32x8( a.zout, gB, vB );
+                acc = df_add_f( acc, trz );
+            }
         }
     }
     if constexpr( P == 3 ) part_publish( acc, DF{ 0.f, 0.f }, a.red.part_rz, nullptr, bid );

@@ -392,7 +392,10 @@ __device__ __forceinline__ void rotate8( float* v, int rho )
 }
 
 // z = M^-1 r of one tile: rA, rB hold the lane's rows of r and return z (both in cell order);
-// mA, mB the rows' squared pivots as stored (rotated). Returns the lane's part of r.z.
+// mA, mB the rows' squared pivots as stored (rotated). Returns the lane's part of r.z. ROLLED: a
+// third of the code, for a kernel whose one warp per SM partition would wait for its instructions
+// (the grid kernel is faster unrolled: 18.3 against 18.7 ms of GPU time per 256^3 step).
+template <bool ROLLED>
 __device__ __forceinline__ float mic_sweeps( float* rA, float* rB, const float* mA, const float* mB )
 {
     constexpr unsigned kAllLanes = 0xffffffffu;
@@ -402,37 +405,52 @@ __device__ __forceinline__ float mic_sweeps( float* rA, float* rB, const float* 
     rotate8( rA, rho );
     rotate8( rB, rho );  // row B's cell of step u is register (u - 1) mod 8
     float wA = 0.f, wB = 0.f, rzA = 0.f, rzB = 0.f;
-#pragma unroll
-    for( int u = 1; u <= 22; ++u )
+    // three rounds of eight steps (none past step 22): a register's steps are eight apart, so the
+    // round can be the body of a loop
+    constexpr int kRounds = ROLLED ? 1 : 3;
+#pragma unroll kRounds
+    for( int round = 0; round < 3; ++round )
     {
-        const bool a = ( live >> u ) & 1u, b = ( live >> ( u - 1 ) ) & 1u;
-        const float yA = __shfl_up_sync( kAllLanes, wA, 1 ), yB = __shfl_up_sync( kAllLanes, wB, 1 );
-        const float zA = __shfl_up_sync( kAllLanes, wB, 8 );
-        float& cA = rA[u & 7];
-        float& cB = rB[( u - 1 ) & 7];
-        const float tA = fmaf( zm, zA, fmaf( ym, yA, cA + wA ) );
-        const float tB = fmaf( ym, yB, ( cB + wB ) + wA );
-        wA = a ? mA[u & 7] * tA : 0.f;
-        wB = b ? mB[u & 7] * tB : 0.f;
-        rzA = fmaf( wA, tA, rzA );
-        rzB = fmaf( wB, tB, rzB );
-        cA = a ? wA : cA;
-        cB = b ? wB : cB;
+        const unsigned lv = live >> ( 8 * round );  // bit v: row A has a cell at step v of the round
+#pragma unroll
+        for( int v = 1; v <= 8; ++v )
+        {
+            if( !ROLLED && 8 * round + v > 22 ) continue;
+            const bool a = ( lv >> v ) & 1u, b = ( lv >> ( v - 1 ) ) & 1u;
+            const float yA = __shfl_up_sync( kAllLanes, wA, 1 ), yB = __shfl_up_sync( kAllLanes, wB, 1 );
+            const float zA = __shfl_up_sync( kAllLanes, wB, 8 );
+            float& cA = rA[v & 7];
+            float& cB = rB[v - 1];
+            const float tA = fmaf( zm, zA, fmaf( ym, yA, cA + wA ) );
+            const float tB = fmaf( ym, yB, ( cB + wB ) + wA );
+            wA = a ? mA[v & 7] * tA : 0.f;
+            wB = b ? mB[v & 7] * tB : 0.f;
+            rzA = fmaf( wA, tA, rzA );
+            rzB = fmaf( wB, tB, rzB );
+            cA = a ? wA : cA;
+            cB = b ? wB : cB;
+        }
     }
     float zA = 0.f, zB = 0.f;
-#pragma unroll
-    for( int u = 22; u >= 1; --u )
+#pragma unroll kRounds
+    for( int round = 2; round >= 0; --round )
     {
-        const bool a = ( live >> u ) & 1u, b = ( live >> ( u - 1 ) ) & 1u;
-        const float yA = __shfl_down_sync( kAllLanes, zA, 1 ), yB = __shfl_down_sync( kAllLanes, zB, 1 );
-        const float nB = __shfl_down_sync( kAllLanes, zA, 8 );
-        float& cA = rA[u & 7];
-        float& cB = rB[( u - 1 ) & 7];
-        const float sumA = fmaf( yp, yA, zA + zB ), sumB = fmaf( zp, nB, fmaf( yp, yB, zB ) );
-        zA = a ? fmaf( mA[u & 7], sumA, cA ) : 0.f;
-        zB = b ? fmaf( mB[u & 7], sumB, cB ) : 0.f;
-        cA = a ? zA : cA;
-        cB = b ? zB : cB;
+        const unsigned lv = live >> ( 8 * round );
+#pragma unroll
+        for( int v = 8; v >= 1; --v )
+        {
+            if( !ROLLED && 8 * round + v > 22 ) continue;
+            const bool a = ( lv >> v ) & 1u, b = ( lv >> ( v - 1 ) ) & 1u;
+            const float yA = __shfl_down_sync( kAllLanes, zA, 1 ), yB = __shfl_down_sync( kAllLanes, zB, 1 );
+            const float nB = __shfl_down_sync( kAllLanes, zA, 8 );
+            float& cA = rA[v & 7];
+            float& cB = rB[v - 1];
+            const float sumA = fmaf( yp, yA, zA + zB ), sumB = fmaf( zp, nB, fmaf( yp, yB, zB ) );
+            zA = a ? fmaf( mA[v & 7], sumA, cA ) : 0.f;
+            zB = b ? fmaf( mB[v & 7], sumB, cB ) : 0.f;
+            cA = a ? zA : cA;
+            cB = b ? zB : cB;
+        }
     }
     rotate8( rA, ( 8 - rho ) & 7 );
     rotate8( rB, ( 8 - rho ) & 7 );
@@ -443,10 +461,11 @@ __device__ __forceinline__ float mic_sweeps( float* rA, float* rB, const float* 
 // r.r accumulated into prz, prr. alpha_of() is called once, by every thread of the block, after
 // the first tile's loads have been issued.
 template <class AlphaOf>
-__device__ __forceinline__ void pcg_update_tiles( const BoraSolveTilesDev& ft, const BoraSolverDev& sv, AlphaOf alpha_of, int first,
-                                                  int tstride, DF& prz, DF& prr )
+__device__ __forceinline__ void pcg_update_tiles( const BoraSolveTilesDev& ft, const BoraSolverDev& sv, AlphaOf alpha_of, unsigned bid,
+                                                  unsigned G, DF& prz, DF& prr )
 {
     // the tiles' slots, read a tile ahead (no kernel of the chain writes the table)
+    const int tstride = (int)G * kUpdWarps, first = (int)bid * kUpdWarps + ( threadIdx.x >> 5 );
     int next = first < ft.n ? solve_slot( ft.tab, first ) : 0;
     const int lane = threadIdx.x & 31;
     const size_t row = 8 * (size_t)( ( lane & 7 ) + 16 * ( lane >> 3 ) );  // row A; row B follows 64 cells on
@@ -481,7 +500,7 @@ __device__ __forceinline__ void pcg_update_tiles( const BoraSolveTilesDev& ft, c
             prr = df_add_f( prr, dot4( make_float4( rA[h], rA[h + 1], rA[h + 2], rA[h + 3] ), make_float4( rA[h], rA[h + 1], rA[h + 2], rA[h + 3] ) ) );
             prr = df_add_f( prr, dot4( make_float4( rB[h], rB[h + 1], rB[h + 2], rB[h + 3] ), make_float4( rB[h], rB[h + 1], rB[h + 2], rB[h + 3] ) ) );
         }
-        prz = df_add_f( prz, mic_sweeps( rA, rB, mA, mB ) );
+        prz = df_add_f( prz, mic_sweeps<false>( rA, rB, mA, mB ) );
         bora_st8( sv.z + o, rA );
         bora_st8( sv.z + o + 64, rB );
     }
@@ -500,7 +519,7 @@ __global__ void __launch_bounds__( 32 * kUpdWarps, 4 ) k_pcg_update( BoraSolveTi
         if( blockIdx.x == 0 && threadIdx.x == 0 ) ring_store( red, slot_dq_in, dq, false );
         return df_ratio( red.ringf[slot_rz_in], make_float2( dq.hi, dq.lo ) );
     };
-    pcg_update_tiles( ft, sv, alpha_of, blockIdx.x * kUpdWarps + ( threadIdx.x >> 5 ), gridDim.x * kUpdWarps, prz, prr );
+    if( ft.n > 0 ) pcg_update_tiles( ft, sv, alpha_of, blockIdx.x, gridDim.x, prz, prr );
     part_publish( prz, prr, red.part_rz, red.part_rr, blockIdx.x );
 }
 
@@ -556,31 +575,36 @@ __device__ __forceinline__ DF pcg_direction_tiles( const BoraSolveTilesDev& ft, 
     constexpr unsigned kAll = 0xffffffffu;
     DF pdq{ 0.f, 0.f };
     float beta = 0.f, alpha = 0.f;
-    float d[8], z[8];
-    const int nh = 2 * ft.n;
-    int h = (int)bid * kDirWarps + ( threadIdx.x >> 5 );
+    float d[8] = {}, z[8] = {};
+    const int nh = 2 * ft.n, stride = (int)G * kDirWarps;
+    const int first = min( (int)bid * kDirWarps + (int)( threadIdx.x >> 5 ), nh - 1 );
     // a half tile's slot, read one ahead (no kernel of the chain writes the table)
-    int next = h < nh ? solve_slot( ft.tab, h >> 1 ) : 0;
-    auto load_rows = [&]( size_t g ) {
+    int next = solve_slot( ft.tab, first >> 1 );
+    auto load_rows = [&]( size_t g, bool mine ) {
+        if( !mine ) return;
         bora_ld8( dold + g, d );
         bora_ld8( sv.z + g, z );
     };
     bora_pdl_wait();  // the previous kernel's results (ring, partial sums, z, d, e) are complete from here
-    if( h < nh ) load_rows( (size_t)next * 512 + ( h & 1 ) * 256 + 8 * lane );
+    load_rows( (size_t)next * 512 + ( first & 1 ) * 256 + 8 * lane, (int)bid * kDirWarps + (int)( threadIdx.x >> 5 ) < nh );
     {
         const float2 c = coef();
         beta = c.x;
         alpha = c.y;
     }
-    for( bool head = true; h < nh; h += (int)G * kDirWarps, head = false )
+    // (a bound of the block's, as in the update; a warp past the last half tile stores nothing)
+#pragma unroll 1
+    for( int base = (int)bid * kDirWarps; base < nh; base += stride )
     {
+        const int h0 = base + (int)( threadIdx.x >> 5 ), h = min( h0, nh - 1 );
+        const bool mine = h0 < nh;
         const int s = next, hi = h & 1;
         const int cA = hi * 256 + 8 * lane;
         const size_t g = (size_t)s * 512 + cA;
-        if( !head ) load_rows( g );
         const int4 n0 = __ldg( ft.tab + 2 * (size_t)( h >> 1 ) ), n1 = __ldg( ft.tab + 2 * (size_t)( h >> 1 ) + 1 );
         const int smx = n0.x, spx = n0.y, smy = n0.z, spy = n0.w, sz = hi ? n1.y : n1.x;
-        if( h + (int)G * kDirWarps < nh ) next = solve_slot( ft.tab, ( h + (int)G * kDirWarps ) >> 1 );
+        const int hn = min( h0 + stride, nh - 1 );
+        next = solve_slot( ft.tab, hn >> 1 );
         const uint4 w = *reinterpret_cast<const uint4*>( code + g );
         float e[8];
         if( upd_e ) bora_ld8( sv.e + g, e );
@@ -605,11 +629,11 @@ __device__ __forceinline__ DF pcg_direction_tiles( const BoraSolveTilesDev& ft, 
         {
 #pragma unroll
             for( int i = 0; i < 8; ++i ) e[i] = fmaf( alpha, d[i], e[i] );
-            bora_st8( sv.e + g, e );
+            if( mine ) bora_st8( sv.e + g, e );
         }
 #pragma unroll
         for( int i = 0; i < 8; ++i ) d[i] = fmaf( beta, d[i], z[i] );
-        bora_st8( dnew + g, d );
+        if( mine ) bora_st8( dnew + g, d );
         const uint32_t cw[4] = { w.x, w.y, w.z, w.w };
 #pragma unroll
         for( int i = 0; i < 8; ++i )
@@ -630,9 +654,13 @@ __device__ __forceinline__ DF pcg_direction_tiles( const BoraSolveTilesDev& ft, 
                 q[i] = fmaf( (float)code_diag( (uint16_t)c ), d[i], -acc );
             }
         }
+        if( mine )
+        {
 #pragma unroll
-        for( int i = 0; i < 8; i += 2 ) pdq = df_add_f( pdq, fmaf( d[i + 1], q[i + 1], d[i] * q[i] ) );
-        bora_st8( sv.q + g, q );
+            for( int i = 0; i < 8; i += 2 ) pdq = df_add_f( pdq, fmaf( d[i + 1], q[i + 1], d[i] * q[i] ) );
+            bora_st8( sv.q + g, q );
+        }
+        load_rows( (size_t)next * 512 + ( hn & 1 ) * 256 + 8 * lane, h0 + stride < nh );
     }
     return pdq;
 }
@@ -792,11 +820,10 @@ __global__ void __launch_bounds__( 32 * kUpdWarps, 3 ) k_pcg_persistent( const _
     double* const pd = a.part;                // d'.q
     double* const pz = a.part + G;            // r.z
     double* const pr = a.part + 2 * (size_t)G;  // r.r
-    const int first = blockIdx.x * kUpdWarps + ( threadIdx.x >> 5 ), stride = G * kUpdWarps;
     double rz_prev = a.slot_rz_prev >= 0 ? a.red.ring[a.slot_rz_prev] : -1.0;
     // the pass's first update: z = M^-1 r (alpha 0)
     DF prz{ 0.f, 0.f }, prr{ 0.f, 0.f };
-    pcg_update_tiles( a.ft, a.sv, [] { return 0.f; }, first, stride, prz, prr );
+    pcg_update_tiles( a.ft, a.sv, [] { return 0.f; }, blockIdx.x, G, prz, prr );
     block_sum_store( df_warp_sum( prz ), pz );
     block_sum_store( df_warp_sum( prr ), pr );
     if( !grid_barrier( a ) ) return;
@@ -816,7 +843,7 @@ __global__ void __launch_bounds__( 32 * kUpdWarps, 3 ) k_pcg_persistent( const _
         prz = DF{ 0.f, 0.f };
         prr = DF{ 0.f, 0.f };
         const float alpha = (float)( rz / dq );
-        pcg_update_tiles( a.ft, a.sv, [=] { return alpha; }, first, stride, prz, prr );
+        pcg_update_tiles( a.ft, a.sv, [=] { return alpha; }, blockIdx.x, G, prz, prr );
         block_sum_store( df_warp_sum( prz ), pz );
         block_sum_store( df_warp_sum( prr ), pr );
         if( !grid_barrier( a ) ) return;
@@ -835,6 +862,311 @@ __global__ void __launch_bounds__( 32 * kUpdWarps, 3 ) k_pcg_persistent( const _
         ring_store( a.red, a.slot_a_dq, pair( a_dq ), false );
         a.red.part_rr[0] = make_float2( pair( rr ).hi, pair( rr ).lo );  // finished by the refinement
         *a.iters = (uint32_t)it;
+    }
+}
+
+// ---------------------------------------------------------------------------------
+// Resident plain PCG: a refinement pass's inner iterations in one cooperative launch for systems
+// whose tiles fit one warp each, every vector of a tile in its warp's registers. Per iteration the
+// blocks meet twice:
+//   direction  d = z + beta d, q = A d; d.q
+//   update     e += alpha d, r -= alpha q, z = M^-1 r (mic_sweeps); r.z, r.r; z stored
+// Only z crosses tiles through memory: a lane that needs a neighbour tile's cells keeps their d
+// as well and forms d = z + beta d for them itself. The stop test runs on the device.
+//
+// A meeting is a sum: a block stores its partial sums as 64-bit words of a float and a tag (the
+// meeting's number), and every block's first warp polls all blocks' words, so a value is its own
+// arrival signal - no counter, no second read. A tag is never reused while a word can hold it
+// (the host hands each launch its own range). z is stored before the block's fence and words, and
+// read past L1 after the poller's fence. Each wait is bounded: a warp that polls `limit` times, or
+// sees another block's error, sets BORA_REDUCE_ERR_BARRIER and its block returns; the other blocks
+// then run out in turn, and the host finds no iteration count.
+//
+// Bound by latency. Of 10.7 K cycles per iteration at 15 tiles the sweeps and sums take 2.7 K, the
+// fence 1.0 K, the two meetings 4.6 K, the stencil 1.2 K. Code that fits the instruction caches
+// matters (one warp per SM partition hides no fetch: 10 x slower at 100 KB): rolled sweeps, one
+// copy of each part, control flow that the compiler knows to be uniform.
+// GPU time of a step against the per-phase form: 0.46 against 0.69 ms at 15 solver tiles, 1.17
+// against 1.40 at 180, 1.73 against 1.95 at 425, 2.45 against 2.54 at 680, 3.74 against 3.47 at 1084.
+struct PcgResidentArgs
+{
+    BoraSolveTilesDev ft;
+    const uint16_t* code;
+    BoraSolverDev sv;
+    BoraReduceDev red;
+    int dsel;               // the buffer of the last search direction (read and left there)
+    int slot_rz_prev;       // r.z before the last update of the previous pass, or -1 (restart)
+    int max_inner;
+    float2 target2;         // stop once r.r <= target2 (a double-float pair)
+    int slot_a_rz;          // out: r.z before the last update; r.r is left as the one partial sum part_rr[0]
+    uint32_t* iters;        // out (mapped host memory): iterations run; not written when a wait ran out
+    ulonglong2* words_rz;   // two per block: r.z, r.r
+    ulonglong2* words_dq;   // one per block
+    uint32_t tag;           // first tag of the launch
+    unsigned expect;        // blocks a meeting waits for (gridDim.x)
+    unsigned limit;         // polls per wait
+};
+
+__device__ __forceinline__ ulonglong2 tagged( DF v, uint32_t tag )
+{
+    const unsigned long long t = (unsigned long long)tag << 32;
+    return make_ulonglong2( t | __float_as_uint( v.hi ), t | __float_as_uint( v.lo ) );
+}
+
+__device__ __forceinline__ void store_words( ulonglong2* p, ulonglong2 v )
+{
+    asm volatile( "st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"( p ), "l"( v.x ), "l"( v.y ) : "memory" );
+}
+
+__device__ __forceinline__ ulonglong2 load_words( const ulonglong2* p )
+{
+    ulonglong2 v;
+    asm volatile( "ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"( v.x ), "=l"( v.y ) : "l"( p ) : "memory" );
+    return v;
+}
+
+// The sums over all blocks of their N double-float words under `tag`, in every thread of the block;
+// false when the wait ran out. The block's first warp polls (lane l blocks l, l + 32, ..., all at
+// once) and adds up in a fixed order. ACQUIRE: what the blocks stored before they published is
+// visible afterwards.
+template <int N, bool ACQUIRE>
+__device__ __forceinline__ bool meet( const ulonglong2* words, const PcgResidentArgs& a, uint32_t tag, DF* sum, float4* out )
+{
+    constexpr int kPer = 5;  // blocks per lane: up to 160
+    if( threadIdx.x < 32 )
+    {
+        const int lane = threadIdx.x;
+        ulonglong2 w[kPer][N];
+        bool ok = false;
+        for( unsigned n = 0;; ++n )  // (the loop's exit is a vote: uniform control flow)
+        {
+            ok = true;
+#pragma unroll
+            for( int q = 0; q < kPer; ++q )
+            {
+                const unsigned b = lane + 32 * q;
+#pragma unroll
+                for( int v = 0; v < N; ++v )
+                    w[q][v] = b < a.expect ? load_words( words + (size_t)b * N + v ) : tagged( DF{ 0.f, 0.f }, tag );
+            }
+#pragma unroll
+            for( int q = 0; q < kPer; ++q )
+#pragma unroll
+                for( int v = 0; v < N; ++v ) ok = ok && (uint32_t)( w[q][v].x >> 32 ) == tag && (uint32_t)( w[q][v].y >> 32 ) == tag;
+            ok = __all_sync( 0xffffffffu, ok );
+            if( ok || n >= a.limit ) break;
+            if( ( n & 255u ) == 255u && __any_sync( 0xffffffffu, *(volatile uint32_t*)a.red.err != 0u ) ) break;
+        }
+        // one fence after the relaxed polls (acquiring loads would wait for one another)
+        if( ACQUIRE && lane == 0 ) asm volatile( "fence.acq_rel.gpu;" ::: "memory" );
+        if( !ok && lane == 0 ) atomicOr( a.red.err, (uint32_t)BORA_REDUCE_ERR_BARRIER );
+        DF t[2] = { { 0.f, 0.f }, { 0.f, 0.f } };
+#pragma unroll
+        for( int v = 0; v < N; ++v )
+        {
+#pragma unroll
+            for( int q = 0; q < kPer; ++q )
+                t[v] = df_add( t[v], DF{ __uint_as_float( (uint32_t)w[q][v].x ), __uint_as_float( (uint32_t)w[q][v].y ) } );
+            t[v] = df_warp_sum_df( t[v] );
+        }
+        // a sum of squares is never negative: r.r = -1 (the second value) says that the wait ran out
+        if( lane == 0 ) *out = ok ? make_float4( t[0].hi, t[0].lo, t[1].hi, t[1].lo ) : make_float4( 0.f, 0.f, -1.f, 0.f );
+    }
+    __syncthreads();
+    const float4 o = *out;
+    sum[0] = DF{ o.x, o.y };
+    if( N > 1 ) sum[1] = DF{ o.z, o.w };
+    return o.z != -1.f;
+}
+
+// The block's sums of N values published under `tag`. FENCE: everything its threads have stored is
+// visible to a warp that acquires the words.
+template <int W, int N, bool FENCE>
+__device__ __forceinline__ void publish( ulonglong2* words, uint32_t tag, const DF* v, float2* w )
+{
+    DF t[N];
+#pragma unroll
+    for( int q = 0; q < N; ++q ) t[q] = df_warp_sum_df( v[q] );
+    const int wid = threadIdx.x >> 5;
+    if( ( threadIdx.x & 31 ) == 0 )
+#pragma unroll
+        for( int q = 0; q < N; ++q ) w[q * W + wid] = make_float2( t[q].hi, t[q].lo );
+    __syncthreads();
+    if( threadIdx.x == 0 )
+    {
+#pragma unroll
+        for( int q = 0; q < N; ++q )
+        {
+            t[q] = DF{ w[q * W].x, w[q * W].y };
+            for( int o = 1; o < W; ++o ) t[q] = df_add( t[q], DF{ w[q * W + o].x, w[q * W + o].y } );
+        }
+        if( FENCE ) asm volatile( "fence.acq_rel.gpu;" ::: "memory" );
+#pragma unroll
+        for( int q = 0; q < N; ++q ) store_words( words + (size_t)blockIdx.x * N + q, tagged( t[q], tag ) );
+    }
+    __syncwarp();  // lanes that went ahead to poll would hold up the one that publishes
+}
+
+template <int W>
+__global__ void __launch_bounds__( 32 * W, 1 ) k_pcg_resident( const __grid_constant__ PcgResidentArgs a )
+{
+    __shared__ float2 s_sum[3][W];  // the warps' r.z and r.r; d.q
+    __shared__ float4 s_met[2];     // the met sums
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, j = lane & 7, kq = lane >> 3;
+    const int cA = 8 * ( j + 16 * kq );  // row A = (j, 2 kq); row B = (j, 2 kq + 1) 64 cells on
+    const int t = blockIdx.x * W + ( threadIdx.x >> 5 );
+    const bool mine = t < a.ft.n;
+    float* const dg = a.dsel ? a.sv.d[1] : a.sv.d[0];
+    int4 n0 = make_int4( -1, -1, -1, -1 ), n1 = n0;
+    float rA[8], rB[8], dA[8], dB[8], eA[8], eB[8], mA[8], mB[8], zA[8], zB[8];
+    uint4 wA = make_uint4( 0u, 0u, 0u, 0u ), wB = wA;
+#pragma unroll
+    for( int i = 0; i < 8; ++i ) rA[i] = rB[i] = dA[i] = dB[i] = eA[i] = eB[i] = mA[i] = mB[i] = 0.f;
+    size_t g = 0;
+    if( mine )
+    {
+        n0 = a.ft.tab[2 * t];
+        n1 = a.ft.tab[2 * t + 1];
+        g = (size_t)n1.z * 512 + cA;
+        bora_ld8( a.sv.r + g, rA ); bora_ld8( a.sv.r + g + 64, rB );
+        bora_ld8( a.sv.minv + g, mA ); bora_ld8( a.sv.minv + g + 64, mB );
+        bora_ld8( dg + g, dA ); bora_ld8( dg + g + 64, dB );
+        wA = *reinterpret_cast<const uint4*>( a.code + g );
+        wB = *reinterpret_cast<const uint4*>( a.code + g + 64 );
+    }
+    // the neighbour tiles' cells that the lane's rows need: the x ends of both rows, the y face rows
+    // of lanes j = 0 / 7, the z face row of row A at k = 0 and of row B at k = 7
+    const int yt = j == 0 ? n0.z : ( j == 7 ? n0.w : -1 ), yc = cA + ( j == 0 ? 56 : -56 );
+    const int zt = kq == 0 ? n1.x : ( kq == 3 ? n1.y : -1 ), zc = 8 * j + ( kq == 0 ? 448 : 0 );
+    float hx[4], hyA[8], hyB[8], hz[8];  // their d
+    auto halo = [&]( const float* v, float* x, float* yA, float* yB, float* z ) {
+        auto one = [&]( int tl, int c ) { return tl < 0 ? 0.f : __ldcg( v + (size_t)tl * 512 + c ); };
+        auto row = [&]( int tl, int c, float* o ) {
+            const float4* p = reinterpret_cast<const float4*>( v + (size_t)( tl < 0 ? 0 : tl ) * 512 + ( tl < 0 ? 0 : c ) );
+            const float4 zero = make_float4( 0.f, 0.f, 0.f, 0.f );
+            const float4 l = tl < 0 ? zero : __ldcg( p ), h = tl < 0 ? zero : __ldcg( p + 1 );
+            o[0] = l.x; o[1] = l.y; o[2] = l.z; o[3] = l.w; o[4] = h.x; o[5] = h.y; o[6] = h.z; o[7] = h.w;
+        };
+        x[0] = one( n0.x, cA + 7 ); x[1] = one( n0.y, cA ); x[2] = one( n0.x, cA + 71 ); x[3] = one( n0.y, cA + 64 );
+        row( yt, yc, yA );
+        row( yt, yc + 64, yB );
+        row( zt, zc, z );
+    };
+    halo( dg, hx, hyA, hyB, hz );
+    // z = M^-1 r, stored for the neighbours, and the sums r.z and r.r
+    auto precondition = [&]( uint32_t tag ) {
+        DF v[2] = { { 0.f, 0.f }, { 0.f, 0.f } };
+#pragma unroll
+        for( int h = 0; h < 8; h += 4 )
+        {
+            const float4 x = make_float4( rA[h], rA[h + 1], rA[h + 2], rA[h + 3] ), y = make_float4( rB[h], rB[h + 1], rB[h + 2], rB[h + 3] );
+            v[1] = df_add_f( df_add_f( v[1], dot4( x, x ) ), dot4( y, y ) );
+        }
+#pragma unroll
+        for( int i = 0; i < 8; ++i ) { zA[i] = rA[i]; zB[i] = rB[i]; }
+        v[0] = df_add_f( v[0], mic_sweeps<true>( zA, zB, mA, mB ) );
+        if( mine )
+        {
+            bora_st8( a.sv.z + g, zA );
+            bora_st8( a.sv.z + g + 64, zB );
+        }
+        publish<W, 2, true>( a.words_rz, tag, v, &s_sum[0][0] );
+    };
+    uint32_t tag = a.tag;
+    DF rz_prev{ 0.f, 0.f }, sum[2];
+    bool cont = a.slot_rz_prev >= 0;  // the recurrence continues from d
+    if( cont ) rz_prev = DF{ a.red.ringf[a.slot_rz_prev].x, a.red.ringf[a.slot_rz_prev].y };
+#pragma unroll 1
+    for( int it = 0;; ++it, ++tag )
+    {
+        precondition( tag );
+        if( !meet<2, true>( a.words_rz, a, tag, sum, &s_met[0] ) ) return;
+        const DF rz = sum[0], rr = sum[1];
+        const bool small = !( rr.hi > 0.f ) || rr.hi < a.target2.x || ( rr.hi == a.target2.x && rr.lo <= a.target2.y );
+        if( it >= a.max_inner || ( it > 0 && __any_sync( kAll, small ) ) )
+        {
+            // the pass is done: it iterations
+            if( mine )
+            {
+                bora_st8( dg + g, dA ); bora_st8( dg + g + 64, dB );
+                bora_st8( a.sv.e + g, eA ); bora_st8( a.sv.e + g + 64, eB );
+            }
+            if( blockIdx.x == 0 && threadIdx.x == 0 )
+            {
+                ring_store( a.red, a.slot_a_rz, rz_prev, false );
+                a.red.part_rr[0] = make_float2( rr.hi, rr.lo );  // finished by the refinement
+                *(volatile uint32_t*)a.iters = (uint32_t)it;
+            }
+            return;
+        }
+        const float beta = cont ? df_ratio( make_float2( rz.hi, rz.lo ), make_float2( rz_prev.hi, rz_prev.lo ) ) : 0.f;
+        float q[8], tA[8], qA[8];
+        {
+            float x[4], yA[8], yB[8], z[8];
+            halo( a.sv.z, x, yA, yB, z );
+#pragma unroll
+            for( int i = 0; i < 8; ++i )
+            {
+                dA[i] = fmaf( beta, dA[i], zA[i] );
+                dB[i] = fmaf( beta, dB[i], zB[i] );
+                if( i < 4 ) hx[i] = fmaf( beta, hx[i], x[i] );
+                hyA[i] = fmaf( beta, hyA[i], yA[i] );
+                hyB[i] = fmaf( beta, hyB[i], yB[i] );
+                hz[i] = fmaf( beta, hz[i], z[i] );
+            }
+        }
+        auto stencil = [&]( const uint4& w, const float* d, const float* hy, const float* zm, const float* zp, float xm, float xp, float* o ) {
+            const uint32_t cw[4] = { w.x, w.y, w.z, w.w };
+#pragma unroll
+            for( int i = 0; i < 8; ++i )
+            {
+                float ym = __shfl_up_sync( kAll, d[i], 1 ), yp = __shfl_down_sync( kAll, d[i], 1 );
+                if( j == 0 ) ym = hy[i];
+                if( j == 7 ) yp = hy[i];
+                const uint32_t c = i & 1 ? cw[i >> 1] >> 16 : cw[i >> 1] & 0xffffu;
+                o[i] = 0.f;
+                if( c & BORA_CODE_FLUID )
+                {
+                    float acc = 0.f;
+                    acc += i > 0 ? d[i > 0 ? i - 1 : 0] : xm; acc += i < 7 ? d[i < 7 ? i + 1 : 7] : xp;
+                    acc += ym; acc += yp; acc += zm[i]; acc += zp[i];
+                    o[i] = fmaf( (float)code_diag( (uint16_t)c ), d[i], -acc );
+                }
+            }
+        };
+        {
+            float zm[8], zp[8];
+#pragma unroll
+            for( int i = 0; i < 8; ++i )
+            {
+                zm[i] = __shfl_up_sync( kAll, dB[i], 8 );
+                zp[i] = __shfl_down_sync( kAll, dA[i], 8 );
+                if( kq == 0 ) zm[i] = hz[i];
+                if( kq == 3 ) zp[i] = hz[i];
+            }
+            stencil( wA, dA, hyA, zm, dB, hx[0], hx[1], qA );
+            stencil( wB, dB, hyB, dA, zp, hx[2], hx[3], q );
+        }
+        DF pdq{ 0.f, 0.f };
+#pragma unroll
+        for( int i = 0; i < 8; ++i )
+        {
+            tA[i] = dA[i] * qA[i];
+            pdq = df_add_f( pdq, fmaf( dB[i], q[i], tA[i] ) );
+        }
+        publish<W, 1, false>( a.words_dq, ++tag, &pdq, &s_sum[2][0] );
+        DF dq;
+        if( !meet<1, false>( a.words_dq, a, tag, &dq, &s_met[1] ) ) return;
+        const float alpha = df_ratio( make_float2( rz.hi, rz.lo ), make_float2( dq.hi, dq.lo ) );
+#pragma unroll
+        for( int i = 0; i < 8; ++i )
+        {
+            eA[i] = fmaf( alpha, dA[i], eA[i] ); eB[i] = fmaf( alpha, dB[i], eB[i] );
+            rA[i] = fmaf( -alpha, qA[i], rA[i] ); rB[i] = fmaf( -alpha, q[i], rB[i] );
+        }
+        rz_prev = rz;
+        cont = true;
     }
 }
 
@@ -1284,6 +1616,57 @@ int bora_launch_pcg_persistent( BoraSolveTilesDev t, const uint16_t* code, BoraS
                    cudaSuccess
                ? 0
                : -1;
+}
+
+namespace {
+constexpr int kResidentBlocks = 152;  // one block per SM; at most 160 (meet)
+template <int W>
+int resident_fits()  // 1 when the device can run the largest grid of k_pcg_resident<W> at once
+{
+    static BoraPerDevice per_sm;
+    const int b = per_sm.get( [] {
+        int v = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor( &v, k_pcg_resident<W>, 32 * W, 0 ) == cudaSuccess && v > 0 ? v : -1;
+    } );
+    return b > 0 && b * num_sms() >= kResidentBlocks;
+}
+}  // namespace
+
+// Warps per block, 0: not for this form. One warp per SM partition up to 256 tiles; above, two, as
+// the blocks poll one another and the meetings grow with their number (464 tiles: 11.2 us per
+// iteration in 116 blocks, 9.6 in 58). From 680 tiles on the per-phase form is level.
+int bora_pcg_resident_warps( int nft )
+{
+    if( nft <= 0 ) return 0;
+    if( nft <= 256 ) return resident_fits<4>() ? 4 : 0;
+    return nft <= 608 && resident_fits<8>() ? 8 : 0;
+}
+
+size_t bora_pcg_resident_words_bytes() { return (size_t)3 * ( kResidentBlocks + 8 ) * sizeof( ulonglong2 ); }
+
+int bora_launch_pcg_resident( BoraSolveTilesDev t, const uint16_t* code, BoraSolverDev s, BoraReduceDev red, int dsel,
+                              int slot_rz_prev, int max_inner, double target, int slot_a_rz, uint32_t* iters, void* words,
+                              uint32_t tag, bool never_release, cudaStream_t st )
+{
+    const int W = bora_pcg_resident_warps( t.n );
+    if( W == 0 ) return -1;
+    PcgResidentArgs a{};
+    a.ft = t; a.code = code; a.sv = s; a.red = red; a.dsel = dsel; a.slot_rz_prev = slot_rz_prev; a.max_inner = max_inner;
+    const double t2 = target * target;
+    const float hi = (float)t2;
+    a.target2 = make_float2( hi, (float)( t2 - (double)hi ) );
+    a.slot_a_rz = slot_a_rz; a.iters = iters;
+    a.words_rz = static_cast<ulonglong2*>( words );
+    a.words_dq = a.words_rz + 2 * ( kResidentBlocks + 8 );
+    a.tag = tag;
+    const int grid = ( t.n + W - 1 ) / W;
+    // a meeting that waits for one block more than there are never ends: every wait runs out (fault
+    // injection for tests), after a short limit
+    a.expect = (unsigned)grid + ( never_release ? 1u : 0u );
+    a.limit = never_release ? ( 1u << 12 ) : ( 1u << 21 );
+    void* args[] = { &a };
+    const void* k = W == 4 ? (const void*)k_pcg_resident<4> : (const void*)k_pcg_resident<8>;
+    return cudaLaunchCooperativeKernel( k, dim3( grid ), dim3( 32 * W ), args, 0, st ) == cudaSuccess ? 0 : -1;
 }
 
 void bora_launch_pcg_direction( BoraSolveTilesDev t, const uint16_t* code, BoraSolverDev s, int dsel_in, BoraReduceDev red, int nparts, int slot_rz_new, int slot_rr, int slot_rz_old,
