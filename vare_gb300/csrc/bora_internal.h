@@ -184,6 +184,10 @@ void bora_launch_p2g( const BoraGridDev& g, int ntiles, BoraTilesDev t, BoraPart
 // tile_fluid: 1 for the tiles with a fluid cell
 void bora_launch_rhs( const BoraGridDev& g, int ntiles, BoraTilesDev t, BoraCellsDev c, uint32_t* nfluid, uint8_t* tile_fluid,
                       cudaStream_t st );
+// list[stride * q + offset] = the q-th flagged of n items (flags 0 or 1, readable up to a multiple of 16);
+// their number on the device and in mapped host memory
+void bora_launch_flag_list( int n, const uint8_t* flags, int32_t* list, int stride, int offset, uint32_t* count,
+                            uint32_t* host_count, cudaStream_t st );
 // the same flags from stencil codes that the caller has set
 void bora_launch_tile_fluid( int ntiles, const uint16_t* code, uint8_t* tile_fluid, cudaStream_t st );
 // the solver's tile table and count (also written to host_count, mapped host memory) from the flags
@@ -209,14 +213,28 @@ void bora_launch_particle_attributes( const BoraGridDev& g, const int32_t* slot_
                                       float3 scale, float dis, cudaStream_t st );
 
 // ---- sparse -> VDB leaf export (FieldCast convertSurfaceVDB / convertVelocityVDB) ------
-// leaf_ijk: 3 ints (voxel origin) per leaf; leaf_slot: its tile's slot or -1 (band leaf);
-// mask: 8 x 64 bits per leaf; val: 512 (surface) or 3 x 512 (velocity) floats per leaf.
-void bora_launch_vdb_surface( const BoraGridDev& g, const float* scale, const float* translate, int nleaves,
-                              const int32_t* leaf_ijk, const int32_t* leaf_slot, const float* surf, float bg, int tank,
-                              float level, uint64_t* mask, float* val, cudaStream_t st );
-void bora_launch_vdb_velocity( const BoraGridDev& g, const float* scale, int nleaves, const int32_t* leaf_ijk,
-                               const int32_t* leaf_slot, const float* vx, const float* vy, const float* vz,
-                               uint64_t* mask, float* val, cudaStream_t st );
+// Candidate leaves: four ints each, the voxel origin and the tile's slot or -1 (band leaf).
+// bora_launch_vdb_leaves: those of the active tiles. A launch with flag != null flags the
+// candidates that have an active voxel; one with keep != null writes the `n` kept ones (indices
+// keep[q]) packed: origin 3 ints, mask 8 x 64 bits, val 512 (surface) or 3 x 512 (velocity) floats.
+struct BoraVdbOut
+{
+    int n;                // leaves of this launch
+    const int4* leaf;
+    uint8_t* flag;
+    const int32_t* keep;
+    int32_t* origin;
+    uint64_t* mask;
+    float* val;
+};
+void bora_launch_vdb_leaves( const BoraGridDev& g, int ntiles, const int32_t* tile_of, int4* leaf, cudaStream_t st );
+void bora_launch_vdb_surface( const BoraGridDev& g, const float* scale, const float* translate, const BoraVdbOut& o,
+                              const float* surf, float bg, int tank, float level, cudaStream_t st );
+void bora_launch_vdb_velocity( const BoraGridDev& g, const float* scale, const BoraVdbOut& o, const float* vx, const float* vy,
+                               const float* vz, cudaStream_t st );
+// three component fields <-> x, y, z interleaved (n cells, a multiple of 4)
+void bora_launch_interleave( size_t n, const float* x, const float* y, const float* z, float* out, cudaStream_t st );
+void bora_launch_deinterleave( size_t n, const float* in, float* x, float* y, float* z, cudaStream_t st );
 int bora_vdb_level_index( float level, float min_y, float dx );
 // tile coordinates (3 ints each) of the water tank's border band (FieldCast.h:398-440)
 void bora_vdb_band_tiles( const BoraGridDev& g, const float* scale, const float* translate, float level,

@@ -2182,27 +2182,19 @@ int bora_flip_export_vdb( bora_flip_handle s, int which, int32_t* origins, uint6
     const float bg = which == BORA_VDB_SURFACE ? kSurfaceBackground : 0.f;
     if( background ) *background = bg * dx;
     // candidate leaves: the active tiles, then (surface, water tank) the band's other tiles
+    cudaStream_t st = s->st;
     const size_t nt = (size_t)s->ntiles;
-    std::vector<int32_t> lin( nt );
-    if( nt )
-    {
-        BORA_TRY( cudaMemcpyAsync( lin.data(), s->tile_of.p, nt * 4, cudaMemcpyDeviceToHost, s->st ) );
-        BORA_TRY( cudaStreamSynchronize( s->st ) );
-    }
-    const int tx = s->g.tx, ty = s->g.ty, tz = s->g.tz;
-    std::vector<int32_t> leaf;  // per leaf: i, j, k origin, slot
-    leaf.reserve( nt * 4 );
-    for( size_t t = 0; t < nt; ++t )
-    {
-        leaf.push_back( 8 * ( lin[t] % tx ) );
-        leaf.push_back( 8 * ( ( lin[t] / tx ) % ty ) );
-        leaf.push_back( 8 * ( lin[t] / ( tx * ty ) ) );
-        leaf.push_back( (int32_t)t );
-    }
     const bool tank = which == BORA_VDB_SURFACE && s->prm.enable_water_tank;
+    std::vector<int32_t> band_leaf;  // i, j, k origin, slot -1
     if( tank )
     {
-        std::vector<int32_t> band;
+        const int tx = s->g.tx, ty = s->g.ty, tz = s->g.tz;
+        std::vector<int32_t> lin( nt ), band;
+        if( nt )
+        {
+            BORA_TRY( cudaMemcpyAsync( lin.data(), s->tile_of.p, nt * 4, cudaMemcpyDeviceToHost, st ) );
+            BORA_TRY( cudaStreamSynchronize( st ) );
+        }
         bora_vdb_band_tiles( s->g, s->scale, s->translate, s->prm.wall_level, band );
         std::vector<uint8_t> active( (size_t)tx * ty * tz, 0 );
         for( size_t t = 0; t < nt; ++t ) active[(size_t)lin[t]] = 1;
@@ -2211,61 +2203,58 @@ int bora_flip_export_vdb( bora_flip_handle s, int which, int32_t* origins, uint6
             const int ti = band[b], tj = band[b + 1], tk = band[b + 2];
             const bool inside = ti >= 0 && tj >= 0 && tk >= 0 && ti < tx && tj < ty && tk < tz;
             if( inside && active[( (size_t)tk * ty + tj ) * tx + ti] ) continue;
-            leaf.push_back( 8 * ti );
-            leaf.push_back( 8 * tj );
-            leaf.push_back( 8 * tk );
-            leaf.push_back( -1 );
+            const int32_t e[4] = { 8 * ti, 8 * tj, 8 * tk, -1 };
+            band_leaf.insert( band_leaf.end(), e, e + 4 );
         }
     }
-    const size_t nl = leaf.size() / 4;
+    const size_t nl = nt + band_leaf.size() / 4;
     if( nl == 0 ) return BORA_OK;
     const size_t comps = which == BORA_VDB_SURFACE ? 1 : 3;
-    BORA_TRY( grow( s->vdb_leaf, nl * 16, false, s->st ) );
-    BORA_TRY( grow( s->vdb_mask, nl * 64, false, s->st ) );
-    BORA_TRY( grow( s->vdb_val, nl * 512 * comps * 4, false, s->st ) );
-    std::vector<int32_t> ijk( nl * 3 ), slot( nl );
-    for( size_t l = 0; l < nl; ++l )
-    {
-        for( int a = 0; a < 3; ++a ) ijk[3 * l + a] = leaf[4 * l + a];
-        slot[l] = leaf[4 * l + 3];
-    }
-    int32_t* d_ijk = P<int32_t>( s->vdb_leaf );
-    int32_t* d_slot = d_ijk + 3 * nl;
-    BORA_TRY( cudaMemcpyAsync( d_ijk, ijk.data(), nl * 12, cudaMemcpyHostToDevice, s->st ) );
-    BORA_TRY( cudaMemcpyAsync( d_slot, slot.data(), nl * 4, cudaMemcpyHostToDevice, s->st ) );
-    if( which == BORA_VDB_SURFACE )
-        bora_launch_vdb_surface( s->g, s->scale, s->translate, (int)nl, d_ijk, d_slot, P<float>( s->surf ), bg, tank ? 1 : 0,
-                                 s->prm.wall_level, P<uint64_t>( s->vdb_mask ), P<float>( s->vdb_val ), s->st );
-    else
-        bora_launch_vdb_velocity( s->g, s->scale, (int)nl, d_ijk, d_slot, P<float>( s->vx ), P<float>( s->vy ),
-                                  P<float>( s->vz ), P<uint64_t>( s->vdb_mask ), P<float>( s->vdb_val ), s->st );
-    s->stats.kernel_launches += 1;
-    BORA_TRYS( check_launch( s ) );
-    std::vector<uint64_t> m( nl * 8 );
-    BORA_TRY( cudaMemcpyAsync( m.data(), s->vdb_mask.p, nl * 64, cudaMemcpyDeviceToHost, s->st ) );
-    BORA_TRY( cudaStreamSynchronize( s->st ) );
+    // per candidate: origin and slot, its place among the kept, its flag (padded to 16)
+    BORA_TRY( grow( s->vdb_leaf, nl * 20 + ( nl + 15 ) / 16 * 16, false, st ) );
+    int4* d_leaf = P<int4>( s->vdb_leaf );
+    uint8_t* d_flag = reinterpret_cast<uint8_t*>( d_leaf + nl );
+    int32_t* d_keep = reinterpret_cast<int32_t*>( d_flag + ( nl + 15 ) / 16 * 16 );
+    BoraVdbOut o{};
+    o.leaf = d_leaf;
+    auto launch = [&] {
+        s->stats.kernel_launches += 1;
+        if( which == BORA_VDB_SURFACE )
+            bora_launch_vdb_surface( s->g, s->scale, s->translate, o, P<float>( s->surf ), bg, tank ? 1 : 0, s->prm.wall_level, st );
+        else bora_launch_vdb_velocity( s->g, s->scale, o, P<float>( s->vx ), P<float>( s->vy ), P<float>( s->vz ), st );
+    };
+    s->stats.kernel_launches += 2;
+    bora_launch_vdb_leaves( s->g, s->ntiles, P<int32_t>( s->tile_of ), d_leaf, st );
+    if( !band_leaf.empty() )
+        BORA_TRY( cudaMemcpyAsync( d_leaf + nt, band_leaf.data(), band_leaf.size() * 4, cudaMemcpyHostToDevice, st ) );
+    o.n = (int)nl;
+    o.flag = d_flag;
+    launch();
     // leaves without an active voxel are not written (OpenVDB creates no leaf for them)
-    std::vector<size_t> keep;
-    keep.reserve( nl );
-    for( size_t l = 0; l < nl; ++l )
-    {
-        uint64_t any = 0;
-        for( int w = 0; w < 8; ++w ) any |= m[8 * l + w];
-        if( any ) keep.push_back( l );
-    }
-    *nleaves = keep.size();
+    ( (volatile uint32_t*)s->h_cnt )[10] = kCountNotArrived;
+    bora_launch_flag_list( (int)nl, d_flag, d_keep, 1, 0, P<uint32_t>( s->counters ) + 10, s->d_cnt + 10, st );
+    BORA_TRYS( check_launch( s ) );
+    uint32_t kept = 0;
+    BORA_TRYS( poll_mapped( (volatile uint32_t*)s->h_cnt + 10, kCountNotArrived, st, &kept ) );
+    if( !band_leaf.empty() ) BORA_TRY( cudaStreamSynchronize( st ) );  // the host list goes out of scope
+    *nleaves = kept;
     if( !origins ) return BORA_OK;
-    if( cap_leaves < keep.size() || !masks || !values ) return cap_leaves < keep.size() ? BORA_ERR_CAPACITY : BORA_ERR_INVALID_ARG;
-    const size_t per = 512 * comps;
-    for( size_t q = 0; q < keep.size(); ++q )
-    {
-        const size_t l = keep[q];
-        for( int a = 0; a < 3; ++a ) origins[3 * q + a] = ijk[3 * l + a];
-        for( int w = 0; w < 8; ++w ) masks[8 * q + w] = m[8 * l + w];
-        BORA_TRY( cudaMemcpyAsync( values + q * per, P<float>( s->vdb_val ) + l * per, per * 4, cudaMemcpyDeviceToHost,
-                                   s->st ) );
-    }
-    BORA_TRY( cudaStreamSynchronize( s->st ) );
+    if( cap_leaves < kept || !masks || !values ) return cap_leaves < kept ? BORA_ERR_CAPACITY : BORA_ERR_INVALID_ARG;
+    if( kept == 0 ) return BORA_OK;
+    BORA_TRY( grow( s->vdb_mask, (size_t)kept * ( 64 + 12 ), false, st ) );
+    BORA_TRY( grow( s->vdb_val, (size_t)kept * 512 * comps * 4, false, st ) );
+    o.n = (int)kept;
+    o.flag = nullptr;
+    o.keep = d_keep;
+    o.mask = P<uint64_t>( s->vdb_mask );
+    o.origin = reinterpret_cast<int32_t*>( o.mask + (size_t)kept * 8 );
+    o.val = P<float>( s->vdb_val );
+    launch();
+    BORA_TRYS( check_launch( s ) );
+    BORA_TRY( cudaMemcpyAsync( origins, o.origin, (size_t)kept * 12, cudaMemcpyDeviceToHost, st ) );
+    BORA_TRY( cudaMemcpyAsync( masks, o.mask, (size_t)kept * 64, cudaMemcpyDeviceToHost, st ) );
+    BORA_TRY( cudaMemcpyAsync( values, o.val, (size_t)kept * 512 * comps * 4, cudaMemcpyDeviceToHost, st ) );
+    BORA_TRY( cudaStreamSynchronize( st ) );
     return BORA_OK;
 }
 
@@ -2302,14 +2291,14 @@ int bora_flip_get_field( bora_flip_handle s, int which, void* out, size_t bytes 
         BORA_TRY( cudaStreamSynchronize( s->st ) );
         return BORA_OK;
     }
-    std::vector<float> tmp( ncell );
-    float* o = (float*)out;
-    for( int c = 0; c < nc; ++c )
-    {
-        BORA_TRY( cudaMemcpyAsync( tmp.data(), b[c]->p, ncell * 4, cudaMemcpyDeviceToHost, s->st ) );
-        BORA_TRY( cudaStreamSynchronize( s->st ) );
-        for( size_t i = 0; i < ncell; ++i ) o[3 * i + c] = tmp[i];
-    }
+    // a vector field is interleaved on the device and copied once
+    if( ncell == 0 ) return BORA_OK;
+    BORA_TRY( grow( s->stage_out, ncell * 12, false, s->st ) );
+    s->stats.kernel_launches += 1;
+    bora_launch_interleave( ncell, P<float>( *b[0] ), P<float>( *b[1] ), P<float>( *b[2] ), P<float>( s->stage_out ), s->st );
+    BORA_TRYS( check_launch( s ) );
+    BORA_TRY( cudaMemcpyAsync( out, s->stage_out.p, ncell * 12, cudaMemcpyDeviceToHost, s->st ) );
+    BORA_TRY( cudaStreamSynchronize( s->st ) );
     return BORA_OK;
 }
 
@@ -2329,14 +2318,13 @@ int bora_flip_set_field( bora_flip_handle s, int which, const void* in, size_t b
         BORA_TRY( cudaStreamSynchronize( s->st ) );
         return BORA_OK;
     }
-    std::vector<float> tmp( ncell );
-    const float* src = (const float*)in;
-    for( int c = 0; c < nc; ++c )
-    {
-        for( size_t i = 0; i < ncell; ++i ) tmp[i] = src[3 * i + c];
-        BORA_TRY( cudaMemcpyAsync( b[c]->p, tmp.data(), ncell * 4, cudaMemcpyHostToDevice, s->st ) );
-        BORA_TRY( cudaStreamSynchronize( s->st ) );
-    }
+    if( ncell == 0 ) return BORA_OK;
+    BORA_TRY( grow( s->stage_in, ncell * 12, false, s->st ) );
+    BORA_TRY( cudaMemcpyAsync( s->stage_in.p, in, ncell * 12, cudaMemcpyHostToDevice, s->st ) );
+    s->stats.kernel_launches += 1;
+    bora_launch_deinterleave( ncell, P<float>( s->stage_in ), P<float>( *b[0] ), P<float>( *b[1] ), P<float>( *b[2] ), s->st );
+    BORA_TRYS( check_launch( s ) );
+    BORA_TRY( cudaStreamSynchronize( s->st ) );  // the caller may free its buffer on return
     return BORA_OK;
 }
 

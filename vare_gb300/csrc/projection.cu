@@ -139,26 +139,26 @@ __global__ void k_tile_fluid( int ntiles, const uint16_t* __restrict__ code, uin
     }
 }
 
-// One CTA: the slots of the flagged tiles, in order, into the own entries of the table, 16 flags
-// per thread and round (a few microseconds for 50 K tiles), and their number.
-__global__ void __launch_bounds__( 1024 ) k_solve_tiles( int ntiles, const uint8_t* __restrict__ tile_fluid, int32_t* __restrict__ tab,
-                                                         uint32_t* count, uint32_t* host_count )
+// One CTA: the indices of the flagged (1, not 0) of n items, in order, into out[stride * q + offset],
+// and their number; 16 flags per thread and round (a few microseconds for 50 K items).
+__global__ void __launch_bounds__( 1024 ) k_flag_list( int n, const uint8_t* __restrict__ flags, int32_t* __restrict__ list,
+                                                       int stride, int offset, uint32_t* count, uint32_t* host_count )
 {
     __shared__ int wsum[32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int carry = 0;
-    for( int base = 0; base < ntiles; base += 16 * 1024 )
+    for( int base = 0; base < n; base += 16 * 1024 )
     {
         const int s0 = base + 16 * (int)threadIdx.x;
         uint32_t w[4] = { 0u, 0u, 0u, 0u };
-        if( s0 < ntiles )  // the flags are padded to a multiple of 16
+        if( s0 < n )  // the flags are padded to a multiple of 16
         {
-            const uint4 f = *reinterpret_cast<const uint4*>( tile_fluid + s0 );
+            const uint4 f = *reinterpret_cast<const uint4*>( flags + s0 );
             w[0] = f.x; w[1] = f.y; w[2] = f.z; w[3] = f.w;
 #pragma unroll
             for( int q = 0; q < 4; ++q )
                 for( int b = 0; b < 4; ++b )
-                    if( s0 + 4 * q + b >= ntiles ) w[q] &= ~( 0xffu << ( 8 * b ) );
+                    if( s0 + 4 * q + b >= n ) w[q] &= ~( 0xffu << ( 8 * b ) );
         }
         const int mine = __popc( w[0] ) + __popc( w[1] ) + __popc( w[2] ) + __popc( w[3] );  // flags are 0 or 1
         int inc = mine;
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__( 1024 ) k_solve_tiles( int ntiles, const uint8
         __syncthreads();
         int out = carry + inc - mine + ( wid ? wsum[wid - 1] : 0 );
         for( int b = 0; b < 16; ++b )
-            if( ( w[b >> 2] >> ( 8 * ( b & 3 ) ) ) & 1u ) tab[8 * (size_t)out++ + 6] = s0 + b;
+            if( ( w[b >> 2] >> ( 8 * ( b & 3 ) ) ) & 1u ) list[stride * (size_t)out++ + offset] = s0 + b;
         carry += wsum[31];
         __syncthreads();  // wsum is rewritten next
     }
@@ -1486,10 +1486,16 @@ void bora_launch_tile_fluid( int ntiles, const uint16_t* code, uint8_t* tile_flu
     if( ntiles > 0 ) k_tile_fluid<<<grid_for( (size_t)ntiles * 32, 256 ), 256, 0, st>>>( ntiles, code, tile_fluid );
 }
 
+void bora_launch_flag_list( int n, const uint8_t* flags, int32_t* list, int stride, int offset, uint32_t* count,
+                            uint32_t* host_count, cudaStream_t st )
+{
+    k_flag_list<<<1, 1024, 0, st>>>( n, flags, list, stride, offset, count, host_count );
+}
+
 void bora_launch_solve_tiles( int ntiles, BoraTilesDev t, const uint8_t* tile_fluid, int4* tab, uint32_t* count,
                               uint32_t* host_count, cudaStream_t st )
 {
-    k_solve_tiles<<<1, 1024, 0, st>>>( ntiles, tile_fluid, reinterpret_cast<int32_t*>( tab ), count, host_count );
+    bora_launch_flag_list( ntiles, tile_fluid, reinterpret_cast<int32_t*>( tab ), 8, 6, count, host_count, st );
     if( ntiles > 0 )
         k_solve_nbrs<<<grid_for( (size_t)ntiles * 8, 256 ), 256, 0, st>>>( count, t.nbr, tile_fluid, reinterpret_cast<int32_t*>( tab ) );
 }
