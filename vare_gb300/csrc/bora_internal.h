@@ -450,12 +450,17 @@ __device__ __forceinline__ int bora_batch_member( const BoraBatchLaunch& L, unsi
 
 // The coarse cluster kernel of a batch: a simulation's descriptor (opaque, desc_bytes each;
 // 0 when its hierarchy does not fit the kernel), and one launch of `blocks` CTAs: one
-// cluster of `ctas` CTAs per simulation taking part (all of the same size; shared memory
-// for the largest).
+// cluster of `ctas` CTAs per simulation taking part (all of the same size; threads and
+// shared memory for the largest: neither they nor ctas change a value's arithmetic).
+struct BoraMidShape
+{
+    int ctas, threads;
+    size_t smem;
+};
 size_t bora_mg_mid_desc_bytes();
 int bora_mg_mid_describe( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t, int ntiles,
-                          const void* image, uint32_t* err, int sweeps, void* desc, size_t* smem, int* ctas );
-void bora_mg_mid_launch_batch( const void* descs, const BoraBatchLaunch& L, int blocks, int ctas, size_t smem,
+                          const void* image, uint32_t* err, int sweeps, void* desc, BoraMidShape* shape );
+void bora_mg_mid_launch_batch( const void* descs, const BoraBatchLaunch& L, int blocks, const BoraMidShape& shape,
                                cudaStream_t st );
 // Batched launches of the solver kernels (projection.cu, multigrid.cu) with `blocks` =
 // start[n] blocks in all.

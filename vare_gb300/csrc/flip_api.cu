@@ -1530,8 +1530,10 @@ int batch_solve( std::vector<BatchMember>& M, cudaStream_t st, BatchBuffers& bb 
     std::vector<BoraMemberSolve> ms( n );
     const size_t dbytes = bora_mg_mid_desc_bytes();
     std::vector<char> mid( dbytes * n );
-    int ctas = 0;
-    size_t smem = 0;
+    // the coarse kernel: one launch for the simulations whose levels run in one CTA, one for
+    // those in a cluster
+    BoraMidShape mid_shape[2] = {};
+    std::vector<int> mid_ctas( n );
     // the launch shapes of the multigrid passes for this batch (the autotuner's choice for
     // the batch's total size; every shape gives the same results)
     int total_tiles = 0;
@@ -1562,18 +1564,18 @@ int batch_solve( std::vector<BatchMember>& M, cudaStream_t st, BatchBuffers& bb 
         for( int l = 0; l < 4; ++l ) m.L[l] = s->levels[l];
         m.z3 = s->levels[3].z0;
         bora_member_grids( s->nft, m.grid, tv );
-        size_t sm = 0;
-        int c = 0;
+        BoraMidShape sh{};
         if( !bora_mg_mid_describe( s->g, s->levels, s->nlevels, s->tiles(), s->ntiles, s->mg_mid.p,
-                                   P<uint32_t>( s->counters ) + 5, 16, mid.data() + dbytes * k, &sm, &c ) )
+                                   P<uint32_t>( s->counters ) + 5, 16, mid.data() + dbytes * k, &sh ) )
             return BORA_ERR_INTERNAL;
-        if( ctas && c != ctas ) return BORA_ERR_INTERNAL;
-        ctas = c;
-        smem = std::max( smem, sm );
+        BoraMidShape& m2 = mid_shape[sh.ctas > 1];
+        if( m2.ctas && sh.ctas != m2.ctas ) return BORA_ERR_INTERNAL;
+        m2 = BoraMidShape{ sh.ctas, std::max( m2.threads, sh.threads ), std::max( m2.smem, sh.smem ) };
+        mid_ctas[k] = sh.ctas;
     }
     // a launch group's arguments: the slots, then per kernel (and the coarse cluster kernel)
     // the n + 1 block offsets of the simulations taking part
-    constexpr int kRows = kGridCount + 1;
+    constexpr int kRows = kGridCount + 2;
     const size_t sl_bytes = sizeof( BoraMemberSlots ) * n;
     const size_t grp_bytes = sl_bytes + sizeof( int ) * kRows * ( n + 1 );
     BORA_TRY( grow( bb.ms, sizeof( BoraMemberSolve ) * n, false, st ) );
@@ -1598,7 +1600,9 @@ int batch_solve( std::vector<BatchMember>& M, cudaStream_t st, BatchBuffers& bb 
             for( int k = 0; k < n; ++k )
             {
                 start[q * ( n + 1 ) + k] = acc;
-                if( sl[k].active ) acc += q < kGridCount ? ms[k].grid[q] : ctas;
+                if( !sl[k].active ) continue;
+                if( q < kGridCount ) acc += ms[k].grid[q];
+                else if( ( q == kGridCount ) == ( mid_ctas[k] == 1 ) ) acc += mid_ctas[k];
             }
             start[q * ( n + 1 ) + n] = acc;
             blocks[q] = acc;
@@ -1619,7 +1623,9 @@ int batch_solve( std::vector<BatchMember>& M, cudaStream_t st, BatchBuffers& bb 
                 bora_launch_mg_pass_batch( l, p, tv[l], launch( q ), blocks[q], st );
             }
         }
-        bora_mg_mid_launch_batch( bb.mid.p, launch( kGridCount ), blocks[kGridCount], ctas, smem, st );
+        for( int q = 0; q < 2; ++q )
+            bora_mg_mid_launch_batch( bb.mid.p, launch( kGridCount + q ), blocks[kGridCount + q], mid_shape[q], st );
+        launches += blocks[kGridCount] > 0 && blocks[kGridCount + 1] > 0;
         for( int l = 2; l >= 0; --l )
             for( int p = 2; p < 4; ++p )
             {

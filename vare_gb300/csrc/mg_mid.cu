@@ -17,6 +17,12 @@
 // shared memory: a CTA reads other cells' values from the owning CTA's shared memory
 // through the cluster window and writes only its own.
 //
+// An operation is one chain of latencies (references, values, store, barrier), so its loads
+// are issued together, without a branch on the neighbour or its owner: 1200-1600 cycles
+// instead of 2400-4400 with one dependent load after another. At 256^3 (9.4 K level-3 cells)
+// the kernel takes 33 K cycles instead of 52 K, at 96^3 (726 cells, one CTA) 15 K instead of
+// 29 K; a whole V-cycle there went from 137 to 128 us and from 57 to 48 us.
+//
 // The arithmetic is the V-cycle of multigrid.cu: per level two Jacobi sweeps before
 // (kOmegaA from zero, then kOmegaB) and after (kOmegaB, then kOmegaA), the residual
 // restricted as 0.5 * sum of the 8 children, injection as prolongation, and damped Jacobi
@@ -47,12 +53,20 @@ constexpr float kOmega = 0.9f;      // coarsest level: damped Jacobi
 constexpr float kOmegaA = 0.5687f;  // Chebyshev pair of the smoothers (multigrid.cu)
 constexpr float kOmegaB = 1.6902f;
 
-constexpr int kMidThreads = 512;
+// Threads per CTA: one per level-3 cell within these bounds (a cluster barrier costs 611
+// cycles with 256 threads a CTA and 924 with 1024, whatever the cluster's size).
+constexpr int kMidThreadsMin = 256, kMidThreadsMax = 1024;
+// Level-3 cells up to which one CTA runs the levels, with its own barrier and loads, instead
+// of a cluster of 16. Cycles from the level-2 residual on: 12.3 K against 16.3 K at 726
+// cells, 15.6 K against 19.7 K at 1526, but 24.0 K against 22.4 K at 2568.
+constexpr int kMidSingleMax = 2048;
 constexpr int kMidMaxLevels = 8;
 constexpr int kMidCtasMax = 16;  // non-portable cluster size where the device allows it
-constexpr size_t kMidSmemMax = 200 * 1024;
+constexpr size_t kMidSmemMax = 200 * 1024 + 512;
 
-// A packed reference to a cell: owning CTA in bits 24-31, local index in bits 0-23; -1 none.
+// A packed reference to a cell: owning CTA in bits 24-31, local index in bits 0-23. Every
+// value array has one more entry than the CTA has cells, which stays 0: a reference that
+// names no cell points there, so an operation issues all of its loads at once.
 __device__ inline int32_t pack_ref( int owner, int local ) { return ( owner << 24 ) | local; }
 
 struct MidLevel
@@ -77,7 +91,7 @@ struct MidDesc
     const __half* r_in;  // level-3 residual (written by the level-2 down kernel)
     __half* z_out;       // level-3 correction (read by the level-2 up kernel)
     int sweeps;
-    int ctas;
+    int ctas, threads;
     int static_bytes;    // bytes of a CTA's static block (a multiple of 16)
     char* image;         // ctas static blocks, built by k_mg_mid_image
     uint32_t* err;       // inconsistent stencil codes are recorded here
@@ -85,11 +99,17 @@ struct MidDesc
 
 extern __shared__ __align__( 16 ) char g_mid_smem[];
 
+// In the image: the code names a fluid neighbour that does not exist. Recorded in d.err when
+// the V-cycle first loads the cell's code; the neighbour counts as 0.
+constexpr uint16_t kCodeBad = 0x4000;
+
 __device__ inline int code_diag( uint16_t c ) { return ( c >> 8 ) & 15; }
 
 // face directions in the 27-entry tile neighbour table: -x +x -y +y -z +z
 __device__ __constant__ int kFaceDir[6] = { 12, 14, 10, 16, 4, 22 };
 
+// ONE: the cluster is one CTA.
+template <bool ONE>
 struct Mid
 {
     const MidDesc& d;
@@ -104,25 +124,28 @@ struct Mid
     }
     __device__ int32_t ref( const MidLevel& L, int c ) const  // packed reference of cell c of L
     {
-        if( c < 0 ) return -1;
         const int o = c / L.chunk;
         return pack_ref( o, c - o * L.chunk );
     }
-    // the value at a packed reference in array `off`: a shared-memory load when this CTA owns
-    // the cell, else a load from the owning CTA's shared memory through the cluster window
+    __device__ int32_t zero_ref( const MidLevel& L ) const { return pack_ref( (int)me, L.chunk ); }
+    // the value at a packed reference in array `off`, from the owning CTA's shared memory
+    // (volatile: stays between the barriers; no branch on the owner, so that the loads of
+    // an operation are in flight together)
     __device__ float ld( int off, int32_t rf ) const
     {
-        const unsigned o = (unsigned)rf >> 24;
-        const int i = rf & 0xFFFFFF;
-        if( o == me ) return arr<float>( off )[i];
-        const uint32_t sa = (uint32_t)__cvta_generic_to_shared( arr<float>( off ) + i );
+        if( ONE ) return arr<float>( off )[rf & 0xFFFFFF];
+        const uint32_t sa = (uint32_t)__cvta_generic_to_shared( g_mid_smem ) + (uint32_t)off + (uint32_t)( rf & 0xFFFFFF ) * 4u;
         uint32_t ra;
         float v;
-        asm volatile( "mapa.shared::cluster.u32 %0, %1, %2;" : "=r"( ra ) : "r"( sa ), "r"( o ) );
-        asm volatile( "ld.shared::cluster.f32 %0, [%1];" : "=f"( v ) : "r"( ra ) : "memory" );
+        asm volatile( "mapa.shared::cluster.u32 %0, %1, %2;" : "=r"( ra ) : "r"( sa ), "r"( (uint32_t)rf >> 24 ) );
+        asm volatile( "ld.shared::cluster.f32 %0, [%1];" : "=f"( v ) : "r"( ra ) );
         return v;
     }
-    __device__ void barrier() const { cl.sync(); }
+    __device__ void barrier() const
+    {
+        if( ONE ) __syncthreads();
+        else cl.sync();
+    }
 
     // static data of level t for the owned cells (codes, neighbours, parent, children),
     // written into the block at `blk` (the CTA's slice of the image)
@@ -132,10 +155,11 @@ struct Mid
         const int n = owned( L ), base = (int)me * L.chunk;
         uint16_t* code = reinterpret_cast<uint16_t*>( blk + L.o_code );
         int32_t* nb = reinterpret_cast<int32_t*>( blk + L.o_nb );
-        for( int i = threadIdx.x; i < n; i += kMidThreads ) code[i] = L.code[base + i];
-        for( int i = threadIdx.x; i < n * 6; i += kMidThreads )
+        for( int i = threadIdx.x; i < n; i += (int)blockDim.x ) code[i] = L.code[base + i];
+        __syncthreads();
+        for( int i = threadIdx.x; i < n * 6; i += (int)blockDim.x )
         {
-            const int c = base + i / 6, q = i % 6;
+            const int lc = i / 6, q = i % 6, c = base + lc;
             int nc;
             if( L.tiled ) nc = d.nbr[(size_t)c * 27 + kFaceDir[q]];
             else
@@ -151,13 +175,16 @@ struct Mid
                     default: nc = z < L.dz - 1 ? c + L.dx * L.dy : -1; break;
                 }
             }
-            nb[i] = ref( L, nc );
+            const uint16_t cc = L.code[c];
+            const bool on = ( cc & BORA_CODE_FLUID ) && ( cc & ( 1u << q ) );
+            if( on && nc < 0 ) code[lc] = cc | kCodeBad;
+            nb[q * L.chunk + lc] = on && nc >= 0 ? ref( L, nc ) : zero_ref( L );
         }
         if( L.o_par >= 0 )
         {
             const MidLevel& P = d.L[t + 1];
             int32_t* par = reinterpret_cast<int32_t*>( blk + L.o_par );
-            for( int i = threadIdx.x; i < n; i += kMidThreads )
+            for( int i = threadIdx.x; i < n; i += (int)blockDim.x )
             {
                 const int c = base + i;
                 int x, y, z;
@@ -177,9 +204,9 @@ struct Mid
         {
             const MidLevel& F = d.L[t - 1];
             int32_t* ch = reinterpret_cast<int32_t*>( blk + L.o_ch );
-            for( int i = threadIdx.x; i < n * 8; i += kMidThreads )
+            for( int i = threadIdx.x; i < n * 8; i += (int)blockDim.x )
             {
-                const int c = base + i / 8, o = i % 8;
+                const int lc = i / 8, o = i % 8, c = base + lc;
                 const int x = c % L.dx, y = ( c / L.dx ) % L.dy, z = c / ( L.dx * L.dy );
                 const int a = 2 * x + ( o & 1 ), b = 2 * y + ( ( o >> 1 ) & 1 ), e = 2 * z + ( o >> 2 );
                 int fc = -1;
@@ -191,71 +218,50 @@ struct Mid
                 {
                     fc = a + F.dx * ( b + F.dy * e );
                 }
-                ch[i] = ref( F, fc );
+                ch[o * L.chunk + lc] = fc >= 0 ? ref( F, fc ) : zero_ref( F );
             }
         }
     }
 
-    // out = in + w[d] (r - (d in - sum of fluid neighbours' in)) on the owned fluid cells, 0 elsewhere
-    __device__ void sweep( int t, int in, int out, const float* w, uint32_t* err ) const
+    // r - S z at an owned cell, from its own value and its fluid neighbours' in array `in`
+    __device__ float defect( const MidLevel& L, int lc, uint16_t cc, int in, float z ) const
+    {
+        const int32_t* nb = arr<int32_t>( L.o_nb ) + lc;
+        int32_t rf[6];
+        float v[6];
+#pragma unroll
+        for( int q = 0; q < 6; ++q ) rf[q] = nb[q * L.chunk];
+#pragma unroll
+        for( int q = 0; q < 6; ++q ) v[q] = ld( in, rf[q] );
+        const float sum = ( ( ( ( v[0] + v[1] ) + v[2] ) + v[3] ) + v[4] ) + v[5];
+        return arr<float>( L.o_r )[lc] - ( (float)code_diag( cc ) * z - sum );
+    }
+    // store( cell, in + w[d] (r - S in) ) on the owned fluid cells, 0 elsewhere
+    template <class Store>
+    __device__ void sweep( int t, int in, const float* w, Store store ) const
     {
         const MidLevel& L = d.L[t];
         const int n = owned( L );
-        const uint16_t* code = arr<uint16_t>( L.o_code );
-        const int32_t* nb = arr<int32_t>( L.o_nb );
-        const float* r = arr<float>( L.o_r );
-        const float* zi = arr<float>( in );
-        float* zo = arr<float>( out );
-        for( int lc = threadIdx.x; lc < n; lc += kMidThreads )
+        for( int lc = threadIdx.x; lc < n; lc += (int)blockDim.x )
         {
-            const uint16_t cc = code[lc];
+            const uint16_t cc = arr<uint16_t>( L.o_code )[lc];
             const int dg = code_diag( cc );
-            float v = 0.f;
-            if( ( cc & BORA_CODE_FLUID ) && dg > 0 )
-            {
-                float sum = 0.f;
-#pragma unroll
-                for( int q = 0; q < 6; ++q )
-                {
-                    if( !( cc & ( 1u << q ) ) ) continue;
-                    const int32_t rf = nb[lc * 6 + q];
-                    if( rf < 0 ) { atomicOr( err, 4u ); continue; }
-                    sum += ld( in, rf );
-                }
-                const float z = zi[lc];
-                v = z + w[dg] * ( r[lc] - ( (float)dg * z - sum ) );
-            }
-            zo[lc] = v;
+            const float z = arr<float>( in )[lc];
+            const float e = defect( L, lc, cc, in, z );
+            store( lc, ( cc & BORA_CODE_FLUID ) && dg > 0 ? z + w[dg] * e : 0.f );
         }
     }
     // A = r - S B on the owned cells (0 on non-fluid cells)
-    __device__ void residual( int t, uint32_t* err ) const
+    __device__ void residual( int t ) const
     {
         const MidLevel& L = d.L[t];
         const int n = owned( L );
-        const uint16_t* code = arr<uint16_t>( L.o_code );
-        const int32_t* nb = arr<int32_t>( L.o_nb );
-        const float* r = arr<float>( L.o_r );
-        const float* zb = arr<float>( L.o_b );
         float* res = arr<float>( L.o_a );
-        for( int lc = threadIdx.x; lc < n; lc += kMidThreads )
+        for( int lc = threadIdx.x; lc < n; lc += (int)blockDim.x )
         {
-            const uint16_t cc = code[lc];
-            float v = 0.f;
-            if( cc & BORA_CODE_FLUID )
-            {
-                float sum = 0.f;
-#pragma unroll
-                for( int q = 0; q < 6; ++q )
-                {
-                    if( !( cc & ( 1u << q ) ) ) continue;
-                    const int32_t rf = nb[lc * 6 + q];
-                    if( rf < 0 ) { atomicOr( err, 8u ); continue; }
-                    sum += ld( L.o_b, rf );
-                }
-                v = r[lc] - ( (float)code_diag( cc ) * zb[lc] - sum );
-            }
-            res[lc] = v;
+            const uint16_t cc = arr<uint16_t>( L.o_code )[lc];
+            const float e = defect( L, lc, cc, L.o_b, arr<float>( L.o_b )[lc] );
+            res[lc] = ( cc & BORA_CODE_FLUID ) ? e : 0.f;
         }
     }
     // level t (>= 1): r = 0.5 * sum of the children's residuals (A of level t - 1), and the
@@ -263,27 +269,24 @@ struct Mid
     __device__ void gather( int t, const float* w ) const
     {
         const MidLevel& L = d.L[t];
-        const MidLevel& F = d.L[t - 1];
+        const int fa = d.L[t - 1].o_a;
         const int n = owned( L );
-        const uint16_t* code = arr<uint16_t>( L.o_code );
-        const int32_t* ch = arr<int32_t>( L.o_ch );
-        float* r = arr<float>( L.o_r );
-        float* a = arr<float>( L.o_a );
-        for( int lc = threadIdx.x; lc < n; lc += kMidThreads )
+        for( int lc = threadIdx.x; lc < n; lc += (int)blockDim.x )
         {
-            float s0 = 0.f, s1 = 0.f;
+            const int32_t* ch = arr<int32_t>( L.o_ch ) + lc;
+            int32_t rf[8];
+            float v[8];
 #pragma unroll
-            for( int o = 0; o < 8; o += 2 )
-            {
-                const int32_t c0 = ch[lc * 8 + o], c1 = ch[lc * 8 + o + 1];
-                if( c0 >= 0 ) s0 += ld( F.o_a, c0 );
-                if( c1 >= 0 ) s1 += ld( F.o_a, c1 );
-            }
+            for( int o = 0; o < 8; ++o ) rf[o] = ch[o * L.chunk];
+#pragma unroll
+            for( int o = 0; o < 8; ++o ) v[o] = ld( fa, rf[o] );
+            const float s0 = ( ( v[0] + v[2] ) + v[4] ) + v[6], s1 = ( ( v[1] + v[3] ) + v[5] ) + v[7];
             const float rv = 0.5f * ( s0 + s1 );
-            const uint16_t cc = code[lc];
+            const uint16_t cc = arr<uint16_t>( L.o_code )[lc];
             const int dg = code_diag( cc );
-            r[lc] = rv;
-            a[lc] = ( ( cc & BORA_CODE_FLUID ) && dg > 0 ) ? w[dg] * rv : 0.f;
+            if( cc & kCodeBad ) atomicOr( d.err, 4u );
+            arr<float>( L.o_r )[lc] = rv;
+            arr<float>( L.o_a )[lc] = ( ( cc & BORA_CODE_FLUID ) && dg > 0 ) ? w[dg] * rv : 0.f;
         }
     }
     // A = B + Z(parent) on the owned fluid cells (Z = array zoff of level t + 1)
@@ -291,34 +294,82 @@ struct Mid
     {
         const MidLevel& L = d.L[t];
         const int n = owned( L );
-        const uint16_t* code = arr<uint16_t>( L.o_code );
-        const int32_t* par = arr<int32_t>( L.o_par );
-        const float* zb = arr<float>( L.o_b );
-        float* a = arr<float>( L.o_a );
-        for( int lc = threadIdx.x; lc < n; lc += kMidThreads )
+        for( int lc = threadIdx.x; lc < n; lc += (int)blockDim.x )
         {
-            const uint16_t cc = code[lc];
-            float v = 0.f;
-            if( ( cc & BORA_CODE_FLUID ) && code_diag( cc ) > 0 ) v = zb[lc] + ld( zoff, par[lc] );
-            a[lc] = v;
+            const uint16_t cc = arr<uint16_t>( L.o_code )[lc];
+            const float z = arr<float>( L.o_b )[lc] + ld( zoff, arr<int32_t>( L.o_par )[lc] );
+            arr<float>( L.o_a )[lc] = ( cc & BORA_CODE_FLUID ) && code_diag( cc ) > 0 ? z : 0.f;
+        }
+    }
+    // The coarsest level's sweeps from the second on, A to B to A. A thread keeps its K
+    // cells' weights, residuals and neighbours' offsets in registers, and the warps that
+    // hold cells meet at a barrier of their own. 16 sweeps of 16 barriers: latency, so the
+    // loop has explicit shared-memory accesses and no branch (107 cycles a sweep at 125
+    // cells and 190 at 512, against 214 and 264 with pointers picked per sweep).
+    template <int K>
+    __device__ __forceinline__ void coarsest( const MidLevel& L, int sweeps, const float* w ) const
+    {
+        const int T = ( ( L.n + K - 1 ) / K + 31 ) / 32 * 32;  // threads that hold cells
+        const int tid = (int)threadIdx.x;
+        if( tid >= T ) return;
+        const uint32_t sa = (uint32_t)__cvta_generic_to_shared( g_mid_smem );
+        const uint32_t A = sa + (uint32_t)L.o_a, B = sa + (uint32_t)L.o_b;
+        uint32_t nb[K][6], own[K];
+        float z[K], rc[K], wd[K], fd[K];
+        bool mine[K], act[K];
+#pragma unroll
+        for( int k = 0; k < K; ++k )
+        {
+            const int c = tid + k * T;
+            mine[k] = c < L.n;
+            own[k] = 4u * (uint32_t)( mine[k] ? c : L.n );
+            const uint16_t cc = mine[k] ? arr<uint16_t>( L.o_code )[c] : (uint16_t)0;
+            act[k] = ( cc & BORA_CODE_FLUID ) && code_diag( cc ) > 0;
+            wd[k] = w[code_diag( cc )];
+            fd[k] = (float)code_diag( cc );
+            rc[k] = mine[k] ? arr<float>( L.o_r )[c] : 0.f;
+            z[k] = mine[k] ? arr<float>( L.o_a )[c] : 0.f;
+#pragma unroll
+            for( int q = 0; q < 6; ++q )  // owner 0: the index is local
+                nb[k][q] = mine[k] ? 4u * (uint32_t)( arr<int32_t>( L.o_nb )[q * L.chunk + c] & 0xFFFFFF ) : 4u * (uint32_t)L.n;
+        }
+        auto step = [&]( uint32_t in, uint32_t out ) {
+            float v[K][6];
+#pragma unroll
+            for( int k = 0; k < K; ++k )
+#pragma unroll
+                for( int q = 0; q < 6; ++q ) asm volatile( "ld.shared.f32 %0, [%1];" : "=f"( v[k][q] ) : "r"( in + nb[k][q] ) );
+#pragma unroll
+            for( int k = 0; k < K; ++k )
+            {
+                const float sum = ( ( ( ( v[k][0] + v[k][1] ) + v[k][2] ) + v[k][3] ) + v[k][4] ) + v[k][5];
+                z[k] = act[k] ? z[k] + wd[k] * ( rc[k] - ( fd[k] * z[k] - sum ) ) : 0.f;
+                if( mine[k] ) asm volatile( "st.shared.f32 [%0], %1;" ::"r"( out + own[k] ), "f"( z[k] ) : "memory" );
+            }
+            asm volatile( "bar.sync 1, %0;" ::"r"( T ) : "memory" );
+        };
+        for( int it = 1; it < sweeps; it += 2 )
+        {
+            step( A, B );
+            if( it + 1 < sweeps ) step( B, A );
         }
     }
 };
 
 // One CTA per cluster CTA: lay out that CTA's static block of the image (once per step).
-__global__ void __launch_bounds__( kMidThreads ) k_mg_mid_image( const __grid_constant__ MidDesc d )
+__global__ void __launch_bounds__( kMidThreadsMax ) k_mg_mid_image( const __grid_constant__ MidDesc d )
 {
-    Mid m{ d, cg::this_cluster(), blockIdx.x };
+    Mid<false> m{ d, cg::this_cluster(), blockIdx.x };
     char* blk = d.image + (size_t)blockIdx.x * d.static_bytes;
     for( int t = 0; t < d.n; ++t ) m.stage( t, blk );
 }
 
+template <bool ONE>
 __device__ __forceinline__ void mg_mid_body( const MidDesc& d )
 {
     __shared__ float wA[16], wB[16], wC[16];
-    uint32_t* err = d.err;
-    Mid m{ d, cg::this_cluster(), 0u };
-    m.me = m.cl.block_rank();
+    Mid<ONE> m{ d, cg::this_cluster(), 0u };
+    if( !ONE ) m.me = m.cl.block_rank();
     const int tid = threadIdx.x;
     bora_pdl_trigger();
     if( tid < 16 )
@@ -332,24 +383,33 @@ __device__ __forceinline__ void mg_mid_body( const MidDesc& d )
     {
         const char* src = d.image + (size_t)m.me * d.static_bytes;
         const uint32_t dst = (uint32_t)__cvta_generic_to_shared( g_mid_smem );
-        for( int i = tid * 16; i < d.static_bytes; i += kMidThreads * 16 )
+        for( int i = tid * 16; i < d.static_bytes; i += (int)blockDim.x * 16 )
             asm volatile( "cp.async.cg.shared.global [%0], [%1], 16;" ::"r"( dst + i ), "l"( src + i ) : "memory" );
-        asm volatile( "cp.async.commit_group;\n\tcp.async.wait_all;" ::: "memory" );
+        asm volatile( "cp.async.commit_group;" ::: "memory" );
+    }
+    // the entry behind each value array that unused references read
+    if( tid < d.n * 2 )
+    {
+        const MidLevel& L = d.L[tid >> 1];
+        m.template arr<float>( tid & 1 ? L.o_b : L.o_a )[L.chunk] = 0.f;
     }
     bora_pdl_wait();  // the level-2 down kernel's restricted residual is complete from here
-    __syncthreads();
     {
         const MidLevel& L = d.L[0];
         const int n = m.owned( L );
-        const uint16_t* code = m.arr<uint16_t>( L.o_code );
-        float* r = m.arr<float>( L.o_r );
-        float* a = m.arr<float>( L.o_a );
+        const uint16_t* code = m.template arr<uint16_t>( L.o_code );
+        float* r = m.template arr<float>( L.o_r );
+        float* a = m.template arr<float>( L.o_a );
         const __half* g = d.r_in + (size_t)m.me * L.chunk;
-        for( int i = tid; i < n; i += kMidThreads )
+        const __half first = tid < n ? g[tid] : __half( 0.f );
+        asm volatile( "cp.async.wait_all;" ::: "memory" );
+        __syncthreads();
+        for( int i = tid; i < n; i += (int)blockDim.x )
         {
             const uint16_t cc = code[i];
             const int dg = code_diag( cc );
-            const float rv = ( cc & BORA_CODE_FLUID ) ? __half2float( g[i] ) : 0.f;
+            if( cc & kCodeBad ) atomicOr( d.err, 4u );
+            const float rv = ( cc & BORA_CODE_FLUID ) ? __half2float( i == tid ? first : g[i] ) : 0.f;
             r[i] = rv;
             a[i] = ( ( cc & BORA_CODE_FLUID ) && dg > 0 ) ? wA[dg] * rv : 0.f;
         }
@@ -360,59 +420,22 @@ __device__ __forceinline__ void mg_mid_body( const MidDesc& d )
     for( int t = 0; t < last; ++t )
     {
         const MidLevel& L = d.L[t];
-        m.sweep( t, L.o_a, L.o_b, wB, err );         // B = second pre-smoothing sweep
+        float* b = m.template arr<float>( L.o_b );
+        m.sweep( t, L.o_a, wB, [&]( int lc, float v ) { b[lc] = v; } );  // second pre-smoothing sweep
         m.barrier();
-        m.residual( t, err );                        // A = r - S B
+        m.residual( t );                             // A = r - S B
         m.barrier();
         m.gather( t + 1, t + 1 == last ? wC : wA );  // coarser r and its pointwise first sweep
         m.barrier();
     }
     // ---- coarsest level: damped Jacobi from zero in CTA 0 (the first sweep, pointwise,
-    // came with the gather). Each thread keeps its cell's code, weight, residual and
-    // neighbours in registers across the sweeps; the values ping-pong between A and B. ----
+    // came with the gather) ----
     const MidLevel& Lc = d.L[last];
     const int zc = ( d.sweeps - 1 ) % 2 == 0 ? Lc.o_a : Lc.o_b;  // the coarsest correction's array
     if( m.me == 0 && d.sweeps > 1 )
     {
-        float* za = m.arr<float>( Lc.o_a );
-        float* zb = m.arr<float>( Lc.o_b );
-        const bool mine = tid < Lc.n;
-        const uint16_t cc = mine ? m.arr<uint16_t>( Lc.o_code )[tid] : 0;
-        const int dg = code_diag( cc );
-        const bool act = mine && ( cc & BORA_CODE_FLUID ) && dg > 0;
-        const float w = wC[dg], rc = mine ? m.arr<float>( Lc.o_r )[tid] : 0.f, fd = (float)dg;
-        int nbl[6];
-#pragma unroll
-        for( int q = 0; q < 6; ++q )
-        {
-            nbl[q] = -1;
-            if( act && ( cc & ( 1u << q ) ) )
-            {
-                const int32_t rf = m.arr<int32_t>( Lc.o_nb )[tid * 6 + q];  // owner 0: the index is local
-                if( rf < 0 ) atomicOr( err, 4u );
-                else nbl[q] = rf & 0xFFFFFF;
-            }
-        }
-        for( int it = 1; it < d.sweeps; ++it )
-        {
-            const float* zi = ( it & 1 ) ? za : zb;
-            float* zo = ( it & 1 ) ? zb : za;
-            if( mine )
-            {
-                float v = 0.f;
-                if( act )
-                {
-                    float sum = 0.f;
-#pragma unroll
-                    for( int q = 0; q < 6; ++q )
-                        if( nbl[q] >= 0 ) sum += zi[nbl[q]];
-                    const float z = zi[tid];
-                    v = z + w * ( rc - ( fd * z - sum ) );
-                }
-                zo[tid] = v;
-            }
-            __syncthreads();
-        }
+        if( Lc.n <= (int)blockDim.x ) m.template coarsest<1>( Lc, d.sweeps, wC );
+        else m.template coarsest<2>( Lc, d.sweeps, wC );
     }
     m.barrier();
     // ---- up ----
@@ -421,30 +444,39 @@ __device__ __forceinline__ void mg_mid_body( const MidDesc& d )
         const MidLevel& L = d.L[t];
         m.inject( t, t + 1 == last ? zc : d.L[t + 1].o_a );  // A = B + Z(parent)
         m.barrier();
-        m.sweep( t, L.o_a, L.o_b, wB, err );                   // B = A + wB (r - S A)
+        float* b = m.template arr<float>( L.o_b );
+        m.sweep( t, L.o_a, wB, [&]( int lc, float v ) { b[lc] = v; } );
         m.barrier();
-        m.sweep( t, L.o_b, L.o_a, wA, err );                   // A = final correction
-        if( t > 0 ) m.barrier();
-    }
-    {
-        const MidLevel& L = d.L[0];
-        const int n = m.owned( L );
-        const float* a = m.arr<float>( L.o_a );
-        __half* g = d.z_out + (size_t)m.me * L.chunk;
-        for( int i = tid; i < n; i += kMidThreads ) g[i] = __float2half_rn( a[i] );
+        // the level's final correction: A, or level 3's result
+        if( t > 0 )
+        {
+            float* a = m.template arr<float>( L.o_a );
+            m.sweep( t, L.o_b, wA, [&]( int lc, float v ) { a[lc] = v; } );
+            m.barrier();
+        }
+        else
+        {
+            __half* g = d.z_out + (size_t)m.me * L.chunk;
+            m.sweep( t, L.o_b, wA, [&]( int lc, float v ) { g[lc] = __float2half_rn( v ); } );
+        }
     }
     m.barrier();  // no CTA leaves while another may still read its shared memory
 }
 
-__global__ void __launch_bounds__( kMidThreads, 1 ) k_mg_mid( const __grid_constant__ MidDesc d ) { mg_mid_body( d ); }
+template <bool ONE>
+__global__ void __launch_bounds__( kMidThreadsMax, 1 ) k_mg_mid( const __grid_constant__ MidDesc d )
+{
+    mg_mid_body<ONE>( d );
+}
 
-// Batched: one cluster per simulation taking part (all clusters of the same size; a
+// Batched: one cluster per simulation taking part (all of the same size; a
 // simulation's offset in the launch is a multiple of it, so a cluster is one simulation's).
-__global__ void __launch_bounds__( kMidThreads, 1 ) k_mg_mid_batch( const MidDesc* __restrict__ descs,
+template <bool ONE>
+__global__ void __launch_bounds__( kMidThreadsMax, 1 ) k_mg_mid_batch( const MidDesc* __restrict__ descs,
                                                                     const __grid_constant__ BoraBatchLaunch L )
 {
     unsigned bid;
-    mg_mid_body( descs[bora_batch_member( L, blockIdx.x, &bid )] );
+    mg_mid_body<ONE>( descs[bora_batch_member( L, blockIdx.x, &bid )] );
 }
 
 // Cluster size: 16 CTAs where the device co-schedules such a cluster of this kernel with
@@ -454,15 +486,17 @@ int mid_cluster_size()
 {
     static BoraPerDevice size;  // 16, 8, or 1 for "none"
     const int v = size.get( [] {
-        cudaFuncSetAttribute( k_mg_mid, cudaFuncAttributeNonPortableClusterSizeAllowed, 1 );
-        cudaFuncSetAttribute( k_mg_mid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMidSmemMax );
-        cudaFuncSetAttribute( k_mg_mid_batch, cudaFuncAttributeNonPortableClusterSizeAllowed, 1 );
-        cudaFuncSetAttribute( k_mg_mid_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMidSmemMax );
+        cudaFuncSetAttribute( k_mg_mid<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1 );
+        cudaFuncSetAttribute( k_mg_mid<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMidSmemMax );
+        cudaFuncSetAttribute( k_mg_mid_batch<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1 );
+        cudaFuncSetAttribute( k_mg_mid_batch<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMidSmemMax );
+        cudaFuncSetAttribute( k_mg_mid<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMidSmemMax );
+        cudaFuncSetAttribute( k_mg_mid_batch<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMidSmemMax );
         cudaGetLastError();
         auto fits = []( int ctas ) {
             cudaLaunchConfig_t cfg{};
             cfg.gridDim = dim3( ctas );
-            cfg.blockDim = dim3( kMidThreads );
+            cfg.blockDim = dim3( kMidThreadsMax );
             cfg.dynamicSmemBytes = kMidSmemMax;
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -472,7 +506,7 @@ int mid_cluster_size()
             cfg.attrs = attr;
             cfg.numAttrs = 1;
             int clusters = 0;
-            const bool ok = cudaOccupancyMaxActiveClusters( &clusters, k_mg_mid, &cfg ) == cudaSuccess && clusters > 0;
+            const bool ok = cudaOccupancyMaxActiveClusters( &clusters, k_mg_mid<false>, &cfg ) == cudaSuccess && clusters > 0;
             cudaGetLastError();  // a refused query leaves no error behind
             return ok;
         };
@@ -493,6 +527,7 @@ size_t mid_layout( MidDesc& d, int ctas )
         return o;
     };
     d.ctas = ctas;
+    d.threads = std::clamp( ( ( ( d.L[0].n + ctas - 1 ) / ctas + 31 ) / 32 ) * 32, kMidThreadsMin, kMidThreadsMax );
     for( int t = 0; t < d.n; ++t )
     {
         MidLevel& L = d.L[t];
@@ -509,8 +544,8 @@ size_t mid_layout( MidDesc& d, int ctas )
         MidLevel& L = d.L[t];
         const size_t c = (size_t)L.chunk;
         L.o_r = take( c * 4 );
-        L.o_a = take( c * 4 );
-        L.o_b = take( c * 4 );
+        L.o_a = take( ( c + 1 ) * 4 );
+        L.o_b = take( ( c + 1 ) * 4 );
     }
     return off;
 }
@@ -545,8 +580,32 @@ bool mid_describe( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels
     d.sweeps = sweeps;
     const int ctas = mid_cluster_size();
     if( ctas == 0 ) return false;
+    smem = 0;
+    if( ntiles <= kMidSingleMax && ( smem = mid_layout( d, 1 ) ) <= kMidSmemMax ) return true;
     smem = mid_layout( d, ctas );
     return smem <= kMidSmemMax;
+}
+
+// One launch of the V-cycle kernel: `blocks` CTAs of `threads` in clusters of `ctas`.
+template <class K1, class KN, class... Args>
+void mid_launch( K1 single, KN clustered, int blocks, int ctas, int threads, size_t smem, cudaStream_t st, const Args&... args )
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3( blocks );
+    cfg.blockDim = dim3( threads );
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = ctas;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ctas == 1 ? 1 : 2;
+    if( ctas == 1 ) cudaLaunchKernelEx( &cfg, single, args... );
+    else cudaLaunchKernelEx( &cfg, clustered, args... );
 }
 
 }  // namespace
@@ -566,7 +625,7 @@ void bora_mg_mid_setup( const BoraGridDev& g, const BoraLevelDev* levels, int nl
     size_t smem = 0;
     if( !image || !mid_describe( g, levels, nlevels, t, ntiles, 16, d, smem ) ) return;
     d.image = static_cast<char*>( image );
-    k_mg_mid_image<<<d.ctas, kMidThreads, 0, st>>>( d );
+    k_mg_mid_image<<<d.ctas, kMidThreadsMax, 0, st>>>( d );
 }
 
 int bora_mg_mid_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t, int ntiles,
@@ -578,28 +637,14 @@ int bora_mg_mid_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nl
     if( !launch ) return 1;
     d.image = static_cast<char*>( const_cast<void*>( image ) );
     d.err = err;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3( d.ctas );
-    cfg.blockDim = dim3( kMidThreads );
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = d.ctas;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 2;
-    cudaLaunchKernelEx( &cfg, k_mg_mid, d );
+    mid_launch( k_mg_mid<true>, k_mg_mid<false>, d.ctas, d.ctas, d.threads, smem, st, d );
     return 1;
 }
 
 size_t bora_mg_mid_desc_bytes() { return sizeof( MidDesc ); }
 
 int bora_mg_mid_describe( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t, int ntiles,
-                          const void* image, uint32_t* err, int sweeps, void* desc, size_t* smem, int* ctas )
+                          const void* image, uint32_t* err, int sweeps, void* desc, BoraMidShape* shape )
 {
     MidDesc d;
     size_t sm = 0;
@@ -607,28 +652,14 @@ int bora_mg_mid_describe( const BoraGridDev& g, const BoraLevelDev* levels, int 
     d.image = static_cast<char*>( const_cast<void*>( image ) );
     d.err = err;
     std::memcpy( desc, &d, sizeof( d ) );
-    *smem = sm;
-    *ctas = d.ctas;
+    *shape = BoraMidShape{ d.ctas, d.threads, sm };
     return 1;
 }
 
-void bora_mg_mid_launch_batch( const void* descs, const BoraBatchLaunch& L, int blocks, int ctas, size_t smem,
+void bora_mg_mid_launch_batch( const void* descs, const BoraBatchLaunch& L, int blocks, const BoraMidShape& shape,
                                cudaStream_t st )
 {
-    if( blocks <= 0 || ctas <= 0 || blocks % ctas ) return;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3( blocks );
-    cfg.blockDim = dim3( kMidThreads );
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ctas;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 2;
-    cudaLaunchKernelEx( &cfg, k_mg_mid_batch, static_cast<const MidDesc*>( descs ), L );
+    if( blocks <= 0 || shape.ctas <= 0 || blocks % shape.ctas ) return;
+    mid_launch( k_mg_mid_batch<true>, k_mg_mid_batch<false>, blocks, shape.ctas, shape.threads, shape.smem, st,
+                static_cast<const MidDesc*>( descs ), L );
 }
