@@ -27,10 +27,13 @@
 // without storing it, and sums r.r over the grid (the convergence check); down 2, which reads no
 // neighbour's r, stores it. This takes the update kernel out of every iteration.
 //
-// Level 0 runs one warp per tile: a lane owns the x-rows (j, k) and (j, k + 4) of the tile as
-// 16-byte vectors (lane = j + 8 k), its x neighbours are in its registers, the y and z
-// neighbours come from other lanes by shuffles, and the lanes of the tile's faces load the face
-// rows of the six neighbour tiles. Levels 1 and 2 run one thread per cell.
+// Level 0 runs one warp per half tile (z layers 0..3 or 4..7): a lane owns one x-row (lane =
+// j + 8 (k mod 4)), read and written as whole vectors; its x neighbours are in its registers, the
+// y and z neighbours come from other lanes by shuffles, and the lanes at the half's faces load
+// the rows across them (the other half, the neighbour tiles). The passes wait on their loads, so
+// they want warps in flight and all of a lane's loads issued before the first is used: with a
+// tile per warp (two rows per lane, 128 registers, 12 warps in flight) the four passes took 33,
+// 18, 28 and 24 us at 256^3 (8.2 K tiles). Levels 1 and 2 run one thread per cell.
 #include <algorithm>
 #include <type_traits>
 
@@ -42,9 +45,15 @@ namespace {
 constexpr float kOmegaA = 0.5687f;  // the Chebyshev pair of the smoothers (multigrid.cu)
 constexpr float kOmegaB = 1.6902f;
 // launch shapes (the autotuner picks one per size class; the results do not depend on it):
-// level 0 tiles (warps) per block, levels 1 and 2 threads (cells) per block
+// level 0 half tiles (warps) per block, levels 1 and 2 threads (cells) per block
 constexpr int kPassWarpsOf[3] = { 2, 4, 8 };
 constexpr int kFlatThreadsOf[4] = { 64, 128, 256, 512 };
+// Warps per SM that level 0 asks registers for: 24 (80 registers) for down 2 and up 1, 16 (128)
+// for the reducing passes (down 1 holds code, r and q of two halo rows). A 256^3 mixed step
+// takes 4.08 ms with 24 / 16, 4.13 with 24 / 20, 4.14 with 24 / 24 (down 1 spills), 4.11 with
+// 16 / 16, 4.15 with 32 / 20 (spills); 4.54 with a whole tile per warp at 128 registers.
+constexpr int kPassWarpsPerSm = 24, kReduceWarpsPerSm = 16;
+constexpr int pass_warps_per_sm( int P ) { return P == 0 || P == 3 ? kReduceWarpsPerSm : kPassWarpsPerSm; }
 constexpr int kReduceWarps = 4;  // level 0's up 2 sums r.z over its blocks: its shape is fixed
 constexpr unsigned kAll = 0xffffffffu;
 
@@ -74,11 +83,10 @@ __device__ __forceinline__ float scale_from( const double* ring, int slot )
     return rr > 0.0 ? (float)( 1.0 / sqrt( rr ) ) : 1.f;
 }
 
-// ---- level 0: one warp per tile ---------------------------------------------------------
+// ---- level 0: one warp per half tile ---------------------------------------------------------
 
-__device__ __forceinline__ void codes8( const uint16_t* __restrict__ code, size_t g, uint16_t* c )
+__device__ __forceinline__ void codes8( uint4 w, uint16_t* c )
 {
-    const uint4 w = *reinterpret_cast<const uint4*>( code + g );
     const uint32_t a[4] = { w.x, w.y, w.z, w.w };
 #pragma unroll
     for( int i = 0; i < 4; ++i )
@@ -88,18 +96,10 @@ __device__ __forceinline__ void codes8( const uint16_t* __restrict__ code, size_
     }
 }
 
-__device__ __forceinline__ void f32x8( const float* __restrict__ p, size_t g, float* v )
-{
-    bora_ld8( p + g, v );
-}
-
-__device__ __forceinline__ void st_f32x8( float* __restrict__ p, size_t g, const float* v ) { bora_st8( p + g, v ); }
-
 __device__ __forceinline__ float hbits( uint32_t w, int q ) { return __half2float( __ushort_as_half( (unsigned short)( w >> ( 16 * q ) ) ) ); }
 
-__device__ __forceinline__ void f16x8( const __half* __restrict__ p, size_t g, float* v )
+__device__ __forceinline__ void f16x8( uint4 w, float* v )
 {
-    const uint4 w = *reinterpret_cast<const uint4*>( p + g );
     const uint32_t a[4] = { w.x, w.y, w.z, w.w };
 #pragma unroll
     for( int i = 0; i < 4; ++i ) { v[2 * i] = hbits( a[i], 0 ); v[2 * i + 1] = hbits( a[i], 1 ); }
@@ -110,147 +110,177 @@ __device__ __forceinline__ uint32_t pack2( float a, float b )
     return (uint32_t)__half_as_ushort( __float2half_rn( a ) ) | ( (uint32_t)__half_as_ushort( __float2half_rn( b ) ) << 16 );
 }
 
-// the fields a pass reads at its neighbours, for 8 cells of a row or one cell of tile slot t
-// (cell index c in the tile; t < 0 gives zeros)
-struct FieldZ1  // down 1: the first sweep's z1 = w_A r' / d of the updated residual r - alpha q
-{
-    const uint16_t* code;
-    const float* r0;
-    const float* q;  // null: no update
-    float alpha;
-    float sc;
-    const float* w;
-    __device__ void row( int t, int c, float* v ) const
-    {
-        if( t < 0 ) { for( int i = 0; i < 8; ++i ) v[i] = 0.f; return; }
-        const size_t g = (size_t)t * 512 + c;
-        uint16_t cc[8];
-        float rr[8];
-        codes8( code, g, cc );
-        f32x8( r0, g, rr );
-        if( q )
-        {
-            float qq[8];
-            f32x8( q, g, qq );
-#pragma unroll
-            for( int i = 0; i < 8; ++i ) rr[i] = fmaf( -alpha, qq[i], rr[i] );
-        }
-#pragma unroll
-        for( int i = 0; i < 8; ++i ) v[i] = cfluid( cc[i] ) ? ( rr[i] * sc ) * w[cdiag( cc[i] )] : 0.f;
-    }
-    __device__ float one( int t, int c ) const
-    {
-        if( t < 0 ) return 0.f;
-        const size_t g = (size_t)t * 512 + c;
-        const uint16_t cc = code[g];
-        const float r = q ? fmaf( -alpha, q[g], r0[g] ) : r0[g];
-        return cfluid( cc ) ? ( r * sc ) * w[cdiag( cc )] : 0.f;
-    }
-};
-
-struct FieldF32  // down 2 and up 2: a scratch value
-{
-    const float* v;
-    __device__ void row( int t, int c, float* o ) const
-    {
-        if( t < 0 ) { for( int i = 0; i < 8; ++i ) o[i] = 0.f; return; }
-        f32x8( v, (size_t)t * 512 + c, o );
-    }
-    __device__ float one( int t, int c ) const { return t < 0 ? 0.f : v[(size_t)t * 512 + c]; }
-};
-
-struct FieldF16  // down 2 and up 2 (level 0): a scratch value stored in FP16
-{
-    const __half* v;
-    __device__ void row( int t, int c, float* o ) const
-    {
-        if( t < 0 ) { for( int i = 0; i < 8; ++i ) o[i] = 0.f; return; }
-        f16x8( v, (size_t)t * 512 + c, o );
-    }
-    __device__ float one( int t, int c ) const { return t < 0 ? 0.f : __half2float( v[(size_t)t * 512 + c] ); }
-};
-
 __device__ __forceinline__ void st_f16x8( __half* __restrict__ p, size_t g, const float* v )
 {
     *reinterpret_cast<uint4*>( p + g ) = make_uint4( pack2( v[0], v[1] ), pack2( v[2], v[3] ), pack2( v[4], v[5] ), pack2( v[6], v[7] ) );
 }
+
+// The fields a pass reads at its neighbours, for 8 cells of a row (Row) or one cell (One) of
+// tile slot t, cell c: load() issues the loads (none for t < 0), value() forms the values, so
+// that a lane's loads are all in flight before the first is waited for. t < 0 gives zeros.
+struct FieldZ1  // down 1: the first sweep's z1 = w_A r' / d of the updated residual r - alpha q
+{
+    const uint16_t* code;
+    const float* r0;
+    const float* q;
+    bool upd;  // r -= alpha q
+    float alpha;
+    float sc;
+    const float* w;
+    struct Row { uint4 c; float r[8], q[8]; };
+    struct One { uint16_t c; float r, q; };
+    __device__ __forceinline__ void load( Row& x, int t, int c ) const
+    {
+        x.c = make_uint4( 0u, 0u, 0u, 0u );
+#pragma unroll
+        for( int i = 0; i < 8; ++i ) x.r[i] = x.q[i] = 0.f;
+        if( t < 0 ) return;
+        const size_t g = (size_t)t * 512 + c;
+        x.c = *reinterpret_cast<const uint4*>( code + g );
+        bora_ld8( r0 + g, x.r );
+        if( upd ) bora_ld8( q + g, x.q );
+    }
+    __device__ __forceinline__ void value( const Row& x, float* v ) const
+    {
+        uint16_t cc[8];
+        codes8( x.c, cc );
+#pragma unroll
+        for( int i = 0; i < 8; ++i )
+        {
+            const float r = upd ? fmaf( -alpha, x.q[i], x.r[i] ) : x.r[i];
+            v[i] = cfluid( cc[i] ) ? ( r * sc ) * w[cdiag( cc[i] )] : 0.f;
+        }
+    }
+    __device__ __forceinline__ void load( One& x, int t, int c ) const
+    {
+        x.c = 0;
+        x.r = x.q = 0.f;
+        if( t < 0 ) return;
+        const size_t g = (size_t)t * 512 + c;
+        x.c = code[g];
+        x.r = r0[g];
+        if( upd ) x.q = q[g];
+    }
+    __device__ __forceinline__ float value( const One& x ) const
+    {
+        const float r = upd ? fmaf( -alpha, x.q, x.r ) : x.r;
+        return cfluid( x.c ) ? ( r * sc ) * w[cdiag( x.c )] : 0.f;
+    }
+};
+
+struct FieldF16  // down 2 and up 2: a scratch value stored in FP16
+{
+    const __half* v;
+    struct Row { uint4 v; };
+    struct One { __half v; };
+    __device__ __forceinline__ void load( Row& x, int t, int c ) const
+    {
+        x.v = make_uint4( 0u, 0u, 0u, 0u );
+        if( t >= 0 ) x.v = *reinterpret_cast<const uint4*>( v + (size_t)t * 512 + c );
+    }
+    __device__ __forceinline__ void value( const Row& x, float* o ) const { f16x8( x.v, o ); }
+    __device__ __forceinline__ void load( One& x, int t, int c ) const
+    {
+        x.v = __half( 0.f );
+        if( t >= 0 ) x.v = v[(size_t)t * 512 + c];
+    }
+    __device__ __forceinline__ float value( const One& x ) const { return __half2float( x.v ); }
+};
 
 struct FieldZa  // up 1: za = z0 + e(parent) on fluid cells
 {
     const uint16_t* code;
     const __half* z0;
     const __half* ec;  // level 1's correction, 64 cells per tile
-    __device__ void row( int t, int c, float* v ) const
+    struct Row { uint4 c, z; uint2 e; };
+    struct One { uint16_t c; __half z, e; };
+    __device__ __forceinline__ void load( Row& x, int t, int c ) const
     {
-        if( t < 0 ) { for( int i = 0; i < 8; ++i ) v[i] = 0.f; return; }
+        x.c = x.z = make_uint4( 0u, 0u, 0u, 0u );
+        x.e = make_uint2( 0u, 0u );
+        if( t < 0 ) return;
         const size_t g = (size_t)t * 512 + c;
+        const int jj = ( c >> 3 ) & 7, kk = c >> 6;
+        x.c = *reinterpret_cast<const uint4*>( code + g );
+        x.z = *reinterpret_cast<const uint4*>( z0 + g );
+        x.e = *reinterpret_cast<const uint2*>( ec + (size_t)t * 64 + 4 * ( ( jj >> 1 ) + 4 * ( kk >> 1 ) ) );
+    }
+    __device__ __forceinline__ void value( const Row& x, float* v ) const
+    {
         uint16_t cc[8];
         float zz[8];
-        codes8( code, g, cc );
-        f16x8( z0, g, zz );
-        const int jj = ( c >> 3 ) & 7, kk = c >> 6;
-        const uint2 e = *reinterpret_cast<const uint2*>( ec + (size_t)t * 64 + 4 * ( ( jj >> 1 ) + 4 * ( kk >> 1 ) ) );
+        codes8( x.c, cc );
+        f16x8( x.z, zz );
 #pragma unroll
         for( int i = 0; i < 8; ++i )
         {
-            const float ev = hbits( ( i >> 2 ) ? e.y : e.x, ( i >> 1 ) & 1 );
+            const float ev = hbits( ( i >> 2 ) ? x.e.y : x.e.x, ( i >> 1 ) & 1 );
             v[i] = cfluid( cc[i] ) ? zz[i] + ev : 0.f;
         }
     }
-    __device__ float one( int t, int c ) const
+    __device__ __forceinline__ void load( One& o, int t, int c ) const
     {
-        if( t < 0 ) return 0.f;
+        o.c = 0;
+        o.z = o.e = __half( 0.f );
+        if( t < 0 ) return;
         const size_t g = (size_t)t * 512 + c;
-        const uint16_t cc = code[g];
         const int x = c & 7, jj = ( c >> 3 ) & 7, kk = c >> 6;
-        const float ev = __half2float( ec[(size_t)t * 64 + ( x >> 1 ) + 4 * ( ( jj >> 1 ) + 4 * ( kk >> 1 ) )] );
-        return cfluid( cc ) ? __half2float( z0[g] ) + ev : 0.f;
+        o.c = code[g];
+        o.z = z0[g];
+        o.e = ec[(size_t)t * 64 + ( x >> 1 ) + 4 * ( ( jj >> 1 ) + 4 * ( kk >> 1 ) )];
+    }
+    __device__ __forceinline__ float value( const One& o ) const
+    {
+        return cfluid( o.c ) ? __half2float( o.z ) + __half2float( o.e ) : 0.f;
     }
 };
 
-// The neighbour sums of a lane's rows A = (j, kq) and B = (j, kq + 4) of tile s from their own
-// values vA, vB (every lane of the warp calls this for the same tile).
-// nf: the face-neighbour slots -x +x -y +y -z +z.
-template <class F>
-__device__ __forceinline__ void row_sums( const F& f, const int* nf, int lane, const float* vA, const float* vB, float* sA,
-                                          float* sB )
+// A half tile: the slots of its face neighbours (-1: none) and of the neighbour across its
+// outer z face, its own slot, and which half (0: z layers 0..3, 1: 4..7).
+struct HalfTile
 {
-    const int j = lane & 7, kq = lane >> 3;
-    const int smx = nf[0], spx = nf[1], smy = nf[2], spy = nf[3], smz = nf[4], spz = nf[5];
-    // the x ends of both rows, the y face row of lanes j = 0 / 7 (both rows), the z face row
-    // of row A at k = 0 (-z) and of row B at k = 7 (+z)
-    const float xmA = f.one( smx, 8 * lane + 7 ), xpA = f.one( spx, 8 * lane );
-    const float xmB = f.one( smx, 256 + 8 * lane + 7 ), xpB = f.one( spx, 256 + 8 * lane );
-    float yhA[8], yhB[8], zh[8];
+    int smx, spx, smy, spy, sz, s, hi;
+};
+
+// The rows and cells around a lane's row that the warp's other lanes do not hold: the x ends,
+// the y face row of lanes j = 0 / 7, and the z row below kk = 0 / above kk = 3 (the other half
+// of the tile or the neighbour tile). load() before the values are needed, sums() from the
+// lane's own values v (every lane of the warp calls both for the same half tile).
+template <class F>
+struct Around
+{
+    typename F::One xm, xp;
+    typename F::Row y, z;
+    __device__ __forceinline__ void load( const F& f, const HalfTile& h, int lane )
     {
-        const int yt = j == 0 ? smy : ( j == 7 ? spy : -1 );
-        const int yc = 8 * ( lane - j ) + ( j == 0 ? 56 : 0 );
-        f.row( yt, yc, yhA );
-        f.row( yt, yc + 256, yhB );
-        const int zt = kq == 0 ? smz : ( kq == 3 ? spz : -1 );
-        f.row( zt, 8 * j + ( kq == 0 ? 448 : 0 ), zh );
+        const int j = lane & 7, kk = lane >> 3, c = h.hi * 256 + 8 * lane;
+        f.load( y, j == 0 ? h.smy : ( j == 7 ? h.spy : -1 ), c + ( j == 0 ? 56 : -56 ) );
+        f.load( z, kk == 0 ? ( h.hi ? h.s : h.sz ) : ( kk == 3 ? ( h.hi ? h.sz : h.s ) : -1 ),
+                8 * j + ( kk == 0 ? ( h.hi ? 192 : 448 ) : ( h.hi ? 0 : 256 ) ) );
+        f.load( xm, h.smx, c + 7 );
+        f.load( xp, h.spx, c );
     }
+    __device__ __forceinline__ void sums( const F& f, int lane, const float* v, float* sum ) const
+    {
+        const int j = lane & 7, kk = lane >> 3;
+        const float xl = f.value( xm ), xr = f.value( xp );
+        float yh[8], zh[8];
+        f.value( y, yh );
+        f.value( z, zh );
 #pragma unroll
-    for( int i = 0; i < 8; ++i )
-    {
-        float ymA = __shfl_up_sync( kAll, vA[i], 1 ), ypA = __shfl_down_sync( kAll, vA[i], 1 );
-        float ymB = __shfl_up_sync( kAll, vB[i], 1 ), ypB = __shfl_down_sync( kAll, vB[i], 1 );
-        if( j == 0 ) { ymA = yhA[i]; ymB = yhB[i]; }
-        if( j == 7 ) { ypA = yhA[i]; ypB = yhB[i]; }
-        float zmA = __shfl_up_sync( kAll, vA[i], 8 );
-        if( kq == 0 ) zmA = zh[i];
-        // the source lane picks the row: lane + 8 wraps from kq = 3 to row B of kq = 0, lane - 8
-        // from kq = 0 to row A of kq = 3
-        const float zpA = __shfl_sync( kAll, kq == 0 ? vB[i] : vA[i], ( lane + 8 ) & 31 );
-        const float zmB = __shfl_sync( kAll, kq == 3 ? vA[i] : vB[i], ( lane + 24 ) & 31 );
-        float zpB = __shfl_down_sync( kAll, vB[i], 8 );
-        if( kq == 3 ) zpB = zh[i];
-        const float xmA_ = i > 0 ? vA[i > 0 ? i - 1 : 0] : xmA, xpA_ = i < 7 ? vA[i < 7 ? i + 1 : 7] : xpA;
-        const float xmB_ = i > 0 ? vB[i > 0 ? i - 1 : 0] : xmB, xpB_ = i < 7 ? vB[i < 7 ? i + 1 : 7] : xpB;
-        sA[i] = ( ( xmA_ + xpA_ ) + ( ymA + ypA ) ) + ( zmA + zpA );
-        sB[i] = ( ( xmB_ + xpB_ ) + ( ymB + ypB ) ) + ( zmB + zpB );
+        for( int i = 0; i < 8; ++i )
+        {
+            float ym = __shfl_up_sync( kAll, v[i], 1 ), yp = __shfl_down_sync( kAll, v[i], 1 );
+            float zm = __shfl_up_sync( kAll, v[i], 8 ), zp = __shfl_down_sync( kAll, v[i], 8 );
+            if( j == 0 ) ym = yh[i];
+            if( j == 7 ) yp = yh[i];
+            if( kk == 0 ) zm = zh[i];
+            if( kk == 3 ) zp = zh[i];
+            const float xm_ = i > 0 ? v[i > 0 ? i - 1 : 0] : xl, xp_ = i < 7 ? v[i < 7 ? i + 1 : 7] : xr;
+            sum[i] = ( ( xm_ + xp_ ) + ( ym + yp ) ) + ( zm + zp );
+        }
     }
-}
+};
 
 struct Pass0Args
 {
@@ -267,7 +297,7 @@ struct Pass0Args
     int ndq;              // down 1: partial sums of dq to finish into slot_dq_in
 };
 
-// pass P of level 0: 0 = down 1, 1 = down 2, 2 = up 1, 3 = up 2; W tiles (warps) per block
+// pass P of level 0: 0 = down 1, 1 = down 2, 2 = up 1, 3 = up 2; W half tiles (warps) per block
 template <int W, int P>
 __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, unsigned G )
 {
@@ -275,29 +305,26 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
     __shared__ float s_sc;
     bora_pdl_trigger();
     init_weights( w );
-    const int lane = threadIdx.x & 31, j = lane & 7, kq = lane >> 3;
-    const int stride = (int)G * W;
-    // what no kernel of the solve writes is read ahead, the first tile's before the dependency
-    // wait: the rows' codes a tile ahead, the tile table (which says where they are) two
-    int4 n0 = make_int4( -1, -1, -1, -1 ), n1 = n0;  // table entry of the tile after the next fetch
-    uint4 cwA = make_uint4( 0u, 0u, 0u, 0u ), cwB = cwA;
-    int nfn[6] = { -1, -1, -1, -1, -1, -1 }, sn = 0;
-    auto entry = [&]( int t ) {
-        if( t >= a.ft.n ) return;
-        n0 = __ldg( a.ft.tab + 2 * (size_t)t );
-        n1 = __ldg( a.ft.tab + 2 * (size_t)t + 1 );
+    const int lane = threadIdx.x & 31, j = lane & 7, kk = lane >> 3;
+    const int nh = 2 * a.ft.n, stride = (int)G * W;
+    // what no kernel of the solve writes - a half tile's table entry and its rows' codes - is
+    // read one ahead, the first one's before the dependency wait
+    HalfTile hn{ -1, -1, -1, -1, -1, 0, 0 };
+    uint4 cwn = make_uint4( 0u, 0u, 0u, 0u );
+    auto entry = [&]( int h ) {
+        hn = HalfTile{ -1, -1, -1, -1, -1, 0, h & 1 };
+        if( h >= nh ) return;
+        const int4 n0 = __ldg( a.ft.tab + 2 * (size_t)( h >> 1 ) ), n1 = __ldg( a.ft.tab + 2 * (size_t)( h >> 1 ) + 1 );
+        hn.smx = n0.x; hn.spx = n0.y; hn.smy = n0.z; hn.spy = n0.w;
+        hn.sz = h & 1 ? n1.y : n1.x;
+        hn.s = n1.z;
     };
-    auto fetch = [&]( int t ) {  // from the entry read before; reads the one after
-        if( t >= a.ft.n ) return;
-        nfn[0] = n0.x; nfn[1] = n0.y; nfn[2] = n0.z; nfn[3] = n0.w; nfn[4] = n1.x; nfn[5] = n1.y;
-        sn = n1.z;
-        cwA = *reinterpret_cast<const uint4*>( a.F.code + (size_t)sn * 512 + 8 * lane );
-        cwB = *reinterpret_cast<const uint4*>( a.F.code + (size_t)sn * 512 + 256 + 8 * lane );
-        entry( t + stride );
+    auto codes = [&]( int h ) {
+        if( h < nh ) cwn = *reinterpret_cast<const uint4*>( a.F.code + (size_t)hn.s * 512 + hn.hi * 256 + 8 * lane );
     };
-    int t = (int)bid * W + ( threadIdx.x >> 5 );
-    entry( t );
-    fetch( t );
+    int h = (int)bid * W + ( threadIdx.x >> 5 );
+    entry( h );
+    codes( h );
     __shared__ float2 s_dq[W];
     bora_pdl_wait();  // the previous kernel's results are complete from here
     if( threadIdx.x == 0 ) s_sc = scale_from( a.red.ring, a.slot_rr );
@@ -311,172 +338,107 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
     }
     if( P == 1 && upd ) alpha = df_ratio( a.red.ringf[a.slot_rz_in], a.red.ringf[a.slot_dq_in] );
     __syncthreads();
-    const float sc = s_sc;
+    const float sc = s_sc, unscale = 1.f / sc;
     DF acc{ 0.f, 0.f };  // down 1: r.r of the updated residual; up 2: r.z
+    __half* const scr = reinterpret_cast<__half*>( a.scratch );
     // the loop's bound is the block's, not the warp's: control flow that the compiler knows to be
-    // uniform, without a reconvergence around each shuffle; a warp past the last tile has no
+    // uniform, without a reconvergence around each shuffle; a warp past the last half tile has no
     // neighbours and neither loads nor stores
 #pragma unroll 1
-    for( int base = (int)bid * W; base < a.ft.n; base += stride, t += stride )
+    for( int base = (int)bid * W; base < nh; base += stride, h += stride )
     {
-        const bool mine = t < a.ft.n;
-        const int s = sn;
-        int nf[6];
-#pragma unroll
-        for( int q = 0; q < 6; ++q ) nf[q] = mine ? nfn[q] : -1;
-        const size_t gA = (size_t)s * 512 + 8 * lane, gB = gA + 256;
-        uint16_t cA[8], cB[8];
-        {
-            const uint32_t wa[4] = { cwA.x, cwA.y, cwA.z, cwA.w }, wb[4] = { cwB.x, cwB.y, cwB.z, cwB.w };
-#pragma unroll
-            for( int i = 0; i < 4; ++i )
-            {
-                cA[2 * i] = (uint16_t)( wa[i] & 0xffffu ); cA[2 * i + 1] = (uint16_t)( wa[i] >> 16 );
-                cB[2 * i] = (uint16_t)( wb[i] & 0xffffu ); cB[2 * i + 1] = (uint16_t)( wb[i] >> 16 );
-            }
-        }
-        fetch( t + stride );
-        float rA[8] = {}, rB[8] = {};  // r' on fluid cells
+        const bool mine = h < nh;
+        const HalfTile ht = hn;
+        const int st = mine ? ht.s : -1, c0 = ht.hi * 256 + 8 * lane;
+        const size_t g = (size_t)ht.s * 512 + c0;
+        const uint4 cw = cwn;
+        entry( h + stride );
+        float r[8] = {}, q[8] = {}, v[8], sum[8];
         if( mine )
         {
-            f32x8( a.r0, gA, rA );
-            f32x8( a.r0, gB, rB );
+            bora_ld8( a.r0 + g, r );
+            if( upd ) bora_ld8( a.q + g, q );
         }
-        if( upd && mine )
-        {
-            float qA[8], qB[8];
-            f32x8( a.q, gA, qA );
-            f32x8( a.q, gB, qB );
+        uint16_t c[8];
+        codes8( cw, c );
+        auto update = [&]() {
+            if( !upd ) return;
 #pragma unroll
-            for( int i = 0; i < 8; ++i )
-            {
-                rA[i] = fmaf( -alpha, qA[i], rA[i] );
-                rB[i] = fmaf( -alpha, qB[i], rB[i] );
-            }
-            if constexpr( P == 1 )
-            {
-                st_f32x8( a.r0, gA, rA );
-                st_f32x8( a.r0, gB, rB );
-            }
-        }
+            for( int i = 0; i < 8; ++i ) r[i] = fmaf( -alpha, q[i], r[i] );
+        };
         if constexpr( P == 0 )
         {
+            const FieldZ1 f{ a.F.code, a.r0, a.q, upd, alpha, sc, w };
+            Around<FieldZ1> ar;
+            ar.load( f, ht, lane );
+            update();
             float p = 0.f;
 #pragma unroll
-            for( int i = 0; i < 8; ++i ) { p = fmaf( rA[i], rA[i], p ); p = fmaf( rB[i], rB[i], p ); }
+            for( int i = 0; i < 8; ++i ) p = fmaf( r[i], r[i], p );
             if( mine ) acc = df_add_f( acc, p );
-        }
 #pragma unroll
-        for( int i = 0; i < 8; ++i )
-        {
-            rA[i] = cfluid( cA[i] ) ? rA[i] * sc : 0.f;
-            rB[i] = cfluid( cB[i] ) ? rB[i] * sc : 0.f;
-        }
-        float vA[8], vB[8], sA[8], sB[8];
-        if constexpr( P == 0 )
-        {
-#pragma unroll
-            for( int i = 0; i < 8; ++i )
-            {
-                vA[i] = cfluid( cA[i] ) ? rA[i] * w[cdiag( cA[i] )] : 0.f;
-                vB[i] = cfluid( cB[i] ) ? rB[i] * w[cdiag( cB[i] )] : 0.f;
-            }
-            row_sums( FieldZ1{ a.F.code, a.r0, upd ? a.q : nullptr, alpha, sc, w }, nf, lane, vA, vB, sA, sB );
-#pragma unroll
-            for( int i = 0; i < 8; ++i )
-            {
-                vA[i] = sweep( vA[i], rA[i], cA[i], sA[i], w + 16 );
-                vB[i] = sweep( vB[i], rB[i], cB[i], sB[i], w + 16 );
-            }
-            if( mine )
-            {
-                st_f16x8( reinterpret_cast<__half*>( a.scratch ), gA, vA );
-                st_f16x8( reinterpret_cast<__half*>( a.scratch ), gB, vB );
-            }
-        }
-        else if constexpr( P == 1 )
-        {
-            const FieldF16 f{ reinterpret_cast<const __half*>( a.scratch ) };
-            f.row( mine ? s : -1, 8 * lane, vA );
-            f.row( mine ? s : -1, 256 + 8 * lane, vB );
-            row_sums( f, nf, lane, vA, vB, sA, sB );
-            float qA[8], qB[8];  // residuals
-#pragma unroll
-            for( int i = 0; i < 8; ++i )
-            {
-                qA[i] = cfluid( cA[i] ) ? rA[i] - ( (float)cdiag( cA[i] ) * vA[i] - sA[i] ) : 0.f;
-                qB[i] = cfluid( cB[i] ) ? rB[i] - ( (float)cdiag( cB[i] ) * vB[i] - sB[i] ) : 0.f;
-            }
-            if( mine )
-            {
-                st_f16x8( a.F.z0, gA, vA );
-                st_f16x8( a.F.z0, gB, vB );
-            }
-            // restriction: x pairs in the row, y pairs from lane j + 1, z pairs from lane + 8
-            float pA[4], pB[4];
-#pragma unroll
-            for( int q = 0; q < 4; ++q )
-            {
-                pA[q] = qA[2 * q] + qA[2 * q + 1];
-                pB[q] = qB[2 * q] + qB[2 * q + 1];
-                pA[q] = pA[q] + __shfl_down_sync( kAll, pA[q], 1 );
-                pB[q] = pB[q] + __shfl_down_sync( kAll, pB[q], 1 );
-                pA[q] = pA[q] + __shfl_down_sync( kAll, pA[q], 8 );
-                pB[q] = pB[q] + __shfl_down_sync( kAll, pB[q], 8 );
-            }
-            if( mine && !( j & 1 ) && !( kq & 1 ) )
-            {
-                __half* cr = a.C.r + (size_t)s * 64 + 4 * ( j >> 1 );
-                *reinterpret_cast<uint2*>( cr + 16 * ( kq >> 1 ) ) =
-                    make_uint2( pack2( 0.5f * pA[0], 0.5f * pA[1] ), pack2( 0.5f * pA[2], 0.5f * pA[3] ) );
-                *reinterpret_cast<uint2*>( cr + 16 * ( 2 + ( kq >> 1 ) ) ) =
-                    make_uint2( pack2( 0.5f * pB[0], 0.5f * pB[1] ), pack2( 0.5f * pB[2], 0.5f * pB[3] ) );
-            }
+            for( int i = 0; i < 8; ++i ) v[i] = cfluid( c[i] ) ? ( r[i] * sc ) * w[cdiag( c[i] )] : 0.f;
+            ar.sums( f, lane, v, sum );
         }
         else if constexpr( P == 2 )
         {
             const FieldZa f{ a.F.code, a.F.z0, a.C.z1 };
-            f.row( mine ? s : -1, 8 * lane, vA );
-            f.row( mine ? s : -1, 256 + 8 * lane, vB );
-            row_sums( f, nf, lane, vA, vB, sA, sB );
-#pragma unroll
-            for( int i = 0; i < 8; ++i )
-            {
-                vA[i] = sweep( vA[i], rA[i], cA[i], sA[i], w + 16 );
-                vB[i] = sweep( vB[i], rB[i], cB[i], sB[i], w + 16 );
-            }
-            if( mine )
-            {
-                st_f16x8( reinterpret_cast<__half*>( a.scratch ), gA, vA );
-                st_f16x8( reinterpret_cast<__half*>( a.scratch ), gB, vB );
-            }
+            typename FieldZa::Row own;
+            f.load( own, st, c0 );
+            Around<FieldZa> ar;
+            ar.load( f, ht, lane );
+            f.value( own, v );
+            ar.sums( f, lane, v, sum );
         }
         else
         {
-            const FieldF16 f{ reinterpret_cast<const __half*>( a.scratch ) };
-            f.row( mine ? s : -1, 8 * lane, vA );
-            f.row( mine ? s : -1, 256 + 8 * lane, vB );
-            row_sums( f, nf, lane, vA, vB, sA, sB );
-            float rawA[8] = {}, rawB[8] = {};
-            if( mine )
+            const FieldF16 f{ scr };
+            typename FieldF16::Row own;
+            f.load( own, st, c0 );
+            Around<FieldF16> ar;
+            ar.load( f, ht, lane );
+            update();
+            if( P == 1 && upd && mine ) bora_st8( a.r0 + g, r );
+            if( P == 1 && mine ) *reinterpret_cast<uint4*>( a.F.z0 + g ) = own.v;  // z0 keeps z2
+            f.value( own, v );
+            ar.sums( f, lane, v, sum );
+        }
+        codes( h + stride );
+        if constexpr( P == 0 || P == 2 )
+        {
+#pragma unroll
+            for( int i = 0; i < 8; ++i ) v[i] = sweep( v[i], r[i] * sc, c[i], sum[i], w + 16 );
+            if( mine ) st_f16x8( scr, g, v );
+        }
+        else if constexpr( P == 1 )
+        {
+            // the residual, restricted: x pairs in the row, y pairs from lane j + 1, z pairs from lane + 8
+            float p[4];
+#pragma unroll
+            for( int i = 0; i < 8; ++i ) sum[i] = cfluid( c[i] ) ? r[i] * sc - ( (float)cdiag( c[i] ) * v[i] - sum[i] ) : 0.f;
+#pragma unroll
+            for( int i = 0; i < 4; ++i )
             {
-                f32x8( a.r0, gA, rawA );
-                f32x8( a.r0, gB, rawB );
+                p[i] = sum[2 * i] + sum[2 * i + 1];
+                p[i] = p[i] + __shfl_down_sync( kAll, p[i], 1 );
+                p[i] = p[i] + __shfl_down_sync( kAll, p[i], 8 );
             }
+            if( mine && !( j & 1 ) && !( kk & 1 ) )
+                *reinterpret_cast<uint2*>( a.C.r + (size_t)ht.s * 64 + 4 * ( j >> 1 ) + 16 * ( 2 * ht.hi + ( kk >> 1 ) ) ) =
+                    make_uint2( pack2( 0.5f * p[0], 0.5f * p[1] ), pack2( 0.5f * p[2], 0.5f * p[3] ) );
+        }
+        else
+        {
             float trz = 0.f;
 #pragma unroll
             for( int i = 0; i < 8; ++i )
             {
-                // undo the FP16 scaling of the residual
-                vA[i] = sweep( vA[i], rA[i], cA[i], sA[i], w ) / sc;
-                vB[i] = sweep( vB[i], rB[i], cB[i], sB[i], w ) / sc;
-                if( cfluid( cA[i] ) ) trz = fmaf( rawA[i], vA[i], trz );
-                if( cfluid( cB[i] ) ) trz = fmaf( rawB[i], vB[i], trz );
+                v[i] = sweep( v[i], r[i] * sc, c[i], sum[i], w ) * unscale;  // undo the FP16 scaling of the residual
+                if( cfluid( c[i] ) ) trz = fmaf( r[i], v[i], trz );
             }
             if( mine )
             {
-                st_f32x8( a.zout, gA, vA );
-                st_f32x8( a.zout, gB, vB );
+                bora_st8( a.zout + g, v );
                 acc = df_add_f( acc, trz );
             }
         }
@@ -486,13 +448,13 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
 }
 
 template <int W, int P>
-__global__ void __launch_bounds__( 32 * W, 16 / W ) k_mg_pass0( const __grid_constant__ Pass0Args a )
+__global__ void __launch_bounds__( 32 * W, pass_warps_per_sm( P ) / W ) k_mg_pass0( const __grid_constant__ Pass0Args a )
 {
     pass0_body<W, P>( a, blockIdx.x, gridDim.x );
 }
 
 template <int W, int P>
-__global__ void __launch_bounds__( 32 * W, 16 / W ) k_mg_pass0_batch( const __grid_constant__ BoraBatchLaunch L )
+__global__ void __launch_bounds__( 32 * W, pass_warps_per_sm( P ) / W ) k_mg_pass0_batch( const __grid_constant__ BoraBatchLaunch L )
 {
     unsigned bid;
     const int k = bora_batch_member( L, blockIdx.x, &bid );
@@ -684,9 +646,9 @@ void launch_pass0( const Pass0Args& a, int v, cudaStream_t st )
 }  // namespace
 
 // Grid of the passes of a level with E cells per tile edge in launch shape v: level 0 as many
-// blocks as make equal rounds of warps over the tiles with up to 16 warps per SM (the up 2 pass,
-// shape kReduceWarps, reduces over them: at most kBoraMaxReduceBlocks); levels 1 and 2 one
-// thread per cell.
+// blocks as make equal rounds of warps over the half tiles with the warps per SM that its
+// registers allow (v < 0: the reducing passes, at most kBoraMaxReduceBlocks); levels 1 and 2
+// one thread per cell.
 int bora_mg_pass_grid( int E, int ntiles, int v )
 {
     if( ntiles <= 0 ) return 0;
@@ -694,9 +656,9 @@ int bora_mg_pass_grid( int E, int ntiles, int v )
     if( E == 8 )
     {
         const int W = v < 0 ? kReduceWarps : kPassWarpsOf[std::min( v, 2 )];
-        const int cap = std::max( 1, std::min( 32 / W * sms, kBoraMaxReduceBlocks ) ) * W;
-        const int rounds = ( ntiles + cap - 1 ) / cap;
-        return std::max( 1, ( ntiles + W * rounds - 1 ) / ( W * rounds ) );
+        const int cap = std::max( 1, std::min( ( v < 0 ? kReduceWarpsPerSm : kPassWarpsPerSm ) / W * sms, kBoraMaxReduceBlocks ) ) * W;
+        const int rounds = ( 2 * ntiles + cap - 1 ) / cap;
+        return std::max( 1, ( 2 * ntiles + W * rounds - 1 ) / ( W * rounds ) );
     }
     const int T = kFlatThreadsOf[std::min( std::max( v, 0 ), 3 )];
     const size_t n = (size_t)ntiles * E * E * E;
@@ -767,14 +729,13 @@ void bora_launch_mg_pass_batch( int l, int pass, int v, const BoraBatchLaunch& L
         }
         const int W = kPassWarpsOf[std::min( std::max( v, 0 ), 2 )];
         const dim3 blk( 32 * W );
-        auto go = [&]( auto k0, auto k1, auto k2 ) {
-            if( pass == 0 ) bora_launch_pdl( k0, grid, blk, 0, st, L );
-            else if( pass == 1 ) bora_launch_pdl( k1, grid, blk, 0, st, L );
+        auto go = [&]( auto k1, auto k2 ) {
+            if( pass == 1 ) bora_launch_pdl( k1, grid, blk, 0, st, L );
             else bora_launch_pdl( k2, grid, blk, 0, st, L );
         };
-        if( W == 2 ) go( k_mg_pass0_batch<2, 0>, k_mg_pass0_batch<2, 1>, k_mg_pass0_batch<2, 2> );
-        else if( W == 4 ) go( k_mg_pass0_batch<4, 0>, k_mg_pass0_batch<4, 1>, k_mg_pass0_batch<4, 2> );
-        else go( k_mg_pass0_batch<8, 0>, k_mg_pass0_batch<8, 1>, k_mg_pass0_batch<8, 2> );
+        if( W == 2 ) go( k_mg_pass0_batch<2, 1>, k_mg_pass0_batch<2, 2> );
+        else if( W == 4 ) go( k_mg_pass0_batch<4, 1>, k_mg_pass0_batch<4, 2> );
+        else go( k_mg_pass0_batch<8, 1>, k_mg_pass0_batch<8, 2> );
         return;
     }
     const int T = kFlatThreadsOf[std::min( std::max( v, 0 ), 3 )];
