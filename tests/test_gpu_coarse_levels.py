@@ -1,9 +1,9 @@
 """The V-cycle's coarse levels (vare_gb300/csrc/mg_mid.cu) in their forms: one CTA or a cluster
 (up to and past 2048 level-3 cells), one or two coarsest cells per thread (a coarsest level
 of more than 256 cells below few tiles), batches that hold both. Every form is the same
-arithmetic: a simulation gives the same bits alone and in the mix, and the iteration count
-is that of the general coarse kernel where a simulation's own hierarchy uses it (levels held
-in 16 bits there: within two iterations)."""
+arithmetic: a simulation gives the same bits alone and in the mix. Its own step outside a
+batch has a shallower hierarchy where it is small (the coarsest level is level 2 or 3, run by
+the same kernel): the iteration count is within two."""
 import numpy as np
 import pytest
 

@@ -372,12 +372,12 @@ void bora_mg_setup( const BoraGridDev& g, BoraLevelDev* levels, int nlevels, Bor
 // Kernel launches of one bora_mg_vcycle call for this hierarchy.
 int bora_mg_vcycle_launches( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t,
                              const void* mid_image );
-// Level 3 .. coarsest of a V-cycle in one thread-block cluster out of distributed shared
+// Level 2 or 3 .. coarsest of a V-cycle in one thread-block cluster out of distributed shared
 // memory (mg_mid.cu). bora_mg_mid_image_bytes: the device buffer its per-step static image
 // needs, 0 when the hierarchy does not have the shape or size it handles;
 // bora_mg_mid_setup: lay the image out (once per step, after bora_mg_setup's codes);
-// bora_mg_mid_vcycle: 1 when it runs these levels (launching the kernel when `launch`), 0
-// when the caller must run them itself.
+// bora_mg_mid_vcycle: the first level that it runs, 2 or 3 (launching the kernel when `launch`),
+// 0 when the caller must run them all itself.
 size_t bora_mg_mid_image_bytes( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t, int ntiles );
 void bora_mg_mid_setup( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t, int ntiles,
                         void* image, cudaStream_t st );

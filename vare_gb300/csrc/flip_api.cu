@@ -591,7 +591,16 @@ int build_hierarchy( bora_flip_sim* s )
         return BORA_OK;
     };
     auto half_up = []( int v ) { return ( v + 1 ) / 2; };
+    // the coarse levels run in one kernel when they fit it; its static image
     s->mg_mid_on = false;
+    auto finish = [&]() -> int {
+        s->nlevels = n;
+        const size_t img = bora_mg_mid_image_bytes( g, s->levels, n, s->tiles(), (int)nt );
+        if( img == 0 ) return BORA_OK;
+        BORA_TRY( grow( s->mg_mid, img, false, s->st ) );
+        s->mg_mid_on = true;
+        return BORA_OK;
+    };
     BORA_TRYS( add( 0, 8, nt * 512, 0, 0, 0 ) );
     for( int E = 4; E >= 1; E /= 2 )
     {
@@ -599,7 +608,7 @@ int build_hierarchy( bora_flip_sim* s )
         BORA_TRYS( add( 0, E, nt * (size_t)E * E * E, 0, 0, 0 ) );
         // a batched step keeps the tiled levels 0-3 and at least one dense level below them
         // (the shape of its launches), whatever the size
-        if( !s->batching && s->levels[n - 1].ncells <= 512 ) { s->nlevels = n; return BORA_OK; }
+        if( !s->batching && s->levels[n - 1].ncells <= 512 ) return finish();
     }
     // level 3 has one cell per tile; its extent is the tile grid
     while( true )
@@ -608,15 +617,7 @@ int build_hierarchy( bora_flip_sim* s )
         BORA_TRYS( add( 1, 0, (size_t)ex * ey * ez, ex, ey, ez ) );
         if( s->levels[n - 1].ncells <= 512 ) break;
     }
-    s->nlevels = n;
-    // the coarse levels run in one cluster kernel when they fit it; its static image
-    const size_t img = bora_mg_mid_image_bytes( g, s->levels, n, s->tiles(), (int)nt );
-    if( img > 0 )
-    {
-        BORA_TRY( grow( s->mg_mid, img, false, s->st ) );
-        s->mg_mid_on = true;
-    }
-    return BORA_OK;
+    return finish();
 }
 
 // The table of the solver's tiles from the per-tile flags; the count reaches the host later

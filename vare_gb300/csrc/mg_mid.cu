@@ -1,5 +1,5 @@
 // The coarse tail of the multigrid V-cycle (level 3, one cell per 8^3 tile, down to the
-// coarsest level and back) in one thread-block cluster whose CTAs keep every value in
+// coarsest level and back; level 2 alone where it is the coarsest) in one thread-block cluster whose CTAs keep every value in
 // distributed shared memory.
 //
 // Levels 0-2 are large and run as grid-wide fused tile kernels (multigrid.cu). Below them
@@ -71,7 +71,7 @@ __device__ inline int32_t pack_ref( int owner, int local ) { return ( owner << 2
 
 struct MidLevel
 {
-    int tiled;       // 1: one cell per active tile (level 3); 0: dense
+    int E;           // cells per tile edge: 2 (level 2, the coarsest), 1 (level 3); 0: dense
     int n;           // cells
     int chunk;       // cells per CTA (the coarsest level: all, in CTA 0)
     int dx, dy, dz;  // dense extent
@@ -83,13 +83,13 @@ struct MidLevel
 struct MidDesc
 {
     MidLevel L[kMidMaxLevels];
-    int n;  // levels; L[0] is level 3 of the hierarchy, then dense; the last is the coarsest
+    int n;  // levels; L[0] is level 2 or 3 of the hierarchy; the last is the coarsest
     const int32_t* nbr;
     const int32_t* tile_of;
     const int32_t* slot_of;
     int tx, ty, tz;
-    const __half* r_in;  // level-3 residual (written by the level-2 down kernel)
-    __half* z_out;       // level-3 correction (read by the level-2 up kernel)
+    const __half* r_in;  // the first level's residual (written by the finer level's down kernel)
+    __half* z_out;       // its correction (read by the finer level's up kernel)
     int sweeps;
     int ctas, threads;
     int static_bytes;    // bytes of a CTA's static block (a multiple of 16)
@@ -147,48 +147,57 @@ struct Mid
         else cl.sync();
     }
 
+    // cell of level L next to cell c in direction q (-x +x -y +y -z +z), or -1
+    __device__ int neighbour( const MidLevel& L, int c, int q ) const
+    {
+        const int s = q & 1 ? 1 : -1, ax = q >> 1;
+        if( L.E )
+        {
+            const int sh = L.E == 2 ? 1 : 0, l = c & ( L.E * L.E * L.E - 1 ), bit = 1 << ax;
+            const int t = c >> ( 3 * sh );
+            const int at = sh ? ( l >> ax ) & 1 : 0;  // the cell's coordinate on the axis inside its tile
+            const int l2 = sh ? l ^ bit : l;          // one cell along the axis, in this tile or wrapped into the next
+            if( at + s >= 0 && at + s < L.E ) return ( t << ( 3 * sh ) ) | l2;
+            const int tn = d.nbr[(size_t)t * 27 + kFaceDir[q]];
+            return tn < 0 ? -1 : ( tn << ( 3 * sh ) ) | l2;
+        }
+        const int x = c % L.dx, y = ( c / L.dx ) % L.dy, z = c / ( L.dx * L.dy );
+        const int at = ax == 0 ? x : ( ax == 1 ? y : z ), n = ax == 0 ? L.dx : ( ax == 1 ? L.dy : L.dz );
+        if( at + s < 0 || at + s >= n ) return -1;
+        return c + s * ( ax == 0 ? 1 : ( ax == 1 ? L.dx : L.dx * L.dy ) );
+    }
     // static data of level t for the owned cells (codes, neighbours, parent, children),
-    // written into the block at `blk` (the CTA's slice of the image)
-    __device__ void stage( int t, char* blk ) const
+    // written into the block at `blk` (the CTA's slice of the image) by `parts` CTAs
+    __device__ void stage( int t, char* blk, int part, int parts ) const
     {
         const MidLevel& L = d.L[t];
         const int n = owned( L ), base = (int)me * L.chunk;
+        const int i0 = part * (int)blockDim.x + (int)threadIdx.x, di = parts * (int)blockDim.x;
         uint16_t* code = reinterpret_cast<uint16_t*>( blk + L.o_code );
         int32_t* nb = reinterpret_cast<int32_t*>( blk + L.o_nb );
-        for( int i = threadIdx.x; i < n; i += (int)blockDim.x ) code[i] = L.code[base + i];
-        __syncthreads();
-        for( int i = threadIdx.x; i < n * 6; i += (int)blockDim.x )
+        for( int i = i0; i < n; i += di )
         {
-            const int lc = i / 6, q = i % 6, c = base + lc;
-            int nc;
-            if( L.tiled ) nc = d.nbr[(size_t)c * 27 + kFaceDir[q]];
-            else
+            const int c = base + i;
+            uint16_t cc = L.code[c], bad = 0;
+#pragma unroll
+            for( int q = 0; q < 6; ++q )
             {
-                const int x = c % L.dx, y = ( c / L.dx ) % L.dy, z = c / ( L.dx * L.dy );
-                switch( q )
-                {
-                    case 0: nc = x > 0 ? c - 1 : -1; break;
-                    case 1: nc = x < L.dx - 1 ? c + 1 : -1; break;
-                    case 2: nc = y > 0 ? c - L.dx : -1; break;
-                    case 3: nc = y < L.dy - 1 ? c + L.dx : -1; break;
-                    case 4: nc = z > 0 ? c - L.dx * L.dy : -1; break;
-                    default: nc = z < L.dz - 1 ? c + L.dx * L.dy : -1; break;
-                }
+                const int nc = neighbour( L, c, q );
+                const bool on = ( cc & BORA_CODE_FLUID ) && ( cc & ( 1u << q ) );
+                if( on && nc < 0 ) bad = kCodeBad;
+                nb[q * L.chunk + i] = on && nc >= 0 ? ref( L, nc ) : zero_ref( L );
             }
-            const uint16_t cc = L.code[c];
-            const bool on = ( cc & BORA_CODE_FLUID ) && ( cc & ( 1u << q ) );
-            if( on && nc < 0 ) code[lc] = cc | kCodeBad;
-            nb[q * L.chunk + lc] = on && nc >= 0 ? ref( L, nc ) : zero_ref( L );
+            code[i] = cc | bad;
         }
         if( L.o_par >= 0 )
         {
             const MidLevel& P = d.L[t + 1];
             int32_t* par = reinterpret_cast<int32_t*>( blk + L.o_par );
-            for( int i = threadIdx.x; i < n; i += (int)blockDim.x )
+            for( int i = i0; i < n; i += di )
             {
                 const int c = base + i;
                 int x, y, z;
-                if( L.tiled )
+                if( L.E )
                 {
                     const int vt = d.tile_of[c];
                     x = vt % d.tx; y = ( vt / d.tx ) % d.ty; z = vt / ( d.tx * d.ty );
@@ -204,13 +213,13 @@ struct Mid
         {
             const MidLevel& F = d.L[t - 1];
             int32_t* ch = reinterpret_cast<int32_t*>( blk + L.o_ch );
-            for( int i = threadIdx.x; i < n * 8; i += (int)blockDim.x )
+            for( int i = i0; i < n * 8; i += di )
             {
                 const int lc = i / 8, o = i % 8, c = base + lc;
                 const int x = c % L.dx, y = ( c / L.dx ) % L.dy, z = c / ( L.dx * L.dy );
                 const int a = 2 * x + ( o & 1 ), b = 2 * y + ( ( o >> 1 ) & 1 ), e = 2 * z + ( o >> 2 );
                 int fc = -1;
-                if( F.tiled )
+                if( F.E )
                 {
                     if( a < d.tx && b < d.ty && e < d.tz ) fc = d.slot_of[( (size_t)e * d.ty + b ) * d.tx + a];
                 }
@@ -356,12 +365,13 @@ struct Mid
     }
 };
 
-// One CTA per cluster CTA: lay out that CTA's static block of the image (once per step).
-__global__ void __launch_bounds__( kMidThreadsMax ) k_mg_mid_image( const __grid_constant__ MidDesc d )
+// kImageParts CTAs per cluster CTA: lay out that CTA's static block of the image (once per step).
+constexpr int kImageParts = 8;
+__global__ void __launch_bounds__( 256 ) k_mg_mid_image( const __grid_constant__ MidDesc d )
 {
-    Mid<false> m{ d, cg::this_cluster(), blockIdx.x };
-    char* blk = d.image + (size_t)blockIdx.x * d.static_bytes;
-    for( int t = 0; t < d.n; ++t ) m.stage( t, blk );
+    Mid<false> m{ d, cg::this_cluster(), blockIdx.x / kImageParts };
+    char* blk = d.image + (size_t)m.me * d.static_bytes;
+    for( int t = 0; t < d.n; ++t ) m.stage( t, blk, (int)( blockIdx.x % kImageParts ), kImageParts );
 }
 
 template <bool ONE>
@@ -393,7 +403,8 @@ __device__ __forceinline__ void mg_mid_body( const MidDesc& d )
         const MidLevel& L = d.L[tid >> 1];
         m.template arr<float>( tid & 1 ? L.o_b : L.o_a )[L.chunk] = 0.f;
     }
-    bora_pdl_wait();  // the level-2 down kernel's restricted residual is complete from here
+    bora_pdl_wait();  // the finer level's restricted residual is complete from here
+    const int last = d.n - 1;
     {
         const MidLevel& L = d.L[0];
         const int n = m.owned( L );
@@ -411,12 +422,11 @@ __device__ __forceinline__ void mg_mid_body( const MidDesc& d )
             if( cc & kCodeBad ) atomicOr( d.err, 4u );
             const float rv = ( cc & BORA_CODE_FLUID ) ? __half2float( i == tid ? first : g[i] ) : 0.f;
             r[i] = rv;
-            a[i] = ( ( cc & BORA_CODE_FLUID ) && dg > 0 ) ? wA[dg] * rv : 0.f;
+            a[i] = ( ( cc & BORA_CODE_FLUID ) && dg > 0 ) ? ( last ? wA : wC )[dg] * rv : 0.f;
         }
     }
     m.barrier();
     // ---- down ----
-    const int last = d.n - 1;
     for( int t = 0; t < last; ++t )
     {
         const MidLevel& L = d.L[t];
@@ -447,7 +457,7 @@ __device__ __forceinline__ void mg_mid_body( const MidDesc& d )
         float* b = m.template arr<float>( L.o_b );
         m.sweep( t, L.o_a, wB, [&]( int lc, float v ) { b[lc] = v; } );
         m.barrier();
-        // the level's final correction: A, or level 3's result
+        // the level's final correction: A, or the first level's result
         if( t > 0 )
         {
             float* a = m.template arr<float>( L.o_a );
@@ -459,6 +469,11 @@ __device__ __forceinline__ void mg_mid_body( const MidDesc& d )
             __half* g = d.z_out + (size_t)m.me * L.chunk;
             m.sweep( t, L.o_b, wA, [&]( int lc, float v ) { g[lc] = __float2half_rn( v ); } );
         }
+    }
+    if( last == 0 && m.me == 0 )
+    {
+        const float* z = m.template arr<float>( zc );
+        for( int i = tid; i < Lc.n; i += (int)blockDim.x ) d.z_out[i] = __float2half_rn( z[i] );
     }
     m.barrier();  // no CTA leaves while another may still read its shared memory
 }
@@ -550,25 +565,30 @@ size_t mid_layout( MidDesc& d, int ctas )
     return off;
 }
 
-// The cluster layout of level 3 .. coarsest, or false when the hierarchy does not have the
-// shape this kernel handles (level 3 with one cell per tile, then dense grids ending at
-// <= 512 cells) or a level does not fit the cluster's shared memory.
-bool mid_describe( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t, int ntiles, int sweeps,
-                   MidDesc& d, size_t& smem )
+// The layout of the first level it takes (2 or 3) .. coarsest, or 0 when the hierarchy does not
+// have the shape this kernel handles (ending at <= 512 cells) or does not fit the cluster's
+// shared memory.
+int mid_describe( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t, int ntiles, int sweeps,
+                  MidDesc& d, size_t& smem )
 {
-    constexpr int first = 3;
-    if( nlevels < first + 2 || nlevels - first > kMidMaxLevels || ntiles <= 0 || sweeps < 1 ) return false;
-    if( levels[first].kind != 0 || levels[first].E != 1 || (int)levels[first].ncells != ntiles ) return false;
-    for( int l = first + 1; l < nlevels; ++l )
-        if( levels[l].kind != 1 ) return false;
-    if( levels[nlevels - 1].ncells > 512 || ntiles >= ( 1 << 24 ) ) return false;
+    if( ntiles <= 0 || ntiles >= ( 1 << 24 ) || sweeps < 1 || nlevels < 3 ) return 0;
+    if( levels[nlevels - 1].ncells > 512 ) return 0;
+    const int cluster = mid_cluster_size();
+    if( cluster == 0 ) return 0;
+    // from level 3, or level 2 where that is the coarsest (with level 2 in it at larger sizes, a
+    // V-cycle is 2 us shorter of 36 at 152 tiles, as long at 304 and 3 us longer at 2568)
+    const int first = nlevels == 3 ? 2 : 3;
+    if( nlevels - first > kMidMaxLevels ) return 0;
     d = MidDesc{};
     d.n = nlevels - first;
     for( int q = 0; q < d.n; ++q )
     {
-        const BoraLevelDev& B = levels[first + q];
+        const int l = first + q;
+        const BoraLevelDev& B = levels[l];
         MidLevel& L = d.L[q];
-        L.tiled = q == 0;
+        if( ( B.kind == 0 ) != ( l <= 3 ) ) return 0;
+        L.E = B.kind == 0 ? B.E : 0;
+        if( l <= 3 && ( L.E != ( l == 2 ? 2 : 1 ) || B.ncells != (size_t)ntiles * L.E * L.E * L.E ) ) return 0;
         L.n = (int)B.ncells;
         L.dx = B.dx; L.dy = B.dy; L.dz = B.dz;
         L.code = B.code;
@@ -578,12 +598,10 @@ bool mid_describe( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels
     d.r_in = levels[first].r;
     d.z_out = levels[first].z0;
     d.sweeps = sweeps;
-    const int ctas = mid_cluster_size();
-    if( ctas == 0 ) return false;
     smem = 0;
-    if( ntiles <= kMidSingleMax && ( smem = mid_layout( d, 1 ) ) <= kMidSmemMax ) return true;
-    smem = mid_layout( d, ctas );
-    return smem <= kMidSmemMax;
+    if( d.L[0].n <= kMidSingleMax && ( smem = mid_layout( d, 1 ) ) <= kMidSmemMax ) return first;
+    smem = mid_layout( d, cluster );
+    return smem <= kMidSmemMax ? first : 0;
 }
 
 // One launch of the V-cycle kernel: `blocks` CTAs of `threads` in clusters of `ctas`.
@@ -625,7 +643,7 @@ void bora_mg_mid_setup( const BoraGridDev& g, const BoraLevelDev* levels, int nl
     size_t smem = 0;
     if( !image || !mid_describe( g, levels, nlevels, t, ntiles, 16, d, smem ) ) return;
     d.image = static_cast<char*>( image );
-    k_mg_mid_image<<<d.ctas, kMidThreadsMax, 0, st>>>( d );
+    k_mg_mid_image<<<d.ctas * kImageParts, 256, 0, st>>>( d );
 }
 
 int bora_mg_mid_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, BoraTilesDev t, int ntiles,
@@ -633,12 +651,13 @@ int bora_mg_mid_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nl
 {
     MidDesc d;
     size_t smem = 0;
-    if( !image || !mid_describe( g, levels, nlevels, t, ntiles, sweeps, d, smem ) ) return 0;
-    if( !launch ) return 1;
+    const int first = image ? mid_describe( g, levels, nlevels, t, ntiles, sweeps, d, smem ) : 0;
+    if( !first ) return 0;
+    if( !launch ) return first;
     d.image = static_cast<char*>( const_cast<void*>( image ) );
     d.err = err;
     mid_launch( k_mg_mid<true>, k_mg_mid<false>, d.ctas, d.ctas, d.threads, smem, st, d );
-    return 1;
+    return first;
 }
 
 size_t bora_mg_mid_desc_bytes() { return sizeof( MidDesc ); }

@@ -700,9 +700,8 @@ int bora_mg_vcycle_launches( const BoraGridDev& g, const BoraLevelDev* levels, i
 {
     if( nlevels < 2 ) return 0;
     const int ntiles = levels[0].kind == 0 ? (int)( levels[0].ncells / 512 ) : 0;
-    const int first = bora_mg_mid_vcycle( g, levels, nlevels, t, ntiles, mid_image, nullptr, 16, nullptr, false )
-                          ? 3
-                          : tail_start( levels, nlevels );
+    const int mid = bora_mg_mid_vcycle( g, levels, nlevels, t, ntiles, mid_image, nullptr, 16, nullptr, false );
+    const int first = mid ? mid : tail_start( levels, nlevels );
     const int stop = std::min( first, nlevels - 1 );
     int n = 1;  // the tail kernel, or the coarsest-level kernel
     for( int l = 0; l < stop; ++l ) n += 4;
@@ -717,10 +716,10 @@ void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nleve
     if( levels[0].ncells == 0 ) return;
     const int last = nlevels - 1;
     const int ntiles = levels[0].kind == 0 ? (int)( levels[0].ncells / 512 ) : 0;
-    // level 3 .. coarsest in one cluster out of distributed shared memory (mg_mid.cu) when
+    // level 2 or 3 .. coarsest in one CTA or cluster out of shared memory (mg_mid.cu) when
     // the hierarchy fits it; otherwise the tail levels run from global memory (k_mg_tail)
-    const bool mid = bora_mg_mid_vcycle( g, levels, nlevels, t, ntiles, mid_image, red.err, coarse_sweeps, st, false ) != 0;
-    const int first = mid ? 3 : tail_start( levels, nlevels );  // levels [first, last] run in one kernel
+    const int mid = bora_mg_mid_vcycle( g, levels, nlevels, t, ntiles, mid_image, red.err, coarse_sweeps, st, false );
+    const int first = mid ? mid : tail_start( levels, nlevels );  // levels [first, last] run in one kernel
     const int stop = std::min( first, last );                     // levels [0, stop) restrict/prolong here
     // down: pre-smooth and restrict
     for( int l = 0; l < stop; ++l )
