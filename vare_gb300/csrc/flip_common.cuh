@@ -106,6 +106,21 @@ __host__ __device__ inline int bora_dir( int dx, int dy, int dz ) { return ( dx 
 // of its dual cell (the base cell max(int(p - 0.5), 0) of the P2G stencil, Rasterization.cu:
 // 139-141); killed particles get BORA_DEAD_KEY, live ones outside the grid (Grid::inside,
 // Grid.h:408-417) BORA_DEAD_KEY - 1 (they still activate their clamped tile).
+// (_inside: for a particle with no coordinate below 0 or beyond the grid; a NaN counts as 0)
+__device__ inline void bora_bin_tile_inside( int tx, int ty, int tz, float x, float y, float z, int& ti, int& tj, int& tk )
+{
+    ti = bora_imin( bora_trunc( x ) >> 3, tx - 1 );
+    tj = bora_imin( bora_trunc( y ) >> 3, ty - 1 );
+    tk = bora_imin( bora_trunc( z ) >> 3, tz - 1 );
+}
+__device__ inline uint32_t bora_bin_inside_key( int tx, int ty, float x, float y, float z )
+{
+    const int di = bora_imax( bora_trunc( x - 0.5f ), 0 );
+    const int dj = bora_imax( bora_trunc( y - 0.5f ), 0 );
+    const int dk = bora_imax( bora_trunc( z - 0.5f ), 0 );
+    const uint32_t vt = (uint32_t)( ( (size_t)( dk >> 3 ) * ty + ( dj >> 3 ) ) * tx + ( di >> 3 ) );
+    return vt * BORA_TILE_CELLS + (uint32_t)bora_local( di, dj, dk );
+}
 __device__ inline void bora_bin_tile( int tx, int ty, int tz, float x, float y, float z, int& ti, int& tj, int& tk )
 {
     ti = bora_imin( bora_imax( bora_trunc( x ) / BORA_TILE, 0 ), tx - 1 );
@@ -115,11 +130,7 @@ __device__ inline void bora_bin_tile( int tx, int ty, int tz, float x, float y, 
 __device__ inline uint32_t bora_bin_live_key( int nx, int ny, int nz, int tx, int ty, float x, float y, float z )
 {
     if( x < 0.f || x > (float)nx || y < 0.f || y > (float)ny || z < 0.f || z > (float)nz ) return BORA_DEAD_KEY - 1;
-    const int di = bora_imax( bora_trunc( x - 0.5f ), 0 );
-    const int dj = bora_imax( bora_trunc( y - 0.5f ), 0 );
-    const int dk = bora_imax( bora_trunc( z - 0.5f ), 0 );
-    const uint32_t vt = (uint32_t)( ( (size_t)( dk >> 3 ) * ty + ( dj >> 3 ) ) * tx + ( di >> 3 ) );
-    return vt * BORA_TILE_CELLS + (uint32_t)bora_local( di, dj, dk );
+    return bora_bin_inside_key( tx, ty, x, y, z );
 }
 // both parts, the tile flag stored in tile_flag
 __device__ inline uint32_t bora_bin_key( int nx, int ny, int nz, int tx, int ty, int tz, int32_t id, float x, float y,

@@ -15,10 +15,11 @@
 
 namespace {
 
-// Grid values of a tile and its high-side halo layer, (8+1)^3 cells, staged in shared
-// memory as two float4 per cell: (comp.x, comp.y, velo.x, velo.y) and (comp.z, velo.z, surf,
-// 0), so that the lerps of both vector fields read two float4 per corner. Cells of inactive
-// tiles hold the field backgrounds (0, and 10 for surf: FLIPMethod.cu:30).
+// Grid values of a tile and its high-side halo layer, (8+1)^3 cells, staged in shared memory: a
+// float4 (comp.x, comp.y, velo.x, velo.y) and a float2 (comp.z, velo.z) per cell, so that the
+// lerps of both vector fields take two loads per corner, and per base cell surf's minimum over
+// the eight corners. Cells of inactive tiles hold the field backgrounds (0, and 10 for surf:
+// FLIPMethod.cu:30).
 constexpr int kG2PThreads = 256;
 constexpr int kStageEdge = BORA_TILE + 1;
 constexpr int kStageCells = kStageEdge * kStageEdge * kStageEdge;
@@ -30,6 +31,7 @@ constexpr int kStageCells = kStageEdge * kStageEdge * kStageEdge;
 struct StagedLerp
 {
     int base;  // staged index of corner (i,j,k)
+    int cell;  // its index in the tile
     float x, y, z;
     __device__ inline void setup( const BoraGridDev& g, int ti, int tj, int tk, float px, float py, float pz )
     {
@@ -39,7 +41,10 @@ struct StagedLerp
         x = bora_clampf( px - ( (float)i + .5f ), 0.f, 1.f );
         y = bora_clampf( py - ( (float)j + .5f ), 0.f, 1.f );
         z = bora_clampf( pz - ( (float)k + .5f ), 0.f, 1.f );
-        base = ( i - ti * BORA_TILE ) + kStageEdge * ( ( j - tj * BORA_TILE ) + kStageEdge * ( k - tk * BORA_TILE ) );
+        // (the frame's extent is a multiple of 4, so that the clamp above leaves i in the tile)
+        const int li = i - ti * BORA_TILE, lj = j - tj * BORA_TILE, lk = k - tk * BORA_TILE;
+        base = li + kStageEdge * ( lj + kStageEdge * lk );
+        cell = li + BORA_TILE * ( lj + BORA_TILE * lk );
     }
     __device__ static inline int off( int q )
     {
@@ -50,28 +55,45 @@ struct StagedLerp
         return make_float4( a.x * ( 1.f - t ) + b.x * t, a.y * ( 1.f - t ) + b.y * t, a.z * ( 1.f - t ) + b.z * t,
                             a.w * ( 1.f - t ) + b.w * t );
     }
-    __device__ static inline float fminf_ref( float a, float b ) { return a < b ? a : b; }  // MathUtils.h:174
-    // comp and velo lerped from the staged cells (comp.xy and velo.xy from fa, comp.z and
-    // velo.z from fb), and lerpMin of surf; the corners' mix order and the min order are
-    // SparseField's
-    __device__ inline void sample( const float4* fa, const float4* fb, float4& comp, float4& velo, float& smin ) const
+    // the same by packed pairs: two FP32 operations an instruction, each rounded as alone. The sum
+    // is a fused b t * one + a (1 - t) with one = 1 from memory, because the compiler would fuse
+    // a packed product into a packed sum, which rounds once.
+    __device__ static inline float2 mix( float2 a, float2 b, float t, float one )
     {
-        auto lerp = [&]( const float4* f ) {
-            const float4 c00 = mix( f[base + off( 0 )], f[base + off( 1 )], x );
-            const float4 c01 = mix( f[base + off( 2 )], f[base + off( 3 )], x );
-            const float4 c10 = mix( f[base + off( 4 )], f[base + off( 5 )], x );
-            const float4 c11 = mix( f[base + off( 6 )], f[base + off( 7 )], x );
-            return mix( mix( c00, c10, y ), mix( c01, c11, y ), z );
-        };
-        const float4 A = lerp( fa ), B = lerp( fb );
-        comp = make_float4( A.x, A.y, B.x, 0.f );
-        velo = make_float4( A.z, A.w, B.y, 0.f );
-        auto w = [&]( int q ) { return fb[base + off( q )].z; };
+        return __ffma2_rn( __fmul2_rn( b, make_float2( t, t ) ), make_float2( one, one ),
+                           __fmul2_rn( a, make_float2( 1.f - t, 1.f - t ) ) );
+    }
+    __device__ static inline float4 mix( float4 a, float4 b, float t, float one )
+    {
+        const float2 lo = mix( make_float2( a.x, a.y ), make_float2( b.x, b.y ), t, one );
+        const float2 hi = mix( make_float2( a.z, a.w ), make_float2( b.z, b.w ), t, one );
+        return make_float4( lo.x, lo.y, hi.x, hi.y );
+    }
+    __device__ static inline float fminf_ref( float a, float b ) { return a < b ? a : b; }  // MathUtils.h:174
+    // the minimum of surf over the corners of the base cell at staged index b, in SparseField's order
+    __device__ static inline float corner_min( const float* surf, int b )
+    {
+        auto w = [&]( int q ) { return surf[b + off( q )]; };
         float v = fminf_ref( w( 0 ), w( 1 ) );
         v = fminf_ref( v, fminf_ref( w( 2 ), w( 3 ) ) );
         v = fminf_ref( v, fminf_ref( w( 4 ), w( 5 ) ) );
-        v = fminf_ref( v, fminf_ref( w( 6 ), w( 7 ) ) );
-        smin = v;
+        return fminf_ref( v, fminf_ref( w( 6 ), w( 7 ) ) );
+    }
+    // comp and velo lerped from the staged cells (comp.xy and velo.xy from fa, comp.z and
+    // velo.z from fb); the corners' mix order is SparseField's
+    __device__ inline void sample( const float4* fa, const float2* fb, float one, float4& comp, float4& velo ) const
+    {
+        auto lerp = [&]( const auto* f ) {
+            const auto c00 = mix( f[base + off( 0 )], f[base + off( 1 )], x, one );
+            const auto c01 = mix( f[base + off( 2 )], f[base + off( 3 )], x, one );
+            const auto c10 = mix( f[base + off( 4 )], f[base + off( 5 )], x, one );
+            const auto c11 = mix( f[base + off( 6 )], f[base + off( 7 )], x, one );
+            return mix( mix( c00, c10, y, one ), mix( c01, c11, y, one ), z, one );
+        };
+        const float4 A = lerp( fa );
+        const float2 B = lerp( fb );
+        comp = make_float4( A.x, A.y, B.x, 0.f );
+        velo = make_float4( A.z, A.w, B.y, 0.f );
     }
 };
 
@@ -180,13 +202,21 @@ __device__ inline float4 comp_at( const BoraGridDev& g, const int32_t* slot_of, 
 // FLIPMethod::updateParticles for one particle (FLIPMethod.cu:60-170); gn and go are the
 // grid's projected and pre-projection velocities lerped at the particle's position. With the
 // RK2 option each substep moves the particle by the midpoint rule in the grid velocity field
-// instead of by its own velocity; everything else is unchanged. kAll = false compiles the
-// common case alone: no water tank, no colliders, Euler advection (the caller checks).
-template <bool kAll>
-__device__ inline bool advance_particle( const BoraGridDev& g, float4 gn, float4 go, const int32_t* slot_of,
+// instead of by its own velocity; everything else is unchanged. The modes compile the common case
+// alone (no water tank, no colliders, Euler advection), the water tank and the colliders with Euler
+// advection, and everything (the caller checks). kCols = false leaves a particle that may meet a
+// collider alone and returns kLater: the collider code's calls would spill the registers of the
+// others. sub[]: dt / iter for iter < kSubTable.
+enum AdvanceMode { kCommon, kEuler, kEverything };
+constexpr int kSubTable = 32;
+constexpr int kLater = 2;
+
+template <int kMode, bool kCols>
+__device__ inline int advance_particle( const BoraGridDev& g, float4 gn, float4 go, const int32_t* slot_of,
                                          const BoraCellsDev& c, float& px, float& py, float& pz, float& vx, float& vy,
-                                         float& vz, float dt )
+                                         float& vz, float dt, const float* sub )
 {
+    constexpr bool kAll = kMode != kCommon, kRk2 = kMode == kEverything;
     const float lx = (float)g.nx + 0.5f, lz = (float)g.nz + 0.5f;
     const float wall = g.voxel_wall;
     {
@@ -212,7 +242,7 @@ __device__ inline bool advance_particle( const BoraGridDev& g, float4 gn, float4
     // particle whose start is farther than 2 |v| dt + 2 cells from every box sees positive
     // collider values all step long. (RK2 moves with the grid velocity: no cull.)
     bool hasCols = kAll && bora_col_active( g.cols );
-    if( hasCols && g.cols.tslot && g.advection != BORA_ADVECT_RK2 && inside_grid( g, px, py, pz ) )
+    if( hasCols && g.cols.tslot && !( kRk2 && g.advection == BORA_ADVECT_RK2 ) && inside_grid( g, px, py, pz ) )
     {
         // sparse collider: every sample outside its tiles is the (positive) background with
         // a zero normal and velocity; a particle whose tile has no collider tile within one
@@ -226,14 +256,15 @@ __device__ inline bool advance_particle( const BoraGridDev& g, float4 gn, float4
             if( !g.cols.tnear[(size_t)ti + (size_t)g.tx * ( (size_t)tj + (size_t)g.ty * tk )] ) hasCols = false;
         }
     }
-    else if( hasCols && !g.cols.fphi && g.advection != BORA_ADVECT_RK2 && inside_grid( g, px, py, pz ) )
+    else if( hasCols && !g.cols.fphi && !( kRk2 && g.advection == BORA_ADVECT_RK2 ) && inside_grid( g, px, py, pz ) )
     {
         const float reach = 2.f * sqrtf( vx * vx + vy * vy + vz * vz ) * dt + 2.f;
         hasCols = false;
         for( int n = 0; n < g.cols.count; ++n )
             if( !( bora_box_sdf( g.cols.box[n], px, py, pz ) > reach ) ) hasCols = true;
     }
-    if( hasCols )
+    if( !kCols && hasCols ) return kLater;
+    if( kCols && hasCols )
     {
         const float3 p = col_carry( &g, make_float3( px, py, pz ), dt );
         px = p.x; py = p.y; pz = p.z;
@@ -242,11 +273,11 @@ __device__ inline bool advance_particle( const BoraGridDev& g, float4 gn, float4
     {
         const float len = sqrtf( vx * vx + vy * vy + vz * vz );
         const int iter = 1 + bora_imin( bora_trunc( len * dt * 1.5f ), bora_imax( g.maxsubsteps, 1 ) );
-        const float sub_dt = dt / (float)iter;
+        const float sub_dt = iter < kSubTable ? sub[iter] : dt / (float)iter;
         bool col = false;
         for( int it = 0; it < iter; ++it )
         {
-            if( kAll && g.advection == BORA_ADVECT_RK2 )
+            if( kRk2 && g.advection == BORA_ADVECT_RK2 )
             {
                 const float h = 0.5f * sub_dt;
                 const float4 k1 = comp_at( g, slot_of, c, px, py, pz );
@@ -266,38 +297,50 @@ __device__ inline bool advance_particle( const BoraGridDev& g, float4 gn, float4
                 if( py > (float)g.ny ) { py = (float)g.ny; if( vy > 0.f ) vy = 0.f; }
                 if( pz > (float)g.nz ) { pz = (float)g.nz; if( vz > 0.f ) vz = 0.f; }
             }
-            if( hasCols )
+            if( kCols && hasCols )
             {
                 const float4 r = col_push( &g, make_float3( px, py, pz ) );
                 px = r.x; py = r.y; pz = r.z;
                 if( r.w != 0.f ) col = true;
             }
         }
-        if( col && col_kill( &g, make_float3( px, py, pz ) ) ) kill = true;
+        if( kCols && col && col_kill( &g, make_float3( px, py, pz ) ) ) kill = true;
         if( !inside_grid( g, px, py, pz ) ) kill = true;
     }
     vx += g.gravity[0] * dt; vy += g.gravity[1] * dt; vz += g.gravity[2] * dt;
-    return kill;
+    return kill ? 1 : 0;
 }
+
+// Mark of a particle left for the collider loop (no key: those are below the dead keys).
+constexpr uint32_t kLaterKey = BORA_DEAD_KEY - 2;
 
 // One CTA per tile: stage the tile's grid values, then advance the particles of the
 // tile's dual cells (a contiguous range of the sorted order). The CTA after the last tile
-// advances the sort's outside bin through the tile table. The common-case kernel (kAll =
-// false) needs 80 registers without spills and runs three CTAs per SM; the one with the
-// collider, water-tank and RK2 paths runs four at 64 registers.
-template <bool kAll>
-__global__ void __launch_bounds__( kG2PThreads, kAll ? 4 : 3 ) k_g2p( const __grid_constant__ BoraGridDev g, BoraTilesDev t, int ntiles,
+// advances the sort's outside bin through the tile table.
+//
+// Bound by the particles' gathers through L1 and by instructions: at 256^3 (24.6 M particles, 8.2
+// K tiles) 435 us in 500 instructions a particle at 80 registers (three CTAs per SM), 384
+// at 64 (four): lerps by packed pairs, surf's minimum once per base cell instead of per particle,
+// dt / iter from a table, the sort key of a particle that is known to be inside the grid. A 640
+// tank with a collider 1097 -> 817, its collider calls in a loop of their own, whose
+// spills the others do not pay for; an RK2 step at 96^3 134 -> 113 at 80 registers (119
+// at 64).
+template <int kMode>
+__global__ void __launch_bounds__( kG2PThreads, kMode == kEverything ? 3 : 4 ) k_g2p( const __grid_constant__ BoraGridDev g, BoraTilesDev t, int ntiles,
                                                        uint32_t nsorted, const uint32_t* __restrict__ start, BoraCellsDev c,
                                                        BoraParticlesDev src, const uint32_t* __restrict__ idx,
                                                        BoraParticlesDev dst, float* __restrict__ adj, float dt,
-                                                       uint32_t* __restrict__ nkilled, uint32_t* __restrict__ vkey,
+                                                       uint32_t* __restrict__ nkilled, uint32_t* vkey,
                                                        uint8_t* __restrict__ tile_flag )
 {
     __shared__ float4 fa[kStageCells];  // comp.x, comp.y, velo.x, velo.y
-    __shared__ float4 fb[kStageCells];  // comp.z, velo.z, surf, 0
+    __shared__ float2 fb[kStageCells];  // comp.z, velo.z
+    __shared__ float surf[kStageCells], surf_min[BORA_TILE_CELLS];
     __shared__ int32_t nb[27];
     __shared__ uint8_t near_flag[27];  // activation flags of the tiles around the CTA's own
+    __shared__ float sub[kSubTable];   // dt / iter; [0] is 1
     const int s = blockIdx.x, tid = threadIdx.x;
+    if( tid < kSubTable ) sub[tid] = tid ? dt / (float)tid : 1.f;
     uint32_t kills = 0;
     int cti = -8, ctj = -8, ctk = -8;  // the CTA's tile (far from every tile: no shared flags)
     auto finish = [&]( uint32_t q, uint32_t pi, int32_t id, float px, float py, float pz, float vx, float vy, float vz,
@@ -308,12 +351,13 @@ __global__ void __launch_bounds__( kG2PThreads, kAll ? 4 : 3 ) k_g2p( const __gr
         uint32_t key = BORA_DEAD_KEY;
         if( !kill && id >= 0 )
         {
+            // (a particle that lives is inside the grid)
             int ti, tj, tk;
-            bora_bin_tile( g.tx, g.ty, g.tz, px, py, pz, ti, tj, tk );
+            bora_bin_tile_inside( g.tx, g.ty, g.tz, px, py, pz, ti, tj, tk );
             const int dx = ti - cti, dy = tj - ctj, dz = tk - ctk;
             if( dx >= -1 && dx <= 1 && dy >= -1 && dy <= 1 && dz >= -1 && dz <= 1 ) near_flag[bora_dir( dx, dy, dz )] = 1;
             else tile_flag[( (size_t)tk * g.ty + tj ) * g.tx + ti] = 1;
-            key = bora_bin_live_key( g.nx, g.ny, g.nz, g.tx, g.ty, px, py, pz );
+            key = bora_bin_inside_key( g.tx, g.ty, px, py, pz );
         }
         vkey[q] = key;
         if( dst.vort )  // post-processing attributes ride along (FLIPMethod.cu:295-296)
@@ -325,6 +369,7 @@ __global__ void __launch_bounds__( kG2PThreads, kAll ? 4 : 3 ) k_g2p( const __gr
     };
     if( s == ntiles )
     {
+        __syncthreads();
         const uint32_t q0 = start[(size_t)ntiles * BORA_TILE_CELLS], q1 = nsorted;
         for( uint32_t q = q0 + tid; q < q1; q += kG2PThreads )
         {
@@ -334,8 +379,8 @@ __global__ void __launch_bounds__( kG2PThreads, kAll ? 4 : 3 ) k_g2p( const __gr
             GlobalLerp smp{ g, t.slot_of, c };
             smp.setup( px, py, pz );
             adj[q] = smp.surf_min();
-            const bool kill = advance_particle<kAll>( g, smp.comp(), smp.velo(), t.slot_of, c, px, py, pz, vx, vy, vz, dt );
-            finish( q, pi, src.id[pi], px, py, pz, vx, vy, vz, kill );
+            const int kill = advance_particle<kMode, true>( g, smp.comp(), smp.velo(), t.slot_of, c, px, py, pz, vx, vy, vz, dt, sub );
+            finish( q, pi, src.id[pi], px, py, pz, vx, vy, vz, kill != 0 );
         }
     }
     else
@@ -368,17 +413,25 @@ __global__ void __launch_bounds__( kG2PThreads, kAll ? 4 : 3 ) k_g2p( const __gr
         {
             const int a = h % kStageEdge, b = ( h / kStageEdge ) % kStageEdge, cz = h / ( kStageEdge * kStageEdge );
             const int ns = nb[bora_dir( a >> 3, b >> 3, cz >> 3 )];
-            float4 va = make_float4( 0.f, 0.f, 0.f, 0.f ), vb = make_float4( 0.f, 0.f, 10.f, 0.f );
+            float4 va = make_float4( 0.f, 0.f, 0.f, 0.f );
+            float2 vb = make_float2( 0.f, 0.f );
+            float vs = 10.f;
             if( ns >= 0 )
             {
                 const size_t q = (size_t)ns * BORA_TILE_CELLS + (size_t)bora_local( a, b, cz );
                 va = make_float4( c.cx[q], c.cy[q], c.vx[q], c.vy[q] );
-                vb = make_float4( c.cz[q], c.vz[q], c.surf[q], 0.f );
+                vb = make_float2( c.cz[q], c.vz[q] );
+                vs = c.surf[q];
             }
             fa[h] = va;
             fb[h] = vb;
+            surf[h] = vs;
         }
         __syncthreads();
+        for( int l = tid; l < BORA_TILE_CELLS; l += kG2PThreads )
+            surf_min[l] = StagedLerp::corner_min( surf, ( l & 7 ) + kStageEdge * ( ( ( l >> 3 ) & 7 ) + kStageEdge * ( l >> 6 ) ) );
+        __syncthreads();
+        uint32_t later = 0;  // particles of this thread that wait for the collider code
         for( uint32_t q = q0 + tid; q < q1; q += kG2PThreads )
         {
             const uint32_t pi = pin;
@@ -394,12 +447,33 @@ __global__ void __launch_bounds__( kG2PThreads, kAll ? 4 : 3 ) k_g2p( const __gr
             StagedLerp l;
             l.setup( g, ti, tj, tk, px, py, pz );
             float4 gn, go;
-            float smin;
-            l.sample( fa, fb, gn, go, smin );
-            adj[q] = smin;  // surf background 10 (FLIPMethod.cu:30)
-            const bool kill = advance_particle<kAll>( g, gn, go, t.slot_of, c, px, py, pz, vx, vy, vz, dt );
-            finish( q, pi, id, px, py, pz, vx, vy, vz, kill );
+            l.sample( fa, fb, sub[0], gn, go );
+            adj[q] = surf_min[l.cell];
+            const int kill = advance_particle<kMode, false>( g, gn, go, t.slot_of, c, px, py, pz, vx, vy, vz, dt, sub );
+            if( kMode != kCommon && kill == kLater )
+            {
+                vkey[q] = kLaterKey;
+                ++later;
+                continue;
+            }
+            finish( q, pi, id, px, py, pz, vx, vy, vz, kill != 0 );
         }
+        if constexpr( kMode != kCommon )
+#pragma unroll 1
+            for( uint32_t q = q0 + tid; later != 0 && q < q1; q += kG2PThreads )
+            {
+                if( vkey[q] != kLaterKey ) continue;
+                --later;
+                const uint32_t pi = idx[q];
+                float px = src.px[pi], py = src.py[pi], pz = src.pz[pi];
+                float vx = src.vx[pi], vy = src.vy[pi], vz = src.vz[pi];
+                StagedLerp l;
+                l.setup( g, ti, tj, tk, px, py, pz );
+                float4 gn, go;
+                l.sample( fa, fb, sub[0], gn, go );
+                const int kill = advance_particle<kMode, true>( g, gn, go, t.slot_of, c, px, py, pz, vx, vy, vz, dt, sub );
+                finish( q, pi, src.id[pi], px, py, pz, vx, vy, vz, kill != 0 );
+            }
         __syncthreads();
         if( tid < 27 && near_flag[tid] )  // a marked tile is a clamped particle tile: inside the table
         {
@@ -419,12 +493,13 @@ void bora_launch_g2p( const BoraGridDev& g, int ntiles, size_t nsorted, BoraTile
                       uint32_t* nkilled, uint32_t* vkey, uint8_t* tile_flag, cudaStream_t st )
 {
     if( nsorted == 0 ) return;
-    // the common case (no water tank, no colliders, Euler advection) in a kernel without the
-    // code of the others
-    if( g.enable_tank || bora_col_active( g.cols ) || g.advection == BORA_ADVECT_RK2 )
-        k_g2p<true><<<ntiles + 1, kG2PThreads, 0, st>>>( g, t, ntiles, (uint32_t)nsorted, start, c, src, idx, dst, adj, dt,
-                                                         nkilled, vkey, tile_flag );
-    else
-        k_g2p<false><<<ntiles + 1, kG2PThreads, 0, st>>>( g, t, ntiles, (uint32_t)nsorted, start, c, src, idx, dst, adj,
-                                                          dt, nkilled, vkey, tile_flag );
+    // the common case in a kernel without the code of the others, and the RK2 lookups (two more
+    // grid samples, inlined) only where they are asked for
+    auto go = [&]( auto kernel ) {
+        kernel<<<ntiles + 1, kG2PThreads, 0, st>>>( g, t, ntiles, (uint32_t)nsorted, start, c, src, idx, dst, adj, dt,
+                                                    nkilled, vkey, tile_flag );
+    };
+    if( g.advection == BORA_ADVECT_RK2 ) go( k_g2p<kEverything> );
+    else if( g.enable_tank || bora_col_active( g.cols ) ) go( k_g2p<kEuler> );
+    else go( k_g2p<kCommon> );
 }
