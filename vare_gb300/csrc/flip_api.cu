@@ -909,7 +909,7 @@ int stage_solve( bora_flip_sim* s )
 
 int stage_update_velocity( bora_flip_sim* s )
 {
-    KTimer t( s, BORA_KERNEL_VELOCITY, s->ntiles > 0 );
+    KTimer t( s, BORA_KERNEL_VELOCITY, s->ntiles > 0 ? 2 : 0 );
     bora_launch_vel_update( s->g, s->ntiles, s->tiles(), s->cells(), s->st );
     const int st = check_launch( s );
     s->pres_valid = st == BORA_OK;  // the solve's pressure (and the air cells' means) over the current tiles

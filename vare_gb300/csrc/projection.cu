@@ -17,31 +17,6 @@
 
 namespace {
 
-// ---------------------------------------------------------------------------------
-// Shared-memory halo of a tile: region of (8+2H)^3 cells around tile s.
-// Cells outside the grid or in inactive tiles read as "background" (air, zero).
-template <int H>
-struct Halo
-{
-    static constexpr int E = BORA_TILE + 2 * H;
-    static constexpr int N = E * E * E;
-    __device__ static inline int at( int a, int b, int c ) { return a + E * ( b + E * c ); }  // a,b,c in [0,E)
-};
-
-// Resolve halo-region cell h (0..N-1) of tile (ti,tj,tk): returns the global field
-// index or -1 (outside the grid or inactive tile).
-template <int H>
-__device__ inline long long halo_index( const BoraGridDev& g, const int32_t* nb, int ti, int tj, int tk, int h )
-{
-    constexpr int E = Halo<H>::E;
-    const int a = h % E, b = ( h / E ) % E, c = h / ( E * E );
-    const int i = ti * BORA_TILE - H + a, j = tj * BORA_TILE - H + b, k = tk * BORA_TILE - H + c;
-    if( i < 0 || j < 0 || k < 0 || i >= g.nx || j >= g.ny || k >= g.nz ) return -1;
-    const int s = nb[bora_dir( ( i >> 3 ) - ti, ( j >> 3 ) - tj, ( k >> 3 ) - tk )];
-    if( s < 0 ) return -1;
-    return (long long)s * BORA_TILE_CELLS + bora_local( i, j, k );
-}
-
 __device__ inline void tile_coords( const BoraGridDev& g, int vt, int& ti, int& tj, int& tk )
 {
     ti = vt % g.tx;
@@ -52,78 +27,177 @@ __device__ inline void tile_coords( const BoraGridDev& g, int vt, int& ti, int& 
 __device__ inline float absr( float x ) { return x < 0.f ? -x : x; }  // MathUtils.h:129 Abs
 
 // ---------------------------------------------------------------------------------
-// Right-hand side and stencil code (FluidProjection.cu:203-266).
-__global__ void __launch_bounds__( 512 ) k_rhs( BoraGridDev g, BoraTilesDev t, BoraCellsDev c, uint32_t* nfluid,
-                                                 uint8_t* __restrict__ tile_fluid )
+// Stencils over the active tiles outside the solve: one warp per half tile (z layers 0..3 or
+// 4..7), a lane per x-row (lane = j + 8 (k mod 4)), as the solve's kernels walk theirs. Cells of
+// inactive tiles and beyond the grid read as air and zero.
+constexpr int kRowWarps = 4;  // half tiles per CTA
+
+struct HalfRow
 {
-    using HL = Halo<1>;
-    __shared__ int32_t nb[27];
-    __shared__ uint8_t sf[HL::N];
-    __shared__ float sx[HL::N], sy[HL::N], sz[HL::N];
-    const int s = blockIdx.x;
-    if( threadIdx.x < 27 ) nb[threadIdx.x] = t.nbr[(size_t)s * 27 + threadIdx.x];
+    bool mine;              // past the last half tile: nothing is stored, every neighbour is inactive
+    int s, hi;              // the tile's slot; the half
+    int xm, xp, yt, zt;     // slots at the row's x ends; of the rows that no other lane holds (-1: none)
+    int c, yc, zc;          // cells of the row, and of those rows, in their tiles
+    int j, kk;              // the lane's row in the half
+    int i0, J, K;           // the row's first cell in the grid
+    __device__ size_t at() const { return (size_t)s * BORA_TILE_CELLS + c; }
+};
+
+__device__ __forceinline__ HalfRow half_row( const BoraGridDev& g, const BoraTilesDev& t, int ntiles )
+{
+    HalfRow r;
+    const int lane = threadIdx.x & 31, h = (int)blockIdx.x * kRowWarps + (int)( threadIdx.x >> 5 );
+    r.mine = h < 2 * ntiles;
+    r.s = r.mine ? h >> 1 : 0;
+    r.hi = h & 1;
+    r.j = lane & 7;
+    r.kk = lane >> 3;
+    r.c = r.hi * 256 + 8 * lane;
+    const int32_t* nb = t.nbr + (size_t)r.s * 27;
+    auto slot = [&]( int d ) { return r.mine ? __ldg( nb + d ) : -1; };
+    r.xm = slot( bora_dir( -1, 0, 0 ) );
+    r.xp = slot( bora_dir( 1, 0, 0 ) );
+    const int ym = slot( bora_dir( 0, -1, 0 ) ), yp = slot( bora_dir( 0, 1, 0 ) ), z = slot( bora_dir( 0, 0, r.hi ? 1 : -1 ) );
+    const int own = r.mine ? r.s : -1;
+    r.yt = r.j == 0 ? ym : ( r.j == 7 ? yp : -1 );
+    r.yc = r.c + ( r.j == 0 ? 56 : -56 );
+    r.zt = r.kk == 0 ? ( r.hi ? own : z ) : ( r.kk == 3 ? ( r.hi ? z : own ) : -1 );
+    r.zc = 8 * r.j + ( r.kk == 0 ? ( r.hi ? 192 : 448 ) : ( r.hi ? 0 : 256 ) );
     int ti, tj, tk;
-    tile_coords( g, t.tile_of[s], ti, tj, tk );
-    __syncthreads();
-#pragma unroll 2
-    for( int h = threadIdx.x; h < HL::N; h += blockDim.x )
-    {
-        const long long gi = halo_index<1>( g, nb, ti, tj, tk, h );
-        if( gi < 0 ) { sf[h] = BORA_AIR; sx[h] = sy[h] = sz[h] = 0.f; }
-        else { sf[h] = c.flag[gi]; sx[h] = c.vx[gi]; sy[h] = c.vy[gi]; sz[h] = c.vz[gi]; }
-    }
-    __syncthreads();
-    const int l = threadIdx.x;
-    const int li = l & 7, lj = ( l >> 3 ) & 7, lk = l >> 6;
-    const int i = ti * 8 + li, j = tj * 8 + lj, k = tk * 8 + lk;
-    const size_t cell = (size_t)s * BORA_TILE_CELLS + l;
-    const int h = HL::at( li + 1, lj + 1, lk + 1 );
-    const bool fluid = sf[h] == BORA_FLUID;
-    const unsigned fl = __ballot_sync( 0xffffffffu, fluid );  // unknowns of the system, counted per warp
-    if( ( threadIdx.x & 31 ) == 0 && fl ) atomicAdd( nfluid, (uint32_t)__popc( fl ) );
-    const int any = __syncthreads_or( fluid );
-    if( threadIdx.x == 0 ) tile_fluid[s] = any ? 1 : 0;
-    if( !fluid )
-    {
-        c.b[cell] = 0.f;
-        c.code[cell] = 0;
-        return;
-    }
-    const int EI = g.nx - 1, EJ = g.ny - 1, EK = g.nz - 1;
-    const int wall = (float)j + 0.5f <= g.voxel_wall + 1.f ? BORA_WALL : BORA_AIR;
-    const int hi0 = h - 1, hi1 = h + 1, hj0 = h - HL::E, hj1 = h + HL::E, hk0 = h - HL::E * HL::E, hk1 = h + HL::E * HL::E;
-    const int t_i0 = i == 0 ? wall : sf[hi0];
-    const int t_i1 = i == EI ? wall : sf[hi1];
-    const int t_j0 = j == 0 ? wall : sf[hj0];
-    const int t_j1 = j == EJ ? wall : sf[hj1];
-    const int t_k0 = k == 0 ? wall : sf[hk0];
-    const int t_k1 = k == EK ? wall : sf[hk1];
-    const float vx = sx[h], vy = sy[h], vz = sz[h];
-    const float i0_j_k = i == 0 ? 2.f * vx - sx[hi1] : sx[hi0];
-    const float i1_j_k = i == EI ? 2.f * vx - sx[hi0] : sx[hi1];
-    const float i_j0_k = j == 0 ? 2.f * vy - sy[hj1] : sy[hj0];
-    const float i_j1_k = j == EJ ? 2.f * vy - sy[hj0] : sy[hj1];
-    const float i_j_k0 = k == 0 ? 2.f * vz - sz[hk1] : sz[hk0];
-    const float i_j_k1 = k == EK ? 2.f * vz - sz[hk0] : sz[hk1];
-    const float v_i0 = t_i0 == BORA_AIR ? 2.f * vx - i1_j_k : t_i0 == BORA_WALL ? absr( vx ) : i0_j_k;
-    const float v_i1 = t_i1 == BORA_AIR ? 2.f * vx - i0_j_k : t_i1 == BORA_WALL ? -absr( vx ) : i1_j_k;
-    const float v_j0 = t_j0 == BORA_AIR ? 2.f * vy - i_j1_k : t_j0 == BORA_WALL ? absr( vy ) : i_j0_k;
-    const float v_j1 = t_j1 == BORA_AIR ? 2.f * vy - i_j0_k : t_j1 == BORA_WALL ? -absr( vy ) : i_j1_k;
-    const float v_k0 = t_k0 == BORA_AIR ? 2.f * vz - i_j_k1 : t_k0 == BORA_WALL ? absr( vz ) : i_j_k0;
-    const float v_k1 = t_k1 == BORA_AIR ? 2.f * vz - i_j_k0 : t_k1 == BORA_WALL ? -absr( vz ) : i_j_k1;
-    const float d = -( ( v_i1 - v_i0 ) * 0.5f + ( v_j1 - v_j0 ) * 0.5f + ( v_k1 - v_k0 ) * 0.5f );
-    int diag = 6;
-    uint32_t mask = 0;
-    const int tt[6] = { t_i0, t_i1, t_j0, t_j1, t_k0, t_k1 };
+    tile_coords( g, t.tile_of[r.s], ti, tj, tk );
+    r.i0 = ti * BORA_TILE;
+    r.J = tj * BORA_TILE + r.j;
+    r.K = tk * BORA_TILE + 4 * r.hi + r.kk;
+    return r;
+}
+
+__device__ __forceinline__ uint2 flags8( const uint8_t* __restrict__ flag, int t, int c )
+{
+    return t < 0 ? make_uint2( 0u, 0u ) : *reinterpret_cast<const uint2*>( flag + (size_t)t * BORA_TILE_CELLS + c );  // BORA_AIR is 0
+}
+__device__ __forceinline__ int flag_of( uint2 w, int i ) { return (int)( ( ( i < 4 ? w.x : w.y ) >> ( 8 * ( i & 3 ) ) ) & 255u ); }
+
+__device__ __forceinline__ void row8( const float* __restrict__ f, int t, int c, float* v )
+{
 #pragma unroll
-    for( int q = 0; q < 6; ++q )
+    for( int i = 0; i < 8; ++i ) v[i] = 0.f;
+    if( t >= 0 ) bora_ld8( f + (size_t)t * BORA_TILE_CELLS + c, v );
+}
+
+__device__ __forceinline__ uint2 shfl2( uint2 w, int lane )
+{
+    return make_uint2( __shfl_sync( 0xffffffffu, w.x, lane ), __shfl_sync( 0xffffffffu, w.y, lane ) );
+}
+
+// A row's flags and those of the rows around it in y and z, and at its x ends.
+struct RowFlags
+{
+    uint2 w, ym, yp, zm, zp;
+    int xm, xp;
+    __device__ __forceinline__ void load( const uint8_t* __restrict__ flag, const HalfRow& r )
     {
-        if( tt[q] == BORA_AIR ) diag += 1;
-        else if( tt[q] == BORA_SOLID || tt[q] == BORA_WALL ) diag -= 1;
-        else if( tt[q] == BORA_FLUID ) mask |= 1u << q;
+        const int lane = threadIdx.x & 31;
+        w = flags8( flag, r.mine ? r.s : -1, r.c );
+        const uint2 y = flags8( flag, r.yt, r.yc ), z = flags8( flag, r.zt, r.zc );
+        xm = r.xm < 0 ? BORA_AIR : flag[(size_t)r.xm * BORA_TILE_CELLS + r.c + 7];
+        xp = r.xp < 0 ? BORA_AIR : flag[(size_t)r.xp * BORA_TILE_CELLS + r.c];
+        ym = shfl2( w, lane - 1 ); yp = shfl2( w, lane + 1 );
+        zm = shfl2( w, lane - 8 ); zp = shfl2( w, lane + 8 );
+        if( r.j == 0 ) ym = y;
+        if( r.j == 7 ) yp = y;
+        if( r.kk == 0 ) zm = z;
+        if( r.kk == 3 ) zp = z;
     }
-    c.b[cell] = d;
-    c.code[cell] = (uint16_t)( BORA_CODE_FLUID | ( (uint32_t)diag << 8 ) | mask );
+};
+
+// the values of a field next to a row in y or z: from the other lanes, or the loaded row
+__device__ __forceinline__ void beside( const float* v, const float* halo, int step, bool first, bool last, float* m, float* p )
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for( int i = 0; i < 8; ++i )
+    {
+        const float a = __shfl_sync( 0xffffffffu, v[i], lane - step ), b = __shfl_sync( 0xffffffffu, v[i], lane + step );
+        m[i] = first ? halo[i] : a;
+        p[i] = last ? halo[i] : b;
+    }
+}
+
+// ---------------------------------------------------------------------------------
+// Right-hand side and stencil code (FluidProjection.cu:203-266). (With a cell per thread from a
+// staged 10^3 region it was bound by index arithmetic: 84 us at 256^3, 35 now.)
+__global__ void __launch_bounds__( 32 * kRowWarps ) k_rhs( BoraGridDev g, BoraTilesDev t, int ntiles, BoraCellsDev c,
+                                                           uint32_t* nfluid, uint8_t* __restrict__ tile_fluid )
+{
+    __shared__ int any[kRowWarps];
+    const HalfRow r = half_row( g, t, ntiles );
+    RowFlags f;
+    f.load( c.flag, r );
+    const int own = r.mine ? r.s : -1;
+    float vx[8], vy[8], vz[8], vym[8], vyp[8], vzm[8], vzp[8], yh[8], zh[8];
+    row8( c.vx, own, r.c, vx );
+    row8( c.vy, own, r.c, vy );
+    row8( c.vz, own, r.c, vz );
+    row8( c.vy, r.yt, r.yc, yh );
+    row8( c.vz, r.zt, r.zc, zh );
+    const float vxm = r.xm < 0 ? 0.f : c.vx[(size_t)r.xm * BORA_TILE_CELLS + r.c + 7];
+    const float vxp = r.xp < 0 ? 0.f : c.vx[(size_t)r.xp * BORA_TILE_CELLS + r.c];
+    beside( vy, yh, 1, r.j == 0, r.j == 7, vym, vyp );
+    beside( vz, zh, 8, r.kk == 0, r.kk == 3, vzm, vzp );
+    const int EI = g.nx - 1, EJ = g.ny - 1, EK = g.nz - 1;
+    const int wall = (float)r.J + 0.5f <= g.voxel_wall + 1.f ? BORA_WALL : BORA_AIR;
+    float b[8];
+    uint32_t cw[8];
+    int count = 0;
+#pragma unroll
+    for( int q = 0; q < 8; ++q )
+    {
+        const bool e_i0 = r.i0 + q == 0, e_i1 = r.i0 + q == EI, e_j0 = r.J == 0, e_j1 = r.J == EJ, e_k0 = r.K == 0, e_k1 = r.K == EK;
+        const int tt[6] = { e_i0 ? wall : ( q ? flag_of( f.w, q ? q - 1 : 0 ) : f.xm ), e_i1 ? wall : ( q < 7 ? flag_of( f.w, q < 7 ? q + 1 : 7 ) : f.xp ),
+                            e_j0 ? wall : flag_of( f.ym, q ), e_j1 ? wall : flag_of( f.yp, q ),
+                            e_k0 ? wall : flag_of( f.zm, q ), e_k1 ? wall : flag_of( f.zp, q ) };
+        // one axis: the two neighbour values, mirrored at the grid's faces, under the ghost rules
+        auto diff = [&]( float v, float lo, float hi, bool e0, bool e1, int t0, int t1 ) {
+            const float n0 = e0 ? 2.f * v - hi : lo, n1 = e1 ? 2.f * v - lo : hi;
+            const float a = t0 == BORA_AIR ? 2.f * v - n1 : t0 == BORA_WALL ? absr( v ) : n0;
+            const float z = t1 == BORA_AIR ? 2.f * v - n0 : t1 == BORA_WALL ? -absr( v ) : n1;
+            return ( z - a ) * 0.5f;
+        };
+        const float dx = diff( vx[q], q ? vx[q ? q - 1 : 0] : vxm, q < 7 ? vx[q < 7 ? q + 1 : 7] : vxp, e_i0, e_i1, tt[0], tt[1] );
+        const float dy = diff( vy[q], vym[q], vyp[q], e_j0, e_j1, tt[2], tt[3] );
+        const float dz = diff( vz[q], vzm[q], vzp[q], e_k0, e_k1, tt[4], tt[5] );
+        const bool fluid = flag_of( f.w, q ) == BORA_FLUID;
+        int diag = 6;
+        uint32_t mask = 0;
+#pragma unroll
+        for( int n = 0; n < 6; ++n )
+        {
+            if( tt[n] == BORA_AIR ) diag += 1;
+            else if( tt[n] == BORA_SOLID || tt[n] == BORA_WALL ) diag -= 1;
+            else if( tt[n] == BORA_FLUID ) mask |= 1u << n;
+        }
+        b[q] = fluid ? -( dx + dy + dz ) : 0.f;
+        cw[q] = fluid ? BORA_CODE_FLUID | ( (uint32_t)diag << 8 ) | mask : 0u;
+        count += fluid ? 1 : 0;
+    }
+    if( r.mine )
+    {
+        bora_st8( c.b + r.at(), b );
+        *reinterpret_cast<uint4*>( c.code + r.at() ) =
+            make_uint4( cw[0] | ( cw[1] << 16 ), cw[2] | ( cw[3] << 16 ), cw[4] | ( cw[5] << 16 ), cw[6] | ( cw[7] << 16 ) );
+    }
+    count = __reduce_add_sync( 0xffffffffu, count );  // unknowns of the system
+    if( ( threadIdx.x & 31 ) == 0 )
+    {
+        any[threadIdx.x >> 5] = count;
+        if( count ) atomicAdd( nfluid, (uint32_t)count );
+    }
+    __syncthreads();
+    if( threadIdx.x < kRowWarps / 2 )
+    {
+        const int tile = (int)blockIdx.x * ( kRowWarps / 2 ) + (int)threadIdx.x;
+        if( tile < ntiles ) tile_fluid[tile] = any[2 * threadIdx.x] || any[2 * threadIdx.x + 1] ? 1 : 0;
+    }
 }
 
 // ---------------------------------------------------------------------------------
@@ -521,27 +595,6 @@ __global__ void __launch_bounds__( 32 * kUpdWarps, 4 ) k_pcg_update( BoraSolveTi
     };
     if( ft.n > 0 ) pcg_update_tiles( ft, sv, alpha_of, blockIdx.x, gridDim.x, prz, prr );
     part_publish( prz, prr, red.part_rz, red.part_rr, blockIdx.x );
-}
-
-// Global index of the face neighbour of cell `cell` (solver tile t, local l) in direction q
-// (0:-x 1:+x 2:-y 3:+y 4:-z 5:+z), or SIZE_MAX when the neighbour tile is not a solver tile
-// (a stencil code that names a fluid neighbour there is inconsistent; callers record
-// it and skip the access).
-__device__ inline size_t face_nbr( const int4* __restrict__ tab, size_t cell, int t, int l, int q )
-{
-    const int li = l & 7, lj = ( l >> 3 ) & 7, lk = l >> 6;
-    int ll;
-    switch( q )
-    {
-        case 0: if( li > 0 ) return cell - 1; ll = l + 7; break;
-        case 1: if( li < 7 ) return cell + 1; ll = l - 7; break;
-        case 2: if( lj > 0 ) return cell - 8; ll = l + 56; break;
-        case 3: if( lj < 7 ) return cell + 8; ll = l - 56; break;
-        case 4: if( lk > 0 ) return cell - 64; ll = l + 448; break;
-        default: if( lk < 7 ) return cell + 64; ll = l - 448; break;
-    }
-    const int ns = __ldg( reinterpret_cast<const int*>( tab + 2 * (size_t)t ) + q );
-    return ns < 0 ? (size_t)-1 : (size_t)ns * 512 + ll;
 }
 
 // ---------------------------------------------------------------------------------
@@ -1295,53 +1348,111 @@ __global__ void k_refine_accumulate_batch( const __grid_constant__ BoraBatchLaun
                             q.a_dq, bid, (unsigned)m.grid[kGridCells] );
 }
 
-// r = b - A x in double-float arithmetic (A from the stencil code, x the double-float
-// iterate); r stored in FP32, ||r||^2 and max|r| reduced. Streaming, one thread per cell.
-// GB300's FP64 pipe is narrow: in FP64 this kernel and the accumulation were bound by it.
+// r = b - A x in double-float arithmetic (A from the stencil code, x the double-float iterate); r
+// stored in FP32, ||r||^2 and max|r| reduced. One warp per half tile and a lane per x-row, as the
+// direction kernel. GB300's FP64 pipe is narrow: in FP64 this kernel and the accumulation were
+// bound by it. (A cell per thread with its neighbours' indices formed one by one: 54 us at 256^3,
+// 35 now.)
+constexpr int kResWarps = 8;
+
 __device__ __forceinline__ void refine_residual_body( const BoraSolveTilesDev& ft, const float* __restrict__ b,
                                                       const uint16_t* __restrict__ code, const BoraSolverDev& sv, const BoraReduceDev& red, int slot_norm2,
                                                       int slot_max, unsigned bid, unsigned G )
 {
     DF n2{ 0.f, 0.f };
     float mx = 0.f;
-    const size_t n = (size_t)ft.n * 512;
-    for( size_t i = bid * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)G * blockDim.x )
-    {
-        const int t = (int)( i >> 9 ), l = (int)( i & 511 );
-        const size_t cell = (size_t)solve_slot( ft.tab, t ) * 512 + l;
-        const uint16_t cc = code[cell];
-        if( !( cc & BORA_CODE_FLUID ) ) { sv.r[cell] = 0.f; continue; }
-        DF acc{ 0.f, 0.f };
+    const int lane = threadIdx.x & 31, j = lane & 7, kk = lane >> 3;
+    const int nh = 2 * ft.n, stride = (int)G * kResWarps;
+    constexpr unsigned kAll = 0xffffffffu;
+    const float* __restrict__ x = reinterpret_cast<const float*>( sv.x );
+    auto load = [&]( int t, int c, float* v ) {  // 8 double-float values
 #pragma unroll
-        for( int q = 0; q < 6; ++q )
+        for( int i = 0; i < 16; ++i ) v[i] = 0.f;
+        if( t < 0 ) return;
+        bora_ld8( x + 2 * ( (size_t)t * 512 + c ), v );
+        bora_ld8( x + 2 * ( (size_t)t * 512 + c ) + 8, v + 8 );
+    };
+    // (a bound of the block's; a warp past the last half tile has no neighbours and stores nothing)
+#pragma unroll 1
+    for( int base = (int)bid * kResWarps; base < nh; base += stride )
+    {
+        const int h = base + (int)( threadIdx.x >> 5 );
+        const bool mine = h < nh;
+        const int t = mine ? h >> 1 : 0, hi = h & 1;
+        int4 n0 = __ldg( ft.tab + 2 * (size_t)t ), n1 = __ldg( ft.tab + 2 * (size_t)t + 1 );
+        const int s = n1.z;
+        if( !mine ) n0 = n1 = make_int4( -1, -1, -1, -1 );
+        const int cA = hi * 256 + 8 * lane;
+        const size_t g = (size_t)s * 512 + cA;
+        const int yt = j == 0 ? n0.z : ( j == 7 ? n0.w : -1 ), yc = cA + ( j == 0 ? 56 : -56 );
+        const int sz = hi ? n1.y : n1.x, own = mine ? s : -1;
+        const int zt = kk == 0 ? ( hi ? own : sz ) : ( kk == 3 ? ( hi ? sz : own ) : -1 );
+        const int zc = 8 * j + ( kk == 0 ? ( hi ? 192 : 448 ) : ( hi ? 0 : 256 ) );
+        uint4 cw = make_uint4( 0u, 0u, 0u, 0u );
+        if( mine ) cw = *reinterpret_cast<const uint4*>( code + g );
+        float v[16], yh[16], zh[16], bv[8] = {};
+        load( own, cA, v );
+        load( yt, yc, yh );
+        load( zt, zc, zh );
+        const float2 zero = make_float2( 0.f, 0.f );
+        const float2 xm = n0.x < 0 ? zero : sv.x[(size_t)n0.x * 512 + cA + 7], xp = n0.y < 0 ? zero : sv.x[(size_t)n0.y * 512 + cA];
+        if( mine ) bora_ld8( b + g, bv );
+        const uint32_t w[4] = { cw.x, cw.y, cw.z, cw.w };
+        float r[8];
+        uint32_t seen = 0;
+#pragma unroll
+        for( int i = 0; i < 8; ++i )
         {
-            if( !( cc & ( 1u << q ) ) ) continue;
-            const size_t nc = face_nbr( ft.tab, cell, t, l, q );
-            if( nc == (size_t)-1 ) { atomicOr( red.err, 2u ); continue; }
-            const float2 xn = sv.x[nc];
-            acc = df_add( acc, DF{ xn.x, xn.y } );
+            const uint32_t c = i & 1 ? w[i >> 1] >> 16 : w[i >> 1] & 0xffffu;
+            const float vh = v[2 * i], vl = v[2 * i + 1];
+            float ymh = __shfl_up_sync( kAll, vh, 1 ), yml = __shfl_up_sync( kAll, vl, 1 );
+            float yph = __shfl_down_sync( kAll, vh, 1 ), ypl = __shfl_down_sync( kAll, vl, 1 );
+            float zmh = __shfl_up_sync( kAll, vh, 8 ), zml = __shfl_up_sync( kAll, vl, 8 );
+            float zph = __shfl_down_sync( kAll, vh, 8 ), zpl = __shfl_down_sync( kAll, vl, 8 );
+            if( j == 0 ) { ymh = yh[2 * i]; yml = yh[2 * i + 1]; }
+            if( j == 7 ) { yph = yh[2 * i]; ypl = yh[2 * i + 1]; }
+            if( kk == 0 ) { zmh = zh[2 * i]; zml = zh[2 * i + 1]; }
+            if( kk == 3 ) { zph = zh[2 * i]; zpl = zh[2 * i + 1]; }
+            // a neighbour that the code does not name counts as 0, which changes no sum
+            DF acc{ 0.f, 0.f };
+            auto add = [&]( int q, float nh_, float nl_ ) {
+                const bool on = ( c >> q ) & 1u;
+                acc = df_add( acc, DF{ on ? nh_ : 0.f, on ? nl_ : 0.f } );
+            };
+            add( 0, i ? v[i ? 2 * i - 2 : 0] : xm.x, i ? v[i ? 2 * i - 1 : 0] : xm.y );
+            add( 1, i < 7 ? v[i < 7 ? 2 * i + 2 : 0] : xp.x, i < 7 ? v[i < 7 ? 2 * i + 3 : 0] : xp.y );
+            add( 2, ymh, yml );
+            add( 3, yph, ypl );
+            add( 4, zmh, zml );
+            add( 5, zph, zpl );
+            const float dg = (float)code_diag( (uint16_t)c );
+            const DF ax = df_add_f( df_prod( vh, dg ), vl * dg );  // diag * x (diag <= 12)
+            const DF y = df_add( ax, DF{ -acc.hi, -acc.lo } );
+            const DF rv = df_add_f( DF{ -y.hi, -y.lo }, bv[i] );
+            const bool fluid = c & BORA_CODE_FLUID;
+            r[i] = fluid ? rv.hi + rv.lo : 0.f;
+            n2 = df_add( n2, df_prod( r[i], r[i] ) );
+            mx = fmaxf( mx, fabsf( r[i] ) );
+            if( fluid ) seen |= c & ( 0x3cu | ( i == 0 ? 1u : 0u ) | ( i == 7 ? 2u : 0u ) );
         }
-        const float2 xc = sv.x[cell];
-        const float dg = (float)code_diag( cc );
-        const DF ax = df_add_f( df_prod( xc.x, dg ), xc.y * dg );  // diag * x (diag <= 12)
-        const DF y = df_add( ax, DF{ -acc.hi, -acc.lo } );
-        const DF rv = df_add_f( DF{ -y.hi, -y.lo }, b[cell] );
-        const float rf = rv.hi + rv.lo;
-        sv.r[cell] = rf;
-        n2 = df_add( n2, df_prod( rf, rf ) );
-        mx = fmaxf( mx, fabsf( rf ) );
+        if( !mine ) continue;
+        bora_st8( sv.r + g, r );
+        // a code that names a fluid neighbour in a tile that is not the solver's is inconsistent
+        if( ( ( seen & 1u ) && n0.x < 0 ) || ( ( seen & 2u ) && n0.y < 0 ) || ( ( seen & 4u ) && j == 0 && yt < 0 ) ||
+            ( ( seen & 8u ) && j == 7 && yt < 0 ) || ( ( seen & 16u ) && kk == 0 && zt < 0 ) || ( ( seen & 32u ) && kk == 3 && zt < 0 ) )
+            atomicOr( red.err, 2u );
     }
     reduce2_publish_dfmax( n2, mx, red, slot_norm2, slot_max, bid, G );
 }
 
-__global__ void __launch_bounds__( 256 ) k_refine_residual( BoraSolveTilesDev ft, const float* __restrict__ b,
+__global__ void __launch_bounds__( 32 * kResWarps, 3 ) k_refine_residual( BoraSolveTilesDev ft, const float* __restrict__ b,
                                                             const uint16_t* __restrict__ code, BoraSolverDev sv,
                                                             BoraReduceDev red, int slot_norm2, int slot_max )
 {
     refine_residual_body( ft, b, code, sv, red, slot_norm2, slot_max, blockIdx.x, gridDim.x );
 }
 
-__global__ void __launch_bounds__( 256 ) k_refine_residual_batch( const __grid_constant__ BoraBatchLaunch L )
+__global__ void __launch_bounds__( 32 * kResWarps, 3 ) k_refine_residual_batch( const __grid_constant__ BoraBatchLaunch L )
 {
     unsigned bid;
     const int k = bora_batch_member( L, blockIdx.x, &bid );
@@ -1369,103 +1480,148 @@ __global__ void k_write_pressure_batch( const __grid_constant__ BoraBatchLaunch 
 }
 
 // ---------------------------------------------------------------------------------
-// Velocity update (FluidProjection.cu:293-378): air cells next to fluid take the mean
-// of their fluid neighbours' pressure, then fluid cells subtract the central-difference
-// pressure gradient with the reference's ghost rules; other cells keep the P2G velocity.
-__global__ void __launch_bounds__( 512 ) k_vel_update( BoraGridDev g, BoraTilesDev t, BoraCellsDev c )
+// Velocity update (FluidProjection.cu:293-378), in two passes over the half tiles: air cells next
+// to fluid take the mean of their fluid neighbours' pressure, in place (the pass reads fluid
+// cells' pressures only, and those it leaves alone); then fluid cells subtract the
+// central-difference pressure gradient with the reference's ghost rules, other cells keep the
+// P2G velocity. (One pass from a 12^3 staged region was bound by index arithmetic: 98 us at
+// 256^3, 48 now.)
+
+// sum of the fluid neighbours' pressures in the order -x +x -y +y -z +z over their number
+struct AirMean
 {
-    using H2 = Halo<2>;
-    using H1 = Halo<1>;
-    __shared__ int32_t nb[27];
-    __shared__ uint8_t sf[H2::N];
-    __shared__ float sp[H2::N];
-    __shared__ float pa[H1::N];
-    __shared__ uint8_t fa[H1::N];
-    const int s = blockIdx.x;
-    if( threadIdx.x < 27 ) nb[threadIdx.x] = t.nbr[(size_t)s * 27 + threadIdx.x];
-    int ti, tj, tk;
-    tile_coords( g, t.tile_of[s], ti, tj, tk );
-    __syncthreads();
-    // the pressure is read with the flag, not after it (every active cell holds a pressure,
-    // 0 off the fluid), so that a cell's two loads are in flight together
-#pragma unroll 4
-    for( int h = threadIdx.x; h < H2::N; h += blockDim.x )
+    float press = 0.f;
+    int count = 0;
+    __device__ __forceinline__ void add( bool in_grid, int flag, float p )
     {
-        const long long gi = halo_index<2>( g, nb, ti, tj, tk, h );
-        if( gi < 0 ) { sf[h] = BORA_AIR; sp[h] = 0.f; }
-        else
-        {
-            const uint8_t f = c.flag[gi];
-            const float pr = c.pres[gi];
-            sf[h] = f;
-            sp[h] = f == BORA_FLUID ? pr : 0.f;
-        }
+        if( in_grid && flag == BORA_FLUID ) { press += p; count++; }
     }
-    __syncthreads();
+    __device__ __forceinline__ float value() const { return count > 0 ? press / (float)count : 0.f; }
+};
+
+__global__ void __launch_bounds__( 32 * kRowWarps ) k_air_pressure( BoraGridDev g, BoraTilesDev t, int ntiles, BoraCellsDev c )
+{
+    const HalfRow r = half_row( g, t, ntiles );
+    RowFlags f;
+    f.load( c.flag, r );
+    constexpr uint32_t kAllFluid = 0x01010101u * BORA_FLUID;
+    if( __all_sync( 0xffffffffu, !r.mine || ( f.w.x == kAllFluid && f.w.y == kAllFluid ) ) ) return;
+    const int own = r.mine ? r.s : -1;
+    float p[8], pym[8], pyp[8], pzm[8], pzp[8], h[8];
+    row8( c.pres, own, r.c, p );
+    row8( c.pres, r.yt, r.yc, h );
+    beside( p, h, 1, r.j == 0, r.j == 7, pym, pyp );
+    row8( c.pres, r.zt, r.zc, h );
+    beside( p, h, 8, r.kk == 0, r.kk == 3, pzm, pzp );
+    const float pxm = r.xm < 0 ? 0.f : c.pres[(size_t)r.xm * BORA_TILE_CELLS + r.c + 7];
+    const float pxp = r.xp < 0 ? 0.f : c.pres[(size_t)r.xp * BORA_TILE_CELLS + r.c];
     const int EI = g.nx - 1, EJ = g.ny - 1, EK = g.nz - 1;
-    for( int h = threadIdx.x; h < H1::N; h += blockDim.x )
+    float out[8];
+#pragma unroll
+    for( int q = 0; q < 8; ++q )
     {
-        const int a = h % H1::E, b = ( h / H1::E ) % H1::E, cc = h / ( H1::E * H1::E );
-        const int i = ti * 8 - 1 + a, j = tj * 8 - 1 + b, k = tk * 8 - 1 + cc;
-        const int h2 = H2::at( a + 1, b + 1, cc + 1 );
-        const uint8_t f = sf[h2];
-        float p = sp[h2];
-        if( f == BORA_AIR && i >= 0 && j >= 0 && k >= 0 && i <= EI && j <= EJ && k <= EK )
-        {
-            float press = 0.f;
-            int count = 0;
-            if( i > 0 && sf[h2 - 1] == BORA_FLUID ) { press += sp[h2 - 1]; count++; }
-            if( i < EI && sf[h2 + 1] == BORA_FLUID ) { press += sp[h2 + 1]; count++; }
-            if( j > 0 && sf[h2 - H2::E] == BORA_FLUID ) { press += sp[h2 - H2::E]; count++; }
-            if( j < EJ && sf[h2 + H2::E] == BORA_FLUID ) { press += sp[h2 + H2::E]; count++; }
-            if( k > 0 && sf[h2 - H2::E * H2::E] == BORA_FLUID ) { press += sp[h2 - H2::E * H2::E]; count++; }
-            if( k < EK && sf[h2 + H2::E * H2::E] == BORA_FLUID ) { press += sp[h2 + H2::E * H2::E]; count++; }
-            if( count > 0 ) p = press / (float)count;
-        }
-        pa[h] = p;
-        fa[h] = f;
+        const int I = r.i0 + q, own_flag = flag_of( f.w, q );
+        AirMean m;
+        m.add( I > 0, q ? flag_of( f.w, q ? q - 1 : 0 ) : f.xm, q ? p[q ? q - 1 : 0] : pxm );
+        m.add( I < EI, q < 7 ? flag_of( f.w, q < 7 ? q + 1 : 7 ) : f.xp, q < 7 ? p[q < 7 ? q + 1 : 7] : pxp );
+        m.add( r.J > 0, flag_of( f.ym, q ), pym[q] );
+        m.add( r.J < EJ, flag_of( f.yp, q ), pyp[q] );
+        m.add( r.K > 0, flag_of( f.zm, q ), pzm[q] );
+        m.add( r.K < EK, flag_of( f.zp, q ), pzp[q] );
+        out[q] = own_flag == BORA_FLUID ? p[q] : ( own_flag == BORA_AIR ? m.value() : 0.f );
     }
-    __syncthreads();
-    const int l = threadIdx.x;
-    const int li = l & 7, lj = ( l >> 3 ) & 7, lk = l >> 6;
-    const int i = ti * 8 + li, j = tj * 8 + lj, k = tk * 8 + lk;
-    const size_t cell = (size_t)s * BORA_TILE_CELLS + l;
-    const int h = H1::at( li + 1, lj + 1, lk + 1 );
-    const uint8_t f = fa[h];
-    if( f == BORA_MASKED ) { c.pres[cell] = 0.f; c.cx[cell] = 0.f; c.cy[cell] = 0.f; c.cz[cell] = 0.f; return; }
-    const float p = pa[h];
-    c.pres[cell] = p;
-    float vx = c.vx[cell], vy = c.vy[cell], vz = c.vz[cell];
-    if( f == BORA_FLUID )
-    {
-        const int wall = (float)j + 0.5f <= g.voxel_wall + 1.f ? BORA_SOLID : BORA_AIR;
-        const int hi0 = h - 1, hi1 = h + 1, hj0 = h - H1::E, hj1 = h + H1::E, hk0 = h - H1::E * H1::E, hk1 = h + H1::E * H1::E;
-        const int t_i0 = i == 0 ? wall : fa[hi0];
-        const int t_i1 = i == EI ? wall : fa[hi1];
-        const int t_j0 = j == 0 ? wall : fa[hj0];
-        const int t_j1 = j == EJ ? wall : fa[hj1];
-        const int t_k0 = k == 0 ? wall : fa[hk0];
-        const int t_k1 = k == EK ? wall : fa[hk1];
-        const float i0_j_k = i == 0 ? 2.f * p - pa[hi1] : pa[hi0];
-        const float i1_j_k = i == EI ? 2.f * p - pa[hi0] : pa[hi1];
-        const float i_j0_k = j == 0 ? 2.f * p - pa[hj1] : pa[hj0];
-        const float i_j1_k = j == EJ ? 2.f * p - pa[hj0] : pa[hj1];
-        const float i_j_k0 = k == 0 ? 2.f * p - pa[hk1] : pa[hk0];
-        const float i_j_k1 = k == EK ? 2.f * p - pa[hk0] : pa[hk1];
-        const float p_i0 = t_i0 == BORA_SOLID ? 2.f * p - i1_j_k : t_i0 == BORA_AIR ? -i0_j_k : i0_j_k;
-        const float p_i1 = t_i1 == BORA_SOLID ? 2.f * p - i0_j_k : t_i1 == BORA_AIR ? -i1_j_k : i1_j_k;
-        const float p_j0 = t_j0 == BORA_SOLID ? 2.f * p - i_j1_k : t_j0 == BORA_AIR ? -i_j0_k : i_j0_k;
-        const float p_j1 = t_j1 == BORA_SOLID ? 2.f * p - i_j0_k : t_j1 == BORA_AIR ? -i_j1_k : i_j1_k;
-        const float p_k0 = t_k0 == BORA_SOLID ? 2.f * p - i_j_k1 : t_k0 == BORA_AIR ? -i_j_k0 : i_j_k0;
-        const float p_k1 = t_k1 == BORA_SOLID ? 2.f * p - i_j_k0 : t_k1 == BORA_AIR ? -i_j_k1 : i_j_k1;
-        vx -= ( p_i1 - p_i0 ) * 0.5f;
-        vy -= ( p_j1 - p_j0 ) * 0.5f;
-        vz -= ( p_k1 - p_k0 ) * 0.5f;
-    }
-    c.cx[cell] = vx;
-    c.cy[cell] = vy;
-    c.cz[cell] = vz;
+    if( !r.mine ) return;
+    // fluid cells are not stored: other warps read them
+#pragma unroll
+    for( int q = 0; q < 8; ++q )
+        if( flag_of( f.w, q ) != BORA_FLUID ) c.pres[r.at() + q] = out[q];
 }
+
+// The air pressure of cell (i, j, k), which lies in the grid and in an inactive tile (only where
+// the caller has set flags: the tiles around every particle are active), out of line.
+__device__ __noinline__ float air_pressure_at( const BoraGridDev* g, const int32_t* slot_of, const uint8_t* flag,
+                                               const float* pres, int i, int j, int k )
+{
+    AirMean m;
+    for( int q = 0; q < 6; ++q )
+    {
+        const int n[3] = { i + ( q == 0 ? -1 : q == 1 ? 1 : 0 ), j + ( q == 2 ? -1 : q == 3 ? 1 : 0 ), k + ( q == 4 ? -1 : q == 5 ? 1 : 0 ) };
+        if( n[0] < 0 || n[1] < 0 || n[2] < 0 || n[0] >= g->nx || n[1] >= g->ny || n[2] >= g->nz ) continue;
+        const int s = slot_of[( (size_t)( n[2] >> 3 ) * g->ty + ( n[1] >> 3 ) ) * g->tx + ( n[0] >> 3 )];
+        if( s < 0 ) continue;
+        const size_t cell = (size_t)s * BORA_TILE_CELLS + bora_local( n[0], n[1], n[2] );
+        m.add( true, flag[cell], pres[cell] );
+    }
+    return m.value();
+}
+
+__global__ void __launch_bounds__( 32 * kRowWarps ) k_vel_update( const __grid_constant__ BoraGridDev g, BoraTilesDev t, int ntiles,
+                                                                  BoraCellsDev c )
+{
+    const HalfRow r = half_row( g, t, ntiles );
+    RowFlags f;
+    f.load( c.flag, r );
+    const int own = r.mine ? r.s : -1;
+    float p[8], pym[8], pyp[8], pzm[8], pzp[8], yh[8], zh[8], vx[8], vy[8], vz[8];
+    row8( c.pres, own, r.c, p );
+    row8( c.pres, r.yt, r.yc, yh );
+    row8( c.pres, r.zt, r.zc, zh );
+    float pxm = r.xm < 0 ? 0.f : c.pres[(size_t)r.xm * BORA_TILE_CELLS + r.c + 7];
+    float pxp = r.xp < 0 ? 0.f : c.pres[(size_t)r.xp * BORA_TILE_CELLS + r.c];
+    row8( c.vx, own, r.c, vx );
+    row8( c.vy, own, r.c, vy );
+    row8( c.vz, own, r.c, vz );
+    const int EI = g.nx - 1, EJ = g.ny - 1, EK = g.nz - 1;
+    // fluid cells next to an inactive tile
+    if( r.mine )
+    {
+        auto outside = [&]( int i, int j, int k ) { return air_pressure_at( &g, t.slot_of, c.flag, c.pres, i, j, k ); };
+        if( r.xm < 0 && r.i0 > 0 && flag_of( f.w, 0 ) == BORA_FLUID ) pxm = outside( r.i0 - 1, r.J, r.K );
+        if( r.xp < 0 && r.i0 + 7 < EI && flag_of( f.w, 7 ) == BORA_FLUID ) pxp = outside( r.i0 + 8, r.J, r.K );
+        const int dy = r.j == 0 ? -1 : 1, dz = r.kk == 0 ? -1 : 1;
+        const bool y_out = ( r.j == 0 || r.j == 7 ) && r.yt < 0 && r.J + dy >= 0 && r.J + dy <= EJ;
+        const bool z_out = ( r.kk == 0 || r.kk == 3 ) && r.zt < 0 && r.K + dz >= 0 && r.K + dz <= EK;
+        if( y_out || z_out )
+#pragma unroll
+            for( int q = 0; q < 8; ++q )
+            {
+                if( flag_of( f.w, q ) != BORA_FLUID ) continue;
+                if( y_out ) yh[q] = outside( r.i0 + q, r.J + dy, r.K );
+                if( z_out ) zh[q] = outside( r.i0 + q, r.J, r.K + dz );
+            }
+    }
+    beside( p, yh, 1, r.j == 0, r.j == 7, pym, pyp );
+    beside( p, zh, 8, r.kk == 0, r.kk == 3, pzm, pzp );
+    const int wall = (float)r.J + 0.5f <= g.voxel_wall + 1.f ? BORA_SOLID : BORA_AIR;
+#pragma unroll
+    for( int q = 0; q < 8; ++q )
+    {
+        const int own_flag = flag_of( f.w, q );
+        const bool e_i0 = r.i0 + q == 0, e_i1 = r.i0 + q == EI, e_j0 = r.J == 0, e_j1 = r.J == EJ, e_k0 = r.K == 0, e_k1 = r.K == EK;
+        auto grad = [&]( float lo, float hi, bool e0, bool e1, int t0, int t1 ) {
+            t0 = e0 ? wall : t0;
+            t1 = e1 ? wall : t1;
+            const float n0 = e0 ? 2.f * p[q] - hi : lo, n1 = e1 ? 2.f * p[q] - lo : hi;
+            const float a = t0 == BORA_SOLID ? 2.f * p[q] - n1 : t0 == BORA_AIR ? -n0 : n0;
+            const float b = t1 == BORA_SOLID ? 2.f * p[q] - n0 : t1 == BORA_AIR ? -n1 : n1;
+            return ( b - a ) * 0.5f;
+        };
+        const float dx = grad( q ? p[q ? q - 1 : 0] : pxm, q < 7 ? p[q < 7 ? q + 1 : 7] : pxp, e_i0, e_i1,
+                               q ? flag_of( f.w, q ? q - 1 : 0 ) : f.xm, q < 7 ? flag_of( f.w, q < 7 ? q + 1 : 7 ) : f.xp );
+        const float dy = grad( pym[q], pyp[q], e_j0, e_j1, flag_of( f.ym, q ), flag_of( f.yp, q ) );
+        const float dz = grad( pzm[q], pzp[q], e_k0, e_k1, flag_of( f.zm, q ), flag_of( f.zp, q ) );
+        const bool fluid = own_flag == BORA_FLUID, masked = own_flag == BORA_MASKED;
+        vx[q] = masked ? 0.f : ( fluid ? vx[q] - dx : vx[q] );
+        vy[q] = masked ? 0.f : ( fluid ? vy[q] - dy : vy[q] );
+        vz[q] = masked ? 0.f : ( fluid ? vz[q] - dz : vz[q] );
+    }
+    if( !r.mine ) return;
+    bora_st8( c.cx + r.at(), vx );
+    bora_st8( c.cy + r.at(), vy );
+    bora_st8( c.cz + r.at(), vz );
+}
+
+int row_grid( int ntiles ) { return ( 2 * ntiles + kRowWarps - 1 ) / kRowWarps; }
 
 int grid_for( size_t n, int threads )
 {
@@ -1478,7 +1634,7 @@ int grid_for( size_t n, int threads )
 void bora_launch_rhs( const BoraGridDev& g, int ntiles, BoraTilesDev t, BoraCellsDev c, uint32_t* nfluid, uint8_t* tile_fluid,
                       cudaStream_t st )
 {
-    if( ntiles > 0 ) k_rhs<<<ntiles, 512, 0, st>>>( g, t, c, nfluid, tile_fluid );
+    if( ntiles > 0 ) k_rhs<<<row_grid( ntiles ), 32 * kRowWarps, 0, st>>>( g, t, ntiles, c, nfluid, tile_fluid );
 }
 
 void bora_launch_tile_fluid( int ntiles, const uint16_t* code, uint8_t* tile_fluid, cudaStream_t st )
@@ -1502,7 +1658,9 @@ void bora_launch_solve_tiles( int ntiles, BoraTilesDev t, const uint8_t* tile_fl
 
 void bora_launch_vel_update( const BoraGridDev& g, int ntiles, BoraTilesDev t, BoraCellsDev c, cudaStream_t st )
 {
-    if( ntiles > 0 ) k_vel_update<<<ntiles, 512, 0, st>>>( g, t, c );
+    if( ntiles <= 0 ) return;
+    k_air_pressure<<<row_grid( ntiles ), 32 * kRowWarps, 0, st>>>( g, t, ntiles, c );
+    k_vel_update<<<row_grid( ntiles ), 32 * kRowWarps, 0, st>>>( g, t, ntiles, c );
 }
 
 void bora_launch_mic_factor( int ntiles, BoraSolveTilesDev t, const uint16_t* code, float* minv, cudaStream_t st )
@@ -1556,14 +1714,19 @@ int bora_pcg_direction_grid( int ntiles )
 }
 
 namespace {
-int residual_grid( size_t nc ) { return (int)std::max<size_t>( 1, std::min<size_t>( ( nc + 255 ) / 256, (size_t)num_sms() * 8 ) ); }
+// equal rounds of the warps that are resident (three CTAs per SM at 80 registers)
+int residual_grid( int nft )
+{
+    const int cap = 3 * num_sms() * kResWarps, rounds = std::max( 1, ( 2 * nft + cap - 1 ) / cap );
+    return std::max( 1, ( 2 * nft + kResWarps * rounds - 1 ) / ( kResWarps * rounds ) );
+}
 }  // namespace
 
 void bora_projection_grids( int nft, int* grid )
 {
     grid[kGridDir] = bora_pcg_direction_grid( nft );
     grid[kGridCells] = grid_for( (size_t)nft * 128, 256 );
-    grid[kGridResidual] = residual_grid( (size_t)nft * 512 );
+    grid[kGridResidual] = residual_grid( nft );
 }
 
 void bora_launch_solve_init_batch( const BoraBatchLaunch& L, int blocks, cudaStream_t st )
@@ -1700,7 +1863,7 @@ void bora_launch_refine_accumulate( BoraSolveTilesDev t, const uint16_t* code, B
 void bora_launch_refine_residual( BoraSolveTilesDev t, const float* b, const uint16_t* code, BoraSolverDev s, BoraReduceDev red,
                                   int slot_norm2, int slot_max, cudaStream_t st )
 {
-    k_refine_residual<<<residual_grid( (size_t)t.n * 512 ), 256, 0, st>>>( t, b, code, s, red, slot_norm2, slot_max );
+    k_refine_residual<<<residual_grid( t.n ), 32 * kResWarps, 0, st>>>( t, b, code, s, red, slot_norm2, slot_max );
 }
 
 void bora_launch_write_pressure( int ntiles, const uint16_t* code, const float2* x, float* pres, cudaStream_t st )
