@@ -33,7 +33,8 @@
 // the rows across them (the other half, the neighbour tiles). The passes wait on their loads, so
 // they want warps in flight and all of a lane's loads issued before the first is used: with a
 // tile per warp (two rows per lane, 128 registers, 12 warps in flight) the four passes took 33,
-// 18, 28 and 24 us at 256^3 (8.2 K tiles). Levels 1 and 2 run one thread per cell.
+// 18, 28 and 24 us at 256^3 (8.2 K tiles). Levels 1 and 2 run one
+// thread per x-row of 4 or 2 cells.
 #include <algorithm>
 #include <type_traits>
 
@@ -45,7 +46,7 @@ namespace {
 constexpr float kOmegaA = 0.5687f;  // the Chebyshev pair of the smoothers (multigrid.cu)
 constexpr float kOmegaB = 1.6902f;
 // launch shapes (the autotuner picks one per size class; the results do not depend on it):
-// level 0 half tiles (warps) per block, levels 1 and 2 threads (cells) per block
+// level 0 half tiles (warps) per block, levels 1 and 2 threads (x-rows) per block
 constexpr int kPassWarpsOf[3] = { 2, 4, 8 };
 constexpr int kFlatThreadsOf[4] = { 64, 128, 256, 512 };
 // Warps per SM that level 0 asks registers for: 24 (80 registers) for down 2 and up 1, 16 (128)
@@ -476,7 +477,7 @@ __global__ void __launch_bounds__( 32 * W, pass_warps_per_sm( P ) / W ) k_mg_pas
     pass0_body<W, P>( a, bid, (unsigned)m.grid[P == 0 || P == 3 ? kGridPass0R : kGridPass0] );
 }
 
-// ---- levels 1 and 2: one thread per cell --------------------------------------------------
+// ---- levels 1 and 2: one thread per x-row --------------------------------------------------
 
 struct PassFArgs
 {
@@ -487,106 +488,171 @@ struct PassFArgs
     float* scratch;
 };
 
-// pass P (0 = down 1, 1 = down 2, 2 = up 1, 3 = up 2) of a level with E = 4 or 2, one cell
-// per thread (the grid covers every cell once; a block holds whole tiles). What no kernel of
-// the solve writes - the cell's code, its neighbours' indices and codes - is read before the
-// dependency wait, so that it overlaps the previous kernel.
-template <int E, int P, int T>
+// E 16-bit values in E / 2 words
+template <int E>
+__device__ __forceinline__ void ld16( const void* p, size_t g, uint32_t* w )
+{
+    const uint16_t* q = static_cast<const uint16_t*>( p ) + g;
+    if constexpr( E == 4 )
+    {
+        const uint2 v = *reinterpret_cast<const uint2*>( q );
+        w[0] = v.x;
+        w[1] = v.y;
+    }
+    else w[0] = *reinterpret_cast<const uint32_t*>( q );
+}
+template <int E>
+__device__ __forceinline__ void st16( __half* p, size_t g, const float* v )
+{
+    if constexpr( E == 4 ) *reinterpret_cast<uint2*>( p + g ) = make_uint2( pack2( v[0], v[1] ), pack2( v[2], v[3] ) );
+    else *reinterpret_cast<uint32_t*>( p + g ) = pack2( v[0], v[1] );
+}
+__device__ __forceinline__ uint16_t word16( const uint32_t* w, int i ) { return (uint16_t)( w[i >> 1] >> ( 16 * ( i & 1 ) ) ); }
+
+// pass P (0 = down 1, 1 = down 2, 2 = up 1, 3 = up 2) of a level with E = 4 or 2: a lane owns an
+// x-row (j, k) of a tile, E * E lanes in a row of the warp own the tile. The neighbours in x are the
+// lane's own, those in y and z other lanes' by shuffles, and the rows and cells across the tile's
+// faces are loaded by the lanes at them. What no kernel of the solve writes - the table entry and
+// the codes - is read before the dependency wait, so that it overlaps the previous kernel. (With
+// a cell per thread, 235 instructions a cell at level 1: a V-cycle of 103 us at 256^3, 95 now, and
+// of 244 us in a 640 tank of 16.8 K tiles, 220 now.)
+template <int E, int P>
 __device__ __forceinline__ void passf_body( const PassFArgs& a, unsigned bid )
 {
-    constexpr int E3 = E * E * E, H = E / 2, H3 = H * H * H;
+    constexpr int R = E * E, E3 = E * E * E, H = E / 2, H3 = H * H * H, W = E / 2;
     constexpr bool kCodes = P == 0 || P == 2;  // the neighbours' values need their codes
     __shared__ float w[32];
-    __shared__ float res[T];
     bora_pdl_trigger();
     init_weights( w );
-    // cell i of the solver's tiles: cell g of the level
-    const size_t base = (size_t)bid * T, i = base + threadIdx.x;
-    const bool live = i < (size_t)a.ft.n * E3;
+    const size_t row = (size_t)bid * blockDim.x + threadIdx.x;
+    const bool live = row < (size_t)a.ft.n * R;
+    const int j = (int)( row % E ), k = (int)( row / E % E );
     const BoraLevelDev& F = a.F;
-    size_t g = 0;
-    int s = 0, x = 0, y = 0, z = 0;
-    uint16_t cc = 0;
-    int64_t gn[6];     // neighbour cells -x +x -y +y -z +z (-1: none)
-    uint16_t cn[6];
-    int pn[6];         // up 1: the neighbours' parents on the coarser level
+    int4 n0 = make_int4( -1, -1, -1, -1 ), n1 = n0;
     if( live )
     {
-        const int l = (int)( i % E3 );
-        const int4 n0 = __ldg( a.ft.tab + 2 * ( i / E3 ) ), n1 = __ldg( a.ft.tab + 2 * ( i / E3 ) + 1 );
-        const int nf[6] = { n0.x, n0.y, n0.z, n0.w, n1.x, n1.y };
-        s = n1.z;
-        g = (size_t)s * E3 + l;
-        x = l % E; y = ( l / E ) % E; z = l / ( E * E );
-        cc = F.code[g];
-#pragma unroll
-        for( int q = 0; q < 6; ++q )
-        {
-            const int dx = q == 0 ? -1 : ( q == 1 ? 1 : 0 ), dy = q == 2 ? -1 : ( q == 3 ? 1 : 0 ),
-                      dz = q == 4 ? -1 : ( q == 5 ? 1 : 0 );
-            int xx = x + dx, yy = y + dy, zz = z + dz, t = s;
-            if( xx < 0 || xx >= E || yy < 0 || yy >= E || zz < 0 || zz >= E )
-            {
-                t = nf[q];
-                xx &= E - 1; yy &= E - 1; zz &= E - 1;
-            }
-            gn[q] = t < 0 ? -1 : (int64_t)t * E3 + xx + E * ( yy + E * zz );
-            pn[q] = t < 0 ? 0 : t * H3 + ( xx >> 1 ) + H * ( ( yy >> 1 ) + H * ( zz >> 1 ) );
-            cn[q] = kCodes && t >= 0 ? F.code[gn[q]] : 0;
-        }
+        n0 = __ldg( a.ft.tab + 2 * ( row / R ) );
+        n1 = __ldg( a.ft.tab + 2 * ( row / R ) + 1 );
+    }
+    // a row of this level: its tile's slot (-1: none) and its j, k
+    struct Row
+    {
+        int t, j, k;
+        __device__ size_t at() const { return (size_t)t * E3 + E * ( j + E * k ); }
+        __device__ size_t parent() const { return (size_t)t * H3 + H * ( ( j >> 1 ) + H * ( k >> 1 ) ); }
+    };
+    const Row own{ live ? n1.z : -1, j, k };
+    const Row ry{ j == 0 ? n0.z : ( j == E - 1 ? n0.w : -1 ), j == 0 ? E - 1 : 0, k };
+    const Row rz{ k == 0 ? n1.x : ( k == E - 1 ? n1.y : -1 ), j, k == 0 ? E - 1 : 0 };
+    const Row rm{ live ? n0.x : -1, j, k }, rp{ live ? n0.y : -1, j, k };  // the x ends: the last / first cell
+    uint32_t co[W] = {}, cy[W] = {}, cz[W] = {};
+    uint16_t cm = 0, cp = 0;
+    if( own.t >= 0 ) ld16<E>( F.code, own.at(), co );
+    if constexpr( kCodes )
+    {
+        if( ry.t >= 0 ) ld16<E>( F.code, ry.at(), cy );
+        if( rz.t >= 0 ) ld16<E>( F.code, rz.at(), cz );
+        if( rm.t >= 0 ) cm = F.code[rm.at() + E - 1];
+        if( rp.t >= 0 ) cp = F.code[rp.at()];
     }
     bora_pdl_wait();  // the previous kernel's results are complete from here
     __syncthreads();
-    // the field value the pass reads at cell gi (code ci, parent pi)
-    auto value = [&]( int64_t gi, uint16_t ci, int pi ) -> float {
-        if( gi < 0 ) return 0.f;
-        if constexpr( P == 0 ) return cfluid( ci ) ? __half2float( F.r[gi] ) * w[cdiag( ci )] : 0.f;
-        else if constexpr( P == 2 ) return cfluid( ci ) ? __half2float( F.z0[gi] ) + __half2float( a.ec[pi] ) : 0.f;
-        else return a.scratch[gi];
-    };
-    float out = 0.f;
-    if( live )
+    // the field that the pass reads at its neighbours: raw loads, then values
+    struct Raw
     {
-        const float rp = cfluid( cc ) ? __half2float( F.r[g] ) : 0.f;
-        const int pg = s * H3 + ( x >> 1 ) + H * ( ( y >> 1 ) + H * ( z >> 1 ) );
-        const float v = value( (int64_t)g, cc, pg );
-        const float sum = ( ( value( gn[0], cn[0], pn[0] ) + value( gn[1], cn[1], pn[1] ) ) +
-                            ( value( gn[2], cn[2], pn[2] ) + value( gn[3], cn[3], pn[3] ) ) ) +
-                          ( value( gn[4], cn[4], pn[4] ) + value( gn[5], cn[5], pn[5] ) );
-        if constexpr( P == 0 ) out = sweep( v, rp, cc, sum, w + 16 );
-        else if constexpr( P == 1 ) out = cfluid( cc ) ? rp - ( (float)cdiag( cc ) * v - sum ) : 0.f;
-        else if constexpr( P == 2 ) out = sweep( v, rp, cc, sum, w + 16 );
-        else out = sweep( v, rp, cc, sum, w );
-        if constexpr( P == 0 || P == 2 ) a.scratch[g] = out;
-        else if constexpr( P == 1 ) F.z0[g] = __float2half_rn( v );
-        else F.z1[g] = __float2half_rn( out );
+        uint32_t h[W], e;  // residual or z0; the parents' correction
+        float f[E];        // scratch
+    };
+    auto load = [&]( const Row& r, Raw& x ) {
+#pragma unroll
+        for( int i = 0; i < W; ++i ) x.h[i] = 0u;
+        x.e = 0u;
+#pragma unroll
+        for( int i = 0; i < E; ++i ) x.f[i] = 0.f;
+        if( r.t < 0 ) return;
+        if constexpr( P == 0 ) ld16<E>( F.r, r.at(), x.h );
+        else if constexpr( P == 2 )
+        {
+            ld16<E>( F.z0, r.at(), x.h );
+            if constexpr( H == 2 ) x.e = *reinterpret_cast<const uint32_t*>( a.ec + r.parent() );
+            else x.e = *reinterpret_cast<const uint16_t*>( a.ec + r.parent() );
+        }
+        else if constexpr( E == 4 )
+        {
+            const float4 v = *reinterpret_cast<const float4*>( a.scratch + r.at() );
+            x.f[0] = v.x; x.f[1] = v.y; x.f[2] = v.z; x.f[3] = v.w;
+        }
+        else
+        {
+            const float2 v = *reinterpret_cast<const float2*>( a.scratch + r.at() );
+            x.f[0] = v.x; x.f[1] = v.y;
+        }
+    };
+    auto value = [&]( const Raw& x, uint16_t c, int i ) -> float {
+        if constexpr( P == 0 ) return cfluid( c ) ? hbits( x.h[i >> 1], i & 1 ) * w[cdiag( c )] : 0.f;
+        else if constexpr( P == 2 ) return cfluid( c ) ? hbits( x.h[i >> 1], i & 1 ) + hbits( x.e, i >> 1 ) : 0.f;
+        else return x.f[i];
+    };
+    auto one = [&]( const Row& r, uint16_t c, int i ) -> float {
+        if( r.t < 0 ) return 0.f;
+        if constexpr( P == 0 ) return cfluid( c ) ? __half2float( F.r[r.at() + i] ) * w[cdiag( c )] : 0.f;
+        else if constexpr( P == 2 ) return cfluid( c ) ? __half2float( F.z0[r.at() + i] ) + __half2float( a.ec[r.parent() + ( i >> 1 )] ) : 0.f;
+        else return a.scratch[r.at() + i];
+    };
+    Raw xo, xy, xz;
+    load( own, xo );
+    load( ry, xy );
+    load( rz, xz );
+    const float xm = one( rm, cm, E - 1 ), xp = one( rp, cp, 0 );
+    uint32_t rw[W] = {};
+    if( own.t >= 0 ) ld16<E>( F.r, own.at(), rw );
+    float v[E], out[E];
+#pragma unroll
+    for( int i = 0; i < E; ++i ) v[i] = value( xo, word16( co, i ), i );
+#pragma unroll
+    for( int i = 0; i < E; ++i )
+    {
+        const uint16_t c = word16( co, i );
+        float ym = __shfl_up_sync( kAll, v[i], 1 ), yp = __shfl_down_sync( kAll, v[i], 1 );
+        float zm = __shfl_up_sync( kAll, v[i], E ), zp = __shfl_down_sync( kAll, v[i], E );
+        const float hy = value( xy, word16( cy, i ), i ), hz = value( xz, word16( cz, i ), i );
+        if( j == 0 ) ym = hy;
+        if( j == E - 1 ) yp = hy;
+        if( k == 0 ) zm = hz;
+        if( k == E - 1 ) zp = hz;
+        const float sum = ( ( ( i ? v[i ? i - 1 : 0] : xm ) + ( i < E - 1 ? v[i < E - 1 ? i + 1 : 0] : xp ) ) + ( ym + yp ) ) + ( zm + zp );
+        const float r = cfluid( c ) ? hbits( rw[i >> 1], i & 1 ) : 0.f;
+        if constexpr( P == 1 ) out[i] = cfluid( c ) ? r - ( (float)cdiag( c ) * v[i] - sum ) : 0.f;
+        else out[i] = sweep( v[i], r, c, sum, P == 3 ? w : w + 16 );
     }
     if constexpr( P == 1 )
     {
-        // restriction of the block's tiles
-        res[threadIdx.x] = out;
-        __syncthreads();
-        constexpr int kParents = T / 8;
-        if( threadIdx.x < kParents )
+        // restriction: x pairs in the row, y pairs from lane j + 1, z pairs from lane + E
+        float q[2];
+#pragma unroll
+        for( int i = 0; i < H; ++i )
         {
-            const int p = threadIdx.x, tl = p / H3, pl = p % H3;
-            if( base / E3 + tl < (size_t)a.ft.n )
-            {
-                const size_t tile = (size_t)__ldg( &a.ft.tab[2 * ( base / E3 + tl ) + 1].z );
-                const int pa = pl % H, pb = ( pl / H ) % H, pc = pl / ( H * H );
-                const int l = tl * E3 + 2 * pa + E * ( 2 * pb + E * 2 * pc );
-                const float sum = ( ( res[l] + res[l + 1] ) + ( res[l + E] + res[l + E + 1] ) ) +
-                                  ( ( res[l + E * E] + res[l + E * E + 1] ) + ( res[l + E * E + E] + res[l + E * E + E + 1] ) );
-                a.C.r[tile * H3 + pl] = __float2half_rn( 0.5f * sum );
-            }
+            q[i] = out[2 * i] + out[2 * i + 1];
+            q[i] = q[i] + __shfl_down_sync( kAll, q[i], 1 );
+            q[i] = q[i] + __shfl_down_sync( kAll, q[i], E );
+        }
+        if( own.t >= 0 && !( j & 1 ) && !( k & 1 ) )
+        {
+            if constexpr( H == 2 ) *reinterpret_cast<uint32_t*>( a.C.r + own.parent() ) = pack2( 0.5f * q[0], 0.5f * q[1] );
+            else a.C.r[own.parent()] = __float2half_rn( 0.5f * q[0] );
         }
     }
+    if( own.t < 0 ) return;
+    if constexpr( P == 1 ) st16<E>( F.z0, own.at(), v );
+    else if constexpr( P == 3 ) st16<E>( F.z1, own.at(), out );
+    else if constexpr( E == 4 ) *reinterpret_cast<float4*>( a.scratch + own.at() ) = make_float4( out[0], out[1], out[2], out[3] );
+    else *reinterpret_cast<float2*>( a.scratch + own.at() ) = make_float2( out[0], out[1] );
 }
 
 template <int E, int P, int T>
 __global__ void __launch_bounds__( T ) k_mg_passf( const __grid_constant__ PassFArgs a )
 {
-    passf_body<E, P, T>( a, blockIdx.x );
+    passf_body<E, P>( a, blockIdx.x );
 }
 
 template <int E, int P, int T>
@@ -602,7 +668,7 @@ __global__ void __launch_bounds__( T ) k_mg_passf_batch( const __grid_constant__
     a.C = m.L[l + 1];
     a.ec = l == 1 ? m.L[2].z1 : m.z3;
     a.scratch = m.sv.minv;
-    passf_body<E, P, T>( a, bid );
+    passf_body<E, P>( a, bid );
 }
 
 int num_sms_pass()
@@ -648,7 +714,7 @@ void launch_pass0( const Pass0Args& a, int v, cudaStream_t st )
 // Grid of the passes of a level with E cells per tile edge in launch shape v: level 0 as many
 // blocks as make equal rounds of warps over the half tiles with the warps per SM that its
 // registers allow (v < 0: the reducing passes, at most kBoraMaxReduceBlocks); levels 1 and 2
-// one thread per cell.
+// one thread per x-row.
 int bora_mg_pass_grid( int E, int ntiles, int v )
 {
     if( ntiles <= 0 ) return 0;
@@ -661,7 +727,7 @@ int bora_mg_pass_grid( int E, int ntiles, int v )
         return std::max( 1, ( 2 * ntiles + W * rounds - 1 ) / ( W * rounds ) );
     }
     const int T = kFlatThreadsOf[std::min( std::max( v, 0 ), 3 )];
-    const size_t n = (size_t)ntiles * E * E * E;
+    const size_t n = (size_t)ntiles * E * E;
     return (int)( ( n + T - 1 ) / T );
 }
 
