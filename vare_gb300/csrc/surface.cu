@@ -32,11 +32,16 @@ __device__ inline void tile_coords( const BoraGridDev& g, int vt, int& ti, int& 
 // sort's key). One CTA per tile owns the tile's 512 cells and walks the 11 dual-cell
 // layers z = -2 .. 8 of its region: each layer's particles (11 x 11 dual cells, one
 // contiguous sorted range each) are staged in shared memory, and the 256 cells the layer
-// can reach (z - 1 .. z + 2) are worked on at once: a pair of z-adjacent cells per thread
-// pair (the pair shares each candidate's x and y distances), the two threads of a pair
-// taking two of the four candidate rows each. Layer sums go into per-cell shared sums in a
-// fixed order, so the result is reproducible; no atomics, and the normalisation of
-// Rasterization.cu:373-395 is applied on the way out.
+// can reach (z - 1 .. z + 2) are worked on at once. A thread takes one of the four candidate
+// rows of a column of four cells (i, j, z - 1 .. z + 2), so that a staged particle is read once
+// for four cells; a warp takes the 32 (column, row) pairs of one i ordered by the row, so that
+// most lanes next to each other read the same particle. The rows' sums are added across the four
+// lanes in a fixed order and go into per-cell shared sums, so the result is reproducible; no
+// atomics, and the normalisation of Rasterization.cu:373-395 is applied on the way out.
+//
+// Bound by shared-memory reads of the staged particles and by FP32 instructions, which work on
+// packed pairs: at 128^3 (1.4 K tiles) 524 us with a thread per two cells and two rows and
+// lanes over 8 columns (10 wavefronts a particle read instead of 5), 346 now.
 constexpr int kSplatThreads = 256;
 constexpr int kSplatCap = 1024;  // staged particles per pass (a layer with more takes several)
 constexpr int kLayerCells = 121;  // 11 x 11 dual cells
@@ -46,7 +51,11 @@ constexpr int kLayerCells = 121;  // 11 x 11 dual cells
 // and the division (one weight's rounding differs by an ulp or two; the sums' order, open
 // in the reference, moves them more). Zero for d^2 >= 2.25; a cell within that radius lies
 // in the reference's 3^3 box around (int)p.
-__global__ void __launch_bounds__( kSplatThreads ) k_splat( const __grid_constant__ BoraGridDev g, BoraTilesDev t,
+// A cell's place in the running sums: the 32 (lj, zc) that a warp adds to at once, zc four
+// consecutive values, lie in 32 banks.
+__device__ inline int splat_at( int li, int lj, int zc ) { return 64 * li + 8 * lj + ( zc ^ ( lj & 4 ) ); }
+
+__global__ void __launch_bounds__( kSplatThreads, 3 ) k_splat( const __grid_constant__ BoraGridDev g, BoraTilesDev t,
                                                             const uint32_t* __restrict__ start,
                                                             const uint32_t* __restrict__ idx, BoraParticlesDev p,
                                                             BoraCellsDev c )
@@ -63,12 +72,19 @@ __global__ void __launch_bounds__( kSplatThreads ) k_splat( const __grid_constan
     for( int h = tid; h < 7 * BORA_TILE_CELLS; h += kSplatThreads ) ( &accs[0][0] )[h] = 0.f;
     int ti, tj, tk;
     tile_coords( g, t.tile_of[s], ti, tj, tk );
-    // work item: cells (li, lj, zz - 1 + 2 pr) and (li, lj, zz + 2 pr); lanes l and l ^ 16
-    // split its four candidate rows
-    const int half = ( tid >> 4 ) & 1;
-    const int item = ( tid & 15 ) | ( ( tid >> 5 ) << 4 );
-    const int li = item & 7, lj = ( item >> 3 ) & 7, pr = item >> 6;
-    const float cx = (float)( ti * BORA_TILE + li ) + .5f, cy = (float)( tj * BORA_TILE + lj ) + .5f;
+    // work item: the column (li, lj), its candidate row yy = lj - 2 + r. Lane of (lj, r) in the
+    // warp of li: the pairs ordered by lj + r, then lj
+    const int li = tid >> 5, lane = tid & 31;
+    auto lane_of = [&]( int j, int r ) {
+        const int y = j + r;
+        const int first = y <= 3 ? y * ( y + 1 ) / 2 : ( y <= 8 ? 4 * y - 6 : 32 - ( 11 - y ) * ( 12 - y ) / 2 );
+        return first + j - max( 0, y - 3 );
+    };
+    int lj = 0, row = 0;
+    for( int q = 0; q < 32; ++q )
+        if( lane_of( q >> 2, q & 3 ) == lane ) { lj = q >> 2; row = q & 3; }
+    const int peer1 = lane_of( lj, row ^ 1 ), peer2 = lane_of( lj, row ^ 2 );
+    const float2 ncxy = make_float2( -( (float)( ti * BORA_TILE + li ) + .5f ), -( (float)( tj * BORA_TILE + lj ) + .5f ) );
     const float fnx = (float)g.nx, fny = (float)g.ny, fnz = (float)g.nz;
     __syncthreads();
     for( int zz = -2; zz <= 8; ++zz )
@@ -91,7 +107,7 @@ __global__ void __launch_bounds__( kSplatThreads ) k_splat( const __grid_constan
         }
         // exclusive scan over the 121 counts (warps 0..3)
         uint32_t inc = cnt;
-        const int lane = tid & 31, wp = tid >> 5;
+        const int wp = tid >> 5;
 #pragma unroll
         for( int o = 1; o < 32; o <<= 1 )
         {
@@ -109,13 +125,13 @@ __global__ void __launch_bounds__( kSplatThreads ) k_splat( const __grid_constan
         }
         __syncthreads();
         const uint32_t total = off[kLayerCells];
-        const int z0 = zz - 1 + 2 * pr, z1 = z0 + 1;  // this item's cells
-        const float cz0 = (float)( tk * BORA_TILE + z0 ) + .5f, cz1 = (float)( tk * BORA_TILE + z1 ) + .5f;
-        float acc[2][7];
+        // the column's cells z = zz - 1 + m; their centres in pairs
+        const float cz = (float)( tk * BORA_TILE + zz - 1 ) + .5f;
+        const float2 ncz[2] = { make_float2( -cz, -( cz + 1.f ) ), make_float2( -( cz + 2.f ), -( cz + 3.f ) ) };
+        float2 aw[2], axy[4], azu[4], avw[4];  // sums of w (cells in pairs), (w x, w y), (w z, w u), (w v, w w)
+        aw[0] = aw[1] = make_float2( 0.f, 0.f );
 #pragma unroll
-        for( int m = 0; m < 2; ++m )
-#pragma unroll
-            for( int v = 0; v < 7; ++v ) acc[m][v] = 0.f;
+        for( int m = 0; m < 4; ++m ) axy[m] = azu[m] = avw[m] = make_float2( 0.f, 0.f );
         for( uint32_t e0 = 0; e0 < total; e0 += kSplatCap )
         {
             const uint32_t e1 = min( total, e0 + kSplatCap );
@@ -138,52 +154,69 @@ __global__ void __launch_bounds__( kSplatThreads ) k_splat( const __grid_constan
                 sb[e - e0] = make_float2( p.vy[pi], p.vz[pi] );
             }
             __syncthreads();
-            // the 4 dual cells xx = li-2 .. li+1 of a row are adjacent in the staging
-            for( int yy = lj - 2 + 2 * half; yy <= lj - 1 + 2 * half; ++yy )
-            {
-                const int d = li + 11 * ( yy + 2 );
-                // the row's part of this pass, as staging indices (empty when the row lies
-                // wholly before or after the pass)
-                const uint32_t ga = max( off[d], e0 ), gb = min( off[d + 4], e1 );
-                const uint32_t a = ga - e0, b = gb > ga ? gb - e0 : a;
-                // branch-free: a particle outside the radius (or the grid) adds weight 0
-                auto add = [&]( uint32_t e ) {
-                    const float4 q = sa[e];
-                    const float2 r = sb[e];
-                    const float dx = q.x - cx, dy = q.y - cy, dz0 = q.z - cz0, dz1 = q.z - cz1;
-                    const float h2 = fmaf( dy, dy, dx * dx );
-                    const float t0 = fmaf( -fmaf( dz0, dz0, h2 ), 1.f / 2.25f, 1.f );
-                    const float t1 = fmaf( -fmaf( dz1, dz1, h2 ), 1.f / 2.25f, 1.f );
-                    const float w0 = t0 > 0.f ? t0 * t0 * t0 : 0.f, w1 = t1 > 0.f ? t1 * t1 * t1 : 0.f;
-                    acc[0][0] += w0; acc[1][0] += w1;
-                    acc[0][1] = fmaf( w0, q.x, acc[0][1] ); acc[1][1] = fmaf( w1, q.x, acc[1][1] );
-                    acc[0][2] = fmaf( w0, q.y, acc[0][2] ); acc[1][2] = fmaf( w1, q.y, acc[1][2] );
-                    acc[0][3] = fmaf( w0, q.z, acc[0][3] ); acc[1][3] = fmaf( w1, q.z, acc[1][3] );
-                    acc[0][4] = fmaf( w0, q.w, acc[0][4] ); acc[1][4] = fmaf( w1, q.w, acc[1][4] );
-                    acc[0][5] = fmaf( w0, r.x, acc[0][5] ); acc[1][5] = fmaf( w1, r.x, acc[1][5] );
-                    acc[0][6] = fmaf( w0, r.y, acc[0][6] ); acc[1][6] = fmaf( w1, r.y, acc[1][6] );
-                };
-                uint32_t e = a;
-                for( ; e + 2 <= b; e += 2 )
+            // the 4 dual cells xx = li-2 .. li+1 of a row are adjacent in the staging; the row's
+            // part of this pass, as staging indices (empty when the row lies wholly before or
+            // after the pass)
+            const int d = li + 11 * ( lj + row );
+            const uint32_t ga = max( off[d], e0 ), gb = min( off[d + 4], e1 );
+            const uint32_t a = ga - e0, b = gb > ga ? gb - e0 : a;
+            // branch-free: a particle outside the radius (or the grid) adds weight 0
+            auto add = [&]( uint32_t e ) {
+                const float4 q = sa[e];
+                const float2 vw = sb[e], xy = make_float2( q.x, q.y ), zu = make_float2( q.z, q.w );
+                const float2 dxy = __fadd2_rn( xy, ncxy );
+                const float h2 = fmaf( dxy.y, dxy.y, dxy.x * dxy.x );
+#pragma unroll
+                for( int n = 0; n < 2; ++n )
                 {
-                    add( e ); add( e + 1 );
+                    const float2 dz = __fadd2_rn( make_float2( q.z, q.z ), ncz[n] );
+                    float2 t = __ffma2_rn( __ffma2_rn( dz, dz, make_float2( h2, h2 ) ), make_float2( -1.f / 2.25f, -1.f / 2.25f ),
+                                           make_float2( 1.f, 1.f ) );
+                    t = make_float2( fmaxf( t.x, 0.f ), fmaxf( t.y, 0.f ) );
+                    const float2 w = __fmul2_rn( __fmul2_rn( t, t ), t );
+                    aw[n] = __fadd2_rn( aw[n], w );
+#pragma unroll
+                    for( int m = 2 * n; m < 2 * n + 2; ++m )
+                    {
+                        const float2 wd = m & 1 ? make_float2( w.y, w.y ) : make_float2( w.x, w.x );
+                        axy[m] = __ffma2_rn( wd, xy, axy[m] );
+                        azu[m] = __ffma2_rn( wd, zu, azu[m] );
+                        avw[m] = __ffma2_rn( wd, vw, avw[m] );
+                    }
                 }
-                if( e < b ) add( e );
+            };
+            uint32_t e = a;
+            for( ; e + 2 <= b; e += 2 )
+            {
+                add( e ); add( e + 1 );
             }
+            if( e < b ) add( e );
+            __syncwarp();
             __syncthreads();  // the staging buffer is reused by the next pass
         }
-        // the two halves' sums, added in a fixed order into the cells' running sums (each
-        // cell is owned by one item in a layer)
+        // the four rows' sums, (0 + 1) + (2 + 3), in two exchanges that leave the cell m = row in
+        // the lane; added into the cells' running sums (a cell is one lane's in a layer)
+        float sum[4][7];
 #pragma unroll
-        for( int m = 0; m < 2; ++m )
+        for( int m = 0; m < 4; ++m )
         {
-            const int zc = m == 0 ? z0 : z1;
+            sum[m][0] = m & 1 ? aw[m >> 1].y : aw[m >> 1].x;
+            sum[m][1] = axy[m].x; sum[m][2] = axy[m].y;
+            sum[m][3] = azu[m].x; sum[m][4] = azu[m].y;
+            sum[m][5] = avw[m].x; sum[m][6] = avw[m].y;
+        }
+        const int zc = zz - 1 + row;
 #pragma unroll
-            for( int v = 0; v < 7; ++v )
-            {
-                const float other = __shfl_xor_sync( 0xffffffffu, acc[m][v], 16 );
-                if( half == 0 && zc >= 0 && zc <= 7 ) accs[v][li + 8 * lj + 64 * zc] += acc[m][v] + other;
-            }
+        for( int v = 0; v < 7; ++v )
+        {
+            // keep the cells of the lane's parity, give the others
+            const bool odd = row & 1, high = row & 2;
+            float k0 = odd ? sum[1][v] : sum[0][v], k1 = odd ? sum[3][v] : sum[2][v];
+            const float g0 = odd ? sum[0][v] : sum[1][v], g1 = odd ? sum[2][v] : sum[3][v];
+            k0 += __shfl_sync( 0xffffffffu, g0, peer1 );
+            k1 += __shfl_sync( 0xffffffffu, g1, peer1 );
+            const float keep = ( high ? k1 : k0 ) + __shfl_sync( 0xffffffffu, high ? k0 : k1, peer2 );
+            if( zc >= 0 && zc <= 7 ) accs[v][splat_at( li, lj, zc )] += keep;
         }
         __syncthreads();  // the layer tables are rewritten next
     }
@@ -195,20 +228,21 @@ __global__ void __launch_bounds__( kSplatThreads ) k_splat( const __grid_constan
         const int l = tid + 256 * m;
         const int i = ti * BORA_TILE + ( l & 7 ), j = tj * BORA_TILE + ( ( l >> 3 ) & 7 ), k = tk * BORA_TILE + ( l >> 6 );
         const size_t n = (size_t)s * BORA_TILE_CELLS + l;
+        const int a = splat_at( l & 7, ( l >> 3 ) & 7, l >> 6 );
         const bool real = i < g.nx && j < g.ny && k < g.nz;
-        const float w = real ? accs[0][l] : 0.f;
+        const float w = real ? accs[0][a] : 0.f;
         c.pres[n] = w;
         if( w > 1e-30f )
         {
-            const float x = accs[1][l] / w, y = accs[2][l] / w, z = accs[3][l] / w;
+            const float x = accs[1][a] / w, y = accs[2][a] / w, z = accs[3][a] / w;
             c.cx[n] = x; c.cy[n] = y; c.cz[n] = z;
             const float dx = x - ( (float)i + .5f ), dy = y - ( (float)j + .5f ), dz = z - ( (float)k + .5f );
             c.surf[n] = sqrtf( dx * dx + dy * dy + dz * dz ) - 0.5f;  // Vec3f::distanceTo, Vector3.h:364-367
-            c.vx[n] = accs[4][l] / w; c.vy[n] = accs[5][l] / w; c.vz[n] = accs[6][l] / w;
+            c.vx[n] = accs[4][a] / w; c.vy[n] = accs[5][a] / w; c.vz[n] = accs[6][a] / w;
         }
         else
         {
-            c.cx[n] = real ? accs[1][l] : 0.f; c.cy[n] = real ? accs[2][l] : 0.f; c.cz[n] = real ? accs[3][l] : 0.f;
+            c.cx[n] = real ? accs[1][a] : 0.f; c.cy[n] = real ? accs[2][a] : 0.f; c.cz[n] = real ? accs[3][a] : 0.f;
             c.surf[n] = 5.f;
             c.vx[n] = 0.f; c.vy[n] = 0.f; c.vz[n] = 0.f;
         }
