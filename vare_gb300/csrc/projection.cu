@@ -13,76 +13,23 @@
 #include <algorithm>
 
 #include "bora_internal.h"
+#include "half_rows.cuh"
 #include "reduce.cuh"
 
 namespace {
 
-__device__ inline void tile_coords( const BoraGridDev& g, int vt, int& ti, int& tj, int& tk )
-{
-    ti = vt % g.tx;
-    tj = ( vt / g.tx ) % g.ty;
-    tk = vt / ( g.tx * g.ty );
-}
-
 __device__ inline float absr( float x ) { return x < 0.f ? -x : x; }  // MathUtils.h:129 Abs
 
 // ---------------------------------------------------------------------------------
-// Stencils over the active tiles outside the solve: one warp per half tile (z layers 0..3 or
-// 4..7), a lane per x-row (lane = j + 8 (k mod 4)), as the solve's kernels walk theirs. Cells of
-// inactive tiles and beyond the grid read as air and zero.
-constexpr int kRowWarps = 4;  // half tiles per CTA
-
-struct HalfRow
-{
-    bool mine;              // past the last half tile: nothing is stored, every neighbour is inactive
-    int s, hi;              // the tile's slot; the half
-    int xm, xp, yt, zt;     // slots at the row's x ends; of the rows that no other lane holds (-1: none)
-    int c, yc, zc;          // cells of the row, and of those rows, in their tiles
-    int j, kk;              // the lane's row in the half
-    int i0, J, K;           // the row's first cell in the grid
-    __device__ size_t at() const { return (size_t)s * BORA_TILE_CELLS + c; }
-};
-
-__device__ __forceinline__ HalfRow half_row( const BoraGridDev& g, const BoraTilesDev& t, int ntiles )
-{
-    HalfRow r;
-    const int lane = threadIdx.x & 31, h = (int)blockIdx.x * kRowWarps + (int)( threadIdx.x >> 5 );
-    r.mine = h < 2 * ntiles;
-    r.s = r.mine ? h >> 1 : 0;
-    r.hi = h & 1;
-    r.j = lane & 7;
-    r.kk = lane >> 3;
-    r.c = r.hi * 256 + 8 * lane;
-    const int32_t* nb = t.nbr + (size_t)r.s * 27;
-    auto slot = [&]( int d ) { return r.mine ? __ldg( nb + d ) : -1; };
-    r.xm = slot( bora_dir( -1, 0, 0 ) );
-    r.xp = slot( bora_dir( 1, 0, 0 ) );
-    const int ym = slot( bora_dir( 0, -1, 0 ) ), yp = slot( bora_dir( 0, 1, 0 ) ), z = slot( bora_dir( 0, 0, r.hi ? 1 : -1 ) );
-    const int own = r.mine ? r.s : -1;
-    r.yt = r.j == 0 ? ym : ( r.j == 7 ? yp : -1 );
-    r.yc = r.c + ( r.j == 0 ? 56 : -56 );
-    r.zt = r.kk == 0 ? ( r.hi ? own : z ) : ( r.kk == 3 ? ( r.hi ? z : own ) : -1 );
-    r.zc = 8 * r.j + ( r.kk == 0 ? ( r.hi ? 192 : 448 ) : ( r.hi ? 0 : 256 ) );
-    int ti, tj, tk;
-    tile_coords( g, t.tile_of[r.s], ti, tj, tk );
-    r.i0 = ti * BORA_TILE;
-    r.J = tj * BORA_TILE + r.j;
-    r.K = tk * BORA_TILE + 4 * r.hi + r.kk;
-    return r;
-}
+// The row stencils (half_rows.cuh) of the right-hand side and the velocity update.
+// Half tiles per CTA: 4 (right-hand side and code 153.6 us, velocity 44.2 at 256^3; 160.4 and 52.1 with 8)
+constexpr int kRowWarps = 4;
 
 __device__ __forceinline__ uint2 flags8( const uint8_t* __restrict__ flag, int t, int c )
 {
     return t < 0 ? make_uint2( 0u, 0u ) : *reinterpret_cast<const uint2*>( flag + (size_t)t * BORA_TILE_CELLS + c );  // BORA_AIR is 0
 }
 __device__ __forceinline__ int flag_of( uint2 w, int i ) { return (int)( ( ( i < 4 ? w.x : w.y ) >> ( 8 * ( i & 3 ) ) ) & 255u ); }
-
-__device__ __forceinline__ void row8( const float* __restrict__ f, int t, int c, float* v )
-{
-#pragma unroll
-    for( int i = 0; i < 8; ++i ) v[i] = 0.f;
-    if( t >= 0 ) bora_ld8( f + (size_t)t * BORA_TILE_CELLS + c, v );
-}
 
 __device__ __forceinline__ uint2 shfl2( uint2 w, int lane )
 {
@@ -110,19 +57,6 @@ struct RowFlags
     }
 };
 
-// the values of a field next to a row in y or z: from the other lanes, or the loaded row
-__device__ __forceinline__ void beside( const float* v, const float* halo, int step, bool first, bool last, float* m, float* p )
-{
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for( int i = 0; i < 8; ++i )
-    {
-        const float a = __shfl_sync( 0xffffffffu, v[i], lane - step ), b = __shfl_sync( 0xffffffffu, v[i], lane + step );
-        m[i] = first ? halo[i] : a;
-        p[i] = last ? halo[i] : b;
-    }
-}
-
 // ---------------------------------------------------------------------------------
 // Right-hand side and stencil code (FluidProjection.cu:203-266). (With a cell per thread from a
 // staged 10^3 region it was bound by index arithmetic: 84 us at 256^3, 35 now.)
@@ -130,7 +64,7 @@ __global__ void __launch_bounds__( 32 * kRowWarps ) k_rhs( BoraGridDev g, BoraTi
                                                            uint32_t* nfluid, uint8_t* __restrict__ tile_fluid )
 {
     __shared__ int any[kRowWarps];
-    const HalfRow r = half_row( g, t, ntiles );
+    const HalfRow r = half_row<kRowWarps>( g, t, ntiles );
     RowFlags f;
     f.load( c.flag, r );
     const int own = r.mine ? r.s : -1;
@@ -1501,7 +1435,7 @@ struct AirMean
 
 __global__ void __launch_bounds__( 32 * kRowWarps ) k_air_pressure( BoraGridDev g, BoraTilesDev t, int ntiles, BoraCellsDev c )
 {
-    const HalfRow r = half_row( g, t, ntiles );
+    const HalfRow r = half_row<kRowWarps>( g, t, ntiles );
     RowFlags f;
     f.load( c.flag, r );
     constexpr uint32_t kAllFluid = 0x01010101u * BORA_FLUID;
@@ -1558,7 +1492,7 @@ __device__ __noinline__ float air_pressure_at( const BoraGridDev* g, const int32
 __global__ void __launch_bounds__( 32 * kRowWarps ) k_vel_update( const __grid_constant__ BoraGridDev g, BoraTilesDev t, int ntiles,
                                                                   BoraCellsDev c )
 {
-    const HalfRow r = half_row( g, t, ntiles );
+    const HalfRow r = half_row<kRowWarps>( g, t, ntiles );
     RowFlags f;
     f.load( c.flag, r );
     const int own = r.mine ? r.s : -1;
@@ -1621,8 +1555,6 @@ __global__ void __launch_bounds__( 32 * kRowWarps ) k_vel_update( const __grid_c
     bora_st8( c.cz + r.at(), vz );
 }
 
-int row_grid( int ntiles ) { return ( 2 * ntiles + kRowWarps - 1 ) / kRowWarps; }
-
 int grid_for( size_t n, int threads )
 {
     const size_t b = ( n + threads - 1 ) / threads;
@@ -1634,7 +1566,7 @@ int grid_for( size_t n, int threads )
 void bora_launch_rhs( const BoraGridDev& g, int ntiles, BoraTilesDev t, BoraCellsDev c, uint32_t* nfluid, uint8_t* tile_fluid,
                       cudaStream_t st )
 {
-    if( ntiles > 0 ) k_rhs<<<row_grid( ntiles ), 32 * kRowWarps, 0, st>>>( g, t, ntiles, c, nfluid, tile_fluid );
+    if( ntiles > 0 ) k_rhs<<<row_grid( ntiles, kRowWarps ), 32 * kRowWarps, 0, st>>>( g, t, ntiles, c, nfluid, tile_fluid );
 }
 
 void bora_launch_tile_fluid( int ntiles, const uint16_t* code, uint8_t* tile_fluid, cudaStream_t st )
@@ -1659,8 +1591,8 @@ void bora_launch_solve_tiles( int ntiles, BoraTilesDev t, const uint8_t* tile_fl
 void bora_launch_vel_update( const BoraGridDev& g, int ntiles, BoraTilesDev t, BoraCellsDev c, cudaStream_t st )
 {
     if( ntiles <= 0 ) return;
-    k_air_pressure<<<row_grid( ntiles ), 32 * kRowWarps, 0, st>>>( g, t, ntiles, c );
-    k_vel_update<<<row_grid( ntiles ), 32 * kRowWarps, 0, st>>>( g, t, ntiles, c );
+    k_air_pressure<<<row_grid( ntiles, kRowWarps ), 32 * kRowWarps, 0, st>>>( g, t, ntiles, c );
+    k_vel_update<<<row_grid( ntiles, kRowWarps ), 32 * kRowWarps, 0, st>>>( g, t, ntiles, c );
 }
 
 void bora_launch_mic_factor( int ntiles, BoraSolveTilesDev t, const uint16_t* code, float* minv, cudaStream_t st )

@@ -9,6 +9,7 @@
 // that lie beyond the grid are never read by a cell inside it (faces use the mirrored or
 // tank rule), so they are left alone.
 #include "bora_internal.h"
+#include "half_rows.cuh"
 
 namespace {
 
@@ -16,13 +17,6 @@ namespace {
 // redistancing update).
 __device__ inline float maxr( float a, float b ) { return a > b ? a : b; }
 __device__ inline float minr( float a, float b ) { return a < b ? a : b; }
-
-__device__ inline void tile_coords( const BoraGridDev& g, int vt, int& ti, int& tj, int& tk )
-{
-    ti = vt % g.tx;
-    tj = ( vt / g.tx ) % g.ty;
-    tk = vt / ( g.tx * g.ty );
-}
 
 // ======================================================================================
 // Rasterization::ParticlesToSurfaceAndVelocity (base/source/Rasterization.cu:311-398),
@@ -463,129 +457,100 @@ __device__ inline size_t halo_index( const int32_t* nb, int h )  // storage inde
 // (base/source/Rasterization.cu:400-486) at a cell with value v and neighbours
 // (i0, i1, j0, j1, k0, k1): phi_t = sign(phi)(1 - |grad phi|), dt 0.3,
 // sign = phi / sqrt(phi^2 + 1). Of the reference's two terms
-// dt max(sign,0)(sqrt(a) - 1) and dt min(sign,0)(sqrt(b) - 1) one has a zero factor; its
-// value is the signed zero (+0) * (sqrt(x) - 1), whose sign is that of x - 1, so only the
-// other square root is taken.
-__device__ inline float godunov_step( float v, float vi0, float vi1, float vj0, float vj1, float vk0, float vk1 )
+// dt max(sign,0)(sqrt(a) - 1) and dt min(sign,0)(sqrt(b) - 1) one has a zero factor and is a
+// signed zero, which changes no other value than -0. a sums max(v - i0, 0)^2 + min(i1 - v, 0)^2
+// over the axes and b the other sides; with the differences' signs flipped for negative phi one
+// expression serves both, since the squares do not see it.
+__device__ __forceinline__ float godunov_step( float v, float vi0, float vi1, float vj0, float vj1, float vk0, float vk1 )
 {
-    const float dx0 = v - vi0, dx1 = vi1 - v, dy0 = v - vj0, dy1 = vj1 - v, dz0 = v - vk0, dz1 = vk1 - v;
+    const uint32_t flip = __float_as_uint( v ) & 0x80000000u;
+    auto up = [&]( float d ) {
+        const float m = fmaxf( __uint_as_float( __float_as_uint( d ) ^ flip ), 0.f );
+        return m * m;
+    };
+    // -(i1 - v) = v - i1 exactly
+    float q = up( v - vi0 );
+    q = q + up( v - vi1 );
+    q = q + up( v - vj0 );
+    q = q + up( v - vj1 );
+    q = q + up( v - vk0 );
+    q = q + up( v - vk1 );
     const float sign = v / sqrtf( v * v + 1.f );
-    const float dt = 0.3f;
-    const float ps = maxr( sign, 0.f ), ns = minr( sign, 0.f );
-    float a = maxr( dx0, 0.f ) * maxr( dx0, 0.f );
-    a = a + minr( dx1, 0.f ) * minr( dx1, 0.f );
-    a = a + maxr( dy0, 0.f ) * maxr( dy0, 0.f );
-    a = a + minr( dy1, 0.f ) * minr( dy1, 0.f );
-    a = a + maxr( dz0, 0.f ) * maxr( dz0, 0.f );
-    a = a + minr( dz1, 0.f ) * minr( dz1, 0.f );
-    float b = minr( dx0, 0.f ) * minr( dx0, 0.f );
-    b = b + maxr( dx1, 0.f ) * maxr( dx1, 0.f );
-    b = b + minr( dy0, 0.f ) * minr( dy0, 0.f );
-    b = b + maxr( dy1, 0.f ) * maxr( dy1, 0.f );
-    b = b + minr( dz0, 0.f ) * minr( dz0, 0.f );
-    b = b + maxr( dz1, 0.f ) * maxr( dz1, 0.f );
-    const float zp = a < 1.f ? -0.f : 0.f, zn = b < 1.f ? -0.f : 0.f;
-    const bool pos = ps != 0.f;  // sign > 0: the first term is live
-    const bool neg = ns != 0.f;  // sign < 0: the second
-    const float t1 = pos ? dt * ps * ( sqrtf( a ) - 1.f ) : zp;
-    const float t2 = neg ? dt * ns * ( sqrtf( b ) - 1.f ) : zn;
-    return ( v - t1 ) - t2;
+    const float res = v - ( 0.3f * sign ) * ( sqrtf( q ) - 1.f );
+    if( sign > 0.f || sign < 0.f ) return res;
+    // v = 0, or so large that its sign is 0 or NaN: (v - t1) - t2 with both terms signed zeros,
+    // (+0) (sqrt(x) - 1) for x = a, b
+    const float di0 = v - vi0, di1 = vi1 - v, dj0 = v - vj0, dj1 = vj1 - v, dk0 = v - vk0, dk1 = vk1 - v;
+    float a = maxr( di0, 0.f ) * maxr( di0, 0.f );
+    a = a + minr( di1, 0.f ) * minr( di1, 0.f );
+    a = a + maxr( dj0, 0.f ) * maxr( dj0, 0.f );
+    a = a + minr( dj1, 0.f ) * minr( dj1, 0.f );
+    a = a + maxr( dk0, 0.f ) * maxr( dk0, 0.f );
+    a = a + minr( dk1, 0.f ) * minr( dk1, 0.f );
+    float b = minr( di0, 0.f ) * minr( di0, 0.f );
+    b = b + maxr( di1, 0.f ) * maxr( di1, 0.f );
+    b = b + minr( dj0, 0.f ) * minr( dj0, 0.f );
+    b = b + maxr( dj1, 0.f ) * maxr( dj1, 0.f );
+    b = b + minr( dk0, 0.f ) * minr( dk0, 0.f );
+    b = b + maxr( dk1, 0.f ) * maxr( dk1, 0.f );
+    return ( v - ( a < 1.f ? -0.f : 0.f ) ) - ( b < 1.f ? -0.f : 0.f );
 }
 
-// Redistancing, one step over all tiles: a persistent grid walks the tiles; each tile's
-// 10^3 region (the tile and a one-cell halo, background 10 for inactive tiles) is read
-// into registers one tile ahead, so the loads of the next tile overlap the arithmetic of
-// the current one.
-constexpr int kRedistThreads = 512;
+// Redistancing, one step over all tiles: a warp per half tile and a lane per x-row
+// (half_rows.cuh; background 10 for inactive tiles). Bound by the step's arithmetic (two square
+// roots and a division a cell); with a tile per CTA staged cell by cell and both of the
+// reference's sums formed, a step at 256^3 (7.9 K tiles) took 33 us, 17 now.
+constexpr int kRedistWarps = 8;  // half tiles per CTA (16.9 us; 17.5 with 4 or 2)
 
 template <bool TANK>
-__global__ void __launch_bounds__( kRedistThreads ) k_redistance( const __grid_constant__ BoraGridDev g, BoraTilesDev t,
+__global__ void __launch_bounds__( 32 * kRedistWarps ) k_redistance( const __grid_constant__ BoraGridDev g, BoraTilesDev t,
                                                                    int ntiles, const float* __restrict__ in,
                                                                    float* __restrict__ out )
 {
-    __shared__ float r[kQN];
-    __shared__ int32_t nbb[2][27];
-    __shared__ int tcb[2][3];  // tile coordinates, double-buffered like the neighbour tables
-    const int tid = threadIdx.x, G = gridDim.x;
     bora_pdl_trigger();
-    if( tid < 27 )
-    {
-        nbb[0][tid] = blockIdx.x < ntiles ? t.nbr[(size_t)blockIdx.x * 27 + tid] : -1;
-        nbb[1][tid] = blockIdx.x + G < ntiles ? t.nbr[(size_t)( blockIdx.x + G ) * 27 + tid] : -1;
-    }
-    else if( tid == 32 || tid == 33 )
-    {
-        const int q = tid - 32, sq = blockIdx.x + q * G;
-        if( sq < ntiles ) tile_coords( g, t.tile_of[sq], tcb[q][0], tcb[q][1], tcb[q][2] );
-    }
-    __syncthreads();
+    const HalfRow r = half_row<kRedistWarps>( g, t, ntiles );
     bora_pdl_wait();  // `in` is the previous step's output
-    // this thread's two region cells: tile direction and local index, the same for every tile
-    int rdir[2], rloc[2];
-    for( int u = 0; u < 2; ++u )
-    {
-        const int hh = tid + u * kRedistThreads;
-        const int a = hh % kQ, b = ( hh / kQ ) % kQ, c = hh / ( kQ * kQ );
-        rdir[u] = hh < kQN ? bora_dir( a == 0 ? -1 : ( a == 9 ? 1 : 0 ), b == 0 ? -1 : ( b == 9 ? 1 : 0 ),
-                                       c == 0 ? -1 : ( c == 9 ? 1 : 0 ) )
-                           : -1;
-        rloc[u] = bora_local( a + 7, b + 7, c + 7 );
-    }
-    float pf[2];
-    auto issue = [&]( const int32_t* nb ) {
-        for( int u = 0; u < 2; ++u )
-        {
-            const int ns = rdir[u] >= 0 ? nb[rdir[u]] : -1;
-            pf[u] = ns >= 0 ? in[(size_t)ns * BORA_TILE_CELLS + rloc[u]] : 10.f;
-        }
-    };
-    issue( nbb[0] );
-    const int li = tid & 7, lj = ( tid >> 3 ) & 7, lk = tid >> 6;
-    const int h = ( li + 1 ) + kQ * ( ( lj + 1 ) + kQ * ( lk + 1 ) );
+    const int own = r.mine ? r.s : -1;
+    float v[8], ym[8], yp[8], zm[8], zp[8], yh[8], zh[8];
+    row8( in, own, r.c, v, 10.f );
+    row8( in, r.yt, r.yc, yh, 10.f );
+    row8( in, r.zt, r.zc, zh, 10.f );
+    const float xm = r.xm < 0 ? 10.f : in[(size_t)r.xm * BORA_TILE_CELLS + r.c + 7];
+    const float xp = r.xp < 0 ? 10.f : in[(size_t)r.xp * BORA_TILE_CELLS + r.c];
+    beside( v, yh, 1, r.j == 0, r.j == 7, ym, yp );
+    beside( v, zh, 8, r.kk == 0, r.kk == 3, zm, zp );
     const int I = g.nx - 1, J = g.ny - 1, K = g.nz - 1;
-    int n = 0;
-    for( int s = blockIdx.x; s < ntiles; s += G, ++n )
+    const bool row_in = r.J <= J && r.K <= K;
+    float res[8];
+#pragma unroll
+    for( int q = 0; q < 8; ++q )
     {
-        for( int u = 0; u < 2; ++u )
-            if( tid + u * kRedistThreads < kQN ) r[tid + u * kRedistThreads] = pf[u];
-        const int32_t nb2 = tid < 27 && s + 2 * G < ntiles ? t.nbr[(size_t)( s + 2 * G ) * 27 + tid] : -1;
-        int tc2[3] = { 0, 0, 0 };
-        if( tid == 32 && s + 2 * G < ntiles ) tile_coords( g, t.tile_of[s + 2 * G], tc2[0], tc2[1], tc2[2] );
-        __syncthreads();
-        if( s + G < ntiles ) issue( nbb[( n + 1 ) & 1] );
-        const int ti = tcb[n & 1][0], tj = tcb[n & 1][1], tk = tcb[n & 1][2];
-        const int i = ti * BORA_TILE + li, j = tj * BORA_TILE + lj, k = tk * BORA_TILE + lk;
-        const float v = r[h];
-        float res = v;
-        if( i < g.nx && j < g.ny && k < g.nz )
+        const int i = r.i0 + q;
+        const float x0 = q ? v[q ? q - 1 : 0] : xm, x1 = q < 7 ? v[q < 7 ? q + 1 : 7] : xp;
+        float vi0, vi1, vj0, vj1, vk0, vk1;
+        if( TANK )
         {
-            float vi0, vi1, vj0, vj1, vk0, vk1;
-            if( TANK )
-            {
-                const float ll = ( (float)j + .5f ) - g.voxel_wall;
-                vj0 = j == 0 ? ll - 1.f : r[h - kQ];
-                vj1 = j == J ? ll + 1.f : r[h + kQ];
-                vi0 = i == 0 ? ll : r[h - 1];
-                vi1 = i == I ? ll : r[h + 1];
-                vk0 = k == 0 ? ll : r[h - kQ * kQ];
-                vk1 = k == K ? ll : r[h + kQ * kQ];
-            }
-            else
-            {
-                vi0 = i == 0 ? 2.f * v - r[h + 1] : r[h - 1];
-                vi1 = i == I ? 2.f * v - r[h - 1] : r[h + 1];
-                vj0 = j == 0 ? 2.f * v - r[h + kQ] : r[h - kQ];
-                vj1 = j == J ? 2.f * v - r[h - kQ] : r[h + kQ];
-                vk0 = k == 0 ? 2.f * v - r[h + kQ * kQ] : r[h - kQ * kQ];
-                vk1 = k == K ? 2.f * v - r[h - kQ * kQ] : r[h + kQ * kQ];
-            }
-            res = godunov_step( v, vi0, vi1, vj0, vj1, vk0, vk1 );
+            const float ll = ( (float)r.J + .5f ) - g.voxel_wall;
+            vj0 = r.J == 0 ? ll - 1.f : ym[q];
+            vj1 = r.J == J ? ll + 1.f : yp[q];
+            vi0 = i == 0 ? ll : x0;
+            vi1 = i == I ? ll : x1;
+            vk0 = r.K == 0 ? ll : zm[q];
+            vk1 = r.K == K ? ll : zp[q];
         }
-        out[(size_t)s * BORA_TILE_CELLS + tid] = res;
-        __syncthreads();  // tile s's tables and region are no longer read
-        if( tid < 27 ) nbb[n & 1][tid] = nb2;
-        if( tid == 32 ) { tcb[n & 1][0] = tc2[0]; tcb[n & 1][1] = tc2[1]; tcb[n & 1][2] = tc2[2]; }
+        else
+        {
+            vi0 = i == 0 ? 2.f * v[q] - x1 : x0;
+            vi1 = i == I ? 2.f * v[q] - x0 : x1;
+            vj0 = r.J == 0 ? 2.f * v[q] - yp[q] : ym[q];
+            vj1 = r.J == J ? 2.f * v[q] - ym[q] : yp[q];
+            vk0 = r.K == 0 ? 2.f * v[q] - zp[q] : zm[q];
+            vk1 = r.K == K ? 2.f * v[q] - zm[q] : zp[q];
+        }
+        const float step = godunov_step( v[q], vi0, vi1, vj0, vj1, vk0, vk1 );
+        res[q] = row_in && i <= I ? step : v[q];
     }
+    if( r.mine ) bora_st8( out + r.at(), res );
 }
 
 // FieldOP::curl of the splatted velocity (base/source/FieldOP.cu:338-369; background 0)
@@ -771,28 +736,14 @@ int bora_tank_scan_launches( const BoraGridDev& g, int ntiles, BoraTilesDev t, f
     return 6;
 }
 
-template <bool TANK>
-int redistance_grid( int ntiles )
-{
-    static BoraPerDevice per_sm;
-    const int b = per_sm.get( [] {
-        int v = 0;
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor( &v, k_redistance<TANK>, kRedistThreads, 0 ) == cudaSuccess && v > 0 ? v : 1;
-    } );
-    int dev = 0, sms = 0;
-    cudaGetDevice( &dev );
-    cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
-    return std::max( 1, std::min( ntiles, b * std::max( sms, 1 ) ) );
-}
-
 cudaError_t bora_launch_redistance( const BoraGridDev& g, int ntiles, BoraTilesDev t, const float* in, float* out,
                                     cudaStream_t st )
 {
     if( ntiles <= 0 ) return cudaSuccess;
     if( g.enable_tank )
-        return bora_launch_pdl( k_redistance<true>, dim3( redistance_grid<true>( ntiles ) ), dim3( kRedistThreads ), 0, st,
+        return bora_launch_pdl( k_redistance<true>, dim3( row_grid( ntiles, kRedistWarps ) ), dim3( 32 * kRedistWarps ), 0, st,
                                 g, t, ntiles, in, out );
-    return bora_launch_pdl( k_redistance<false>, dim3( redistance_grid<false>( ntiles ) ), dim3( kRedistThreads ), 0, st,
+    return bora_launch_pdl( k_redistance<false>, dim3( row_grid( ntiles, kRedistWarps ) ), dim3( 32 * kRedistWarps ), 0, st,
                             g, t, ntiles, in, out );
 }
 
