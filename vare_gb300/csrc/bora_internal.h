@@ -362,10 +362,10 @@ struct BoraTuneTimer
 // Fold the timings of completed launches into the table (call after a stream synchronize).
 void bora_tune_resolve();
 
-// Cell types and stencil codes of level c from level c-1 (levels[0] = fine, given).
-// mid_image: the buffer for the coarse levels' cluster image (bora_mg_mid_image_bytes), or null
-void bora_mg_setup( const BoraGridDev& g, BoraLevelDev* levels, int nlevels, BoraTilesDev t, void* mid_image,
-                    uint32_t* err, cudaStream_t st );
+// Cell types and stencil codes of levels 1 .. nlevels - 1 (levels[0] = fine, given; at most 16).
+// mid_image: the buffer for the coarse levels' cluster image (bora_mg_mid_image_bytes), or null.
+// Returns its kernel launches.
+int bora_mg_setup( const BoraGridDev& g, BoraLevelDev* levels, int nlevels, BoraTilesDev t, void* mid_image, cudaStream_t st );
 // One preconditioned PCG update: r -= alpha q (alpha = rz / dq of slots slot_rz_in and slot_dq_in,
 // none when slot_rz_in < 0), then one V-cycle z = M^-1 r (FP32 in and out, FP16 inside, scaled by
 // 1 / sqrt(ring[slot_scale])); partial sums of r.r and r.z, bora_mg_pass_grid( 8, ntiles, -1 ) blocks each.

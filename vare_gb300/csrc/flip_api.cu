@@ -651,9 +651,8 @@ int stage_build_system( bora_flip_sim* s )
     if( s->prm.solver == BORA_SOLVER_MIXED )
     {
         BORA_TRYS( build_hierarchy( s ) );
-        s->stats.kernel_launches += 2 * (uint64_t)( s->nlevels - 1 ) + ( s->mg_mid_on ? 1 : 0 );
-        bora_mg_setup( s->g, s->levels, s->nlevels, s->tiles(), s->mg_mid_on ? s->mg_mid.p : nullptr,
-                       P<uint32_t>( s->counters ) + 5, s->st );
+        s->stats.kernel_launches += (uint64_t)bora_mg_setup( s->g, s->levels, s->nlevels, s->tiles(),
+                                                             s->mg_mid_on ? s->mg_mid.p : nullptr, s->st );
     }
     else
     {

@@ -44,139 +44,239 @@ constexpr float kOmegaB = 1.6902f;  // 1 / (1.175 - 0.825 cos(pi/4))
 
 __device__ inline int code_diag( uint16_t c ) { return ( c >> 8 ) & 15; }
 
-// Index of the face neighbour q (0:-x 1:+x 2:-y 3:+y 4:-z 5:+z) of a cell on level L,
-// or -1 when it lies in an inactive tile / beyond the stored grid.
-struct LevelNav
+// ---- set-up: cell types and stencil codes of coarse levels ---------------------------
+//
+// A coarse cell is air when one of its children is, else fluid when one is, else solid; beyond
+// the domain it is masked. Children beyond the finer level's domain count as none (wall-like).
+// Three launches: the tiled levels' types, the dense levels' types, all levels' codes (with two
+// launches a level and a cell per thread the set-up was 8 to 14 launches. With the right-hand side
+// and the solver's tile table: 83 -> 50 us at 96^3, 155 -> 101 at 256^3, 237 -> 140 in a 640 tank.)
+constexpr size_t kDenseOneCta = 16384;  // dense cells up to which one CTA forms a level's types
+
+struct SetupLevels
 {
-    BoraLevelDev L;
-    const int32_t* nbr;      // tile neighbour table (tiled levels)
-    const int32_t* tile_of;  // slot -> virtual tile (tiled levels)
-    int tx, ty;              // tile grid (tiled levels)
-
-    __device__ inline void coords( long long cell, int& i, int& j, int& k ) const
-    {
-        if( L.kind == 1 )
-        {
-            i = (int)( cell % L.dx );
-            j = (int)( ( cell / L.dx ) % L.dy );
-            k = (int)( cell / ( (long long)L.dx * L.dy ) );
-            return;
-        }
-        const int E = L.E, E3 = E * E * E;
-        const int s = (int)( cell / E3 ), loc = (int)( cell % E3 );
-        const int vt = tile_of[s];
-        i = ( vt % tx ) * E + loc % E;
-        j = ( ( vt / tx ) % ty ) * E + ( loc / E ) % E;
-        k = ( vt / ( tx * ty ) ) * E + loc / ( E * E );
-    }
-    __device__ inline bool real( int i, int j, int k ) const { return i < L.nx && j < L.ny && k < L.nz; }
-
-    // neighbour cell index, -1 inactive/outside storage; *edge = true beyond the domain
-    __device__ inline long long nbr_index( long long cell, int i, int j, int k, int q, bool* edge ) const
-    {
-        const int di = q == 0 ? -1 : ( q == 1 ? 1 : 0 );
-        const int dj = q == 2 ? -1 : ( q == 3 ? 1 : 0 );
-        const int dk = q == 4 ? -1 : ( q == 5 ? 1 : 0 );
-        const int a = i + di, b = j + dj, c = k + dk;
-        *edge = ( a < 0 || b < 0 || c < 0 || a >= L.nx || b >= L.ny || c >= L.nz );
-        if( *edge ) return -1;
-        if( L.kind == 1 ) return (long long)a + (long long)L.dx * ( b + (long long)L.dy * c );
-        const int E = L.E, E3 = E * E * E;
-        const int s = (int)( cell / E3 );
-        const int la = ( ( i % E ) + di ), lb = ( ( j % E ) + dj ), lc = ( ( k % E ) + dk );
-        if( la >= 0 && la < E && lb >= 0 && lb < E && lc >= 0 && lc < E )
-            return (long long)s * E3 + la + E * ( lb + E * lc );
-        const int ox = la < 0 ? -1 : ( la >= E ? 1 : 0 );
-        const int oy = lb < 0 ? -1 : ( lb >= E ? 1 : 0 );
-        const int oz = lc < 0 ? -1 : ( lc >= E ? 1 : 0 );
-        const int ns = nbr[(size_t)s * 27 + bora_dir( ox, oy, oz )];
-        if( ns < 0 ) return -1;
-        const int wa = ( la + E ) % E, wb = ( lb + E ) % E, wc = ( lc + E ) % E;
-        return (long long)ns * E3 + wa + E * ( wb + E * wc );
-    }
+    BoraLevelDev L[16];
+    int n;
+    const int32_t* nbr;
+    const int32_t* slot_of;
+    const int32_t* tile_of;
+    int tx, ty, tz;
+    float voxel_wall;
 };
 
-// ---- set-up: cell types and stencil codes of coarse levels ---------------------------
+__device__ __forceinline__ int coarse_type( bool air, bool fluid ) { return air ? BORA_AIR : ( fluid ? BORA_FLUID : BORA_SOLID ); }
 
-// Types of level `C` from level `F` (one finer). C tiled with E_C = E_F / 2 (children in
-// the same tile), or C dense: children are the finer level's cells (dense) or tiles
-// (F tiled with E = 1, through slot_of).
-__global__ void k_mg_types( BoraLevelDev F, BoraLevelDev C, const int32_t* __restrict__ slot_of,
-                            const int32_t* __restrict__ tile_of, int tx, int ty, int tz )
+// Types of levels 1, 2, 3 (4^3, 2^3, 1 cells per tile), 16 lanes per tile: a lane owns the four
+// level-1 cells of a row (y, z), lane = y + 4 z.
+__global__ void __launch_bounds__( 256 ) k_mg_types_tiled( const __grid_constant__ SetupLevels d, int ntiles )
 {
-    for( long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < (long long)C.ncells;
-         cell += (long long)gridDim.x * blockDim.x )
+    const int s0 = (int)( ( blockIdx.x * (size_t)blockDim.x + threadIdx.x ) >> 4 ), s = min( s0, ntiles - 1 );
+    const bool mine = s0 < ntiles;
+    const int y = threadIdx.x & 3, z = ( threadIdx.x >> 2 ) & 3;
+    const int vt = d.tile_of[s];
+    const int ti = vt % d.tx, tj = ( vt / d.tx ) % d.ty, tk = vt / ( d.tx * d.ty );
+    const BoraLevelDev& F = d.L[0];
+    uint32_t air = 0, fluid = 0;  // bit x: a child of cell x is air / fluid
+#pragma unroll
+    for( int o = 0; o < 4; ++o )
     {
-        int i, j, k;
-        if( C.kind == 1 )
+        const int b = 2 * y + ( o & 1 ), c = 2 * z + ( o >> 1 );
+        if( tj * 8 + b >= F.ny || tk * 8 + c >= F.nz ) continue;
+        const uint2 w = *reinterpret_cast<const uint2*>( F.type + (size_t)s * 512 + 8 * b + 64 * c );
+#pragma unroll
+        for( int a = 0; a < 8; ++a )
         {
-            i = (int)( cell % C.dx ); j = (int)( ( cell / C.dx ) % C.dy ); k = (int)( cell / ( (long long)C.dx * C.dy ) );
+            const int t = (int)( ( ( a < 4 ? w.x : w.y ) >> ( 8 * ( a & 3 ) ) ) & 255u );
+            if( ti * 8 + a >= F.nx ) continue;
+            if( t == BORA_AIR ) air |= 1u << ( a >> 1 );
+            else if( t == BORA_FLUID ) fluid |= 1u << ( a >> 1 );
         }
-        else
+    }
+    int n = 4;  // the level's cells along the row and per tile edge
+#pragma unroll
+    for( int l = 1; l <= 3; ++l )
+    {
+        if( l >= d.n || d.L[l].kind != 0 ) return;
+        const BoraLevelDev& C = d.L[l];
+        const int step = 1 << ( l - 1 ), yy = y / step, zz = z / step;
+        uint32_t types = 0, na = 0, nf = 0;
+        for( int x = 0; x < n; ++x )
         {
-            const int E = C.E, E3 = E * E * E;
-            const int s = (int)( cell / E3 ), loc = (int)( cell % E3 );
-            const int vt = tile_of[s];
-            i = ( vt % tx ) * E + loc % E;
-            j = ( ( vt / tx ) % ty ) * E + ( loc / E ) % E;
-            k = ( vt / ( tx * ty ) ) * E + loc / ( E * E );
+            const bool real = ti * n + x < C.nx && tj * n + yy < C.ny && tk * n + zz < C.nz;
+            const int t = real ? coarse_type( ( air >> x ) & 1u, ( fluid >> x ) & 1u ) : BORA_MASKED;
+            types |= (uint32_t)t << ( 8 * x );
+            if( t == BORA_AIR ) na |= 1u << ( x >> 1 );
+            else if( t == BORA_FLUID ) nf |= 1u << ( x >> 1 );
         }
-        if( i >= C.nx || j >= C.ny || k >= C.nz ) { C.type[cell] = BORA_MASKED; continue; }
-        bool anyF = false, anyA = false;
-        for( int o = 0; o < 8; ++o )
+        if( mine && !( y & ( step - 1 ) ) && !( z & ( step - 1 ) ) )
         {
-            const int a = 2 * i + ( o & 1 ), b = 2 * j + ( ( o >> 1 ) & 1 ), c = 2 * k + ( o >> 2 );
-            if( a >= F.nx || b >= F.ny || c >= F.nz ) continue;  // beyond the finer grid: wall-like
-            uint8_t t;
-            if( C.kind == 0 )
-            {
-                const int E = F.E;
-                const int s = (int)( cell / ( C.E * C.E * C.E ) );
-                t = F.type[(long long)s * E * E * E + ( a % E ) + E * ( ( b % E ) + E * ( c % E ) )];
-            }
-            else if( F.kind == 1 )
-            {
-                t = F.type[(long long)a + (long long)F.dx * ( b + (long long)F.dy * c )];
-            }
-            else  // F tiled with one cell per tile: children are tiles
-            {
-                if( a >= tx || b >= ty || c >= tz ) continue;
-                const int s = slot_of[( (size_t)c * ty + b ) * tx + a];
-                t = s < 0 ? (uint8_t)BORA_AIR : F.type[s];
-            }
-            if( t == BORA_FLUID ) anyF = true;
-            else if( t == BORA_AIR ) anyA = true;
+            uint8_t* out = C.type + (size_t)s * ( n * n * n ) + n * ( yy + n * zz );
+            if( n == 4 ) *reinterpret_cast<uint32_t*>( out ) = types;
+            else if( n == 2 ) *reinterpret_cast<uint16_t*>( out ) = (uint16_t)types;
+            else *out = (uint8_t)types;
         }
-        C.type[cell] = anyA ? BORA_AIR : ( anyF ? BORA_FLUID : BORA_SOLID );
+        // the next level's children: the cells of the row and of the rows y, z + step
+        air = na;
+        fluid = nf;
+        air |= __shfl_xor_sync( 0xffffffffu, air, step );
+        fluid |= __shfl_xor_sync( 0xffffffffu, fluid, step );
+        air |= __shfl_xor_sync( 0xffffffffu, air, 4 * step );
+        fluid |= __shfl_xor_sync( 0xffffffffu, fluid, 4 * step );
+        n >>= 1;
     }
 }
 
-// Stencil codes of level L from its types (same bit layout as the fine code).
-__global__ void k_mg_codes( LevelNav nav, float voxel_wall )
+// Type of cell `cell` of dense level l from the finer level (dense, or level 3: tiles).
+__device__ __forceinline__ void dense_type( const SetupLevels& d, int l, long long cell )
 {
-    const BoraLevelDev& L = nav.L;
-    for( long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < (long long)L.ncells;
-         cell += (long long)gridDim.x * blockDim.x )
+    const BoraLevelDev &C = d.L[l], &F = d.L[l - 1];
+    const int i = (int)( cell % C.dx ), j = (int)( ( cell / C.dx ) % C.dy ), k = (int)( cell / ( (long long)C.dx * C.dy ) );
+    if( i >= C.nx || j >= C.ny || k >= C.nz ) { C.type[cell] = BORA_MASKED; return; }
+    int t[8];
+#pragma unroll
+    for( int o = 0; o < 8; ++o )
     {
-        if( L.type[cell] != BORA_FLUID ) { L.code[cell] = 0; continue; }
-        int i, j, k;
-        nav.coords( cell, i, j, k );
-        // FluidProjection.cu:208 evaluated at the cell's lowest fine row
-        const int wall = (float)( j << L.level ) + 0.5f <= voxel_wall + 1.f ? BORA_WALL : BORA_AIR;
-        int diag = 6;
-        uint32_t mask = 0;
-        for( int q = 0; q < 6; ++q )
+        const int a = 2 * i + ( o & 1 ), b = 2 * j + ( ( o >> 1 ) & 1 ), c = 2 * k + ( o >> 2 );
+        t[o] = BORA_MASKED;
+        if( a >= F.nx || b >= F.ny || c >= F.nz ) continue;
+        if( F.kind == 1 ) t[o] = F.type[(long long)a + (long long)F.dx * ( b + (long long)F.dy * c )];
+        else if( a < d.tx && b < d.ty && c < d.tz )
         {
-            bool edge;
-            const long long n = nav.nbr_index( cell, i, j, k, q, &edge );
-            int t = edge ? wall : ( n < 0 ? BORA_AIR : (int)L.type[n] );
-            if( t == BORA_MASKED ) t = BORA_SOLID;
-            if( t == BORA_AIR ) diag += 1;
-            else if( t == BORA_SOLID || t == BORA_WALL ) diag -= 1;
-            else if( t == BORA_FLUID ) mask |= 1u << q;
+            const int s = d.slot_of[( (size_t)c * d.ty + b ) * d.tx + a];
+            t[o] = s < 0 ? BORA_AIR : F.type[s];
         }
-        L.code[cell] = (uint16_t)( BORA_CODE_FLUID | ( (uint32_t)diag << 8 ) | mask );
     }
+    bool air = false, fluid = false;
+#pragma unroll
+    for( int o = 0; o < 8; ++o )
+    {
+        air = air || t[o] == BORA_AIR;
+        fluid = fluid || t[o] == BORA_FLUID;
+    }
+    C.type[cell] = (uint8_t)coarse_type( air, fluid );
+}
+
+// Types of dense levels [first, d.n), one after the other, in one CTA.
+__global__ void __launch_bounds__( 1024 ) k_mg_types_dense( const __grid_constant__ SetupLevels d, int first )
+{
+    for( int l = first; l < d.n; ++l )
+    {
+        for( long long cell = threadIdx.x; cell < (long long)d.L[l].ncells; cell += blockDim.x ) dense_type( d, l, cell );
+        __syncthreads();
+    }
+}
+
+// Types of one dense level over the grid (levels too large for one CTA).
+__global__ void k_mg_types_level( const __grid_constant__ SetupLevels d, int l )
+{
+    for( long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < (long long)d.L[l].ncells;
+         cell += (long long)gridDim.x * blockDim.x )
+        dense_type( d, l, cell );
+}
+
+// The stencil code (same bit layout as the fine code) of a fluid cell from its neighbours' types;
+// wall: FluidProjection.cu:208 evaluated at the cell's lowest fine row.
+__device__ __forceinline__ uint32_t stencil_code( const int* t )
+{
+    int diag = 6;
+    uint32_t mask = 0;
+#pragma unroll
+    for( int q = 0; q < 6; ++q )
+    {
+        if( t[q] == BORA_AIR ) diag += 1;
+        else if( t[q] == BORA_FLUID ) mask |= 1u << q;
+        else diag -= 1;  // solid, wall, masked
+    }
+    return BORA_CODE_FLUID | ( (uint32_t)diag << 8 ) | mask;
+}
+
+// Codes of a tiled level with E = 4, 2 or 1 cells per tile edge, a thread per x-row.
+template <int E>
+__device__ __forceinline__ void codes_tiled( const SetupLevels& d, const BoraLevelDev& L, size_t row )
+{
+    constexpr int R = E * E, E3 = E * E * E;
+    if( row >= L.ncells / E ) return;
+    const int s = (int)( row / R ), y = (int)( row % E ), z = (int)( row / E % E );
+    const int vt = d.tile_of[s];
+    const int i0 = ( vt % d.tx ) * E, j = ( ( vt / d.tx ) % d.ty ) * E + y, k = ( vt / ( d.tx * d.ty ) ) * E + z;
+    const int32_t* nb = d.nbr + (size_t)s * 27;
+    // types of E cells from cell c of slot t (air in an inactive tile)
+    auto types = [&]( int t, int c ) -> uint32_t {
+        if( t < 0 ) return 0u;  // BORA_AIR is 0
+        const uint8_t* p = L.type + (size_t)t * E3 + c;
+        if constexpr( E == 4 ) return *reinterpret_cast<const uint32_t*>( p );
+        else if constexpr( E == 2 ) return *reinterpret_cast<const uint16_t*>( p );
+        else return *p;
+    };
+    const uint32_t w = types( s, E * ( y + E * z ) );
+    uint32_t code[E] = {};
+    bool any = false;
+#pragma unroll
+    for( int x = 0; x < E; ++x ) any = any || ( ( w >> ( 8 * x ) ) & 255u ) == BORA_FLUID;
+    if( any )
+    {
+        const uint32_t ym = y > 0 ? types( s, E * ( y - 1 + E * z ) ) : types( nb[bora_dir( 0, -1, 0 )], E * ( E - 1 + E * z ) );
+        const uint32_t yp = y < E - 1 ? types( s, E * ( y + 1 + E * z ) ) : types( nb[bora_dir( 0, 1, 0 )], E * ( E * z ) );
+        const uint32_t zm = z > 0 ? types( s, E * ( y + E * ( z - 1 ) ) ) : types( nb[bora_dir( 0, 0, -1 )], E * ( y + E * ( E - 1 ) ) );
+        const uint32_t zp = z < E - 1 ? types( s, E * ( y + E * ( z + 1 ) ) ) : types( nb[bora_dir( 0, 0, 1 )], E * y );
+        const int sm = nb[bora_dir( -1, 0, 0 )], sp = nb[bora_dir( 1, 0, 0 )];
+        const int xm = sm < 0 ? BORA_AIR : L.type[(size_t)sm * E3 + E * ( y + E * z ) + E - 1];
+        const int xp = sp < 0 ? BORA_AIR : L.type[(size_t)sp * E3 + E * ( y + E * z )];
+        const int wall = (float)( j << L.level ) + 0.5f <= d.voxel_wall + 1.f ? BORA_WALL : BORA_AIR;
+        auto at = [&]( uint32_t v, int x ) { return (int)( ( v >> ( 8 * x ) ) & 255u ); };
+#pragma unroll
+        for( int x = 0; x < E; ++x )
+        {
+            if( at( w, x ) != BORA_FLUID ) continue;
+            const int t[6] = { i0 + x == 0 ? wall : ( x ? at( w, x ? x - 1 : 0 ) : xm ), i0 + x + 1 >= L.nx ? wall : ( x < E - 1 ? at( w, x < E - 1 ? x + 1 : 0 ) : xp ),
+                               j == 0 ? wall : at( ym, x ), j + 1 >= L.ny ? wall : at( yp, x ),
+                               k == 0 ? wall : at( zm, x ), k + 1 >= L.nz ? wall : at( zp, x ) };
+            code[x] = stencil_code( t );
+        }
+    }
+    uint16_t* out = L.code + row * E;
+    if constexpr( E == 4 ) *reinterpret_cast<uint2*>( out ) = make_uint2( code[0] | ( code[1] << 16 ), code[2] | ( code[3] << 16 ) );
+    else if constexpr( E == 2 ) *reinterpret_cast<uint32_t*>( out ) = code[0] | ( code[1] << 16 );
+    else *out = (uint16_t)code[0];
+}
+
+__device__ __forceinline__ void codes_dense( const SetupLevels& d, const BoraLevelDev& L, size_t cell )
+{
+    if( cell >= L.ncells ) return;
+    if( L.type[cell] != BORA_FLUID ) { L.code[cell] = 0; return; }
+    const int i = (int)( cell % L.dx ), j = (int)( ( cell / L.dx ) % L.dy ), k = (int)( cell / ( (size_t)L.dx * L.dy ) );
+    const size_t sy = L.dx, sz = (size_t)L.dx * L.dy;
+    const int wall = (float)( j << L.level ) + 0.5f <= d.voxel_wall + 1.f ? BORA_WALL : BORA_AIR;
+    const int t[6] = { i == 0 ? wall : L.type[cell - 1], i + 1 >= L.nx ? wall : L.type[cell + 1],
+                       j == 0 ? wall : L.type[cell - sy], j + 1 >= L.ny ? wall : L.type[cell + sy],
+                       k == 0 ? wall : L.type[cell - sz], k + 1 >= L.nz ? wall : L.type[cell + sz] };
+    L.code[cell] = (uint16_t)stencil_code( t );
+}
+
+// Blocks of 256 threads that level L takes in k_mg_codes.
+__host__ __device__ inline size_t code_blocks( const BoraLevelDev& L )
+{
+    const size_t n = L.kind == 0 ? L.ncells / L.E : L.ncells;
+    return ( n + 255 ) / 256;
+}
+
+// Codes of levels 1 .. d.n - 1, a level after the other in the grid.
+__global__ void __launch_bounds__( 256 ) k_mg_codes( const __grid_constant__ SetupLevels d )
+{
+    size_t b = blockIdx.x;
+    int l = 1;
+    for( ; l < d.n - 1; ++l )
+    {
+        const size_t n = code_blocks( d.L[l] );
+        if( b < n ) break;
+        b -= n;
+    }
+    const BoraLevelDev& L = d.L[l];
+    const size_t at = b * 256 + threadIdx.x;
+    if( L.kind == 1 ) codes_dense( d, L, at );
+    else if( L.E == 4 ) codes_tiled<4>( d, L, at );
+    else if( L.E == 2 ) codes_tiled<2>( d, L, at );
+    else codes_tiled<1>( d, L, at );
 }
 
 // ---- V-cycle -----------------------------------------------------------------------
@@ -604,26 +704,37 @@ int blocks_for( size_t n )
     return (int)std::max<size_t>( 1, std::min<size_t>( ( n + 255 ) / 256, (size_t)sm_count() * 8 ) );
 }
 
-LevelNav nav_of( const BoraGridDev& g, const BoraLevelDev& L, BoraTilesDev t )
-{
-    return LevelNav{ L, t.nbr, t.tile_of, g.tx, g.ty };
-}
-
 }  // namespace
 
-void bora_mg_setup( const BoraGridDev& g, BoraLevelDev* levels, int nlevels, BoraTilesDev t, void* mid_image,
-                    uint32_t* err, cudaStream_t st )
+int bora_mg_setup( const BoraGridDev& g, BoraLevelDev* levels, int nlevels, BoraTilesDev t, void* mid_image,
+                   cudaStream_t st )
 {
-    (void)err;
-    for( int l = 1; l < nlevels; ++l )
-    {
-        const BoraLevelDev& F = levels[l - 1];
-        const BoraLevelDev& C = levels[l];
-        k_mg_types<<<blocks_for( C.ncells ), 256, 0, st>>>( F, C, t.slot_of, t.tile_of, g.tx, g.ty, g.tz );
-        k_mg_codes<<<blocks_for( C.ncells ), 256, 0, st>>>( nav_of( g, C, t ), g.voxel_wall );
-    }
     const int ntiles = levels[0].kind == 0 ? (int)( levels[0].ncells / 512 ) : 0;
+    SetupLevels d{};
+    d.n = nlevels;
+    for( int l = 0; l < nlevels; ++l ) d.L[l] = levels[l];
+    d.nbr = t.nbr; d.slot_of = t.slot_of; d.tile_of = t.tile_of;
+    d.tx = g.tx; d.ty = g.ty; d.tz = g.tz;
+    d.voxel_wall = g.voxel_wall;
+    int launches = 0;
+    if( nlevels < 2 ) return 0;
+    k_mg_types_tiled<<<(unsigned)( ( (size_t)ntiles * 16 + 255 ) / 256 ), 256, 0, st>>>( d, ntiles );
+    ++launches;
+    int dense = 1;
+    while( dense < nlevels && levels[dense].kind == 0 ) ++dense;
+    for( ; dense < nlevels && levels[dense].ncells > kDenseOneCta; ++dense, ++launches )
+        k_mg_types_level<<<blocks_for( levels[dense].ncells ), 256, 0, st>>>( d, dense );
+    if( dense < nlevels )
+    {
+        k_mg_types_dense<<<1, 1024, 0, st>>>( d, dense );
+        ++launches;
+    }
+    size_t blocks = 0;
+    for( int l = 1; l < nlevels; ++l ) blocks += code_blocks( levels[l] );
+    k_mg_codes<<<(unsigned)blocks, 256, 0, st>>>( d );
+    ++launches;
     bora_mg_mid_setup( g, levels, nlevels, t, ntiles, mid_image, st );
+    return launches + ( mid_image ? 1 : 0 );
 }
 
 namespace {
