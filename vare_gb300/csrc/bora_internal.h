@@ -87,7 +87,7 @@ cudaError_t bora_launch_pdl( void ( *kernel )( KArgs... ), dim3 grid, dim3 block
 
 // ---- scan ---------------------------------------------------------------------------
 size_t bora_scan_scratch_elems( size_t n );
-void bora_device_scan( const uint32_t* in, uint32_t* out, size_t n, uint32_t* scratch, uint32_t* total, cudaStream_t st );
+int bora_device_scan( const uint32_t* in, uint32_t* out, size_t n, uint32_t* scratch, uint32_t* total, cudaStream_t st );
 
 // ---- particle arrays (structure of arrays) -------------------------------------------
 struct BoraParticlesDev

@@ -487,10 +487,10 @@ int rebuild_tiles( bora_flip_sim* s )
     }
     s->keys_valid = false;
     {
-        KTimer t( s, BORA_KERNEL_TILES, 4 );
+        KTimer t( s, BORA_KERNEL_TILES, 1 );
         bora_launch_activate( s->g, P<uint8_t>( s->tile_flag ), P<uint32_t>( s->tile_act ), st );
-        bora_device_scan( P<uint32_t>( s->tile_act ), P<uint32_t>( s->tile_excl ), s->ntv, P<uint32_t>( s->scan_scratch ),
-                       P<uint32_t>( s->counters ) + 0, st );
+        s->stats.kernel_launches += (uint64_t)bora_device_scan( P<uint32_t>( s->tile_act ), P<uint32_t>( s->tile_excl ), s->ntv,
+                                                                P<uint32_t>( s->scan_scratch ), P<uint32_t>( s->counters ) + 0, st );
     }
     BORA_TRYS( check_launch( s ) );
     return issue_counters( s, 0, 1, st );
@@ -512,11 +512,12 @@ int rebuild_sort( bora_flip_sim* s )
         bora_launch_tile_nbrs( s->g, ntiles, P<int32_t>( s->slot_of ), P<int32_t>( s->tile_of ), P<int32_t>( s->nbr ), st );
     }
     {
-        KTimer t( s, BORA_KERNEL_SORT, s->np ? 6 : 3 );
+        KTimer t( s, BORA_KERNEL_SORT, s->np ? 3 : 0 );
         bora_launch_hist( s->np, P<uint32_t>( s->vkey ), P<int32_t>( s->slot_of ), ncell, P<uint32_t>( s->key ),
                           P<uint32_t>( s->cell_count ), P<uint32_t>( s->counters ) + 2, st );
-        bora_device_scan( P<uint32_t>( s->cell_count ), P<uint32_t>( s->cell_start ), (size_t)ncell + 1,
-                       P<uint32_t>( s->scan_scratch ), P<uint32_t>( s->counters ) + 1, st );
+        s->stats.kernel_launches += (uint64_t)bora_device_scan( P<uint32_t>( s->cell_count ), P<uint32_t>( s->cell_start ),
+                                                                (size_t)ncell + 1, P<uint32_t>( s->scan_scratch ),
+                                                                P<uint32_t>( s->counters ) + 1, st );
         bora_launch_scatter( s->np, P<uint32_t>( s->key ), P<uint32_t>( s->cell_start ), P<uint32_t>( s->cell_count ),
                              P<uint32_t>( s->idx ), st );
         if( s->np ) bora_launch_order_bins( (size_t)ncell + 1, P<uint32_t>( s->cell_start ), P<uint32_t>( s->idx ), st );

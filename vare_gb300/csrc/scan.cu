@@ -1,7 +1,11 @@
 // Device exclusive prefix sum of uint32 counts (tile activation flags, per-dual-cell
-// particle counts). Three passes: per-block sums, one-block scan of the block sums,
-// per-block scan with the block's offset. Each pass reads its input with 128-bit
-// loads; the block-sum scratch array (2048 elements per block) is owned by the caller.
+// particle counts). Up to 8192 counts: one block. Up to 16 M: per-block sums (2048 elements per
+// block), then a scan per block whose offset the block sums up itself from the block sums before
+// it, its elements read ahead of the wait for them. Beyond, where those sums would be most of the
+// traffic: a one-block scan of the block sums in between. Each pass reads its input with 128-bit
+// loads; the block-sum scratch array is owned by the caller. Latency bounds the small ones: 11.3 us
+// with three launches up to 100 K counts, 4.2 in one block (8192), 6.1 with two launches; 20.5 and
+// 12.3 us for 4 M.
 #include "bora_internal.h"
 
 namespace {
@@ -9,6 +13,9 @@ namespace {
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;  // per thread -> 2048 elements per block
 constexpr int kScanChunk = kScanThreads * kScanItems;
+constexpr int kScanOneThreads = 1024;
+constexpr size_t kScanOneMax = (size_t)kScanOneThreads * kScanItems;
+constexpr int kScanSelfMax = 8192;  // blocks up to which a block sums up its own offset (16 M counts: 41.0 us, 53.3 with three launches)
 
 __device__ inline uint32_t warp_incl_scan( uint32_t v )
 {
@@ -24,22 +31,23 @@ __device__ inline uint32_t warp_incl_scan( uint32_t v )
 
 // Block-wide exclusive scan of one value per thread; returns the exclusive prefix and
 // the block total in *total.
+template <int T>
 __device__ inline uint32_t block_excl_scan( uint32_t v, uint32_t* total )
 {
-    __shared__ uint32_t warp_sums[kScanThreads / 32];
+    __shared__ uint32_t warp_sums[T / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t inc = warp_incl_scan( v );
     if( lane == 31 ) warp_sums[wid] = inc;
     __syncthreads();
     if( wid == 0 )
     {
-        uint32_t s = lane < kScanThreads / 32 ? warp_sums[lane] : 0u;
+        uint32_t s = lane < T / 32 ? warp_sums[lane] : 0u;
         s = warp_incl_scan( s );
-        if( lane < kScanThreads / 32 ) warp_sums[lane] = s;
+        if( lane < T / 32 ) warp_sums[lane] = s;
     }
     __syncthreads();
     const uint32_t base = wid > 0 ? warp_sums[wid - 1] : 0u;
-    *total = warp_sums[kScanThreads / 32 - 1];
+    *total = warp_sums[T / 32 - 1];
     __syncthreads();
     return base + inc - v;
 }
@@ -61,45 +69,17 @@ __device__ inline void load_items( const uint32_t* __restrict__ in, size_t n, si
     }
 }
 
-__global__ void k_scan_reduce( const uint32_t* __restrict__ in, size_t n, uint32_t* __restrict__ block_sums )
+__device__ inline uint32_t item_sum( const uint32_t v[kScanItems] )
 {
-    uint32_t v[kScanItems];
-    load_items( in, n, (size_t)blockIdx.x * kScanChunk, v );
     uint32_t s = 0;
 #pragma unroll
     for( int q = 0; q < kScanItems; ++q ) s += v[q];
-    uint32_t total;
-    block_excl_scan( s, &total );
-    if( threadIdx.x == 0 ) block_sums[blockIdx.x] = total;
+    return s;
 }
 
-// One block scans the nb block sums in place (exclusive) and writes the grand total.
-__global__ void k_scan_blocks( uint32_t* __restrict__ block_sums, int nb, uint32_t* __restrict__ grand_total )
+// the thread's items as prefix sums from `run`
+__device__ inline void store_items( uint32_t* __restrict__ out, size_t n, size_t base, const uint32_t v[kScanItems], uint32_t run )
 {
-    uint32_t carry = 0;
-    for( int base = 0; base < nb; base += kScanThreads )
-    {
-        const int i = base + threadIdx.x;
-        const uint32_t v = i < nb ? block_sums[i] : 0u;
-        uint32_t total;
-        const uint32_t ex = block_excl_scan( v, &total );
-        if( i < nb ) block_sums[i] = carry + ex;
-        carry += total;
-    }
-    if( threadIdx.x == 0 && grand_total ) *grand_total = carry;
-}
-
-__global__ void k_scan_down( const uint32_t* __restrict__ in, size_t n, const uint32_t* __restrict__ block_sums,
-                             uint32_t* __restrict__ out )
-{
-    uint32_t v[kScanItems];
-    const size_t base = (size_t)blockIdx.x * kScanChunk;
-    load_items( in, n, base, v );
-    uint32_t s = 0;
-#pragma unroll
-    for( int q = 0; q < kScanItems; ++q ) s += v[q];
-    uint32_t total;
-    uint32_t run = block_excl_scan( s, &total ) + block_sums[blockIdx.x];
     const size_t i0 = base + (size_t)threadIdx.x * kScanItems;
     uint32_t o[kScanItems];
 #pragma unroll
@@ -117,23 +97,96 @@ __global__ void k_scan_down( const uint32_t* __restrict__ in, size_t n, const ui
     }
 }
 
+// n <= kScanOneMax
+__global__ void __launch_bounds__( kScanOneThreads ) k_scan_one( const uint32_t* in, size_t n, uint32_t* out,
+                                                                 uint32_t* __restrict__ grand_total )
+{
+    uint32_t v[kScanItems];
+    load_items( in, n, 0, v );
+    uint32_t total;
+    const uint32_t run = block_excl_scan<kScanOneThreads>( item_sum( v ), &total );
+    store_items( out, n, 0, v, run );
+    if( threadIdx.x == 0 && grand_total ) *grand_total = total;
+}
+
+__global__ void k_scan_reduce( const uint32_t* __restrict__ in, size_t n, uint32_t* __restrict__ block_sums )
+{
+    bora_pdl_trigger();
+    uint32_t v[kScanItems];
+    load_items( in, n, (size_t)blockIdx.x * kScanChunk, v );
+    uint32_t total;
+    block_excl_scan<kScanThreads>( item_sum( v ), &total );
+    if( threadIdx.x == 0 ) block_sums[blockIdx.x] = total;
+}
+
+// One block scans the nb block sums in place (exclusive) and writes the grand total.
+__global__ void k_scan_blocks( uint32_t* __restrict__ block_sums, int nb, uint32_t* __restrict__ grand_total )
+{
+    uint32_t carry = 0;
+    for( int base = 0; base < nb; base += kScanThreads )
+    {
+        const int i = base + threadIdx.x;
+        const uint32_t v = i < nb ? block_sums[i] : 0u;
+        uint32_t total;
+        const uint32_t ex = block_excl_scan<kScanThreads>( v, &total );
+        if( i < nb ) block_sums[i] = carry + ex;
+        carry += total;
+    }
+    if( threadIdx.x == 0 && grand_total ) *grand_total = carry;
+}
+
+// SELF: block_sums are the blocks' sums (the kernel follows k_scan_reduce, which no longer reads
+// `in` when a block of this one writes); else they are scanned already.
+template <bool SELF>
+__global__ void __launch_bounds__( kScanThreads ) k_scan_down( const uint32_t* in, size_t n, const uint32_t* block_sums,
+                                                               uint32_t* out, uint32_t* __restrict__ grand_total )
+{
+    uint32_t v[kScanItems];
+    const size_t base = (size_t)blockIdx.x * kScanChunk;
+    load_items( in, n, base, v );
+    uint32_t total, offset = 0;
+    uint32_t run = block_excl_scan<kScanThreads>( item_sum( v ), &total );
+    if( SELF )
+    {
+        bora_pdl_wait();
+        uint32_t before = 0;
+        for( unsigned b = threadIdx.x; b < blockIdx.x; b += kScanThreads ) before += block_sums[b];
+        block_excl_scan<kScanThreads>( before, &offset );
+        if( grand_total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0 ) *grand_total = offset + total;
+    }
+    else offset = block_sums[blockIdx.x];
+    store_items( out, n, base, v, run + offset );
+}
+
 }  // namespace
 
 size_t bora_scan_scratch_elems( size_t n ) { return ( n + kScanChunk - 1 ) / kScanChunk + 1; }
 
 // out[i] = sum_{j<i} in[i]; *total = sum of all (device pointer, may be null).
 // in and out may alias. scratch holds bora_scan_scratch_elems(n) uint32.
-void bora_device_scan( const uint32_t* in, uint32_t* out, size_t n, uint32_t* scratch, uint32_t* total, cudaStream_t st )
+// Returns its kernel launches.
+int bora_device_scan( const uint32_t* in, uint32_t* out, size_t n, uint32_t* scratch, uint32_t* total, cudaStream_t st )
 {
     if( n == 0 )
     {
         if( total ) cudaMemsetAsync( total, 0, sizeof( uint32_t ), st );
-        return;
+        return 0;
+    }
+    if( n <= kScanOneMax )
+    {
+        k_scan_one<<<1, kScanOneThreads, 0, st>>>( in, n, out, total );
+        return 1;
     }
     const int nb = (int)( ( n + kScanChunk - 1 ) / kScanChunk );
     k_scan_reduce<<<nb, kScanThreads, 0, st>>>( in, n, scratch );
+    if( nb <= kScanSelfMax )
+    {
+        bora_launch_pdl( k_scan_down<true>, dim3( nb ), dim3( kScanThreads ), 0, st, in, n, (const uint32_t*)scratch, out, total );
+        return 2;
+    }
     k_scan_blocks<<<1, kScanThreads, 0, st>>>( scratch, nb, total );
-    k_scan_down<<<nb, kScanThreads, 0, st>>>( in, n, scratch, out );
+    k_scan_down<false><<<nb, kScanThreads, 0, st>>>( in, n, scratch, out, nullptr );
+    return 3;
 }
 
 // ---- public C ABI: device exclusive prefix sum -------------------------------------
