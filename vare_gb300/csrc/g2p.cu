@@ -32,6 +32,7 @@ struct StagedLerp
 {
     int base;  // staged index of corner (i,j,k)
     int cell;  // its index in the tile
+    bool staged;  // the base cell lies in the tile
     float x, y, z;
     __device__ inline void setup( const BoraGridDev& g, int ti, int tj, int tk, float px, float py, float pz )
     {
@@ -41,10 +42,12 @@ struct StagedLerp
         x = bora_clampf( px - ( (float)i + .5f ), 0.f, 1.f );
         y = bora_clampf( py - ( (float)j + .5f ), 0.f, 1.f );
         z = bora_clampf( pz - ( (float)k + .5f ), 0.f, 1.f );
-        // (the frame's extent is a multiple of 4, so that the clamp above leaves i in the tile)
+        // (for the particles of the tile's dual cells it does: the frame's extent is a multiple of
+        // 4, so that the clamp above leaves i in the tile)
         const int li = i - ti * BORA_TILE, lj = j - tj * BORA_TILE, lk = k - tk * BORA_TILE;
         base = li + kStageEdge * ( lj + kStageEdge * lk );
         cell = li + BORA_TILE * ( lj + BORA_TILE * lk );
+        staged = ( (unsigned)li | (unsigned)lj | (unsigned)lk ) < (unsigned)BORA_TILE;
     }
     __device__ static inline int off( int q )
     {
@@ -78,6 +81,19 @@ struct StagedLerp
         v = fminf_ref( v, fminf_ref( w( 2 ), w( 3 ) ) );
         v = fminf_ref( v, fminf_ref( w( 4 ), w( 5 ) ) );
         return fminf_ref( v, fminf_ref( w( 6 ), w( 7 ) ) );
+    }
+    // comp alone
+    __device__ inline float4 comp( const float4* fa, const float2* fb, float one ) const
+    {
+        auto xy = [&]( int q ) { return *reinterpret_cast<const float2*>( fa + base + off( q ) ); };
+        auto cz = [&]( int q ) { return make_float2( fb[base + off( q )].x, 0.f ); };
+        auto lerp = [&]( auto f ) {
+            const float2 c00 = mix( f( 0 ), f( 1 ), x, one ), c01 = mix( f( 2 ), f( 3 ), x, one );
+            const float2 c10 = mix( f( 4 ), f( 5 ), x, one ), c11 = mix( f( 6 ), f( 7 ), x, one );
+            return mix( mix( c00, c10, y, one ), mix( c01, c11, y, one ), z, one );
+        };
+        const float2 a = lerp( xy ), b = lerp( cz );
+        return make_float4( a.x, a.y, b.x, 0.f );
     }
     // comp and velo lerped from the staged cells (comp.xy and velo.xy from fa, comp.z and
     // velo.z from fb); the corners' mix order is SparseField's
@@ -190,10 +206,26 @@ __device__ __noinline__ bool col_kill( const BoraGridDev* g, float3 p )
     return phi > 3.f || phi < 0.f;
 }
 
-// Grid velocity ("comp") at an arbitrary point, for the RK2 option.
-__device__ inline float4 comp_at( const BoraGridDev& g, const int32_t* slot_of, const BoraCellsDev& c, float x, float y,
-                                  float z )
+// The CTA's staged tile, for lookups away from the particle's own position (fa null: none).
+struct StagedTile
 {
+    const float4* fa;
+    const float2* fb;
+    float one;
+    int ti, tj, tk;
+};
+
+// Grid velocity ("comp") at an arbitrary point, for the RK2 option: from the staged tile where the
+// point's base cell lies in it, else through the tile table.
+__device__ inline float4 comp_at( const BoraGridDev& g, const int32_t* slot_of, const BoraCellsDev& c, const StagedTile& st,
+                                  float x, float y, float z )
+{
+    if( st.fa )
+    {
+        StagedLerp l;
+        l.setup( g, st.ti, st.tj, st.tk, x, y, z );
+        if( l.staged ) return l.comp( st.fa, st.fb, st.one );
+    }
     GlobalLerp l{ g, slot_of, c };
     l.setup( x, y, z );
     return l.comp();
@@ -214,7 +246,7 @@ constexpr int kLater = 2;
 template <int kMode, bool kCols>
 __device__ inline int advance_particle( const BoraGridDev& g, float4 gn, float4 go, const int32_t* slot_of,
                                          const BoraCellsDev& c, float& px, float& py, float& pz, float& vx, float& vy,
-                                         float& vz, float dt, const float* sub )
+                                         float& vz, float dt, const float* sub, const StagedTile& st )
 {
     constexpr bool kAll = kMode != kCommon, kRk2 = kMode == kEverything;
     const float lx = (float)g.nx + 0.5f, lz = (float)g.nz + 0.5f;
@@ -280,8 +312,9 @@ __device__ inline int advance_particle( const BoraGridDev& g, float4 gn, float4 
             if( kRk2 && g.advection == BORA_ADVECT_RK2 )
             {
                 const float h = 0.5f * sub_dt;
-                const float4 k1 = comp_at( g, slot_of, c, px, py, pz );
-                const float4 k2 = comp_at( g, slot_of, c, px + k1.x * h, py + k1.y * h, pz + k1.z * h );
+                // the first substep starts where gn was sampled, unless a collider carried the particle
+                const float4 k1 = it == 0 && !( kCols && hasCols ) ? gn : comp_at( g, slot_of, c, st, px, py, pz );
+                const float4 k2 = comp_at( g, slot_of, c, st, px + k1.x * h, py + k1.y * h, pz + k1.z * h );
                 px += k2.x * sub_dt; py += k2.y * sub_dt; pz += k2.z * sub_dt;
             }
             else
@@ -324,7 +357,8 @@ constexpr uint32_t kLaterKey = BORA_DEAD_KEY - 2;
 // dt / iter from a table, the sort key of a particle that is known to be inside the grid. A 640
 // tank with a collider 1097 -> 817, its collider calls in a loop of their own, whose
 // spills the others do not pay for; an RK2 step at 96^3 134 -> 113 at 80 registers (119
-// at 64).
+// at 64), and 82 with its lookups from the staged tile instead of through the tile table, the
+// first one being the sample that the particle already has.
 template <int kMode>
 __global__ void __launch_bounds__( kG2PThreads, kMode == kEverything ? 3 : 4 ) k_g2p( const __grid_constant__ BoraGridDev g, BoraTilesDev t, int ntiles,
                                                        uint32_t nsorted, const uint32_t* __restrict__ start, BoraCellsDev c,
@@ -379,7 +413,8 @@ __global__ void __launch_bounds__( kG2PThreads, kMode == kEverything ? 3 : 4 ) k
             GlobalLerp smp{ g, t.slot_of, c };
             smp.setup( px, py, pz );
             adj[q] = smp.surf_min();
-            const int kill = advance_particle<kMode, true>( g, smp.comp(), smp.velo(), t.slot_of, c, px, py, pz, vx, vy, vz, dt, sub );
+            const int kill = advance_particle<kMode, true>( g, smp.comp(), smp.velo(), t.slot_of, c, px, py, pz, vx, vy, vz, dt, sub,
+                                                               StagedTile{} );
             finish( q, pi, src.id[pi], px, py, pz, vx, vy, vz, kill != 0 );
         }
     }
@@ -431,6 +466,7 @@ __global__ void __launch_bounds__( kG2PThreads, kMode == kEverything ? 3 : 4 ) k
         for( int l = tid; l < BORA_TILE_CELLS; l += kG2PThreads )
             surf_min[l] = StagedLerp::corner_min( surf, ( l & 7 ) + kStageEdge * ( ( ( l >> 3 ) & 7 ) + kStageEdge * ( l >> 6 ) ) );
         __syncthreads();
+        const StagedTile st{ fa, fb, sub[0], ti, tj, tk };
         uint32_t later = 0;  // particles of this thread that wait for the collider code
         for( uint32_t q = q0 + tid; q < q1; q += kG2PThreads )
         {
@@ -449,7 +485,7 @@ __global__ void __launch_bounds__( kG2PThreads, kMode == kEverything ? 3 : 4 ) k
             float4 gn, go;
             l.sample( fa, fb, sub[0], gn, go );
             adj[q] = surf_min[l.cell];
-            const int kill = advance_particle<kMode, false>( g, gn, go, t.slot_of, c, px, py, pz, vx, vy, vz, dt, sub );
+            const int kill = advance_particle<kMode, false>( g, gn, go, t.slot_of, c, px, py, pz, vx, vy, vz, dt, sub, st );
             if( kMode != kCommon && kill == kLater )
             {
                 vkey[q] = kLaterKey;
@@ -471,7 +507,7 @@ __global__ void __launch_bounds__( kG2PThreads, kMode == kEverything ? 3 : 4 ) k
                 l.setup( g, ti, tj, tk, px, py, pz );
                 float4 gn, go;
                 l.sample( fa, fb, sub[0], gn, go );
-                const int kill = advance_particle<kMode, true>( g, gn, go, t.slot_of, c, px, py, pz, vx, vy, vz, dt, sub );
+                const int kill = advance_particle<kMode, true>( g, gn, go, t.slot_of, c, px, py, pz, vx, vy, vz, dt, sub, st );
                 finish( q, pi, src.id[pi], px, py, pz, vx, vy, vz, kill != 0 );
             }
         __syncthreads();
