@@ -1,6 +1,6 @@
 """The multigrid hierarchy's set-up (cell types and stencil codes, vare_gb300/csrc/multigrid.cu): the
 same pool of fluid, away from the walls, in grids whose hierarchies have from three levels to
-dense levels of more than 16384 cells (types formed by one CTA, or over the grid). The levels are
+dense levels of more than 2048 cells (types formed by one CTA, or over the grid). The levels are
 aligned with the grid's origin, so the pool's cells have the same types in every grid but for the
 coarsest levels: the solver converges in the same number of iterations within two."""
 import numpy as np

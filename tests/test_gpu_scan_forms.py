@@ -31,3 +31,29 @@ def test_scan_forms(gpu, n, shift, in_place):
         np.testing.assert_array_equal(out[shift:shift + n].cpu().numpy().view(np.uint32), want)
         assert int(tot.cpu().numpy().view(np.uint32)[0]) == int(host.astype(np.uint64).sum() & 0xFFFFFFFF)
         assert int(out[n + shift]) == (0 if in_place else -1)
+
+
+@pytest.mark.parametrize("n", [5000, 100000])
+def test_scan_in_a_graph(gpu, n):
+    """The form without allocation recorded into a CUDA graph and replayed on new counts."""
+    import torch
+    lib = gpu.load()
+    d = torch.zeros(n, dtype=torch.int32, device="cuda")
+    out, tot = torch.empty_like(d), torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def scan():
+        assert lib.bora_scan_u32_noalloc(ctypes.c_void_p(d.data_ptr()), ctypes.c_void_p(out.data_ptr()), n,
+                                         ctypes.c_void_p(tot.data_ptr()),
+                                         ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    scan()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        scan()
+    for seed in range(3):
+        host = np.random.default_rng(seed).integers(0, 1000, n, dtype=np.int32)
+        d.copy_(torch.from_numpy(host))
+        graph.replay()
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(out.cpu().numpy(), np.cumsum(host, dtype=np.int32) - host)
+        assert int(tot[0]) == int(host.sum())

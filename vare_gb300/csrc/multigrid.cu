@@ -50,8 +50,10 @@ __device__ inline int code_diag( uint16_t c ) { return ( c >> 8 ) & 15; }
 // the domain it is masked. Children beyond the finer level's domain count as none (wall-like).
 // Three launches: the tiled levels' types, the dense levels' types, all levels' codes (with two
 // launches a level and a cell per thread the set-up was 8 to 14 launches. With the right-hand side
-// and the solver's tile table: 83 -> 50 us at 96^3, 155 -> 101 at 256^3, 237 -> 140 in a 640 tank.)
-constexpr size_t kDenseOneCta = 16384;  // dense cells up to which one CTA forms a level's types
+// and the solver's tile table: 83 -> 50 us at 96^3, 155 -> 94 at 256^3, 237 -> 136 in a 640 tank.)
+// dense cells up to which one CTA forms a level's types (the 4096 of a 256^3 grid: 102 us in one CTA
+// with the right-hand side, 94 over the grid)
+constexpr size_t kDenseOneCta = 2048;
 
 struct SetupLevels
 {
