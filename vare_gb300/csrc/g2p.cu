@@ -10,6 +10,8 @@
 // is also binned for the next rebuild (its sort key and tile flag, the rule of k_bin), so
 // that the next step need not read the particles again to bin them; a tile's CTA marks the
 // flags of the 27 tiles around its own in shared memory and stores each marked one once.
+#include <algorithm>
+
 #include "bora_internal.h"
 #include "../../include/bora_flip.h"
 
@@ -21,6 +23,7 @@ namespace {
 // the eight corners. Cells of inactive tiles hold the field backgrounds (0, and 10 for surf:
 // FLIPMethod.cu:30).
 constexpr int kG2PThreads = 256;
+constexpr int kG2PSplitMax = 4;  // CTAs per tile at most
 constexpr int kStageEdge = BORA_TILE + 1;
 constexpr int kStageCells = kStageEdge * kStageEdge * kStageEdge;
 
@@ -374,6 +377,8 @@ __global__ void __launch_bounds__( kG2PThreads, kMode == kEverything ? 3 : 4 ) k
     __shared__ uint8_t near_flag[27];  // activation flags of the tiles around the CTA's own
     __shared__ float sub[kSubTable];   // dt / iter; [0] is 1
     const int s = blockIdx.x, tid = threadIdx.x;
+    // a tile's CTAs (grid y) take its particles in turns
+    const uint32_t first = blockIdx.y * kG2PThreads + tid, stride = gridDim.y * kG2PThreads;
     if( tid < kSubTable ) sub[tid] = tid ? dt / (float)tid : 1.f;
     uint32_t kills = 0;
     int cti = -8, ctj = -8, ctk = -8;  // the CTA's tile (far from every tile: no shared flags)
@@ -405,7 +410,7 @@ __global__ void __launch_bounds__( kG2PThreads, kMode == kEverything ? 3 : 4 ) k
     {
         __syncthreads();
         const uint32_t q0 = start[(size_t)ntiles * BORA_TILE_CELLS], q1 = nsorted;
-        for( uint32_t q = q0 + tid; q < q1; q += kG2PThreads )
+        for( uint32_t q = q0 + first; q < q1; q += stride )
         {
             const uint32_t pi = idx[q];
             float px = src.px[pi], py = src.py[pi], pz = src.pz[pi];
@@ -437,12 +442,12 @@ __global__ void __launch_bounds__( kG2PThreads, kMode == kEverything ? 3 : 4 ) k
             vxn = src.vx[pi]; vyn = src.vy[pi]; vzn = src.vz[pi];
             idn = src.id[pi];
         };
-        if( q0 + tid < q1 )
+        if( q0 + first < q1 )
         {
-            pin = idx[q0 + tid];
+            pin = idx[q0 + first];
             fetch( pin );
         }
-        if( q0 + tid + kG2PThreads < q1 ) pin2 = idx[q0 + tid + kG2PThreads];
+        if( q0 + first + stride < q1 ) pin2 = idx[q0 + first + stride];
         __syncthreads();
         for( int h = tid; h < kStageCells; h += kG2PThreads )
         {
@@ -468,17 +473,17 @@ __global__ void __launch_bounds__( kG2PThreads, kMode == kEverything ? 3 : 4 ) k
         __syncthreads();
         const StagedTile st{ fa, fb, sub[0], ti, tj, tk };
         uint32_t later = 0;  // particles of this thread that wait for the collider code
-        for( uint32_t q = q0 + tid; q < q1; q += kG2PThreads )
+        for( uint32_t q = q0 + first; q < q1; q += stride )
         {
             const uint32_t pi = pin;
             const int32_t id = idn;
             float px = pxn, py = pyn, pz = pzn;
             float vx = vxn, vy = vyn, vz = vzn;
-            if( q + kG2PThreads < q1 )
+            if( q + stride < q1 )
             {
                 pin = pin2;
                 fetch( pin );
-                if( q + 2 * kG2PThreads < q1 ) pin2 = idx[q + 2 * kG2PThreads];
+                if( q + 2 * stride < q1 ) pin2 = idx[q + 2 * stride];
             }
             StagedLerp l;
             l.setup( g, ti, tj, tk, px, py, pz );
@@ -496,7 +501,7 @@ __global__ void __launch_bounds__( kG2PThreads, kMode == kEverything ? 3 : 4 ) k
         }
         if constexpr( kMode != kCommon )
 #pragma unroll 1
-            for( uint32_t q = q0 + tid; later != 0 && q < q1; q += kG2PThreads )
+            for( uint32_t q = q0 + first; later != 0 && q < q1; q += stride )
             {
                 if( vkey[q] != kLaterKey ) continue;
                 --later;
@@ -531,8 +536,12 @@ void bora_launch_g2p( const BoraGridDev& g, int ntiles, size_t nsorted, BoraTile
     if( nsorted == 0 ) return;
     // the common case in a kernel without the code of the others, and the RK2 lookups (two more
     // grid samples, inlined) only where they are asked for
+    // Few tiles: up to four CTAs each, so that two rounds of the chip's 608 places are taken (a tile's
+    // particles are a chain of 16 rounds in one CTA): 26 us at 24^3 (27 tiles) and 30 at 64^3 (240)
+    // with one, 14 and 22 with four.
+    const int split = std::max( 1, std::min( kG2PSplitMax, 1216 / ( ntiles + 1 ) ) );
     auto go = [&]( auto kernel ) {
-        kernel<<<ntiles + 1, kG2PThreads, 0, st>>>( g, t, ntiles, (uint32_t)nsorted, start, c, src, idx, dst, adj, dt,
+        kernel<<<dim3( ntiles + 1, split ), kG2PThreads, 0, st>>>( g, t, ntiles, (uint32_t)nsorted, start, c, src, idx, dst, adj, dt,
                                                     nkilled, vkey, tile_flag );
     };
     if( g.advection == BORA_ADVECT_RK2 ) go( k_g2p<kEverything> );
