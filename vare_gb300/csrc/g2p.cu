@@ -241,7 +241,7 @@ __device__ inline float4 comp_at( const BoraGridDev& g, const int32_t* slot_of, 
 // alone (no water tank, no colliders, Euler advection), the water tank and the colliders with Euler
 // advection, and everything (the caller checks). kCols = false leaves a particle that may meet a
 // collider alone and returns kLater: the collider code's calls would spill the registers of the
-// others. sub[]: dt / iter for iter < kSubTable.
+// others. sub[]: dt / iter for 0 < iter < kSubTable.
 enum AdvanceMode { kCommon, kEuler, kEverything };
 constexpr int kSubTable = 32;
 constexpr int kLater = 2;
@@ -308,7 +308,8 @@ __device__ inline int advance_particle( const BoraGridDev& g, float4 gn, float4 
     {
         const float len = sqrtf( vx * vx + vy * vy + vz * vz );
         const int iter = 1 + bora_imin( bora_trunc( len * dt * 1.5f ), bora_imax( g.maxsubsteps, 1 ) );
-        const float sub_dt = iter < kSubTable ? sub[iter] : dt / (float)iter;
+        // (iter is 0 or negative for a negative dt: the loop does not run, and the table is not read)
+        const float sub_dt = (unsigned)iter < (unsigned)kSubTable ? sub[iter] : dt / (float)iter;
         bool col = false;
         for( int it = 0; it < iter; ++it )
         {
