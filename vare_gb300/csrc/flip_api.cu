@@ -680,6 +680,11 @@ int stage_solve( bora_flip_sim* s )
         s->stats.kernel_launches += 1;
         bora_launch_tile_fluid( s->ntiles, code, P<uint8_t>( s->tile_fluid ), st );
         issue_solve_tiles( s );
+        if( p.solver == BORA_SOLVER_PLAIN && s->ntiles > 0 )  // a tile that was not the solver's has no pivots yet
+        {
+            s->stats.kernel_launches += 1;
+            bora_launch_mic_factor( s->ntiles, s->solve_tiles(), code, P<float>( s->sminv ), st );
+        }
     }
     const int s_b2 = s->slot(), s_bmax = s->slot();
     arm_mirror( s, s_b2 );
