@@ -140,6 +140,7 @@ struct BoraSolveTilesDev
     const int4* tab;
     const uint32_t* count;  // their number, on the device
     int n;                  // the same on the host, once known
+    const int32_t* nbr;     // the active tiles' neighbour table (BoraTilesDev), for the check of the codes
 };
 
 // Scalars that the solver kernels exchange on the device (ring of FP64 reductions).

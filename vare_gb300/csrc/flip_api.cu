@@ -237,7 +237,7 @@ struct bora_flip_sim
                              P<float>( vz ), P<float>( cx ), P<float>( cy ), P<float>( cz ), P<uint8_t>( flag ),
                              P<uint16_t>( code ), P<float>( rhs ) };
     }
-    BoraSolveTilesDev solve_tiles() { return BoraSolveTilesDev{ P<int4>( solve_tab ), P<uint32_t>( counters ) + 9, nft }; }
+    BoraSolveTilesDev solve_tiles() { return BoraSolveTilesDev{ P<int4>( solve_tab ), P<uint32_t>( counters ) + 9, nft, P<int32_t>( nbr ) }; }
     BoraTilesDev tiles() { return BoraTilesDev{ P<int32_t>( slot_of ), P<int32_t>( tile_of ), P<int32_t>( nbr ) }; }
     BoraSolverDev solver()
     {

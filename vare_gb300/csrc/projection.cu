@@ -1371,9 +1371,12 @@ __device__ __forceinline__ void refine_residual_body( const BoraSolveTilesDev& f
         }
         if( !mine ) continue;
         bora_st8( sv.r + g, r );
-        // a code that names a fluid neighbour in a tile that is not the solver's is inconsistent
-        if( ( ( seen & 1u ) && n0.x < 0 ) || ( ( seen & 2u ) && n0.y < 0 ) || ( ( seen & 4u ) && j == 0 && yt < 0 ) ||
-            ( ( seen & 8u ) && j == 7 && yt < 0 ) || ( ( seen & 16u ) && kk == 0 && zt < 0 ) || ( ( seen & 32u ) && kk == 3 && zt < 0 ) )
+        // a code that names a fluid neighbour in an inactive tile is inconsistent (in an active tile
+        // without fluid, where only a caller's codes name one, the neighbour counts as 0)
+        auto bad = [&]( uint32_t bit, bool missing, int dir ) { return ( seen & bit ) && missing && ft.nbr[(size_t)s * 27 + dir] < 0; };
+        if( bad( 1u, n0.x < 0, bora_dir( -1, 0, 0 ) ) || bad( 2u, n0.y < 0, bora_dir( 1, 0, 0 ) ) ||
+            bad( 4u, j == 0 && yt < 0, bora_dir( 0, -1, 0 ) ) || bad( 8u, j == 7 && yt < 0, bora_dir( 0, 1, 0 ) ) ||
+            bad( 16u, kk == 0 && zt < 0, bora_dir( 0, 0, -1 ) ) || bad( 32u, kk == 3 && zt < 0, bora_dir( 0, 0, 1 ) ) )
             atomicOr( red.err, 2u );
     }
     reduce2_publish_dfmax( n2, mx, red, slot_norm2, slot_max, bid, G );
