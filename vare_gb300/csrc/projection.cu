@@ -944,8 +944,9 @@ __device__ __forceinline__ bool meet( const ulonglong2* words, const PcgResident
             if( ok || n >= a.limit ) break;
             if( ( n & 255u ) == 255u && __any_sync( 0xffffffffu, *(volatile uint32_t*)a.red.err != 0u ) ) break;
         }
-        // one fence after the relaxed polls (acquiring loads would wait for one another)
-        if( ACQUIRE && lane == 0 ) asm volatile( "fence.acq_rel.gpu;" ::: "memory" );
+        // one fence after the relaxed polls (acquiring loads would wait for one another), by every lane:
+        // each has polled other blocks' words, and a fence orders what its own thread has read
+        if( ACQUIRE ) asm volatile( "fence.acq_rel.gpu;" ::: "memory" );
         if( !ok && lane == 0 ) atomicOr( a.red.err, (uint32_t)BORA_REDUCE_ERR_BARRIER );
         DF t[2] = { { 0.f, 0.f }, { 0.f, 0.f } };
 #pragma unroll
