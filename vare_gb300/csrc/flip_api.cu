@@ -511,12 +511,13 @@ int rebuild_sort( bora_flip_sim* s )
                                  P<int32_t>( s->tile_of ), st );
         bora_launch_tile_nbrs( s->g, ntiles, P<int32_t>( s->slot_of ), P<int32_t>( s->tile_of ), P<int32_t>( s->nbr ), st );
     }
+    // (one count past the outside bin, always 0: its prefix sum is the outside bin's end)
     {
         KTimer t( s, BORA_KERNEL_SORT, s->np ? 3 : 0 );
         bora_launch_hist( s->np, P<uint32_t>( s->vkey ), P<int32_t>( s->slot_of ), ncell, P<uint32_t>( s->key ),
                           P<uint32_t>( s->cell_count ), P<uint32_t>( s->counters ) + 2, st );
         s->stats.kernel_launches += (uint64_t)bora_device_scan( P<uint32_t>( s->cell_count ), P<uint32_t>( s->cell_start ),
-                                                                (size_t)ncell + 1, P<uint32_t>( s->scan_scratch ),
+                                                                (size_t)ncell + 2, P<uint32_t>( s->scan_scratch ),
                                                                 P<uint32_t>( s->counters ) + 1, st );
         bora_launch_scatter( s->np, P<uint32_t>( s->key ), P<uint32_t>( s->cell_start ), P<uint32_t>( s->cell_count ),
                              P<uint32_t>( s->idx ), st );
