@@ -5,6 +5,7 @@
 // grown geometrically and reused across steps; nothing is allocated inside a step
 // unless the particle count or the active-tile count outgrows its capacity.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -438,7 +439,9 @@ int read_counters( bora_flip_sim* s, int first, int count )
 }
 
 // A value that a kernel writes to mapped host memory (BoraReduceDev::mirror): marked as not
-// arrived before the launch, then polled. Sums of squares and maxima are never negative.
+// arrived before the launch, then polled. Sums of squares and maxima are never negative. A value
+// that has arrived says nothing about another one's store, so each is marked and polled itself; the
+// fence keeps what the caller reads next behind the poll (the host's loads may pass one another).
 constexpr double kNotArrived = -1.0;
 template <class T>
 int poll_mapped( volatile T* p, T none, cudaStream_t st, T* v )
@@ -446,11 +449,12 @@ int poll_mapped( volatile T* p, T none, cudaStream_t st, T* v )
     for( unsigned n = 1;; ++n )
     {
         *v = *p;
-        if( *v != none ) return BORA_OK;
+        if( *v != none ) { std::atomic_thread_fence( std::memory_order_acquire ); return BORA_OK; }
         if( n % 8192 ) continue;
         const cudaError_t e = cudaStreamQuery( st );  // an error, or nothing left that could write it
         if( e == cudaErrorNotReady ) continue;
         if( e != cudaSuccess ) return cuda_status( e );
+        std::atomic_thread_fence( std::memory_order_acquire );
         *v = *p;
         return *v != none ? BORA_OK : BORA_ERR_INTERNAL;
     }
@@ -874,13 +878,15 @@ int stage_solve( bora_flip_sim* s )
         const int s_n2 = s->slot(), s_mx = s->slot();
         arm_mirror( s, s_n2 );
         arm_mirror( s, s_mx );
+        arm_mirror( s, rr_cur );
         {
             KTimer t( s, BORA_KERNEL_REFINE, 2 );
             bora_launch_refine_accumulate( ft, code, sv, dsel, red, nparts, rr_cur, a_rz, a_dq, st );
             bora_launch_refine_residual( ft, b, code, sv, red, s_n2, s_mx, st );
         }
         BORA_TRYS( check_launch( s ) );
-        double n2 = 0.0;
+        double n2 = 0.0, rr_rec = 0.0;
+        BORA_TRYS( poll_mirror( s, rr_cur, st, &rr_rec ) );
         BORA_TRYS( poll_mirror( s, s_n2, st, &n2 ) );
         BORA_TRYS( poll_mirror( s, s_mx, st, &rmax ) );
         rnorm = std::sqrt( n2 );
@@ -893,9 +899,8 @@ int stage_solve( bora_flip_sim* s )
         }
         if( !std::isfinite( rnorm ) ) break;
         // Continue the recurrence only while the refined residual still agrees with the
-        // recursive one (the device finished the pass, so its last r.r is in mapped memory);
-        // a larger drift would break conjugacy, so the next pass restarts (beta = 0).
-        const double rr_rec = ( (volatile double*)s->h_mirror )[rr_cur];
+        // recursive one (the pass's last r.r, finished by the accumulation); a larger drift would
+        // break conjugacy, so the next pass restarts (beta = 0).
         const double rec = rr_rec > 0.0 ? std::sqrt( rr_rec ) : 0.0;
         if( !( rec > 0.0 ) || rnorm > 1.5 * rec ) rz_prev = -1;
     }
