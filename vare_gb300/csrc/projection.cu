@@ -36,15 +36,21 @@ __device__ __forceinline__ uint2 shfl2( uint2 w, int lane )
     return make_uint2( __shfl_sync( 0xffffffffu, w.x, lane ), __shfl_sync( 0xffffffffu, w.y, lane ) );
 }
 
-// A row's flags and those of the rows around it in y and z, and at its x ends.
+// A row's flags and those of the rows around it in y and z, and at its x ends. A cell beyond the grid
+// (the frame's extents are multiples of 4, so half a row or all of it) is air, whatever flag the
+// caller may have set there.
 struct RowFlags
 {
     uint2 w, ym, yp, zm, zp;
     int xm, xp;
-    __device__ __forceinline__ void load( const uint8_t* __restrict__ flag, const HalfRow& r )
+    bool in_grid[2];  // the row's cells 0..3, 4..7
+    __device__ __forceinline__ void load( const BoraGridDev& g, const uint8_t* __restrict__ flag, const HalfRow& r )
     {
         const int lane = threadIdx.x & 31;
         w = flags8( flag, r.mine ? r.s : -1, r.c );
+        in_grid[0] = r.J < g.ny && r.K < g.nz;
+        in_grid[1] = in_grid[0] && r.i0 + 4 < g.nx;
+        w = make_uint2( in_grid[0] ? w.x : 0u, in_grid[1] ? w.y : 0u );
         const uint2 y = flags8( flag, r.yt, r.yc ), z = flags8( flag, r.zt, r.zc );
         xm = r.xm < 0 ? BORA_AIR : flag[(size_t)r.xm * BORA_TILE_CELLS + r.c + 7];
         xp = r.xp < 0 ? BORA_AIR : flag[(size_t)r.xp * BORA_TILE_CELLS + r.c];
@@ -66,7 +72,7 @@ __global__ void __launch_bounds__( 32 * kRowWarps ) k_rhs( BoraGridDev g, BoraTi
     __shared__ int any[kRowWarps];
     const HalfRow r = half_row<kRowWarps>( g, t, ntiles );
     RowFlags f;
-    f.load( c.flag, r );
+    f.load( g, c.flag, r );
     const int own = r.mine ? r.s : -1;
     float vx[8], vy[8], vz[8], vym[8], vyp[8], vzm[8], vzp[8], yh[8], zh[8];
     row8( c.vx, own, r.c, vx );
@@ -1441,7 +1447,7 @@ __global__ void __launch_bounds__( 32 * kRowWarps ) k_air_pressure( BoraGridDev 
 {
     const HalfRow r = half_row<kRowWarps>( g, t, ntiles );
     RowFlags f;
-    f.load( c.flag, r );
+    f.load( g, c.flag, r );
     constexpr uint32_t kAllFluid = 0x01010101u * BORA_FLUID;
     if( __all_sync( 0xffffffffu, !r.mine || ( f.w.x == kAllFluid && f.w.y == kAllFluid ) ) ) return;
     const int own = r.mine ? r.s : -1;
@@ -1466,7 +1472,7 @@ __global__ void __launch_bounds__( 32 * kRowWarps ) k_air_pressure( BoraGridDev 
         m.add( r.J < EJ, flag_of( f.yp, q ), pyp[q] );
         m.add( r.K > 0, flag_of( f.zm, q ), pzm[q] );
         m.add( r.K < EK, flag_of( f.zp, q ), pzp[q] );
-        out[q] = own_flag == BORA_FLUID ? p[q] : ( own_flag == BORA_AIR ? m.value() : 0.f );
+        out[q] = own_flag == BORA_FLUID ? p[q] : ( own_flag == BORA_AIR && f.in_grid[q >> 2] ? m.value() : 0.f );
     }
     if( !r.mine ) return;
     // fluid cells are not stored: other warps read them
@@ -1498,7 +1504,7 @@ __global__ void __launch_bounds__( 32 * kRowWarps ) k_vel_update( const __grid_c
 {
     const HalfRow r = half_row<kRowWarps>( g, t, ntiles );
     RowFlags f;
-    f.load( c.flag, r );
+    f.load( g, c.flag, r );
     const int own = r.mine ? r.s : -1;
     float p[8], pym[8], pyp[8], pzm[8], pzp[8], yh[8], zh[8], vx[8], vy[8], vz[8];
     row8( c.pres, own, r.c, p );
