@@ -378,8 +378,9 @@ __global__ void __launch_bounds__( 32 * kTilesPerCta ) k_mic_factor( BoraSolveTi
 // shuffles. A row's cells sit in eight registers rotated by (j + k + 1) mod 8, so that step u
 // finds its cell in register u mod 8 in every lane (r is rotated in three select stages; M2 is
 // stored rotated). Steps outside a row's eight cells yield 0, which feeds the row's first cell a
-// zero neighbour. r.z = sum of w t (r.M^-1 r = y.y), all terms >= 0. Non-fluid
-// cells have M2 = 0 and r = 0.
+// zero neighbour. r.z = sum of w t (r.M^-1 r = y.y), all terms >= 0, in FP32 over four cells (a
+// row's eight lie at consecutive steps, so exactly four of them at steps with bit 2 set), then in
+// double-float. Non-fluid cells have M2 = 0 and r = 0.
 //
 // Bound by latency and issue: 44 dependent steps of a shuffle and three arithmetic
 // instructions, about 900 warp instructions per tile. The earlier form kept the tile in shared
@@ -406,11 +407,11 @@ __device__ __forceinline__ void rotate8( float* v, int rho )
 }
 
 // z = M^-1 r of one tile: rA, rB hold the lane's rows of r and return z (both in cell order);
-// mA, mB the rows' squared pivots as stored (rotated). Returns the lane's part of r.z. ROLLED: a
+// mA, mB the rows' squared pivots as stored (rotated). Adds the lane's part of r.z to prz. ROLLED: a
 // third of the code, for a kernel whose one warp per SM partition would wait for its instructions
 // (the grid kernel is faster unrolled: 18.3 against 18.7 ms of GPU time per 256^3 step).
 template <bool ROLLED>
-__device__ __forceinline__ float mic_sweeps( float* rA, float* rB, const float* mA, const float* mB )
+__device__ __forceinline__ void mic_sweeps( float* rA, float* rB, const float* mA, const float* mB, DF& prz )
 {
     constexpr unsigned kAllLanes = 0xffffffffu;
     const int lane = threadIdx.x & 31, j = lane & 7, kq = lane >> 3, sA = j + 2 * kq, rho = ( sA + 1 ) & 7;
@@ -418,7 +419,7 @@ __device__ __forceinline__ float mic_sweeps( float* rA, float* rB, const float* 
     const unsigned live = 0xffu << ( sA + 1 );  // bit u: row A has a cell at step u (row B: at step u + 1)
     rotate8( rA, rho );
     rotate8( rB, rho );  // row B's cell of step u is register (u - 1) mod 8
-    float wA = 0.f, wB = 0.f, rzA = 0.f, rzB = 0.f;
+    float wA = 0.f, wB = 0.f, rzA[2] = { 0.f, 0.f }, rzB[2] = { 0.f, 0.f };
     // three rounds of eight steps (none past step 22): a register's steps are eight apart, so the
     // round can be the body of a loop
     constexpr int kRounds = ROLLED ? 1 : 3;
@@ -439,8 +440,8 @@ __device__ __forceinline__ float mic_sweeps( float* rA, float* rB, const float* 
             const float tB = fmaf( ym, yB, ( cB + wB ) + wA );
             wA = a ? mA[v & 7] * tA : 0.f;
             wB = b ? mB[v & 7] * tB : 0.f;
-            rzA = fmaf( wA, tA, rzA );
-            rzB = fmaf( wB, tB, rzB );
+            rzA[( v >> 2 ) & 1] = fmaf( wA, tA, rzA[( v >> 2 ) & 1] );
+            rzB[( v >> 2 ) & 1] = fmaf( wB, tB, rzB[( v >> 2 ) & 1] );
             cA = a ? wA : cA;
             cB = b ? wB : cB;
         }
@@ -468,7 +469,8 @@ __device__ __forceinline__ float mic_sweeps( float* rA, float* rB, const float* 
     }
     rotate8( rA, ( 8 - rho ) & 7 );
     rotate8( rB, ( 8 - rho ) & 7 );
-    return rzA + rzB;
+#pragma unroll
+    for( int q = 0; q < 2; ++q ) prz = df_add_f( df_add_f( prz, rzA[q] ), rzB[q] );
 }
 
 // The update of the warp's tiles first, first + tstride, ...: r -= alpha q, z = M^-1 r; r.z and
@@ -514,7 +516,7 @@ __device__ __forceinline__ void pcg_update_tiles( const BoraSolveTilesDev& ft, c
             prr = df_add_f( prr, dot4( make_float4( rA[h], rA[h + 1], rA[h + 2], rA[h + 3] ), make_float4( rA[h], rA[h + 1], rA[h + 2], rA[h + 3] ) ) );
             prr = df_add_f( prr, dot4( make_float4( rB[h], rB[h + 1], rB[h + 2], rB[h + 3] ), make_float4( rB[h], rB[h + 1], rB[h + 2], rB[h + 3] ) ) );
         }
-        prz = df_add_f( prz, mic_sweeps<false>( rA, rB, mA, mB ) );
+        mic_sweeps<false>( rA, rB, mA, mB, prz );
         bora_st8( sv.z + o, rA );
         bora_st8( sv.z + o + 64, rB );
     }
@@ -1059,7 +1061,7 @@ __global__ void __launch_bounds__( 32 * W, 1 ) k_pcg_resident( const __grid_cons
         }
 #pragma unroll
         for( int i = 0; i < 8; ++i ) { zA[i] = rA[i]; zB[i] = rB[i]; }
-        v[0] = df_add_f( v[0], mic_sweeps<true>( zA, zB, mA, mB ) );
+        mic_sweeps<true>( zA, zB, mA, mB, v[0] );
         if( mine )
         {
             bora_st8( a.sv.z + g, zA );
