@@ -22,7 +22,7 @@ __device__ __forceinline__ DF df_prod( float a, float b )
     const float p = __fmul_rn( a, b );
     return DF{ p, fmaf( a, b, -p ) };
 }
-__device__ __forceinline__ DF df_add( DF a, DF b )
+__host__ __device__ __forceinline__ DF df_add( DF a, DF b )
 {
     const float s = a.hi + b.hi;
     const float bb = s - a.hi;
@@ -197,13 +197,19 @@ __device__ __forceinline__ DF df_warp_sum_df( DF v )
 }
 
 // (float)( a / b ) of two double-float values: the quotient of the high parts corrected by one
-// residual step (within an ulp of the rounded quotient).
-__device__ __forceinline__ float df_ratio( float2 a, float2 b )
+// residual step, which rounds the quotient of the pairs once (off by 0.5 + 2^-22 ulp at most, as
+// the FP64 quotient rounded to FP32). Small operands are scaled by a power of two, so that the
+// remainder does not lose bits below FP32's smallest normal number.
+__host__ __device__ __forceinline__ float df_ratio( float2 a, float2 b )
 {
+    constexpr float kSmall = 1e-20f, kUp = 1.152921504606847e18f, kDown = 1.f / kUp;  // 2^60
+    float back = 1.f;
+    if( fabsf( a.x ) < kSmall ) { a.x *= kUp; a.y *= kUp; back = kDown; }
+    if( fabsf( b.x ) < kSmall ) { b.x *= kUp; b.y *= kUp; back *= kUp; }
     const float q = a.x / b.x;
     const float rem = fmaf( -q, b.x, a.x ) + fmaf( -q, b.y, a.y );
     const float c = rem / b.x;
-    return isfinite( c ) ? q + c : q;
+    return ( isfinite( c ) ? q + c : q ) * back;
 }
 
 // The block's sums of v0 and v1 into part0[bid] and part1[bid] (part1 may be null). Called once per
