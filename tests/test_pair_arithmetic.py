@@ -8,7 +8,10 @@ exponent that a sum of squares in FP32 can have.
 
 df_add: partial sums of up to kBoraMaxReduceBlocks blocks, added as part_collect does. An addition of
 two pairs of one sign is off by 3 * 2^-48 at most (Joldes, Muller and Popescu, ACM TOMS 44, 2017);
-19 + 5 + 3 of them follow one another, so the sum is off by 2^-41 at most."""
+19 + 5 + 3 of them follow one another, so the sum is off by 2^-41 at most.
+
+residual_scale: a power of two, so that the V-cycle's scaling of the residual and its undoing round
+nothing, with the scaled norm in [1, 2)."""
 import ctypes
 import math
 import os
@@ -34,6 +37,10 @@ extern "C" void add( int n, const float* a, const float* b, float* out )
         out[2 * i] = s.hi;
         out[2 * i + 1] = s.lo;
     }
+}
+extern "C" void scales( int n, const double* rr, float* out )
+{
+    for( int i = 0; i < n; ++i ) out[i] = residual_scale( rr[i] );
 }
 """
 
@@ -92,3 +99,19 @@ def test_partial_sums(lib, n, spread):
         t = _call(lib.add, t, acc[32 * w:32 * w + 1], 2)
     want = math.fsum(p.astype(np.float64).ravel())
     assert abs(float(t.astype(np.float64).sum()) - want) <= 2.0 ** -41 * want
+
+
+def test_scale(lib):
+    rng = np.random.default_rng(2)
+    rr = np.concatenate([10.0 ** rng.uniform(-70, 70, 20000), 4.0 ** np.arange(-100, 100), 2.0 * 4.0 ** np.arange(-100, 100)])
+    sc = np.zeros(len(rr), np.float32)
+    lib.scales(len(rr), rr.ctypes.data_as(ctypes.c_void_p), sc.ctypes.data_as(ctypes.c_void_p))
+    assert (np.frexp(sc)[0] == 0.5).all()
+    norm = sc.astype(np.float64) * np.sqrt(rr)
+    assert norm.min() >= 1.0 and norm.max() < 2.0
+    r = rng.standard_normal(len(rr)).astype(np.float32) * np.float32(1e-3) / sc
+    np.testing.assert_array_equal(r * sc * (np.float32(1) / sc), r)
+    rr = np.array([0.0, np.inf, np.nan, 1e-300, 1e300])
+    sc = np.zeros(len(rr), np.float32)
+    lib.scales(len(rr), rr.ctypes.data_as(ctypes.c_void_p), sc.ctypes.data_as(ctypes.c_void_p))
+    assert (sc[:3] == 1).all() and np.isfinite(sc).all() and (sc > 0).all()

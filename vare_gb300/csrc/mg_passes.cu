@@ -11,9 +11,9 @@
 //           neighbours' za).                                                    zb -> scratch
 //   up 2    z = S_A(zb) (the neighbours' zb); level 0 unscales into the FP32 z of the PCG and
 //           sums r.z, the other levels store FP16 z1 for the finer level's up 1
-// where r' = r * sc on level 0 (sc = 1 / ||r|| of the latest residual whose norm is known: it
-// keeps the FP16 levels' values O(1), and the V-cycle is linear in r, so any scale serves) and r
-// on the others,
+// where r' = r * sc on level 0 (sc = the power of two that brings ||r|| of the latest residual whose
+// norm is known to [1, 2): it keeps the FP16 levels' values O(1), scaling and unscaling are exact,
+// and the V-cycle is linear in r, so any scale serves) and r on the others,
 // S_w(v) = v + (w / d) (r' - (d v - sum of the neighbours' v)) on fluid cells and 0 elsewhere,
 // neighbour sums in the order ((x- + x+) + (y- + y+)) + (z- + z+), and the 8 children summed as
 // ((x pairs) + (y pairs)) + (z pairs). Every cell is computed once per pass; the scratch is
@@ -76,16 +76,6 @@ __device__ __forceinline__ void init_weights( float* w )
 __device__ __forceinline__ float sweep( float v, float r, uint16_t c, float sum, const float* w )
 {
     return cfluid( c ) ? v + w[cdiag( c )] * ( r - ( (float)cdiag( c ) * v - sum ) ) : 0.f;
-}
-
-__device__ __forceinline__ float scale_from( const double* ring, int slot )
-{
-    // in FP64 only where FP32 may not hold it: the root and the quotient are half a microsecond of
-    // latency in each of level 0's passes (V-cycle 43.6 us at 96^3, 41.9 so; 86.9 and 84.2 at 192^3)
-    const double rr = ring[slot];
-    const float f = (float)rr;
-    if( f >= 1e-36f && f <= 1e36f ) return 1.f / sqrtf( f );
-    return rr > 0.0 ? (float)( 1.0 / sqrt( rr ) ) : 1.f;
 }
 
 // ---- level 0: one warp per half tile ---------------------------------------------------------
@@ -332,7 +322,7 @@ __device__ __forceinline__ void pass0_body( const Pass0Args& a, unsigned bid, un
     codes( h );
     __shared__ float2 s_dq[W];
     bora_pdl_wait();  // the previous kernel's results are complete from here
-    if( threadIdx.x == 0 ) s_sc = scale_from( a.red.ring, a.slot_rr );
+    if( threadIdx.x == 0 ) s_sc = residual_scale( a.red.ring[a.slot_rr] );
     const bool upd = ( P == 0 || P == 1 ) && a.slot_rz_in >= 0;  // down 1, 2 apply r -= alpha q
     float alpha = 0.f;
     if( P == 0 && upd )

@@ -1,6 +1,8 @@
 // FP64-accurate, deterministic reductions shared by the solver kernels.
 #pragma once
 
+#include <cstring>
+
 #include "bora_internal.h"
 
 namespace bora_reduce {
@@ -210,6 +212,21 @@ __host__ __device__ __forceinline__ float df_ratio( float2 a, float2 b )
     const float rem = fmaf( -q, b.x, a.x ) + fmaf( -q, b.y, a.y );
     const float c = rem / b.x;
     return ( isfinite( c ) ? q + c : q ) * back;
+}
+
+// The V-cycle's scale of a residual with r.r = rr: the power of two 2^-k with 2^k <= sqrt( rr ) < 2^(k + 1),
+// within FP32's normal range (1 for rr = 0 or not finite). A product with it, and with its
+// reciprocal, is exact; a quotient by the norm's root would be rounded twice per cell.
+__host__ __device__ __forceinline__ float residual_scale( double rr )
+{
+    unsigned long long u;
+    memcpy( &u, &rr, 8 );
+    if( !( rr > 0.0 ) || u >> 52 == 0x7ffu ) return 1.f;
+    const int k = ( (int)( u >> 52 ) - 1023 ) >> 1;  // from the exponents' bits: 2^(2k) <= rr < 2^(2k + 2)
+    const unsigned w = (unsigned)( 127 - ( k < -126 ? -126 : ( k > 126 ? 126 : k ) ) ) << 23;
+    float sc;
+    memcpy( &sc, &w, 4 );
+    return sc;
 }
 
 // The block's sums of v0 and v1 into part0[bid] and part1[bid] (part1 may be null). Called once per
