@@ -892,7 +892,8 @@ struct PcgResidentArgs
     int dsel;               // the buffer of the last search direction (read and left there)
     int slot_rz_prev;       // r.z before the last update of the previous pass, or -1 (restart)
     int max_inner;
-    float2 target2;         // stop once r.r <= target2 (a double-float pair)
+    double target2;         // stop once r.r <= target2
+    float above;            // an r.r that is not: its FP64 test, 0.2 us (0.8 with a root), is only formed at the end
     int slot_a_rz;          // out: r.z before the last update; r.r is left as the one partial sum part_rr[0]
     uint32_t* iters;        // out (mapped host memory): iterations run; not written when a wait ran out
     ulonglong2* words_rz;   // two per block: r.z, r.r
@@ -1079,8 +1080,13 @@ __global__ void __launch_bounds__( 32 * W, 1 ) k_pcg_resident( const __grid_cons
         precondition( tag );
         if( !meet<2, true>( a.words_rz, a, tag, sum, &s_met[0] ) ) return;
         const DF rz = sum[0], rr = sum[1];
-        const bool small = !( rr.hi > 0.f ) || rr.hi < a.target2.x || ( rr.hi == a.target2.x && rr.lo <= a.target2.y );
-        if( it >= a.max_inner || ( it > 0 && __any_sync( kAll, small ) ) )
+        bool small = false;
+        if( __any_sync( kAll, !( rr.hi > a.above ) ) )
+        {
+            const double rrd = (double)rr.hi + (double)rr.lo;
+            small = __any_sync( kAll, !( rrd > 0.0 ) || rrd <= a.target2 );
+        }
+        if( it >= a.max_inner || ( it > 0 && small ) )
         {
             // the pass is done: it iterations
             if( mine )
@@ -1765,9 +1771,8 @@ int bora_launch_pcg_resident( BoraSolveTilesDev t, const uint16_t* code, BoraSol
     if( W == 0 ) return -1;
     PcgResidentArgs a{};
     a.ft = t; a.code = code; a.sv = s; a.red = red; a.dsel = dsel; a.slot_rz_prev = slot_rz_prev; a.max_inner = max_inner;
-    const double t2 = target * target;
-    const float hi = (float)t2;
-    a.target2 = make_float2( hi, (float)( t2 - (double)hi ) );
+    a.target2 = target * target;
+    a.above = (float)( a.target2 * ( 1.0 + 1e-6 ) );
     a.slot_a_rz = slot_a_rz; a.iters = iters;
     a.words_rz = static_cast<ulonglong2*>( words );
     a.words_dq = a.words_rz + 2 * ( kResidentBlocks + 8 );
