@@ -97,8 +97,10 @@ typedef struct bora_flip_params
                                 PCG in one cooperative launch whose phases meet at bounded grid
                                 barriers and which checks convergence itself, every iteration. Small
                                 systems (up to 608 tiles with fluid, proj_iteration up to 2^24) run
-                                that way with either value, where it is the faster form, unless the
-                                PCG's phases are being timed (bora_flip_set_profiling) */
+                                in one launch with either value, where it is the faster form, and stop
+                                by the rule of the value (with 0: every check_every-th iteration is
+                                tested and one more follows), unless the PCG's phases are being timed
+                                (bora_flip_set_profiling) */
     int warm_start;          /* 0: every pressure solve starts from p = 0, as the reference's does
                                 (its pressure field is re-created with the frame each step,
                                 FLIPMethod.cu:28-33, FluidProjection.cu:265); 1: from the last

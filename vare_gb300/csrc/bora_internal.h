@@ -278,14 +278,15 @@ int bora_launch_pcg_persistent( BoraSolveTilesDev t, const uint16_t* code, BoraS
                                 int dsel, int slot_rz_prev, int max_inner, double target, int slot_a_rz, int slot_a_dq,
                                 uint32_t* iters, unsigned* bar, double* part, bool never_release, cudaStream_t st );
 // The same for systems of up to 608 solver tiles, one warp per tile with its vectors in
-// registers (projection.cu). No update is pending afterwards (e is complete); slot_a_rz: r.z before
+// registers (projection.cu). ||r|| is tested every `check` iterations; `beyond` more follow one that
+// reaches the target. No update is pending afterwards (e is complete); slot_a_rz: r.z before
 // the last update. words: bora_pcg_resident_words_bytes() of device memory, zeroed once; the launch
 // uses the tags tag .. tag + 2 max_inner, which no earlier launch over these words may have used.
 int bora_pcg_resident_warps( int nft );  // warps per block, 0: too large
 size_t bora_pcg_resident_words_bytes();
 int bora_launch_pcg_resident( BoraSolveTilesDev t, const uint16_t* code, BoraSolverDev s, BoraReduceDev red, int dsel,
-                              int slot_rz_prev, int max_inner, double target, int slot_a_rz, uint32_t* iters, void* words,
-                              uint32_t tag, bool never_release, cudaStream_t st );
+                              int slot_rz_prev, int max_inner, int check, int beyond, double target, int slot_a_rz,
+                              uint32_t* iters, void* words, uint32_t tag, bool never_release, cudaStream_t st );
 // d' = z + beta d; q = A d'; partial sums of dq (beta = rz_new / rz_old, or 0 when slot_rz_old < 0). Finishes rz
 // and rr from nparts producer blocks' partials into slot_rz_new and slot_rr (host_rr: rr also for the host).
 void bora_launch_pcg_direction( BoraSolveTilesDev t, const uint16_t* code, BoraSolverDev s, int dsel_in, BoraReduceDev red, int nparts, int slot_rz_new, int slot_rr, int slot_rz_old,

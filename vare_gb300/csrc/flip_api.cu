@@ -784,8 +784,11 @@ int stage_solve( bora_flip_sim* s )
             }
             ( (volatile uint32_t*)s->h_cnt )[8] = kCountNotArrived;
             s->stats.kernel_launches += 1;
-            resident = bora_launch_pcg_resident( ft, code, sv, red, dsel, rz_prev, max_inner, target, s_a_rz, s->d_cnt + 8,
-                                                 s->meet.p, s->meet_tag, p.persistent && s->fault == BORA_FAULT_BARRIER, st ) == 0;
+            // stopped by the rule of the form whose place it takes: every check-th iteration is tested, and one
+            // more follows (it is queued when the host reads the test); the persistent form's each, at once
+            resident = bora_launch_pcg_resident( ft, code, sv, red, dsel, rz_prev, max_inner, p.persistent ? 1 : check,
+                                                 p.persistent ? 0 : 1, target, s_a_rz, s->d_cnt + 8, s->meet.p, s->meet_tag,
+                                                 p.persistent && s->fault == BORA_FAULT_BARRIER, st ) == 0;
             if( resident )
             {
                 s->meet_tag += tags;

@@ -892,6 +892,7 @@ struct PcgResidentArgs
     int dsel;               // the buffer of the last search direction (read and left there)
     int slot_rz_prev;       // r.z before the last update of the previous pass, or -1 (restart)
     int max_inner;
+    int check, beyond;      // iterations between stop tests; iterations that a pass runs on after one that holds
     double target2;         // stop once r.r <= target2
     float above;            // an r.r that is not: its FP64 test, 0.2 us (0.8 with a root), is only formed at the end
     int slot_a_rz;          // out: r.z before the last update; r.r is left as the one partial sum part_rr[0]
@@ -1073,6 +1074,7 @@ __global__ void __launch_bounds__( 32 * W, 1 ) k_pcg_resident( const __grid_cons
     uint32_t tag = a.tag;
     DF rz_prev{ 0.f, 0.f }, sum[2];
     bool cont = a.slot_rz_prev >= 0;  // the recurrence continues from d
+    int last = a.max_inner, due = a.check;  // the pass's last iteration; the next one to be tested
     if( cont ) rz_prev = DF{ a.red.ringf[a.slot_rz_prev].x, a.red.ringf[a.slot_rz_prev].y };
 #pragma unroll 1
     for( int it = 0;; ++it, ++tag )
@@ -1080,13 +1082,16 @@ __global__ void __launch_bounds__( 32 * W, 1 ) k_pcg_resident( const __grid_cons
         precondition( tag );
         if( !meet<2, true>( a.words_rz, a, tag, sum, &s_met[0] ) ) return;
         const DF rz = sum[0], rr = sum[1];
-        bool small = false;
-        if( __any_sync( kAll, !( rr.hi > a.above ) ) )
+        if( it == due )
         {
-            const double rrd = (double)rr.hi + (double)rr.lo;
-            small = __any_sync( kAll, !( rrd > 0.0 ) || rrd <= a.target2 );
+            due += a.check;
+            if( __any_sync( kAll, !( rr.hi > a.above ) ) )
+            {
+                const double rrd = (double)rr.hi + (double)rr.lo;
+                if( __any_sync( kAll, !( rrd > 0.0 ) || rrd <= a.target2 ) ) last = min( last, it + a.beyond );
+            }
         }
-        if( it >= a.max_inner || ( it > 0 && small ) )
+        if( it >= last )
         {
             // the pass is done: it iterations
             if( mine )
@@ -1764,13 +1769,15 @@ int bora_pcg_resident_warps( int nft )
 size_t bora_pcg_resident_words_bytes() { return (size_t)3 * ( kResidentBlocks + 8 ) * sizeof( ulonglong2 ); }
 
 int bora_launch_pcg_resident( BoraSolveTilesDev t, const uint16_t* code, BoraSolverDev s, BoraReduceDev red, int dsel,
-                              int slot_rz_prev, int max_inner, double target, int slot_a_rz, uint32_t* iters, void* words,
-                              uint32_t tag, bool never_release, cudaStream_t st )
+                              int slot_rz_prev, int max_inner, int check, int beyond, double target, int slot_a_rz,
+                              uint32_t* iters, void* words, uint32_t tag, bool never_release, cudaStream_t st )
 {
     const int W = bora_pcg_resident_warps( t.n );
     if( W == 0 ) return -1;
     PcgResidentArgs a{};
     a.ft = t; a.code = code; a.sv = s; a.red = red; a.dsel = dsel; a.slot_rz_prev = slot_rz_prev; a.max_inner = max_inner;
+    a.check = check;
+    a.beyond = beyond;
     a.target2 = target * target;
     a.above = (float)( a.target2 * ( 1.0 + 1e-6 ) );
     a.slot_a_rz = slot_a_rz; a.iters = iters;
