@@ -99,8 +99,8 @@ typedef struct bora_flip_params
                                 systems (up to 608 tiles with fluid, proj_iteration up to 2^24) run
                                 in one launch with either value, where it is the faster form, and stop
                                 by the rule of the value (with 0: every check_every-th iteration is
-                                tested and one more follows), unless the PCG's phases are being timed
-                                (bora_flip_set_profiling) */
+                                tested and one more follows), unless the PCG's two phases are being
+                                timed (bora_flip_set_profiling) */
     int warm_start;          /* 0: every pressure solve starts from p = 0, as the reference's does
                                 (its pressure field is re-created with the frame each step,
                                 FLIPMethod.cu:28-33, FluidProjection.cu:265); 1: from the last
@@ -146,6 +146,7 @@ typedef struct bora_flip_stats
 #define BORA_KERNEL_G2P 9
 #define BORA_KERNEL_MG 10          /* multigrid V-cycle (mixed solver) */
 #define BORA_KERNEL_POST 11        /* post-processing: splat, tank scan, redistancing, attributes */
+#define BORA_KERNEL_PCG_PASS 12    /* a refinement pass in one launch (small plain systems; see persistent) */
 #define BORA_KERNEL_CLASSES 16
 
 /* Simulation frame description (after padding). */
@@ -330,9 +331,11 @@ int bora_flip_set_field( bora_flip_handle h, int which, const void* in, size_t b
 int bora_flip_get_stats( bora_flip_handle h, bora_flip_stats* out );
 
 /* Record CUDA events around every launch of the kernel classes in `class_mask` (bit c =
- * class c) and accumulate their device time; setting a mask resets the totals. Timing the PCG's
- * direction or update class makes small plain systems run per phase too (see persistent), whose
- * results differ from the one-launch form's by the solver's tolerance. */
+ * class c) and accumulate their device time; setting a mask resets the totals. A small plain
+ * system's pressure solve runs in one launch per pass (see persistent): BORA_KERNEL_PCG_PASS times
+ * it as it runs. Asking for the PCG's direction or update class instead makes such a system run
+ * per phase, stopped by the same rule; its sums are rounded differently, so its results differ from
+ * the one-launch form's by the solver's tolerance. No other class changes a result. */
 int bora_flip_set_profiling( bora_flip_handle h, uint32_t class_mask );
 /* Time only one in `every` brackets of each profiled class (1, the default: all). A bracket
  * records an event on the handle's stream before and after the class's kernels, which ends the

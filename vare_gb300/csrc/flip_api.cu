@@ -783,7 +783,7 @@ int stage_solve( bora_flip_sim* s )
                 s->meet_tag = 1;
             }
             ( (volatile uint32_t*)s->h_cnt )[8] = kCountNotArrived;
-            s->stats.kernel_launches += 1;
+            KTimer t( s, BORA_KERNEL_PCG_PASS, 1 );
             // stopped by the rule of the form whose place it takes: every check-th iteration is tested, and one
             // more follows (it is queued when the host reads the test); the persistent form's each, at once
             resident = bora_launch_pcg_resident( ft, code, sv, red, dsel, rz_prev, max_inner, p.persistent ? 1 : check,
