@@ -168,11 +168,10 @@ __global__ void k_scatter( size_t n, const uint32_t* __restrict__ key, const uin
     }
 }
 
-// Order the particles of every dual cell by their source index (insertion sort of each
-// bin of the permutation, in place). The counting-sort scatter fills a bin in atomic
-// arrival order; this makes the order - and so every floating-point sum over a bin - a
-// function of the input only. Bins larger than `max_bin` (possible only for the bin of
-// particles outside the grid) keep their arrival order.
+// Order the particles of every dual cell by their source index, in place in the permutation. The
+// counting-sort scatter fills a bin in atomic arrival order; this makes the order - and so every
+// floating-point sum over a bin - a function of the input only. Bins larger than `max_bin`
+// keep their arrival order.
 // Batcher's odd-even merge sort (Knuth, TAOCP vol. 3, 5.3.4) on 16 inputs: comparator pairs
 // (a, b), a < b, in the order applied.
 constexpr int kSortNet16 = 63;
@@ -212,10 +211,43 @@ __device__ __forceinline__ void warp_sort( uint32_t* idx, uint32_t n )
         if( 32 * m + lane < n ) idx[r[m]] = v[m];
 }
 
+// Orders a bin of any n by the warp: pieces of 128 by warp_sort, then merged in the bin's memory by
+// bitonic steps that only ever put the smaller entry first (Knuth, TAOCP vol. 3, 5.3.4, with the
+// first step of a merge reversed), so that a place past the end counts as larger than all.
+__device__ __forceinline__ void warp_merge_sort( uint32_t* idx, uint32_t n )
+{
+    const uint32_t lane = threadIdx.x & 31;
+    for( uint32_t b = 0; b < n; b += 32 * kWarpSort ) warp_sort( idx + b, min( n - b, 32u * kWarpSort ) );
+    __syncwarp();
+    auto order = [&]( uint32_t i, uint32_t j ) {
+        if( j >= n ) return;
+        const uint32_t a = idx[i], c = idx[j];
+        if( a > c ) { idx[i] = c; idx[j] = a; }
+    };
+    for( int lg = 8; ( n - 1 ) >> ( lg - 1 ); ++lg )  // merges into sorted pieces of 2^lg
+    {
+        for( int h = lg - 1; h >= 0; --h )
+        {
+            const uint32_t low = ( 1u << h ) - 1u;
+#pragma unroll 4
+            for( uint32_t p = lane; ; p += 32 )  // pair p: its first place grows with p
+            {
+                const uint32_t i = ( ( p & ~low ) << 1 ) | ( p & low );
+                if( i >= n ) break;
+                order( i, h == lg - 1 ? i ^ ( 2 * low + 1u ) : i + low + 1u );
+            }
+            __syncwarp();
+        }
+    }
+}
+
 // A lane sorts a bin of up to 16 entries in registers; larger ones (the dual cells at the domain's
 // faces hold up to 27 particles at 8 a cell, dense emissions more) are ordered by the warp one
 // after the other, because a lane's insertion sort in memory is a chain of loads and stores: the
 // whole sort took 36 us at 24^3, 63 at 96^3, 352 at 256^3 with these few bins, 26, 47 and 323 now.
+// Dense emissions, 100, 140, 200, 500 and 1000 particles in each of 8192 (4096, 2048) neighbouring
+// bins: 0.13, 0.29, 0.38, 1.1 and 2.2 ms (a lane's insertion sort per bin, the lanes side by side, 0.91,
+// 1.7, 3.1, 32 and 116 ms; one such lane after the other from 129 particles on 0.65, 11, 21, 122 and 481).
 __global__ void k_order_bins( size_t nbins, const uint32_t* __restrict__ start, uint32_t* idx, uint32_t max_bin )
 {
     constexpr int kReg = 16;  // bins up to this size are sorted in registers
@@ -254,14 +286,7 @@ __global__ void k_order_bins( size_t nbins, const uint32_t* __restrict__ start, 
             const int src = __ffs( big ) - 1;
             const uint32_t qb = __shfl_sync( 0xffffffffu, q0, src ), nb = __shfl_sync( 0xffffffffu, n, src );
             if( nb <= 32 * kWarpSort ) warp_sort( idx + qb, nb );
-            else if( lane == src )
-                for( uint32_t q = q0 + 1; q < q0 + n; ++q )
-                {
-                    const uint32_t v = idx[q];
-                    uint32_t r = q;
-                    while( r > q0 && idx[r - 1] > v ) { idx[r] = idx[r - 1]; --r; }
-                    idx[r] = v;
-                }
+            else warp_merge_sort( idx + qb, nb );
         }
     }
 }
