@@ -11,7 +11,9 @@
 // summation order of a reduction are never tuned.
 //
 // The table can be loaded from and saved to a text file (BORA_TUNE_FILE: one line per entry,
-// "group device size_class variant median_ms"), so a deployment reuses measured shapes.
+// "code device size_class variant median_ms", code = 100 kLayout + group), so a deployment reuses
+// measured shapes. kLayout counts up with every change of what a shape or a unit is; a line of
+// another layout (the first had the bare group) is passed over, and its shape measured again.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -29,6 +31,9 @@
 namespace {
 
 constexpr int kSamples = 3;
+// 1: shapes in tiles per block and cells per block, units active tiles; 2: half tiles and rows per
+// block, units solver tiles
+constexpr int kLayout = 2;
 
 struct Entry
 {
@@ -68,6 +73,8 @@ struct Tuner
         double m;
         while( std::fscanf( f, "%d %d %d %d %lf", &g, &d, &c, &v, &m ) == 5 )
         {
+            if( g / 100 != kLayout ) continue;
+            g %= 100;
             if( g < 0 || g >= kBoraTuneGroups || v < 0 || v >= bora_tune_variants( g ) ) continue;
             Entry& e = table[std::make_tuple( g, d, c )];
             e.nvar = bora_tune_variants( g );
@@ -85,7 +92,7 @@ struct Tuner
         if( !f ) return;
         for( const auto& kv : table )
             if( kv.second.chosen >= 0 )
-                std::fprintf( f, "%d %d %d %d %.6f\n", std::get<0>( kv.first ), std::get<1>( kv.first ),
+                std::fprintf( f, "%d %d %d %d %.6f\n", 100 * kLayout + std::get<0>( kv.first ), std::get<1>( kv.first ),
                               std::get<2>( kv.first ), kv.second.chosen, kv.second.best_ms );
         std::fclose( f );
     }
@@ -128,7 +135,7 @@ int bora_tune_variants( int group )
 {
     switch( group )
     {
-    case kBoraTuneL0: case kBoraTuneL0Batch: return 3;  // 2, 4, 8 warps (tiles) per block
+    case kBoraTuneL0: case kBoraTuneL0Batch: return 3;  // 2, 4, 8 half tiles (warps) per block
     case kBoraTuneL1: case kBoraTuneL2: case kBoraTuneL1Batch: case kBoraTuneL2Batch: return 4;  // 64 .. 512 threads
     default: return 1;
     }
