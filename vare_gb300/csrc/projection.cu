@@ -881,8 +881,6 @@ __global__ void __launch_bounds__( 32 * kUpdWarps, 3 ) k_pcg_persistent( const _
 // fence 1.0 K, the two meetings 4.6 K, the stencil 1.2 K. Code that fits the instruction caches
 // matters (one warp per SM partition hides no fetch: 10 x slower at 100 KB): rolled sweeps, one
 // copy of each part, control flow that the compiler knows to be uniform.
-// GPU time of a step against the per-phase form: 0.46 against 0.69 ms at 15 solver tiles, 1.17
-// against 1.40 at 180, 1.73 against 1.95 at 425, 2.45 against 2.54 at 680, 3.74 against 3.47 at 1084.
 struct PcgResidentArgs
 {
     BoraSolveTilesDev ft;
@@ -1743,27 +1741,33 @@ int bora_launch_pcg_persistent( BoraSolveTilesDev t, const uint16_t* code, BoraS
 }
 
 namespace {
-constexpr int kResidentBlocks = 152;  // one block per SM; at most 160 (meet)
+// One warp per SM partition up to 256 tiles; above, two, as the blocks poll one another and the
+// meetings grow with their number (464 tiles: 11.2 us per iteration in 116 blocks, 9.6 in 58).
+constexpr int kResidentTiles4 = 256, kResidentTiles8 = 608;
+constexpr int kResidentBlocks = std::max( ( kResidentTiles4 + 3 ) / 4, ( kResidentTiles8 + 7 ) / 8 );  // the largest grid (meet: 160)
+
+// blocks of k_pcg_resident<W> that the device can run at once
 template <int W>
-int resident_fits()  // 1 when the device can run the largest grid of k_pcg_resident<W> at once
+int resident_blocks()
 {
     static BoraPerDevice per_sm;
     const int b = per_sm.get( [] {
         int v = 0;
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor( &v, k_pcg_resident<W>, 32 * W, 0 ) == cudaSuccess && v > 0 ? v : -1;
     } );
-    return b > 0 && b * num_sms() >= kResidentBlocks;
+    return b > 0 ? b * num_sms() : 0;
 }
 }  // namespace
 
-// Warps per block, 0: not for this form. One warp per SM partition up to 256 tiles; above, two, as
-// the blocks poll one another and the meetings grow with their number (464 tiles: 11.2 us per
-// iteration in 116 blocks, 9.6 in 58). From 680 tiles on the per-phase form is level.
+// Warps per block, 0: not for this form (too many tiles, or the device cannot run the grid at once). The
+// step's GPU time against the per-phase form: 0.45 against 0.58 ms at 18 solver tiles, 1.10 against 1.28
+// at 196, 1.43 against 1.60 at 356, 1.82 against 1.88 at 488, 2.05 against 2.11 at 632, level at 715 (2.28
+// and 2.25) and 776 (2.51 and 2.54): the line lies where it stops to gain, at four tiles per SM.
 int bora_pcg_resident_warps( int nft )
 {
-    if( nft <= 0 ) return 0;
-    if( nft <= 256 ) return resident_fits<4>() ? 4 : 0;
-    return nft <= 608 && resident_fits<8>() ? 8 : 0;
+    if( nft <= 0 || nft > kResidentTiles8 ) return 0;
+    if( nft <= kResidentTiles4 ) return resident_blocks<4>() >= ( nft + 3 ) / 4 ? 4 : 0;
+    return resident_blocks<8>() >= ( nft + 7 ) / 8 ? 8 : 0;
 }
 
 size_t bora_pcg_resident_words_bytes() { return (size_t)3 * ( kResidentBlocks + 8 ) * sizeof( ulonglong2 ); }
