@@ -288,10 +288,10 @@ __global__ void __launch_bounds__( 256 ) k_mg_codes( const __grid_constant__ Set
 // neighbour table), dense levels use their small extents. Kernels only visit the
 // neighbours that the stencil code marks as fluid, which always exist.
 
-template <int E>
+template <int E>  // 4, 2, 1
 struct TiledNav
 {
-    static constexpr int LE = E == 8 ? 3 : ( E == 4 ? 2 : ( E == 2 ? 1 : 0 ) );
+    static constexpr int LE = E == 4 ? 2 : ( E == 2 ? 1 : 0 );
     static constexpr int E3 = E * E * E;
     const int32_t* nbr;
     // dense parent level (E == 1 only)
@@ -316,18 +316,11 @@ struct TiledNav
         const int ns = nbr[s * 27 + dir];
         return ns < 0 ? -1 : (long long)ns * E3 + ll;
     }
-    // parent on the next coarser level: same tile with edge E/2, or (E == 1) a dense cell
+    // parent on the next coarser level, a dense cell (E == 1: the cell is the tile)
     __device__ inline long long parent( long long cell ) const
     {
-        const long long s = cell >> ( 3 * LE );
-        const int l = (int)( cell & ( E3 - 1 ) );
-        if( E > 1 )
-        {
-            constexpr int H = E > 1 ? E / 2 : 1;
-            const int li = l & ( E - 1 ), lj = ( l >> LE ) & ( E - 1 ), lk = l >> ( 2 * LE );
-            return s * ( H * H * H ) + ( li >> 1 ) + H * ( ( lj >> 1 ) + H * ( lk >> 1 ) );
-        }
-        const int vt = tile_of[s];
+        static_assert( E == 1, "finer tiled levels run in mg_passes.cu" );
+        const int vt = tile_of[cell];
         const int ti = vt % tx, tj = ( vt / tx ) % ty, tk = vt / ( tx * ty );
         return (long long)( ti >> 1 ) + (long long)cdx * ( ( tj >> 1 ) + (long long)cdy * ( tk >> 1 ) );
     }
@@ -406,13 +399,11 @@ __device__ inline void smooth0_cells( const Nav& nav, const BoraLevelDev& L, con
 
 // Restriction, one thread per (coarse cell, child): each thread forms its child's
 // residual r' - S z (z = the pre-smoothed z0), the 8 lanes of a coarse cell add up by
-// shuffles, and r'_C = 4 * mean = 0.5 * sum. Child enumeration:
-//   mode 0: C tiled (edge EC), F tiled (edge 2 EC) in the same tile;
-//   mode 1: C dense, F tiled with one cell per tile (children are tiles, via slot_of);
-//   mode 2: C dense, F dense.
+// shuffles, and r'_C = 4 * mean = 0.5 * sum. C is dense; TILED: F is tiled with one cell per tile
+// (children are tiles, via slot_of), else dense.
 // i0 and stride are multiples of 8 apart within a warp (every lane of a warp runs the
 // same number of iterations).
-template <class FNav, int MODE, int EC>
+template <class FNav, bool TILED>
 __device__ inline void restrict_cells( const FNav& fnav, const BoraLevelDev& F, const BoraLevelDev& C, const RIn& R,
                                        const int32_t* __restrict__ slot_of, int tx, int ty, int tz, uint32_t* err,
                                        long long i0, long long stride )
@@ -427,28 +418,15 @@ __device__ inline void restrict_cells( const FNav& fnav, const BoraLevelDev& F, 
         if( t < total )  // the value of a non-fluid coarse cell is never read
         {
             long long fc = -1;
-            if( MODE == 0 )
+            const int I = (int)( pc % C.dx ), J = (int)( ( pc / C.dx ) % C.dy ), K = (int)( pc / ( (long long)C.dx * C.dy ) );
+            const int a = 2 * I + ( o & 1 ), b = 2 * J + ( ( o >> 1 ) & 1 ), c = 2 * K + ( o >> 2 );
+            if( TILED )
             {
-                constexpr int LC = EC == 4 ? 2 : ( EC == 2 ? 1 : 0 );
-                constexpr int EF = 2 * EC;
-                const long long s = pc >> ( 3 * LC );
-                const int l = (int)( pc & ( EC * EC * EC - 1 ) );
-                const int ci = l & ( EC - 1 ), cj = ( l >> LC ) & ( EC - 1 ), ck = l >> ( 2 * LC );
-                fc = s * ( EF * EF * EF ) + ( 2 * ci + ( o & 1 ) ) + EF * ( ( 2 * cj + ( ( o >> 1 ) & 1 ) ) +
-                                                                           EF * ( 2 * ck + ( o >> 2 ) ) );
+                if( a < tx && b < ty && c < tz ) fc = slot_of[( (size_t)c * ty + b ) * tx + a];
             }
-            else
+            else if( a < F.dx && b < F.dy && c < F.dz )
             {
-                const int I = (int)( pc % C.dx ), J = (int)( ( pc / C.dx ) % C.dy ), K = (int)( pc / ( (long long)C.dx * C.dy ) );
-                const int a = 2 * I + ( o & 1 ), b = 2 * J + ( ( o >> 1 ) & 1 ), c = 2 * K + ( o >> 2 );
-                if( MODE == 1 )
-                {
-                    if( a < tx && b < ty && c < tz ) fc = slot_of[( (size_t)c * ty + b ) * tx + a];
-                }
-                else if( a < F.dx && b < F.dy && c < F.dz )
-                {
-                    fc = (long long)a + (long long)F.dx * ( b + (long long)F.dy * c );
-                }
+                fc = (long long)a + (long long)F.dx * ( b + (long long)F.dy * c );
             }
             if( fc >= 0 )  // children beyond the domain are masked cells: their code is 0
             {
@@ -595,12 +573,12 @@ __global__ void __launch_bounds__( 256 ) k_mg_smooth0( Nav nav, BoraLevelDev L, 
     smooth0_cells( nav, L, RIn{ L.r }, err, gtid(), gstride() );
 }
 
-template <class FNav, int MODE, int EC>
+template <class FNav, bool TILED>
 __global__ void __launch_bounds__( 256 ) k_mg_restrict( FNav fnav, BoraLevelDev F, BoraLevelDev C,
                                                         const int32_t* __restrict__ slot_of, int tx, int ty, int tz,
                                                         uint32_t* err )
 {
-    restrict_cells<FNav, MODE, EC>( fnav, F, C, RIn{ F.r }, slot_of, tx, ty, tz, err, gtid(), gstride() );
+    restrict_cells<FNav, TILED>( fnav, F, C, RIn{ F.r }, slot_of, tx, ty, tz, err, gtid(), gstride() );
 }
 
 template <class Nav>
@@ -669,9 +647,9 @@ __global__ void __launch_bounds__( kTailThreads ) k_mg_tail( const __grid_consta
         cluster_barrier();
         with_level( t, [&]( auto nav ) {
             if( t == 0 && d.first_tiled )
-                restrict_cells<decltype( nav ), 1, 1>( nav, d.L[t], d.L[t + 1], R, d.slot_of, d.tx, d.ty, d.tz, err, i0, st );
+                restrict_cells<decltype( nav ), true>( nav, d.L[t], d.L[t + 1], R, d.slot_of, d.tx, d.ty, d.tz, err, i0, st );
             else
-                restrict_cells<decltype( nav ), 2, 1>( nav, d.L[t], d.L[t + 1], R, d.slot_of, d.tx, d.ty, d.tz, err, i0, st );
+                restrict_cells<decltype( nav ), false>( nav, d.L[t], d.L[t + 1], R, d.slot_of, d.tx, d.ty, d.tz, err, i0, st );
         } );
         cluster_barrier();
     }
@@ -741,23 +719,16 @@ int bora_mg_setup( const BoraGridDev& g, BoraLevelDev* levels, int nlevels, Bora
 
 namespace {
 
-TiledNav<8> tnav8( BoraTilesDev t ) { return TiledNav<8>{ t.nbr, t.tile_of, 0, 0, 0, 0 }; }
-
-// Launch a level-templated kernel with the navigation of level l.
+// Launch a level-templated kernel with the navigation of level l, dense or tiled with one cell
+// per tile (the finer tiled levels run in mg_passes.cu).
 template <class F>
 void with_nav( const BoraGridDev& g, const BoraLevelDev* levels, int nlevels, int l, BoraTilesDev t, F&& f )
 {
     const BoraLevelDev& L = levels[l];
     const int cdx = l + 1 < nlevels ? levels[l + 1].dx : 0;
     const int cdy = l + 1 < nlevels ? levels[l + 1].dy : 0;
-    if( L.kind == 1 ) { f( DenseNav{ L.dx, L.dy, L.dz, cdx, cdy } ); return; }
-    switch( L.E )
-    {
-        case 8: f( TiledNav<8>{ t.nbr, t.tile_of, g.tx, g.ty, cdx, cdy } ); break;
-        case 4: f( TiledNav<4>{ t.nbr, t.tile_of, g.tx, g.ty, cdx, cdy } ); break;
-        case 2: f( TiledNav<2>{ t.nbr, t.tile_of, g.tx, g.ty, cdx, cdy } ); break;
-        default: f( TiledNav<1>{ t.nbr, t.tile_of, g.tx, g.ty, cdx, cdy } ); break;
-    }
+    if( L.kind == 1 ) f( DenseNav{ L.dx, L.dy, L.dz, cdx, cdy } );
+    else f( TiledNav<1>{ t.nbr, t.tile_of, g.tx, g.ty, cdx, cdy } );
 }
 
 }  // namespace
@@ -848,15 +819,10 @@ void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nleve
             k_mg_smooth0<<<blocks_for( F.ncells ), 256, 0, st>>>( nav, F, red.err );
             const int nb = blocks_for( C.ncells * 8 );
             using N = decltype( nav );
-            if( C.kind == 1 )
-            {
-                if( F.kind == 1 )
-                    k_mg_restrict<N, 2, 1><<<nb, 256, 0, st>>>( nav, F, C, t.slot_of, g.tx, g.ty, g.tz, red.err );
-                else
-                    k_mg_restrict<N, 1, 1><<<nb, 256, 0, st>>>( nav, F, C, t.slot_of, g.tx, g.ty, g.tz, red.err );
-            }
+            if( F.kind == 1 )
+                k_mg_restrict<N, false><<<nb, 256, 0, st>>>( nav, F, C, t.slot_of, g.tx, g.ty, g.tz, red.err );
             else
-                k_mg_restrict<N, 0, 1><<<nb, 256, 0, st>>>( nav, F, C, t.slot_of, g.tx, g.ty, g.tz, red.err );
+                k_mg_restrict<N, true><<<nb, 256, 0, st>>>( nav, F, C, t.slot_of, g.tx, g.ty, g.tz, red.err );
         } );
     }
     if( mid )
@@ -890,9 +856,10 @@ void bora_mg_vcycle( const BoraGridDev& g, const BoraLevelDev* levels, int nleve
     }
     else
     {
-        with_nav( g, levels, nlevels, last, t, [&]( auto nav ) {
-            k_mg_coarsest<<<1, 512, 0, st>>>( nav, levels[last], coarse_sweeps, red.err );
-        } );
+        // a tiled level with four or two cells per tile's edge (a tail level would be in the tail)
+        auto coarsest = [&]( auto nav ) { k_mg_coarsest<<<1, 512, 0, st>>>( nav, levels[last], coarse_sweeps, red.err ); };
+        if( levels[last].E == 4 ) coarsest( TiledNav<4>{ t.nbr, t.tile_of, g.tx, g.ty, 0, 0 } );
+        else coarsest( TiledNav<2>{ t.nbr, t.tile_of, g.tx, g.ty, 0, 0 } );
     }
     // up: prolong + two sweeps
     for( int l = stop - 1; l >= 0; --l )

@@ -85,12 +85,11 @@ __device__ __forceinline__ double warp_max( double v )
     return v;
 }
 
-// op1: 0 = sum, 1 = max for the second value. Slots < 0 are skipped. Inputs are the
-// per-warp totals (already reduced across the warp, valid in every lane). The block takes
-// part as block `bid` of `nblocks` (blockIdx.x of gridDim.x unless a batched launch runs
-// several simulations' blocks side by side in y).
-__device__ __forceinline__ void reduce2_publish_warp( double v0, double v1, int op1, BoraReduceDev red, int slot0, int slot1,
-                                                      unsigned bid, unsigned nblocks )
+// A sum (v0) and a maximum (v1), the per-warp totals (already reduced across the warp, valid in
+// every lane). The block takes part as block `bid` of `nblocks` (blockIdx.x of gridDim.x unless a
+// batched launch runs several simulations' blocks side by side).
+__device__ __forceinline__ void reduce2_publish_warp( double v0, double v1, BoraReduceDev red, int slot0, int slot1, unsigned bid,
+                                                      unsigned nblocks )
 {
     __shared__ double w0[32], w1[32];
     __shared__ bool last;
@@ -100,12 +99,11 @@ __device__ __forceinline__ void reduce2_publish_warp( double v0, double v1, int 
     if( threadIdx.x == 0 )
     {
         double a = 0.0, b = 0.0;
-        for( int q = 0; q < nw; ++q ) { a += w0[q]; b = op1 ? fmax( b, w1[q] ) : b + w1[q]; }
+        for( int q = 0; q < nw; ++q ) { a += w0[q]; b = fmax( b, w1[q] ); }
         red.partials[2 * (size_t)bid] = a;
         red.partials[2 * (size_t)bid + 1] = b;
         __threadfence();
-        const int key = slot0 >= 0 ? slot0 : slot1;
-        const unsigned prev = atomicAdd( &red.done[key % BORA_RING], 1u );
+        const unsigned prev = atomicAdd( &red.done[slot0 % BORA_RING], 1u );
         last = ( prev == nblocks - 1 );
     }
     __syncthreads();
@@ -120,61 +118,37 @@ __device__ __forceinline__ void reduce2_publish_warp( double v0, double v1, int 
     {
         const double2 pq = __ldcg( reinterpret_cast<const double2*>( red.partials ) + q );
         a += pq.x;
-        b = op1 ? fmax( b, pq.y ) : b + pq.y;
+        b = fmax( b, pq.y );
     }
     a = warp_sum( a );
-    b = op1 ? warp_max( b ) : warp_sum( b );
+    b = warp_max( b );
     if( lane == 0 ) { w0[wid] = a; w1[wid] = b; }
     __syncthreads();
     if( threadIdx.x == 0 )
     {
         double ta = 0.0, tb = 0.0;
-        for( int q = 0; q < nw; ++q ) { ta += w0[q]; tb = op1 ? fmax( tb, w1[q] ) : tb + w1[q]; }
-        if( slot0 >= 0 )
+        for( int q = 0; q < nw; ++q ) { ta += w0[q]; tb = fmax( tb, w1[q] ); }
+        red.ring[slot0] = ta;
+        const float hi = (float)ta;
+        red.ringf[slot0] = make_float2( hi, (float)( ta - (double)hi ) );
+        red.ring[slot1] = tb;
+        if( red.mirror )  // the host polls them
         {
-            red.ring[slot0] = ta;
-            const float hi = (float)ta;
-            red.ringf[slot0] = make_float2( hi, (float)( ta - (double)hi ) );
+            red.mirror[slot0] = ta;
+            red.mirror[slot1] = tb;
         }
-        if( slot1 >= 0 ) red.ring[slot1] = tb;
-        if( red.mirror )  // host-visible once the kernel has completed
-        {
-            if( slot0 >= 0 ) red.mirror[slot0] = ta;
-            if( slot1 >= 0 ) red.mirror[slot1] = tb;
-        }
-        const int key = slot0 >= 0 ? slot0 : slot1;
-        red.done[key % BORA_RING] = 0;
+        red.done[slot0 % BORA_RING] = 0;
         __threadfence();
     }
 }
 
-__device__ __forceinline__ void reduce2_publish_warp( double v0, double v1, int op1, BoraReduceDev red, int slot0, int slot1 )
-{
-    reduce2_publish_warp( v0, v1, op1, red, slot0, slot1, blockIdx.x, gridDim.x );
-}
-
-// Per-thread double-float sums (op1 = 0) or a float max in v1 (op1 = 1).
-__device__ __forceinline__ void reduce2_publish_df( DF v0, DF v1, BoraReduceDev red, int slot0, int slot1,
-                                                    unsigned bid, unsigned nblocks )
-{
-    const double a = df_warp_sum( v0 );
-    const double b = df_warp_sum( v1 );
-    reduce2_publish_warp( a, b, 0, red, slot0, slot1, bid, nblocks );
-}
-__device__ __forceinline__ void reduce2_publish_df( DF v0, DF v1, BoraReduceDev red, int slot0, int slot1 )
-{
-    reduce2_publish_df( v0, v1, red, slot0, slot1, blockIdx.x, gridDim.x );
-}
+// Per-thread double-float sums and float maxima.
 __device__ __forceinline__ void reduce2_publish_dfmax( DF v0, float vmax, BoraReduceDev red, int slot0, int slot1,
                                                        unsigned bid, unsigned nblocks )
 {
     const double a = df_warp_sum( v0 );
     const double b = (double)warp_maxf( vmax );
-    reduce2_publish_warp( a, b, 1, red, slot0, slot1, bid, nblocks );
-}
-__device__ __forceinline__ void reduce2_publish_dfmax( DF v0, float vmax, BoraReduceDev red, int slot0, int slot1 )
-{
-    reduce2_publish_dfmax( v0, vmax, red, slot0, slot1, blockIdx.x, gridDim.x );
+    reduce2_publish_warp( a, b, red, slot0, slot1, bid, nblocks );
 }
 
 
