@@ -354,6 +354,12 @@ const char* bora_flip_status_string( int status );
 #define BORA_FAULT_NONE 0
 #define BORA_FAULT_BARRIER 1
 int bora_flip_set_fault( bora_flip_handle h, int fault );
+/* Read back a level of the mixed form's hierarchy as the last system's build left it (tests of its
+ * set-up; no counterpart in the reference). info: cells per tile edge (0: a dense grid), the level's
+ * extent in cells (x, y, z), and the stored cells; types and codes (null: not wanted) take that many
+ * entries, tile after tile in slot order, x fastest, or the dense grid. level 0 is the fine grid; a
+ * level that does not exist is an invalid argument. */
+int bora_flip_get_mg_level( bora_flip_handle h, int level, int info[5], uint8_t* types, uint16_t* codes );
 
 /* Launch-shape autotuner (process-wide; no counterpart in the reference). Kernels with
  * several launch shapes that compute the same bits (the multigrid passes of levels 0-2:

@@ -2379,6 +2379,19 @@ int bora_flip_get_stats( bora_flip_handle s, bora_flip_stats* o )
     return BORA_OK;
 }
 
+int bora_flip_get_mg_level( bora_flip_handle s, int level, int info[5], uint8_t* types, uint16_t* codes )
+{
+    if( !s || !info || level < 0 || level >= s->nlevels ) return BORA_ERR_INVALID_ARG;
+    const BoraLevelDev& L = s->levels[level];
+    info[0] = L.kind == 0 ? L.E : 0;
+    info[1] = L.nx; info[2] = L.ny; info[3] = L.nz;
+    info[4] = (int)L.ncells;
+    if( types ) BORA_TRY( cudaMemcpyAsync( types, L.type, L.ncells, cudaMemcpyDeviceToHost, s->st ) );
+    if( codes ) BORA_TRY( cudaMemcpyAsync( codes, L.code, L.ncells * 2, cudaMemcpyDeviceToHost, s->st ) );
+    BORA_TRY( cudaStreamSynchronize( s->st ) );
+    return BORA_OK;
+}
+
 int bora_flip_set_fault( bora_flip_handle s, int fault )
 {
     if( !s || ( fault != BORA_FAULT_NONE && fault != BORA_FAULT_BARRIER ) ) return BORA_ERR_INVALID_ARG;

@@ -122,6 +122,7 @@ _SIGS = {
     "bora_flip_get_kernel_times": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int]),
     "bora_flip_set_tuning": (ctypes.c_int, [ctypes.c_int]),
     "bora_flip_set_fault": (ctypes.c_int, [_vp, ctypes.c_int]),
+    "bora_flip_get_mg_level": (ctypes.c_int, [_vp, ctypes.c_int, _vp, _vp, _vp]),
     "bora_flip_tune_table": (ctypes.c_int, [_vp, ctypes.c_size_t, _vp]),
     "bora_scan_u32": (ctypes.c_int, [_vp, _vp, ctypes.c_size_t, _vp, _vp]),
     "bora_scan_u32_noalloc": (ctypes.c_int, [_vp, _vp, ctypes.c_size_t, _vp, _vp]),
@@ -443,6 +444,14 @@ class FlipSim:
     def set_profiling_sampling(self, every: int) -> None:
         """Time one in `every` brackets of each profiled kernel class (1: all)."""
         _check(self.lib.bora_flip_set_profiling_sampling(self.h, every), "set_profiling_sampling")
+
+    def mg_level(self, level: int):
+        """bora_flip_get_mg_level: (cells per tile edge or 0, extent (x, y, z), types, codes)."""
+        info = np.zeros(5, np.int32)
+        _check(self.lib.bora_flip_get_mg_level(self.h, level, _ptr(info), None, None), "get_mg_level")
+        types, codes = np.zeros(info[4], np.uint8), np.zeros(info[4], np.uint16)
+        _check(self.lib.bora_flip_get_mg_level(self.h, level, _ptr(info), _ptr(types), _ptr(codes)), "get_mg_level")
+        return int(info[0]), tuple(int(v) for v in info[1:4]), types, codes
 
     def kernel_times(self):
         ms = np.zeros(16, np.float64)
