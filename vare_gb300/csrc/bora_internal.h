@@ -291,13 +291,14 @@ int bora_launch_pcg_resident( BoraSolveTilesDev t, const uint16_t* code, BoraSol
 // and rr from nparts producer blocks' partials into slot_rz_new and slot_rr (host_rr: rr also for the host).
 void bora_launch_pcg_direction( BoraSolveTilesDev t, const uint16_t* code, BoraSolverDev s, int dsel_in, BoraReduceDev red, int nparts, int slot_rz_new, int slot_rr, int slot_rz_old,
                                 int slot_a_rz, int slot_a_dq, bool host_rr, cudaStream_t st );
-// x += e (FP64); e = 0; d = 0; q = 0; finishes the last update's rr into slot_rr (also for the host)
 // x = the last step's pressure on fluid cells, read through the previous tile table (the warm start)
 void bora_launch_solve_warm( int ntiles, const uint16_t* code, const int32_t* tile_of, const int32_t* slot_prev,
                              const float* pres, BoraSolverDev s, cudaStream_t st );
+// x += e (and the last update's pending alpha d) in double-float; e = 0; q = 0; finishes that update's rr into
+// slot_rr (also for the host)
 void bora_launch_refine_accumulate( BoraSolveTilesDev t, const uint16_t* code, BoraSolverDev s, int dsel, BoraReduceDev red,
                                     int nparts, int slot_rr, int slot_a_rz, int slot_a_dq, cudaStream_t st );
-// r = b - A x in FP64 (stored FP32); ||r||^2 and max|r| -> ring slots
+// r = b - A x in double-float (stored FP32); ||r||^2 and max|r| -> ring slots
 void bora_launch_refine_residual( BoraSolveTilesDev t, const float* b, const uint16_t* code, BoraSolverDev s,
                                   BoraReduceDev red, int slot_norm2, int slot_max, cudaStream_t st );
 // pres = (float) x on fluid cells, 0 elsewhere

@@ -535,12 +535,13 @@ void bora_launch_g2p( const BoraGridDev& g, int ntiles, size_t nsorted, BoraTile
                       uint32_t* nkilled, uint32_t* vkey, uint8_t* tile_flag, cudaStream_t st )
 {
     if( nsorted == 0 ) return;
-    // the common case in a kernel without the code of the others, and the RK2 lookups (two more
-    // grid samples, inlined) only where they are asked for
     // Few tiles: up to four CTAs each, so that two rounds of the chip's 608 places are taken (a tile's
     // particles are a chain of 16 rounds in one CTA): 26 us at 24^3 (27 tiles) and 30 at 64^3 (240)
-    // with one, 14 and 22 with four.
+    // with one, 14 and 22 with four; at 360 tiles 25 with one, 23 with three; at 432, 504 and 576
+    // tiles 31, 33 and 35 with one, 27, 28 and 31 with two; one from 608 tiles on.
     const int split = std::max( 1, std::min( kG2PSplitMax, 1216 / ( ntiles + 1 ) ) );
+    // the common case in a kernel without the code of the others, and the RK2 lookups (two more
+    // grid samples, inlined) only where they are asked for
     auto go = [&]( auto kernel ) {
         kernel<<<dim3( ntiles + 1, split ), kG2PThreads, 0, st>>>( g, t, ntiles, (uint32_t)nsorted, start, c, src, idx, dst, adj, dt,
                                                     nkilled, vkey, tile_flag );

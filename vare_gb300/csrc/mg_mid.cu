@@ -2,7 +2,7 @@
 // coarsest level and back; level 2 alone where it is the coarsest) in one thread-block cluster whose CTAs keep every value in
 // distributed shared memory.
 //
-// Levels 0-2 are large and run as grid-wide fused tile kernels (multigrid.cu). Below them
+// Levels 0-2 are large and run as grid-wide stencil passes (mg_passes.cu). Below them
 // the hierarchy is tiny (level 3 has one cell per active tile, then dense grids halved per
 // level down to <= 512 cells). Run from global memory every operation of these levels is a
 // chain of dependent global loads (tile tables, codes, neighbours' values) followed by a

@@ -22,7 +22,8 @@ __device__ inline float absr( float x ) { return x < 0.f ? -x : x; }  // MathUti
 
 // ---------------------------------------------------------------------------------
 // The row stencils (half_rows.cuh) of the right-hand side and the velocity update.
-// Half tiles per CTA: 4 (right-hand side and code 153.6 us, velocity 44.2 at 256^3; 160.4 and 52.1 with 8)
+// Half tiles per CTA: 4 (the system's build 94.7 us, of which the right-hand side is 35, the velocity update
+// 44.5 at 256^3; 102 and 53 with 8)
 constexpr int kRowWarps = 4;
 
 __device__ __forceinline__ uint2 flags8( const uint8_t* __restrict__ flag, int t, int c )
@@ -383,10 +384,10 @@ __global__ void __launch_bounds__( 32 * kTilesPerCta ) k_mic_factor( BoraSolveTi
 // double-float. Non-fluid cells have M2 = 0 and r = 0.
 //
 // Bound by latency and issue: 44 dependent steps of a shuffle and three arithmetic
-// instructions, about 900 warp instructions per tile. The earlier form kept the tile in shared
-// memory (11 shared accesses per row and step pair, 78 % of the shared pipe): 32.5 us per launch
-// at 256^3 (7926 tiles), now 22 us with an event on either side, 3.7 TB/s of its 20 B per cell;
-// 8.4 against 11.9 us at 64^3 (240 tiles). 16 warps per SM without spills beat 20 .. 32 with
+// instructions, about 900 warp instructions per tile. With the tile in shared memory (11 shared
+// accesses per row and step pair, 78 % of the shared pipe) a launch took 32.5 us at 256^3 (7926 tiles)
+// with an event on either side, in registers 22 (3.7 TB/s of its 20 B per cell), and 18 over the
+// solver's tiles alone; 8.4 against 11.9 us at 64^3 (240 tiles). 16 warps per SM without spills beat 20 .. 32 with
 // (23.3 against 23.5 .. 26.1 ms per 256^3 step), and loading the next tile during the sweeps
 // gains nothing (23.3 .. 24.3 ms).
 constexpr int kUpdWarps = 4;
@@ -552,7 +553,7 @@ __global__ void __launch_bounds__( 32 * kUpdWarps, 4 ) k_pcg_update( BoraSolveTi
 //
 // Waits on its loads (long scoreboard), so it wants warps in flight and few sectors per load: a
 // lane with two rows needs 122 registers for the same loads in flight (31.2 us per launch with
-// 16-byte loads at 72 registers, 256^3, an event on either side; 26.8 us now).
+// 16-byte loads at 72 registers, 256^3, an event on either side; 26.8 us so, 20.6 over the solver's tiles alone).
 constexpr int kDirWarps = 4;
 
 // The direction step of the warp's half tiles bid * kDirWarps + warp, then every G * kDirWarps:

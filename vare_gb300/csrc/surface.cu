@@ -40,15 +40,15 @@ constexpr int kSplatThreads = 256;
 constexpr int kSplatCap = 1024;  // staged particles per pass (a layer with more takes several)
 constexpr int kLayerCells = 121;  // 11 x 11 dual cells
 
+// A cell's place in the running sums: the 32 (lj, zc) that a warp adds to at once, zc four
+// consecutive values, lie in 32 banks.
+__device__ inline int splat_at( int li, int lj, int zc ) { return 64 * li + 8 * lj + ( zc ^ ( lj & 4 ) ); }
+
 // Kernel weight of Rasterization.cu:343-349, max(0, (1 - (d/1.5)^2)^3), evaluated as
 // (1 - d^2 / 2.25)^3 with fused multiply-adds: the same function without the square root
 // and the division (one weight's rounding differs by an ulp or two; the sums' order, open
 // in the reference, moves them more). Zero for d^2 >= 2.25; a cell within that radius lies
 // in the reference's 3^3 box around (int)p.
-// A cell's place in the running sums: the 32 (lj, zc) that a warp adds to at once, zc four
-// consecutive values, lie in 32 banks.
-__device__ inline int splat_at( int li, int lj, int zc ) { return 64 * li + 8 * lj + ( zc ^ ( lj & 4 ) ); }
-
 __global__ void __launch_bounds__( kSplatThreads, 3 ) k_splat( const __grid_constant__ BoraGridDev g, BoraTilesDev t,
                                                             const uint32_t* __restrict__ start,
                                                             const uint32_t* __restrict__ idx, BoraParticlesDev p,
