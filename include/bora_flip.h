@@ -368,8 +368,8 @@ int bora_flip_get_mg_level( bora_flip_handle h, int level, int info[5], uint8_t*
  * fastest median is kept. Tuning never changes a result. mode 1 = tune (the default),
  * 0 = the default shapes everywhere. With the environment variable BORA_TUNE_FILE set,
  * the table is read from that file on first use and written back when an entry is
- * decided; entries whose shapes meant something else in the library that wrote them are
- * passed over. */
+ * decided; entries whose shapes may have meant something else (written by a library with
+ * other shapes, or by hand without a layout) are a first guess and measured again. */
 int bora_flip_set_tuning( int mode );
 /* The table as text, one line per entry: "group device size_class shape median_ms"
  * (shape -1: still measuring). *len = its length; cap = 0 asks for the length only;

@@ -12,8 +12,9 @@
 //
 // The table can be loaded from and saved to a text file (BORA_TUNE_FILE: one line per entry,
 // "code device size_class variant median_ms", code = 100 kLayout + group), so a deployment reuses
-// measured shapes. kLayout counts up with every change of what a shape or a unit is; a line of
-// another layout (the first had the bare group) is passed over, and its shape measured again.
+// measured shapes. kLayout counts up with every change of what a shape or a unit is. A line with the
+// bare group (the first layout, or written by hand) is taken as a first guess: it is listed, and the
+// shapes are measured again on live launches; lines of any other layout are passed over.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -39,6 +40,7 @@ struct Entry
 {
     int nvar = 0;
     int chosen = -1;
+    bool guess = false;  // chosen is a file's guess: still to be measured
     std::vector<std::vector<float>> ms;  // samples per variant
     std::vector<int> inflight;           // timed launches not yet resolved, per variant
     double best_ms = 0.0;
@@ -73,12 +75,14 @@ struct Tuner
         double m;
         while( std::fscanf( f, "%d %d %d %d %lf", &g, &d, &c, &v, &m ) == 5 )
         {
-            if( g / 100 != kLayout ) continue;
+            const bool guess = g >= 0 && g < 100;
+            if( g / 100 != kLayout && !guess ) continue;
             g %= 100;
             if( g < 0 || g >= kBoraTuneGroups || v < 0 || v >= bora_tune_variants( g ) ) continue;
             Entry& e = table[std::make_tuple( g, d, c )];
             e.nvar = bora_tune_variants( g );
             e.chosen = v;
+            e.guess = guess;
             e.best_ms = m;
         }
         std::fclose( f );
@@ -92,7 +96,7 @@ struct Tuner
         if( !f ) return;
         for( const auto& kv : table )
             if( kv.second.chosen >= 0 )
-                std::fprintf( f, "%d %d %d %d %.6f\n", 100 * kLayout + std::get<0>( kv.first ), std::get<1>( kv.first ),
+                std::fprintf( f, "%d %d %d %d %.6f\n", ( kv.second.guess ? 0 : 100 * kLayout ) + std::get<0>( kv.first ), std::get<1>( kv.first ),
                               std::get<2>( kv.first ), kv.second.chosen, kv.second.best_ms );
         std::fclose( f );
     }
@@ -158,7 +162,7 @@ BoraTunePick bora_tune_pick( int group, int units )
     std::lock_guard<std::mutex> lk( t.mu );
     if( !t.mode ) return p;
     Entry& e = t.entry_locked( group, current_device(), units );
-    if( e.chosen >= 0 ) { p.variant = e.chosen; return p; }
+    if( e.chosen >= 0 && !e.guess ) { p.variant = e.chosen; return p; }
     // the candidate with the fewest samples so far, counting launches still in flight
     int v = 0;
     for( int q = 1; q < e.nvar; ++q )
@@ -210,7 +214,7 @@ void bora_tune_resolve()
         if( !ok ) continue;
         Entry& e = t.entry_locked( p.group, p.device, p.units );
         if( p.variant < e.nvar && e.inflight[p.variant] > 0 ) --e.inflight[p.variant];
-        if( e.chosen >= 0 || p.variant >= e.nvar ) continue;
+        if( ( e.chosen >= 0 && !e.guess ) || p.variant >= e.nvar ) continue;
         e.ms[p.variant].push_back( ms );
         bool done = true;
         for( const auto& v : e.ms ) done = done && v.size() >= (size_t)kSamples;
@@ -225,6 +229,7 @@ void bora_tune_resolve()
             if( v == 0 || med < best_ms ) { best = v; best_ms = med; }
         }
         e.chosen = best;
+        e.guess = false;
         e.best_ms = best_ms;
         frozen = true;
     }
