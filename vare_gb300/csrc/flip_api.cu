@@ -565,6 +565,7 @@ int build_hierarchy( bora_flip_sim* s )
 {
     const BoraGridDev& g = s->g;
     const size_t nt = (size_t)s->ntiles;
+    s->nlevels = 0;  // an allocation below may fail: no level may name a buffer that has been replaced
     int n = 0;
     int ex = g.nx, ey = g.ny, ez = g.nz;
     auto add = [&]( int kind, int E, size_t ncells, int dx, int dy, int dz ) -> int {
